@@ -1,0 +1,58 @@
+"""Linear layers of at most 128 rows (csrc/gemm_skinny.cuh): edges of the row tiles (16, 32, 64, 128), of the 128-column tiles and of
+the split contraction, with every epilogue, against 64-bit products."""
+import pytest
+import torch
+
+from vllm_omni_b200.ops import _native as nv, gemm
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(y, ref, mass, act_err=0.0):
+    # bf16 result: half an ulp; fp32 sums: K / 16 additions of at most 2^-23 of the products' mass each, K <= 12288; the
+    # activations are 1.13-Lipschitz and use tanh.approx (2^-11 relative)
+    bound = 1.2 * (ref.abs() * 2.0 ** -8 + mass * (12288 / 16) * 2.0 ** -23) + act_err
+    assert torch.isfinite(y).all()
+    assert ((y.double() - ref).abs() <= bound + 1e-6).all()
+
+
+@pytest.mark.parametrize("rows", [1, 15, 16, 17, 32, 33, 64, 65, 127, 128])
+@pytest.mark.parametrize("n,k", [(8, 8), (136, 72), (2048, 64), (2048, 2048), (1000, 12288), (5120, 136), (40000, 128)])
+def test_plain(rows, n, k):
+    g = torch.Generator(device="cuda").manual_seed(rows * 7 + n + k)
+    x = torch.randn(rows, k + 8, generator=g, device="cuda").bfloat16()[:, :k]          # a row pitch wider than the row
+    w = torch.randn(n, k, generator=g, device="cuda").bfloat16()
+    buf = torch.full((rows + 1, n + 8), 7.0, device="cuda", dtype=torch.bfloat16)
+    y = gemm.linear(x, w, out=buf[:rows, :n])
+    _check(y, x.double() @ w.double().T, x.double().abs() @ w.double().abs().T)
+    assert (buf[rows] == 7).all() and (buf[:, n:] == 7).all()
+    nv.check_status()
+
+
+@pytest.mark.parametrize("rows", [2, 16, 48, 128])
+@pytest.mark.parametrize("act", [None, "gelu_tanh", "silu", "relu2", "xielu"])
+def test_epilogue(rows, act):
+    n, k = 264, 1024
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    x, w, b, res, gate = rnd(rows, k), rnd(n, k) * 0.03, rnd(n), rnd(rows, n), rnd(2, n)
+    coef = (0.4, 0.7)
+    z = x.double() @ w.double().T + b.double()
+    ref = {None: lambda t: t, "gelu_tanh": lambda t: torch.nn.functional.gelu(t, approximate="tanh"), "silu": torch.nn.functional.silu,
+           "relu2": lambda t: t.clamp(min=0) ** 2, "xielu": lambda t: gemm.xielu(t, coef)}[act](z)
+    y = (ref.view(2, rows // 2, n) * gate.double()[:, None]).view(rows, n) + res.double()
+    slope = {None: 1.0, "relu2": 2 * z.abs(), "xielu": z.abs() + 1}.get(act, 1.0)
+    err = z.abs() * 2.0 ** -11 * (act in ("gelu_tanh", "silu")) + 1e-5 * (act == "xielu")
+    mass = (x.double().abs() @ w.double().abs().T) * slope
+    big = gate.double().abs().max()
+    out = gemm.linear(x, w, b, act=act, residual=res, gate=gate, coef=coef)
+    _check(out, y, mass * big, err * big)
+    inplace = res.clone()
+    gemm.linear(x, w, b, act=act, residual=inplace, gate=gate, coef=coef, out=inplace)
+    assert torch.equal(inplace, out)
+    # rows of two batches into one joint buffer
+    joint = torch.zeros(2, rows // 2 + 3, n, device="cuda", dtype=torch.bfloat16)
+    gemm.linear(x, w, b, act=act, residual=res, gate=gate, coef=coef, out=joint[:, 1:], out_rows_per_batch=rows // 2,
+                out_batch_stride=joint.stride(0))
+    assert torch.equal(joint[:, 1:1 + rows // 2].reshape(rows, n), out) and (joint[:, 0] == 0).all() and (joint[:, 1 + rows // 2:] == 0).all()
+    nv.check_status()

@@ -1,0 +1,369 @@
+// Linear layers of few rows (decoded tokens, short text streams): C[M, N] = epilogue(A[M, K] W[N, K]^T) for M <= 128.  The time
+// is that of streaming W from HBM plus a launch's fixed chain of latencies, and a tile per 128..256 columns leaves most SMs
+// idle (16 tiles of 128 columns for a 2048-wide layer).
+//
+// gemm_rows_kernel     M <= 16: 16 columns of C per block, the contraction dealt out to its warps.  W goes from HBM straight into
+//                      MMA fragments: no shared-memory ring, no barriers and no tensor memory to set up, which is what a
+//                      launch of a few microseconds is made of.
+// gemm_skinny_kernel   17 <= M <= 128: the operands change places, 128 rows of W are the M side of a tcgen05 MMA and MT = 32 / 64 /
+//                      128 rows of A its N side; the contraction is split over the S = 1, 2, 4 or 8 CTAs of a cluster, each
+//                      streaming its own K range through a TMA ring.  Partial sums (fp32) meet over distributed shared
+//                      memory in rank order: the result does not depend on timing.
+#pragma once
+#include "host_util.h"
+#include "ptx_sm100.cuh"
+
+namespace omni {
+
+template <int MT, bool ALONE>
+struct SkinnyCfg {
+  static constexpr int A_BYTES = 128 * 128;                 // 128 rows of W x 64 bf16
+  static constexpr int STAGE_BYTES = A_BYTES + MT * 128;
+  static constexpr int STAGES = (ALONE ? 200 * 1024 : 108 * 1024) / STAGE_BYTES;
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024;
+  static constexpr int TMEM_COLS = MT < 32 ? 32 : MT;
+  static_assert(MT * 128 * 4 <= STAGES * STAGE_BYTES, "partial sums reuse the ring");
+};
+constexpr int SKINNY_THREADS = 192;   // warp 0 TMA, warp 1 MMA, warps 2-5 epilogue (TMEM quadrant = warp & 3)
+
+__device__ __forceinline__ float ld_shared_cluster_f32(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
+
+// bias, activation, gate, residual and the store of B rows m, m + step, ... of column n.  All operands are read before the
+// first store, because the residual may be the output.
+template <int B>
+__device__ __forceinline__ void skinny_finish(float (&x)[B], int m, int step, int M, int n, __nv_bfloat16* __restrict__ C, int ldc,
+                                              const GemmEpilogue& epi, float bias) {
+  float add[B];
+#pragma unroll
+  for (int j = 0; j < B; ++j) {
+    x[j] += bias;
+    const int r = m + j * step;
+    add[j] = epi.residual && r < M ? __bfloat162float(epi.residual[(size_t)r * epi.ldr + n]) : 0.f;
+  }
+  if (epi.act == ACT_GELU_TANH) {
+#pragma unroll
+    for (int j = 0; j < B; ++j) x[j] = gelu_tanh(x[j]);
+  } else if (epi.act == ACT_SILU) {
+#pragma unroll
+    for (int j = 0; j < B; ++j) x[j] = silu(x[j]);
+  } else if (epi.act == ACT_RELU2) {
+#pragma unroll
+    for (int j = 0; j < B; ++j) x[j] = fmaxf(x[j], 0.f) * fmaxf(x[j], 0.f);
+  } else if (epi.act == ACT_XIELU) {
+#pragma unroll
+    for (int j = 0; j < B; ++j) x[j] = xielu(x[j], epi.act_c0, epi.act_c1);
+  }
+  if (epi.gate) {
+#pragma unroll
+    for (int j = 0; j < B; ++j) {
+      const int r = m + j * step;
+      if (r < M) x[j] *= __bfloat162float(epi.gate[(size_t)(r / epi.rows_per_batch) * epi.gate_stride + n]);
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < B; ++j) {
+    const int r = m + j * step;
+    if (r < M) {
+      __nv_bfloat16* out = C + (size_t)r * ldc;
+      if (epi.c_rows_per_batch > 0) {
+        const int cb = r / epi.c_rows_per_batch;
+        out = C + (size_t)cb * epi.c_batch_stride + (size_t)(r - cb * epi.c_rows_per_batch) * ldc;
+      }
+      out[n] = __float2bfloat16(x[j] + add[j]);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------- at most 16 rows
+__device__ __forceinline__ uint4 ldg_stream(const __nv_bfloat16* p) {   // read once: past L1
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.L2::256B.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ void mma_bf16_16x8(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// NT * 8 rows of A; NW warps, warp w takes the 32-channel chunks w, w + NW, ...  Lane group j of a quad owns channels 8 j .. 8 j + 7 of
+// a chunk for both operands: one 16-byte load per row, and the contraction is permuted alike on both sides.  U chunks are
+// in flight per warp: 16 resident warps x 8 chunks x 1 KB = 128 KB per SM.
+template <int NT, int NW>
+__global__ void __launch_bounds__(32 * NW, NW == 16 ? 1 : 2)
+gemm_rows_kernel(const __nv_bfloat16* __restrict__ A, int lda, const __nv_bfloat16* __restrict__ W, int ldw, __nv_bfloat16* C, int ldc,
+                 int M, int N, int K, const __grid_constant__ GemmEpilogue epi) {
+  constexpr int U = NT == 1 ? 8 : 4;
+  __shared__ float part[NW][NT * 8][16];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, j = lane & 3;
+  const int n0 = blockIdx.x * 16;
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  const __nv_bfloat16* w0 = W + (size_t)min(n0 + g, N - 1) * ldw;          // columns past N repeat the last one and are not stored
+  const __nv_bfloat16* w1 = W + (size_t)min(n0 + 8 + g, N - 1) * ldw;
+  float acc[NT][4];
+#pragma unroll
+  for (int t = 0; t < NT; ++t)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) acc[t][i] = 0.f;
+#pragma unroll 1
+  for (int c = warp * 32; c < K; c += 32 * NW * U) {
+    uint4 a[U][2], b[U][NT];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int ch = c + u * 32 * NW + j * 8;                              // K is a multiple of 8
+      const bool in = ch < K;
+      a[u][0] = in ? ldg_stream(w0 + ch) : zero;
+      a[u][1] = in ? ldg_stream(w1 + ch) : zero;
+#pragma unroll
+      for (int t = 0; t < NT; ++t)
+        b[u][t] = in && t * 8 + g < M ? *reinterpret_cast<const uint4*>(A + (size_t)(t * 8 + g) * lda + ch) : zero;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        mma_bf16_16x8(acc[t], a[u][0].x, a[u][1].x, a[u][0].y, a[u][1].y, b[u][t].x, b[u][t].y);
+        mma_bf16_16x8(acc[t], a[u][0].z, a[u][1].z, a[u][0].w, a[u][1].w, b[u][t].z, b[u][t].w);
+      }
+  }
+#pragma unroll
+  for (int t = 0; t < NT; ++t)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) part[warp][t * 8 + j * 2 + (i & 1)][g + 8 * (i >> 1)] = acc[t][i];
+  __syncthreads();
+  if (threadIdx.x < NT * 128) {
+    const int n = n0 + (threadIdx.x & 15), m = threadIdx.x >> 4;
+    if (n < N && m < M) {
+      const float bias = epi.bias ? __bfloat162float(epi.bias[n]) : 0.f;
+      float x[1] = {0.f};
+#pragma unroll
+      for (int w = 0; w < NW; ++w) x[0] += part[w][m][threadIdx.x & 15];
+      skinny_finish<1>(x, m, 1, M, n, C, ldc, epi, bias);
+    }
+  }
+}
+
+static int launch_rows(const void* A, int lda, const void* W, int ldw, __nv_bfloat16* C, int ldc, int M, int N, int K,
+                       const GemmEpilogue& epi, cudaStream_t stream) {
+  if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15) return RC_BAD_ARG;
+  const auto a = static_cast<const __nv_bfloat16*>(A), w = static_cast<const __nv_bfloat16*>(W);
+  const int tiles = (N + 15) / 16;
+  // one block per SM: 16 warps, so that a long contraction still is one or two rounds of loads; else two blocks of 8
+  const bool wide = tiles <= sm_count() && K > 1024;
+  if (M <= 8) {
+    if (wide) gemm_rows_kernel<1, 16><<<tiles, 512, 0, stream>>>(a, lda, w, ldw, C, ldc, M, N, K, epi);
+    else gemm_rows_kernel<1, 8><<<tiles, 256, 0, stream>>>(a, lda, w, ldw, C, ldc, M, N, K, epi);
+  } else {
+    if (wide) gemm_rows_kernel<2, 16><<<tiles, 512, 0, stream>>>(a, lda, w, ldw, C, ldc, M, N, K, epi);
+    else gemm_rows_kernel<2, 8><<<tiles, 256, 0, stream>>>(a, lda, w, ldw, C, ldc, M, N, K, epi);
+  }
+  return (int)cudaGetLastError();
+}
+
+// ------------------------------------------------------------------------------------------------------- 17 to 128 rows
+template <int MT, int S, bool ALONE>
+__global__ void __launch_bounds__(SKINNY_THREADS)
+gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, __nv_bfloat16* __restrict__ C,
+                   int ldc, int M, int N, int K, const __grid_constant__ GemmEpilogue epi, int* status) {
+  using Cfg = SkinnyCfg<MT, ALONE>;
+  constexpr int STAGES = Cfg::STAGES;
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ __align__(8) uint64_t full_bar[STAGES];
+  __shared__ __align__(8) uint64_t empty_bar[STAGES];
+  __shared__ __align__(8) uint64_t done_bar;
+  __shared__ uint32_t tmem_base_s;
+  __shared__ int s_abort;
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = S > 1 ? (int)cluster_ctarank() : 0;
+  const int n0 = (blockIdx.x / S) * 128;
+  const int num_kb = (K + 63) / 64;
+  const int kb0 = rank * num_kb / S, kb1 = (rank + 1) * num_kb / S;      // never empty: the launcher keeps num_kb >= S
+  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+
+  if (threadIdx.x == 0) {
+    s_abort = 0;
+    for (int i = 0; i < STAGES; ++i) {
+      mbar_init(smem_u32(&full_bar[i]), 1);
+      mbar_init(smem_u32(&empty_bar[i]), 1);
+    }
+    mbar_init(smem_u32(&done_bar), 1);
+    fence_mbar_init();
+    tma_prefetch_desc(&tmX);
+    tma_prefetch_desc(&tmW);
+  }
+  if (warp == 1) {
+    tmem_alloc(smem_u32(&tmem_base_s), Cfg::TMEM_COLS);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = tmem_base_s;
+
+  if (warp == 0) {
+    if (elect_one()) {
+      int stage = 0;
+      uint32_t phase = 0;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        mbar_wait(smem_u32(&empty_bar[stage]), phase ^ 1, &s_abort, status, ERR_WAIT_EMPTY);
+        const uint32_t fb = smem_u32(&full_bar[stage]);
+        const uint32_t sa = smem_base + stage * Cfg::STAGE_BYTES;
+        mbar_expect_tx(fb, Cfg::STAGE_BYTES);
+        tma_load_2d(sa, &tmW, fb, kb * 64, n0);
+        tma_load_2d(sa + Cfg::A_BYTES, &tmX, fb, kb * 64, 0);
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
+      }
+    }
+  } else if (warp == 1) {
+    if (elect_one()) {
+      constexpr uint32_t idesc = umma_idesc(128, MT, 1, 1, 0, 0);
+      int stage = 0;
+      uint32_t phase = 0;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        mbar_wait(smem_u32(&full_bar[stage]), phase, &s_abort, status, ERR_WAIT_FULL);
+        tc_fence_after_sync();
+        const uint32_t sa = smem_base + stage * Cfg::STAGE_BYTES;
+        const uint64_t w_desc = umma_desc_kmajor_sw128(sa), x_desc = umma_desc_kmajor_sw128(sa + Cfg::A_BYTES);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) mma_f16_ss(tmem_base, w_desc + 2 * k, x_desc + 2 * k, idesc, kb != kb0 || k != 0);
+        tc_commit(smem_u32(&empty_bar[stage]));
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
+      }
+      tc_commit(smem_u32(&done_bar));
+    }
+  } else {
+    const int q = warp & 3;
+    const int n = n0 + q * 32 + lane;
+    const float bias = epi.bias && n < N ? __bfloat162float(epi.bias[n]) : 0.f;
+    mbar_wait(smem_u32(&done_bar), 0, &s_abort, status, ERR_WAIT_TMEM_FULL);
+    tc_fence_after_sync();
+    // a lane holds one column of C, the registers 16 of its rows
+#pragma unroll 1
+    for (int c = 0; c < MT && (S > 1 || c < M); c += 16) {
+      uint32_t v[16];
+      tmem_ld_32x16(tmem_base + ((uint32_t)(q * 32) << 16) + c, v);
+      tmem_wait_ld();
+      if (S > 1) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+          asm volatile("st.shared.b32 [%0], %1;" ::"r"(smem_base + ((c + j) * 128 + q * 32 + lane) * 4), "r"(v[j]) : "memory");
+      } else if (n < N) {
+        float x[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) x[j] = __uint_as_float(v[j]);
+        skinny_finish<16>(x, c, 1, M, n, C, ldc, epi, bias);
+      }
+    }
+    tc_fence_before_sync();
+  }
+  __syncthreads();
+  if (S > 1) {
+    cluster_sync_all();                                     // every rank's partial sums lie in its shared memory
+    if (warp >= 2) {
+      const int col = (warp & 3) * 32 + lane, n = n0 + col;
+      const float bias = epi.bias && n < N ? __bfloat162float(epi.bias[n]) : 0.f;
+      uint32_t src[S];
+#pragma unroll
+      for (int s = 0; s < S; ++s) src[s] = mapa_shared(smem_base + col * 4, s);
+      if (n < N) {
+        constexpr int B = MT / S < 8 ? MT / S : 8;
+#pragma unroll 1
+        for (int m = rank; m < M; m += B * S) {             // rows of C are dealt out to the ranks, B at a time
+          float x[B];
+#pragma unroll
+          for (int j = 0; j < B; ++j) {
+            float p[S];                                     // rows past M are zero products: there to be read, never stored
+#pragma unroll
+            for (int s = 0; s < S; ++s) p[s] = ld_shared_cluster_f32(src[s] + (m + j * S) * 512);
+            x[j] = p[0];
+#pragma unroll
+            for (int s = 1; s < S; ++s) x[j] += p[s];
+          }
+          skinny_finish<B>(x, m, S, M, n, C, ldc, epi, bias);
+        }
+      }
+    }
+    __syncthreads();
+    cluster_sync_all();                                     // no rank leaves while another reads its shared memory
+  }
+  if (s_abort) {                                            // copies and MMAs in flight land before the memory is handed back
+    const unsigned long long t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 200000ull) {
+    }
+  }
+  if (warp == 1) {
+    tc_fence_after_sync();
+    tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
+  }
+}
+
+template <int MT, int S, bool ALONE>
+static int launch_skinny_s(const CUtensorMap& tmX, const CUtensorMap& tmW, __nv_bfloat16* C, int ldc, int M, int N, int K,
+                           const GemmEpilogue& epi, int* status, cudaStream_t stream) {
+  static unsigned long long prepared = 0;
+  if (int e = ensure_dynamic_smem((const void*)gemm_skinny_kernel<MT, S, ALONE>, SkinnyCfg<MT, ALONE>::SMEM_BYTES, prepared)) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((N + 127) / 128 * S));
+  cfg.blockDim = dim3(SKINNY_THREADS);
+  cfg.dynamicSmemBytes = SkinnyCfg<MT, ALONE>::SMEM_BYTES;
+  cfg.stream = stream;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = S; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = S > 1 ? 1 : 0;
+  return (int)cudaLaunchKernelEx(&cfg, gemm_skinny_kernel<MT, S, ALONE>, tmX, tmW, C, ldc, M, N, K, epi, status);
+}
+
+// CTAs per tile: up to about 200 in all (two share an SM), each with at least two K blocks
+static int skinny_split(int N, int K) {
+  const int tiles = (N + 127) / 128, num_kb = (K + 63) / 64;
+  for (int s = 8; s > 1; s >>= 1)
+    if (tiles * s <= 200 && num_kb >= 2 * s) return s;
+  return 1;
+}
+
+template <int MT>
+static int launch_skinny_mt(const CUtensorMap& tmW, const void* A, int lda, __nv_bfloat16* C, int ldc, int M, int N, int K,
+                            const GemmEpilogue& epi, int split, int* status, cudaStream_t stream) {
+  CUtensorMap tmX;
+  if (int rc = make_tmap_2d(&tmX, A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)M, (uint64_t)K, (uint64_t)lda * 2, MT, 64)) return rc;
+  const bool alone = split <= 4 && (N + 127) / 128 * split <= sm_count();   // clusters of 8 CTAs do not fit every GPC's SMs one by one
+#define OMNI_SKINNY(S)                                                                                       \
+  return alone ? launch_skinny_s<MT, S, true>(tmX, tmW, C, ldc, M, N, K, epi, status, stream)                \
+               : launch_skinny_s<MT, S, false>(tmX, tmW, C, ldc, M, N, K, epi, status, stream)
+  switch (split) {
+    case 8: OMNI_SKINNY(8);
+    case 4: OMNI_SKINNY(4);
+    case 2: OMNI_SKINNY(2);
+    default: OMNI_SKINNY(1);
+  }
+#undef OMNI_SKINNY
+}
+
+// Which problems leave the general kernels (tiles of 128 or 256 rows).  M <= 16: all.  Above, the split needs room: with half as
+// many tiles as SMs or more the general kernels stream W as fast, and their wider tiles read A less often.
+enum class FewRows { no, rows, skinny };
+static FewRows few_rows(int M, int N) {
+  const int tiles = (N + 127) / 128;
+  if (M <= 16) return FewRows::rows;
+  if ((M <= 64 && tiles * 2 <= sm_count()) || (M <= 128 && tiles * 3 <= sm_count())) return FewRows::skinny;
+  return FewRows::no;
+}
+
+static int launch_skinny(const void* A, int lda, const void* W, int ldw, __nv_bfloat16* C, int ldc, int M, int N, int K,
+                         const GemmEpilogue& epi, int* status, cudaStream_t stream) {
+  CUtensorMap tmW;
+  if (int rc = make_tmap_2d(&tmW, W, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)N, (uint64_t)K, (uint64_t)ldw * 2, 128, 64)) return rc;
+  const int s = skinny_split(N, K);
+  if (M <= 32) return launch_skinny_mt<32>(tmW, A, lda, C, ldc, M, N, K, epi, s, status, stream);
+  if (M <= 64) return launch_skinny_mt<64>(tmW, A, lda, C, ldc, M, N, K, epi, s, status, stream);
+  return launch_skinny_mt<128>(tmW, A, lda, C, ldc, M, N, K, epi, s, status, stream);
+}
+
+}  // namespace omni

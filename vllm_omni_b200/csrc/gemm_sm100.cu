@@ -1043,6 +1043,8 @@ static int pick_bn(int M, int N, int ctas) {
 
 }  // namespace omni
 
+#include "gemm_skinny.cuh"
+
 // C ABI.  All pointers are device pointers; `status` is a device int32 that receives the
 // first timeout code (0 = none).  Strides are in elements.  force_bn = 0 lets the launcher
 // choose the tile width.
@@ -1060,10 +1062,6 @@ extern "C" int omni_gemm_bf16_coef(const void* A, int lda, const void* W, int ld
   if ((K & 7) || (N & 7) || (lda & 7) || (ldw & 7) || (ldc & 7) || (ldr & 7) || (gate_stride & 7))
     return RC_BAD_ARG;
   if (gate && rows_per_batch <= 0) return RC_BAD_ARG;
-  CUtensorMap tmA;
-  int rc = make_tmap_2d(&tmA, A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)M, (uint64_t)K,
-                        (uint64_t)lda * 2, BM, BK);
-  if (rc) return rc;
   GemmEpilogue epi;
   epi.bias = static_cast<const __nv_bfloat16*>(bias);
   epi.residual = static_cast<const __nv_bfloat16*>(residual);
@@ -1096,6 +1094,17 @@ extern "C" int omni_gemm_bf16_coef(const void* A, int lda, const void* W, int ld
   const int ctas = sm_count();
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   __nv_bfloat16* c = static_cast<__nv_bfloat16*>(C);
+  if (force_bn == 0 && !sync && epi.scatter_P == 0 && epi.scatter_rows == 0) {
+    switch (few_rows(M, N)) {
+      case FewRows::rows: return launch_rows(A, lda, W, ldw, c, ldc, M, N, K, epi, s);
+      case FewRows::skinny: return launch_skinny(A, lda, W, ldw, c, ldc, M, N, K, epi, status, s);
+      default: break;
+    }
+  }
+  CUtensorMap tmA;
+  int rc = make_tmap_2d(&tmA, A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)M, (uint64_t)K,
+                        (uint64_t)lda * 2, BM, BK);
+  if (rc) return rc;
   // force_bn = 576 / 448 / 384 selects the CTA-pair kernel with a 256 / 192 / 128 wide tile on two
   // SMs, 512 the pair kernel with the launcher's choice of width; in automatic mode the pair kernel takes every
   // problem with at least one full wave of 256 x 256 tiles
