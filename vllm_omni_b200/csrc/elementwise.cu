@@ -42,90 +42,99 @@ __device__ __forceinline__ float warp_sum(float v) {
 }
 
 // ---------------------------------------------------------------- norm + modulate
-// One CTA (256 threads) per row; each thread keeps up to MAXV 8-element chunks in
-// registers, so the row is read exactly once.  D % 8 == 0, D <= 256 * 8 * MAXV.
-constexpr int NM_THREADS = 256;
-constexpr int NM_MAXV = 4;
-
-__global__ void __launch_bounds__(NM_THREADS)
-norm_modulate_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, int rows,
-                     int D, int ldx, int ldy, const __nv_bfloat16* __restrict__ weight,
-                     const __nv_bfloat16* __restrict__ bias, const __nv_bfloat16* __restrict__ shift,
-                     const __nv_bfloat16* __restrict__ scale, int mod_stride, int rows_per_batch,
-                     int rms, float eps) {
-  __shared__ float red[2][NM_THREADS / 32];
-  const int row = blockIdx.x;
-  if (row >= rows) return;
-  const __nv_bfloat16* xr = x + (size_t)row * ldx;
-  float v[NM_MAXV][8];
+// Few rows of more than 1024 channels: one block per row, CPT 16-byte chunks per thread.  Gains and modulation are fetched
+// together with the row, so a launch is one round trip to memory and one reduction; short code matters as much, because a
+// launch of a few rows spends its time fetching instructions.  Caches cold, launch included: 8 rows of 4096 8 us (one
+// warp per row with all chunks unrolled: 18), 512 rows of 3072 10 us (14).
+template <int CPT>
+__global__ void __launch_bounds__(512)
+norm_modulate_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, int D, int ldx, int ldy,
+                     const __nv_bfloat16* __restrict__ weight, const __nv_bfloat16* __restrict__ bias,
+                     const __nv_bfloat16* __restrict__ shift, const __nv_bfloat16* __restrict__ scale, int mod_stride,
+                     int rows_per_batch, int rms, float eps) {
+  __shared__ float2 red[16];
+  const int row = blockIdx.x, nchunk = D >> 3, warps = blockDim.x >> 5;
+  const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)row * ldx);
+  const size_t mod = (size_t)(row / rows_per_batch) * mod_stride;
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  uint4 v[CPT], wv[CPT], bv[CPT], sh[CPT], sc[CPT];
+#pragma unroll
+  for (int i = 0; i < CPT; ++i) {
+    const int c = threadIdx.x + i * blockDim.x;
+    const bool in = c < nchunk;
+    v[i] = in ? xr[c] : zero;
+    if (weight) wv[i] = in ? *reinterpret_cast<const uint4*>(weight + c * 8) : zero;
+    if (bias) bv[i] = in ? *reinterpret_cast<const uint4*>(bias + c * 8) : zero;
+    if (scale) sc[i] = in ? *reinterpret_cast<const uint4*>(scale + mod + c * 8) : zero;
+    if (shift) sh[i] = in ? *reinterpret_cast<const uint4*>(shift + mod + c * 8) : zero;
+  }
   float s = 0.f, ss = 0.f;
-  const int nchunk = D >> 3;
 #pragma unroll
-  for (int i = 0; i < NM_MAXV; ++i) {
-    const int c = threadIdx.x + i * NM_THREADS;
-    if (c < nchunk) {
-      load8(xr + c * 8, v[i]);
+  for (int i = 0; i < CPT; ++i) {
+    const uint32_t w[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
 #pragma unroll
-      for (int e = 0; e < 8; ++e) { s += v[i][e]; ss += v[i][e] * v[i][e]; }
+    for (int j = 0; j < 4; ++j) {
+      const float2 f = unpack_bf16(w[j]);
+      s += f.x + f.y;
+      ss = fmaf(f.x, f.x, fmaf(f.y, f.y, ss));
     }
   }
   s = warp_sum(s);
   ss = warp_sum(ss);
-  if ((threadIdx.x & 31) == 0) { red[0][threadIdx.x >> 5] = s; red[1][threadIdx.x >> 5] = ss; }
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = make_float2(s, ss);
   __syncthreads();
   s = 0.f; ss = 0.f;
-#pragma unroll
-  for (int w = 0; w < NM_THREADS / 32; ++w) { s += red[0][w]; ss += red[1][w]; }
+  for (int w = 0; w < warps; ++w) { s += red[w].x; ss += red[w].y; }
   const float inv_d = 1.0f / (float)D;
-  float mean = rms ? 0.f : s * inv_d;
-  float var = rms ? ss * inv_d : fmaxf(ss * inv_d - mean * mean, 0.f);
+  const float mean = rms ? 0.f : s * inv_d;
+  const float var = rms ? ss * inv_d : fmaxf(ss * inv_d - mean * mean, 0.f);
   const float rstd = rsqrtf(var + eps);
-  const int b = row / rows_per_batch;
-  const __nv_bfloat16* sh = shift ? shift + (size_t)b * mod_stride : nullptr;
-  const __nv_bfloat16* sc = scale ? scale + (size_t)b * mod_stride : nullptr;
-  __nv_bfloat16* yr = y + (size_t)row * ldy;
+  uint4* yr = reinterpret_cast<uint4*>(y + (size_t)row * ldy);
 #pragma unroll
-  for (int i = 0; i < NM_MAXV; ++i) {
-    const int c = threadIdx.x + i * NM_THREADS;
-    if (c < nchunk) {
-      float o[8];
+  for (int i = 0; i < CPT; ++i) {
+    const int c = threadIdx.x + i * blockDim.x;
+    if (c >= nchunk) break;
+    uint32_t o[4];
+    const uint32_t vv[4] = {v[i].x, v[i].y, v[i].z, v[i].w}, ww[4] = {wv[i].x, wv[i].y, wv[i].z, wv[i].w};
+    const uint32_t bb[4] = {bv[i].x, bv[i].y, bv[i].z, bv[i].w}, cc[4] = {sc[i].x, sc[i].y, sc[i].z, sc[i].w};
+    const uint32_t hh[4] = {sh[i].x, sh[i].y, sh[i].z, sh[i].w};
 #pragma unroll
-      for (int e = 0; e < 8; ++e) o[e] = (v[i][e] - mean) * rstd;
-      if (weight) { float w[8]; load8(weight + c * 8, w);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) o[e] *= w[e]; }
-      if (bias) { float w[8]; load8(bias + c * 8, w);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) o[e] += w[e]; }
-      if (sc) { float w[8]; load8(sc + c * 8, w);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) o[e] *= (1.0f + w[e]); }
-      if (sh) { float w[8]; load8(sh + c * 8, w);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) o[e] += w[e]; }
-      store8(yr + c * 8, o);
+    for (int j = 0; j < 4; ++j) {
+      float2 f = unpack_bf16(vv[j]);
+      f.x = (f.x - mean) * rstd;
+      f.y = (f.y - mean) * rstd;
+      if (weight) { const float2 t = unpack_bf16(ww[j]); f.x *= t.x; f.y *= t.y; }
+      if (bias) { const float2 t = unpack_bf16(bb[j]); f.x += t.x; f.y += t.y; }
+      if (scale) { const float2 t = unpack_bf16(cc[j]); f.x = fmaf(f.x, t.x, f.x); f.y = fmaf(f.y, t.y, f.y); }
+      if (shift) { const float2 t = unpack_bf16(hh[j]); f.x += t.x; f.y += t.y; }
+      o[j] = pack_bf16(f.x, f.y);
     }
+    yr[c] = make_uint4(o[0], o[1], o[2], o[3]);
   }
 }
 
-// Warp-per-row variant: the row stays packed (bf16) in VPL 16-byte registers per lane, all
-// loads of a row are in flight at once, no shared memory and no block barrier.
-template <int VPL>
+// Many rows, or rows of up to 1024 channels: WPR warps per row, the row packed (bf16) in VPL 16-byte registers per lane.  All loads of a
+// row are in flight at once and 40 to 60 registers leave room for 32 warps and more per SM.  8192 rows of 4096 (134 MB): 39 us, with one
+// warp per row and 16 chunks per lane 53 us; keeping rows in flight through shared memory instead (bulk copies,
+// 200 KB per SM) did not help: 16 warps issue too little.
+template <int VPL, int WPR>
 __global__ void __launch_bounds__(256)
 norm_modulate_warp_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, int rows,
                           int D, int ldx, int ldy, const __nv_bfloat16* __restrict__ weight,
                           const __nv_bfloat16* __restrict__ bias, const __nv_bfloat16* __restrict__ shift,
                           const __nv_bfloat16* __restrict__ scale, int mod_stride, int rows_per_batch,
                           int rms, float eps) {
-  const int row = blockIdx.x * 8 + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (row >= rows) return;
-  const int nchunk = D >> 3;
+  __shared__ float2 red[8];
+  const int warp = threadIdx.x >> 5, row = blockIdx.x * (8 / WPR) + warp / WPR;
+  const int lane = (threadIdx.x & 31) + (warp % WPR) * 32;
+  if (WPR == 1 && row >= rows) return;
+  const bool live = row < rows;
+  const int nchunk = live ? D >> 3 : 0;
   const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)row * ldx);
   uint4 v[VPL];
 #pragma unroll
   for (int i = 0; i < VPL; ++i) {
-    const int c = lane + i * 32;
+    const int c = lane + i * 32 * WPR;
     v[i] = c < nchunk ? xr[c] : make_uint4(0u, 0u, 0u, 0u);
   }
   float s = 0.f, ss = 0.f;
@@ -141,6 +150,16 @@ norm_modulate_warp_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __
   }
   s = warp_sum(s);
   ss = warp_sum(ss);
+  if (WPR > 1) {
+    if ((threadIdx.x & 31) == 0) red[warp] = make_float2(s, ss);
+    __syncthreads();
+    s = 0.f; ss = 0.f;
+#pragma unroll
+    for (int w = 0; w < WPR; ++w) {
+      const float2 p = red[warp / WPR * WPR + w];
+      s += p.x; ss += p.y;
+    }
+  }
   const float inv_d = 1.0f / (float)D;
   const float mean = rms ? 0.f : s * inv_d;
   const float var = rms ? ss * inv_d : fmaxf(ss * inv_d - mean * mean, 0.f);
@@ -151,7 +170,7 @@ norm_modulate_warp_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __
   __nv_bfloat16* yr = y + (size_t)row * ldy;
 #pragma unroll
   for (int i = 0; i < VPL; ++i) {
-    const int c = lane + i * 32;
+    const int c = lane + i * 32 * WPR;
     if (c < nchunk) {
       const uint32_t w[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
       float o[8];
@@ -178,16 +197,100 @@ norm_modulate_warp_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __
   }
 }
 
-// Fast q/k norm + rope for D = 128: one warp per (batch, position) row walks all q and k heads
-// of that row; half a warp owns one head (8 contiguous elements per lane, one 16-byte access),
-// four heads-pairs are in flight per iteration.
+// Where the heads of a row also go: key and value pages (null: nowhere), at slots[r], < 0 = none.
+struct HeadPages {
+  __nv_bfloat16 *k, *v;
+  const int* slots;
+};
+
+// Norm and rotation of one head held by half a warp, 8 consecutive elements per lane (D = 128).  c, s: this lane's rotation
+// coefficients, 4 pairs of neighbours (interleaved) or the 8 frequencies of its elements (halves, the sign already on s).
+__device__ __forceinline__ uint4 head_norm_rope(const uint4& v, bool norm, const uint4& gain, bool rope, int interleaved, const float (&c)[8],
+                                                const float (&s)[8], float eps) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+  float x[8];
+  float ss = 0.f;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float2 f = unpack_bf16(w[j]);
+    x[2 * j] = f.x; x[2 * j + 1] = f.y;
+    ss = fmaf(f.x, f.x, fmaf(f.y, f.y, ss));
+  }
+  if (norm) {
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    const float r = rsqrtf(ss * (1.0f / 128) + eps);
+    const uint32_t g[4] = {gain.x, gain.y, gain.z, gain.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 f = unpack_bf16(g[j]);
+      x[2 * j] = x[2 * j] * r * f.x;
+      x[2 * j + 1] = x[2 * j + 1] * r * f.y;
+    }
+  }
+  if (rope) {
+    if (interleaved) {
+#pragma unroll
+      for (int e = 0; e < 8; e += 2) {
+        const float a = x[e], b = x[e + 1];
+        x[e] = fmaf(a, c[e >> 1], -b * s[e >> 1]);
+        x[e + 1] = fmaf(b, c[e >> 1], a * s[e >> 1]);
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float partner = __shfl_xor_sync(0xffffffffu, x[e], 8);
+        x[e] = fmaf(x[e], c[e], partner * s[e]);
+      }
+    }
+  }
+  return make_uint4(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]), pack_bf16(x[4], x[5]), pack_bf16(x[6], x[7]));
+}
+
+struct HeadRows {
+  __nv_bfloat16* qkv;
+  long rows;
+  int S, H, Hkv, ld;
+  const __nv_bfloat16 *wq, *wk, *wq_alt, *wk_alt;
+  int s_alt;
+  const float *cosb, *sinb;
+  int interleaved;
+  float eps;
+  const int* positions;
+  HeadPages pages;
+};
+
+__device__ __forceinline__ void rope_coefficients(const HeadRows& a, long row, int s, int l16, float (&cs)[8], float (&sn)[8]) {
+#pragma unroll
+  for (int e = 0; e < 8; ++e) cs[e] = sn[e] = 0.f;
+  if (!a.cosb) return;
+  const int pos = a.positions ? a.positions[row] : s;
+  const int f0 = a.interleaved ? 4 * l16 : (l16 & 7) * 8, n = a.interleaved ? 4 : 8;
+  const float* cr = a.cosb + (size_t)pos * 64 + f0;
+  const float* sr = a.sinb + (size_t)pos * 64 + f0;
+#pragma unroll
+  for (int e = 0; e < 8; ++e)
+    if (e < n) {
+      cs[e] = cr[e];
+      sn[e] = a.interleaved || l16 >= 8 ? sr[e] : -sr[e];
+    }
+}
+
+// A result to its places: back to the row, and key and value heads to their page.
+__device__ __forceinline__ void store_head(const HeadRows& a, long row, int h, int l16, int slot, const uint4& raw, const uint4& done) {
+  const int heads = a.H + a.Hkv;
+  if (h < heads) *reinterpret_cast<uint4*>(a.qkv + (size_t)row * a.ld + (size_t)h * 128 + l16 * 8) = done;
+  if (slot >= 0 && h >= a.H) {
+    __nv_bfloat16* page = h < heads ? a.pages.k + (size_t)(h - a.H) * 128 : a.pages.v + (size_t)(h - heads) * 128;
+    *reinterpret_cast<uint4*>(page + (size_t)slot * a.Hkv * 128 + l16 * 8) = h < heads ? done : raw;
+  }
+}
+
+// Head norms and rotation for D = 128, a few rows: two heads to a warp, half a warp each.  With pages the key heads go there as
+// well and the value heads that follow them are copied.  8 rows of 40 heads, caches cold, launch included: 8 us, 14 us
+// with one warp per row; 560 rows of 48 heads 12 us (16).
 __global__ void __launch_bounds__(256)
-qk_norm_rope128_kernel(__nv_bfloat16* __restrict__ qkv, long rows, int S, int H, int Hkv, int ld,
-                       const __nv_bfloat16* __restrict__ wq, const __nv_bfloat16* __restrict__ wk,
-                       const __nv_bfloat16* __restrict__ wq_alt, const __nv_bfloat16* __restrict__ wk_alt,
-                       int s_alt, const float* __restrict__ cosb, const float* __restrict__ sinb,
-                       int interleaved, float eps, const int* __restrict__ positions, PeerWait wt, int* status) {
-  constexpr int D = 128;
+qk_norm_rope128_kernel(const __grid_constant__ HeadRows a, PeerWait wt, int* status) {
   if (wt.counter) {
     // fused exchange: the rows come from the peers' QKV GEMM epilogues; wait for their arrivals
     // here instead of in a barrier kernel of its own
@@ -197,82 +300,64 @@ qk_norm_rope128_kernel(__nv_bfloat16* __restrict__ qkv, long rows, int S, int H,
     }
     __syncthreads();
   }
-  const long row = (long)blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (row >= rows) return;
-  const int lane = threadIdx.x & 31;
-  const int l16 = lane & 15;
-  const int hsel = lane >> 4;
-  const int s = (int)(row % S);
-  const int pos = positions ? positions[row] : s;
-  const bool alt = s >= s_alt;
-  const __nv_bfloat16* wqq = (alt && wq_alt) ? wq_alt : wq;
-  const __nv_bfloat16* wkk = (alt && wk_alt) ? wk_alt : wk;
-  float wqf[8], wkf[8];
-  if (wqq) { load8(wqq + l16 * 8, wqf); load8(wkk + l16 * 8, wkf); }
-  // rotation coefficients of this lane's elements
-  float cs[8], sn[8];
-  if (cosb) {
-    const float* cr = cosb + (size_t)pos * (D / 2);
-    const float* sr = sinb + (size_t)pos * (D / 2);
-    if (interleaved) {   // elements 8*l16 .. +7 = pairs 4*l16 .. +3
-      const float4 c4 = *reinterpret_cast<const float4*>(cr + 4 * l16);
-      const float4 s4 = *reinterpret_cast<const float4*>(sr + 4 * l16);
-      cs[0] = cs[1] = c4.x; cs[2] = cs[3] = c4.y; cs[4] = cs[5] = c4.z; cs[6] = cs[7] = c4.w;
-      sn[0] = -s4.x; sn[1] = s4.x; sn[2] = -s4.y; sn[3] = s4.y; sn[4] = -s4.z; sn[5] = s4.z; sn[6] = -s4.w; sn[7] = s4.w;
-    } else {             // element i pairs with i +- 64; frequency index i mod 64
-      const int f0 = (l16 & 7) * 8;
-      const float sign = l16 < 8 ? -1.f : 1.f;
-#pragma unroll
-      for (int e = 0; e < 8; ++e) { cs[e] = cr[f0 + e]; sn[e] = sign * sr[f0 + e]; }
-    }
+  const int all = a.H + (a.pages.k ? 2 : 1) * a.Hkv, pairs = (all + 1) / 2;
+  const long unit = (long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  const long row = unit / pairs;
+  if (row >= a.rows) return;
+  const int lane = threadIdx.x & 31, l16 = lane & 15;
+  const int h = (int)(unit - row * pairs) * 2 + (lane >> 4);
+  uint4 v = make_uint4(0u, 0u, 0u, 0u), gain = v;
+  if (h < all) v = *reinterpret_cast<const uint4*>(a.qkv + (size_t)row * a.ld + (size_t)h * 128 + l16 * 8);
+  const int s = (int)(row % a.S);
+  const bool alt = s >= a.s_alt;
+  if (a.wq) {
+    const __nv_bfloat16* g = h < a.H ? ((alt && a.wq_alt) ? a.wq_alt : a.wq) : ((alt && a.wk_alt) ? a.wk_alt : a.wk);
+    gain = *reinterpret_cast<const uint4*>(g + l16 * 8);
   }
-  __nv_bfloat16* base = qkv + (size_t)row * ld;
-  const int heads = H + Hkv;
+  float cs[8], sn[8];
+  rope_coefficients(a, row, s, l16, cs, sn);
+  const uint4 o = head_norm_rope(v, a.wq != nullptr, gain, a.cosb != nullptr, a.interleaved, cs, sn, a.eps);
+  if (h < all) store_head(a, row, h, l16, a.pages.k ? a.pages.slots[row] : -1, v, o);
+}
+
+// The same for many rows: a warp walks all heads of its row, 8 at a time, and fetches the rotation coefficients once.
+__global__ void __launch_bounds__(256)
+qk_norm_rope128_rows_kernel(const __grid_constant__ HeadRows a, PeerWait wt, int* status) {
+  if (wt.counter) {
+    if (threadIdx.x == 0) {
+      peer_wait_arrivals(wt, nullptr, status);
+      peer_wait_cta_exit(wt, gridDim.x);
+    }
+    __syncthreads();
+  }
+  const long row = (long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (row >= a.rows) return;
+  const int all = a.H + (a.pages.k ? 2 : 1) * a.Hkv;
+  const int lane = threadIdx.x & 31, l16 = lane & 15, hsel = lane >> 4;
+  const int s = (int)(row % a.S);
+  const bool alt = s >= a.s_alt;
+  uint4 gq = make_uint4(0u, 0u, 0u, 0u), gk = gq;
+  if (a.wq) {
+    gq = *reinterpret_cast<const uint4*>(((alt && a.wq_alt) ? a.wq_alt : a.wq) + l16 * 8);
+    gk = *reinterpret_cast<const uint4*>(((alt && a.wk_alt) ? a.wk_alt : a.wk) + l16 * 8);
+  }
+  float cs[8], sn[8];
+  rope_coefficients(a, row, s, l16, cs, sn);
+  const int page = a.pages.k ? a.pages.slots[row] : -1;
   constexpr int U = 4;
-  for (int h0 = 0; h0 < heads; h0 += 2 * U) {
+#pragma unroll 1
+  for (int h0 = hsel; h0 < all; h0 += 2 * U) {
     uint4 v[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int h = h0 + 2 * u + hsel;
-      v[u] = h < heads ? *reinterpret_cast<const uint4*>(base + (size_t)h * D + l16 * 8) : make_uint4(0u, 0u, 0u, 0u);
+      const int h = h0 + 2 * u;
+      v[u] = h < all ? *reinterpret_cast<const uint4*>(a.qkv + (size_t)row * a.ld + (size_t)h * 128 + l16 * 8) : make_uint4(0u, 0u, 0u, 0u);
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int h = h0 + 2 * u + hsel;
-      const uint32_t w[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
-      float xv[8];
-      float ss = 0.f;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 f = unpack_bf16(w[j]);
-        xv[2 * j] = f.x; xv[2 * j + 1] = f.y;
-        ss = fmaf(f.x, f.x, fmaf(f.y, f.y, ss));
-      }
-      if (wqq) {
-#pragma unroll
-        for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        const float r = rsqrtf(ss * (1.0f / D) + eps);
-        const bool is_k = h >= H;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) xv[e] = xv[e] * r * (is_k ? wkf[e] : wqf[e]);
-      }
-      if (cosb) {
-        if (interleaved) {
-#pragma unroll
-          for (int e = 0; e < 8; e += 2) {
-            const float a = xv[e], bb = xv[e + 1];
-            xv[e] = fmaf(a, cs[e], bb * sn[e]);          // a*c - b*s
-            xv[e + 1] = fmaf(bb, cs[e + 1], a * sn[e + 1]);  // b*c + a*s
-          }
-        } else {
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            const float partner = __shfl_xor_sync(0xffffffffu, xv[e], 8);
-            xv[e] = fmaf(xv[e], cs[e], partner * sn[e]);
-          }
-        }
-      }
-      if (h < heads) store8(base + (size_t)h * D + l16 * 8, xv);
+      const int h = h0 + 2 * u;
+      const uint4 o = head_norm_rope(v[u], a.wq != nullptr, h < a.H ? gq : gk, a.cosb != nullptr, a.interleaved, cs, sn, a.eps);
+      if (h < all) store_head(a, row, h, l16, page, v[u], o);
     }
   }
 }
@@ -498,58 +583,77 @@ extern "C" int omni_norm_modulate(const void* x, void* y, int rows, int D, int l
                                   const void* scale, int mod_stride, int rows_per_batch, int rms,
                                   float eps, void* stream) {
   if (rows <= 0) return RC_OK;
-  if ((D & 7) || D > NM_THREADS * 8 * NM_MAXV || (ldx & 7) || (ldy & 7) || (mod_stride & 7)) return RC_BAD_ARG;
+  if ((D & 7) || D > 8192 || (ldx & 7) || (ldy & 7) || (mod_stride & 7)) return RC_BAD_ARG;
   if (rows_per_batch <= 0) rows_per_batch = rows;
   auto xx = (const __nv_bfloat16*)x; auto yy = (__nv_bfloat16*)y;
   auto w = (const __nv_bfloat16*)weight; auto bb = (const __nv_bfloat16*)bias;
   auto sh = (const __nv_bfloat16*)shift; auto sc = (const __nv_bfloat16*)scale;
   cudaStream_t st = (cudaStream_t)stream;
-  const int vpl = ((D >> 3) + 31) / 32;
-  const unsigned wgrid = (unsigned)((rows + 7) / 8);
-#define OMNI_NM_WARP(V) norm_modulate_warp_kernel<V><<<wgrid, 256, 0, st>>>(xx, yy, rows, D, ldx, ldy, w, bb, sh, sc, mod_stride, rows_per_batch, rms, eps)
-  if (vpl <= 2) OMNI_NM_WARP(2);
-  else if (vpl <= 4) OMNI_NM_WARP(4);
-  else if (vpl <= 8) OMNI_NM_WARP(8);
-  else if (vpl <= 12) OMNI_NM_WARP(12);
-  else if (vpl <= 16) OMNI_NM_WARP(16);
-  else if (vpl <= 20) OMNI_NM_WARP(20);
-  else
-    norm_modulate_kernel<<<rows, NM_THREADS, 0, st>>>(xx, yy, rows, D, ldx, ldy, w, bb, sh, sc, mod_stride,
-                                                      rows_per_batch, rms, eps);
+  const int nchunk = D >> 3;
+#define OMNI_NM_WARP(V, W) norm_modulate_warp_kernel<V, W><<<(unsigned)((rows + 8 / W - 1) / (8 / W)), 256, 0, st>>>(xx, yy, rows, D, ldx, ldy, w, bb, sh, sc, mod_stride, rows_per_batch, rms, eps)
+  if (nchunk <= 64) OMNI_NM_WARP(2, 1);
+  else if (nchunk <= 128) OMNI_NM_WARP(4, 1);
+  else if (rows < 8 * sm_count() || nchunk > 640)
+    // up to 8 rows per SM a block per row is one round of latencies
+    norm_modulate_kernel<2><<<rows, ((nchunk + 1) / 2 + 31) / 32 * 32, 0, st>>>(xx, yy, D, ldx, ldy, w, bb, sh, sc, mod_stride,
+                                                                               rows_per_batch, rms, eps);
+  else if (nchunk <= 256) OMNI_NM_WARP(4, 2);
+  else if (nchunk <= 384) OMNI_NM_WARP(6, 2);
+  else if (nchunk <= 512) OMNI_NM_WARP(8, 2);
+  else OMNI_NM_WARP(5, 4);
 #undef OMNI_NM_WARP
   return (int)cudaGetLastError();
 }
 
 // `sync` (may be null, head_dim 128 only): arrivals from the peers' QKV epilogues that the kernel
 // waits for before it touches the buffer (see peer_signal.cuh); `status` receives a timeout code.
-extern "C" int omni_qk_norm_rope_sync(void* qkv, int B, int S, int H, int Hkv, int D, int ld, const void* wq,
-                                      const void* wk, const void* wq_alt, const void* wk_alt, int s_alt,
-                                      const float* cosb, const float* sinb, int interleaved, float eps,
-                                      const int* positions, const OmniSync* sync, int* status, void* stream) {
+// `kc`, `vc` (both or neither; head_dim 128): pages [slots, Hkv, D] that the key heads, as they leave the kernel, and the value
+// heads of row r are written to at slots[r] (< 0: not).
+extern "C" int omni_qk_norm_rope_pages(void* qkv, int B, int S, int H, int Hkv, int D, int ld, const void* wq,
+                                       const void* wk, const void* wq_alt, const void* wk_alt, int s_alt,
+                                       const float* cosb, const float* sinb, int interleaved, float eps,
+                                       const int* positions, void* kc, void* vc, const int* slots, const OmniSync* sync,
+                                       int* status, void* stream) {
   const long total = (long)B * S * (H + Hkv);
   if (total <= 0) return sync ? RC_BAD_ARG : RC_OK;
   PeerSignal unused;
   PeerWait wt;
   unpack_sync(sync, unused, wt);
-  if (wt.counter && !(D == 128 && (ld & 7) == 0 && (wq != nullptr) == (wk != nullptr))) return RC_BAD_ARG;
+  const bool fast = D == 128 && (ld & 7) == 0 && (wq != nullptr) == (wk != nullptr);
+  if ((wt.counter || kc) && !fast) return RC_BAD_ARG;
+  if ((kc != nullptr) != (vc != nullptr) || (kc && !slots)) return RC_BAD_ARG;
   const int wpb = 8;
   const unsigned grid = (unsigned)((total + wpb - 1) / wpb);
   auto q = (__nv_bfloat16*)qkv;
   auto a = (const __nv_bfloat16*)wq; auto b = (const __nv_bfloat16*)wk;
   auto c = (const __nv_bfloat16*)wq_alt; auto d = (const __nv_bfloat16*)wk_alt;
-  const bool have_w = wq != nullptr;
-  if (D == 128 && (ld & 7) == 0 && (wq != nullptr) == (wk != nullptr)) {
+  cudaStream_t st = (cudaStream_t)stream;
+  if (fast) {
     const long rows = (long)B * S;
-    (void)have_w;
-    qk_norm_rope128_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, (cudaStream_t)stream>>>(
-        q, rows, S, H, Hkv, ld, a, b, c, d, s_alt, cosb, sinb, interleaved, eps, positions, wt, status);
+    const HeadRows r = {q, rows, S, H, Hkv, ld, a, b, c, d, s_alt, cosb, sinb, interleaved, eps, positions,
+                        {(__nv_bfloat16*)kc, (__nv_bfloat16*)vc, slots}};
+    const int all = H + Hkv + (kc ? Hkv : 0);
+    const long pairs = rows * ((all + 1) / 2);
+    // two heads to a warp up to about 600 rows of 48 heads; from there on a warp per row, which loads the coefficients once
+    if (pairs <= 2L * 64 * sm_count())
+      qk_norm_rope128_kernel<<<(unsigned)((pairs + 7) / 8), 256, 0, st>>>(r, wt, status);
+    else
+      qk_norm_rope128_rows_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(r, wt, status);
   } else if (D == 128)
-    qk_norm_rope_kernel<128><<<grid, wpb * 32, 0, (cudaStream_t)stream>>>(q, B, S, H, Hkv, ld, a, b, c, d, s_alt, cosb, sinb, interleaved, eps, positions);
+    qk_norm_rope_kernel<128><<<grid, wpb * 32, 0, st>>>(q, B, S, H, Hkv, ld, a, b, c, d, s_alt, cosb, sinb, interleaved, eps, positions);
   else if (D == 64)
-    qk_norm_rope_kernel<64><<<grid, wpb * 32, 0, (cudaStream_t)stream>>>(q, B, S, H, Hkv, ld, a, b, c, d, s_alt, cosb, sinb, interleaved, eps, positions);
+    qk_norm_rope_kernel<64><<<grid, wpb * 32, 0, st>>>(q, B, S, H, Hkv, ld, a, b, c, d, s_alt, cosb, sinb, interleaved, eps, positions);
   else
     return RC_BAD_ARG;
   return (int)cudaGetLastError();
+}
+
+extern "C" int omni_qk_norm_rope_sync(void* qkv, int B, int S, int H, int Hkv, int D, int ld, const void* wq,
+                                      const void* wk, const void* wq_alt, const void* wk_alt, int s_alt,
+                                      const float* cosb, const float* sinb, int interleaved, float eps,
+                                      const int* positions, const OmniSync* sync, int* status, void* stream) {
+  return omni_qk_norm_rope_pages(qkv, B, S, H, Hkv, D, ld, wq, wk, wq_alt, wk_alt, s_alt, cosb, sinb, interleaved, eps,
+                                 positions, nullptr, nullptr, nullptr, sync, status, stream);
 }
 
 extern "C" int omni_qk_norm_rope(void* qkv, int B, int S, int H, int Hkv, int D, int ld, const void* wq,

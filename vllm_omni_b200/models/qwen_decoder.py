@@ -293,8 +293,6 @@ class QwenDecoderModel(nn.Module):
         q = qkv[:, :H * Dh].view(T, H, Dh)
         k = qkv[:, H * Dh:(H + Hkv) * Dh].view(T, Hkv, Dh)
         v = qkv[:, (H + Hkv) * Dh:].view(T, Hkv, Dh)
-        if k_cache is not None:
-            KC.kv_write(k, v, k_cache, v_cache, batch.slot_mapping)
         scale = 1.0 / math.sqrt(Dh)
         o = out.view(T, H, Dh)
         for seg in batch.prefills:
@@ -339,9 +337,10 @@ class QwenDecoderModel(nn.Module):
         for li, layer in enumerate(self.layers):
             fused.norm_modulate(x, weight=layer.input_layernorm, rms=True, eps=cfg.rms_norm_eps, out=xn)
             qkv = layer.qkv_proj(xn)
-            fused.qk_norm_rope_(qkv.view(1, T, -1), H, Hkv, Dh, wq=layer.q_norm, wk=layer.k_norm, cos=cos, sin=sin,
-                                interleaved=False, eps=cfg.rms_norm_eps)
             kc, vc = kv_caches[li] if kv_caches is not None else (None, None)
+            fused.qk_norm_rope_(qkv.view(1, T, -1), H, Hkv, Dh, wq=layer.q_norm, wk=layer.k_norm, cos=cos, sin=sin,
+                                interleaved=False, eps=cfg.rms_norm_eps,
+                                pages=None if kc is None else (kc, vc, batch.slot_mapping))
             self.attention_block(layer, qkv, batch, kc, vc, attn)
             if self.tp_reduce is not None:
                 self.tp_reduce.linear(layer.o_proj, attn, residual=x, out=x, capacity=tp_cap)   # sum over ranks

@@ -117,26 +117,41 @@ def qk_norm_rope_reference(qkv, H, Hkv, D, wq, wk, wq_alt, wk_alt, s_alt, cos, s
 
 
 def qk_norm_rope_(qkv, H, Hkv, D, wq=None, wk=None, wq_alt=None, wk_alt=None, s_alt=1 << 30, cos=None, sin=None,
-                  interleaved=True, eps=1e-6, positions=None, sync=None):
+                  interleaved=True, eps=1e-6, positions=None, sync=None, pages=None):
     """In place on a packed qkv buffer [B, S, (H + 2*Hkv) * D]: q,k <- rope(rmsnorm(q,k)).
 
     Rows s >= s_alt use the norm weights ``wq_alt`` / ``wk_alt`` (the text rows that follow
     the image rows of a joint sequence).  ``sync``: an ``OmniSync`` whose waiting half names the
-    arrivals (peers' QKV epilogues) the kernel waits for before it touches the buffer."""
+    arrivals (peers' QKV epilogues) the kernel waits for before it touches the buffer.
+
+    ``pages = (k_cache, v_cache, slots)`` (one batch, B = 1): the key heads, as they come out, and the value heads of row t are
+    written to the pages [blocks, block size, Hkv, D] at slots[t] as well (int32 [S], < 0 = skip)."""
+    B, S = qkv.shape[:2]
+    kc = vc = slots = None
+    if pages is not None:
+        kc, vc, slots = pages
+        one_pass = qkv.is_cuda and D == 128 and (wq is None) == (wk is None) and qkv.stride(1) % 8 == 0 and not nv.bounds_check_enabled()
+        if not one_pass:
+            from .kv_cache import kv_write
+            qk_norm_rope_(qkv, H, Hkv, D, wq, wk, wq_alt, wk_alt, s_alt, cos, sin, interleaved, eps, positions, sync)
+            rows = qkv.view(B * S, -1)
+            kv_write(rows[:, H * D:(H + Hkv) * D].view(B * S, Hkv, D), rows[:, (H + Hkv) * D:].view(B * S, Hkv, D), kc, vc, slots)
+            return qkv
+        assert slots.dtype == torch.int32 and slots.is_contiguous() and slots.numel() == B * S
+        assert kc.is_contiguous() and vc.is_contiguous() and kc.shape[2:] == (Hkv, D) == vc.shape[2:] and kc.dtype == vc.dtype == qkv.dtype
     if not qkv.is_cuda:
         qkv.copy_(qk_norm_rope_reference(qkv, H, Hkv, D, wq, wk, wq_alt, wk_alt, s_alt, cos, sin, interleaved, eps, positions))
         return qkv
-    B, S = qkv.shape[:2]
     assert qkv.dtype == torch.bfloat16 and qkv.stride(-1) == 1 and qkv.is_contiguous()
     ld = qkv.stride(1)
     if cos is not None:
         assert cos.dtype == torch.float32 and cos.is_contiguous() and sin.is_contiguous() and cos.shape[-1] == D // 2
     if positions is not None:
         assert positions.dtype == torch.int32 and positions.is_contiguous()
-    rc = nv.lib("elementwise").omni_qk_norm_rope_sync(
+    rc = nv.lib("elementwise").omni_qk_norm_rope_pages(
         nv.ptr(qkv), c_int(B), c_int(S), c_int(H), c_int(Hkv), c_int(D), c_int(ld), nv.ptr(wq), nv.ptr(wk),
         nv.ptr(wq_alt), nv.ptr(wk_alt), c_int(min(s_alt, 1 << 30)), nv.ptr(cos), nv.ptr(sin), c_int(1 if interleaved else 0),
-        c_float(eps), nv.ptr(positions), ctypes.byref(sync) if sync is not None else None,
+        c_float(eps), nv.ptr(positions), nv.ptr(kc), nv.ptr(vc), nv.ptr(slots), ctypes.byref(sync) if sync is not None else None,
         nv.ptr(nv.status_word(qkv.device)), nv.stream_ptr())
     nv.check_rc(rc, "omni_qk_norm_rope")
     return qkv
