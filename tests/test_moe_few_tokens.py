@@ -1,0 +1,104 @@
+"""Experts of few tokens (csrc/moe.cu, tiles of 16 rows gathered in place): one row to several tiles per expert, experts of another
+rank, ragged widths, both activations; and the plan of the 128-row tiles."""
+import pytest
+import torch
+
+from vllm_omni_b200.ops import _native as nv
+from vllm_omni_b200.ops.moe import MoEWorkspace, Router, _few, expert_rows, moe_forward
+
+pytestmark = pytest.mark.gpu
+
+
+def _problem(T, E, k, D, F, crowd, seed=0):
+    g = torch.Generator(device="cuda").manual_seed(seed + T * 31 + E)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    x, w13, w2 = rnd(T, D).bfloat16(), (rnd(E, 2 * F, D) * D ** -0.5).bfloat16(), (rnd(E, D, F) * F ** -0.5).bfloat16()
+    # distinct logits (no ties to break); with ``crowd`` every token wants expert 1
+    logits = torch.stack([torch.randperm(E, generator=g, device="cuda") for _ in range(T)]).float() / 16
+    if crowd:
+        logits[:, 1] = E / 16 + 1
+    return x, logits.bfloat16(), w13, w2
+
+
+def _expected(x, ids, w, up, down, act, lo=0, hi=1 << 30):
+    """(result, bound): bf16 rounding of h, of every pair's row and of the result, tanh.approx in silu, fp32 sums."""
+    T, F = x.shape[0], down.shape[2]
+    y, bound = torch.zeros(T, down.shape[1], dtype=torch.float64, device="cuda"), 0
+    bound = torch.zeros_like(y)
+    for t in range(T):
+        for j in range(ids.shape[1]):
+            e = int(ids[t, j])
+            if not lo <= e < hi:
+                continue
+            a = x[t].double() @ up[e - lo].double().T
+            if act == "swiglu":
+                h = torch.nn.functional.silu(a[:F]) * a[F:]
+                eh = h.abs() * 2.0 ** -8 + (a[:F] * a[F:]).abs() * 2.0 ** -11 + 1e-4
+            else:
+                h = a.clamp(min=0) ** 2
+                eh = h * 2.0 ** -8 + 1e-4
+            d = down[e - lo].double()
+            y[t] += w[t, j].double() * (h @ d.T)
+            bound[t] += w[t, j].double() * (eh @ d.abs().T + (h @ d.T).abs() * 2.0 ** -8 + 1e-4)
+    return y, 1.2 * bound + y.abs() * 2.0 ** -8
+
+
+@pytest.mark.parametrize("T,E,k,D,F,crowd", [(1, 128, 8, 2048, 768, False), (32, 128, 8, 256, 96, False), (16, 8, 1, 72, 40, True),
+                                              (16, 16, 2, 1032, 136, True), (32, 128, 8, 128, 64, True), (17, 256, 16, 64, 1096, True)])
+def test_moe_forward(T, E, k, D, F, crowd):
+    x, logits, w13, w2 = _problem(T, E, k, D, F, crowd)
+    assert _few(T, k, E, False)
+    p = torch.softmax(logits.double(), -1)
+    w, ids = p.topk(k, -1)
+    w = w / w.sum(-1, keepdim=True)
+    res = torch.randn(T, D, device="cuda").bfloat16()
+    ref, bound = _expected(x, ids, w, w13, w2, "swiglu")
+    y = moe_forward(x, logits, w13, w2, k, ws=MoEWorkspace(), residual=res)
+    assert ((y.double() - ref - res.double()).abs() <= bound + res.double().abs() * 2.0 ** -8).all()
+    half = E // 2
+    parts = [moe_forward(x, logits, w13[a:b], w2[a:b], k, e_lo=a, e_hi=b).double() for a, b in ((0, half), (half, E))]
+    for (a, b), got in zip(((0, half), (half, E)), parts):
+        ref, bound = _expected(x, ids, w, w13[a:b], w2[a:b], "swiglu", a, b)
+        assert ((got - ref).abs() <= bound).all()
+    nv.check_status()
+
+
+@pytest.mark.parametrize("act", ["relu2", "swiglu"])
+def test_expert_rows(act):
+    T, E, k, D, F = 33, 72, 4, 200, 72
+    x, logits, up, down = _problem(T, E, k, D, F, False)
+    up = up if act == "swiglu" else up[:, :F].contiguous()
+    router = Router(E, k)
+    rw = torch.randn(E, D, device="cuda").bfloat16()
+    got = expert_rows(x, rw, None, router, up, down, act, MoEWorkspace())
+    ids, w = router.choose(x.double() @ rw.double().T)
+    y = torch.zeros(T, D, dtype=torch.float64, device="cuda")
+    for t in range(T):
+        for j in range(k):
+            y[t] += got.weights[t, j].double() * got.y[got.row_of_pair[t * k + j]].double()
+    ref, bound = _expected(x, ids, w, up, down, act)
+    same = (got.weights.double() - w.double()).abs().max(1).values < 1e-3      # rows whose choice is not a rounding
+    assert same.sum() >= T - 2 and ((y - ref).abs() <= bound + 0.01 * ref.abs())[same].all()
+
+
+@pytest.mark.parametrize("n_pairs,E,lo,hi", [(1, 1, 0, 1), (5000, 128, 0, 128), (3000, 7, 2, 5), (2048, 1024, 0, 1024), (70001, 64, 0, 64)])
+def test_compact_plan(n_pairs, E, lo, hi):
+    g = torch.Generator(device="cuda").manual_seed(n_pairs)
+    ids = (torch.rand(n_pairs, generator=g, device="cuda") ** 2 * E).int().clamp(max=E - 1)
+    tiles = E + n_pairs // 128 + 1
+    row, te, t0, tn, n = (torch.full((m,), -7, dtype=torch.int32, device="cuda") for m in (n_pairs, tiles, tiles, tiles, 1))
+    from ctypes import c_int
+    nv.check_rc(nv.lib("moe").omni_moe_plan_compact(nv.ptr(ids), c_int(n_pairs), c_int(E), c_int(lo), c_int(hi), c_int(tiles), nv.ptr(row),
+                                                    nv.ptr(te), nv.ptr(t0), nv.ptr(tn), nv.ptr(n), nv.stream_ptr()), "plan")
+    local = (ids >= lo) & (ids < hi)
+    assert int(n) == int(local.sum()) and (row[~local] == -1).all()
+    assert torch.equal(row[local].sort().values, torch.arange(int(n), device="cuda", dtype=torch.int32))
+    of_row = torch.empty(int(n), dtype=torch.int32, device="cuda")
+    of_row[row[local].long()] = ids[local]
+    assert torch.equal(of_row, of_row.sort().values)                            # experts in order, rows back to back
+    at = 0
+    for e, r0, rn in zip(te.tolist(), t0.tolist(), tn.tolist()):
+        if e >= 0:
+            assert r0 == at and 1 <= rn <= 128 and (of_row[r0:r0 + rn] == e).all()
+            at += rn
+    assert at == int(n)

@@ -1,0 +1,40 @@
+"""Paged attention of single tokens straight from the pages (csrc/decode_attn.cu): group sizes, head counts that do not fill a block,
+page sizes, lengths around tiles of 16 keys, one and many shares; page rows past a sequence's end hold NaN."""
+import pytest
+import torch
+
+from vllm_omni_b200.ops import kv_cache as KC
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("H,Hkv", [(8, 1), (32, 4), (32, 8), (12, 3), (20, 10), (16, 1), (36, 3), (5, 5)])
+@pytest.mark.parametrize("bs", [8, 16, 48, 128])
+@pytest.mark.parametrize("lens", [[1], [7, 8, 9, 16, 17, 33], [1000, 1, 333, 2047] * 5])
+def test_against_64_bits(H, Hkv, bs, lens):
+    D, n, G = 128, len(lens), H // Hkv
+    g = torch.Generator(device="cuda").manual_seed(H * 100 + bs + n)
+    per = [-(-l // bs) for l in lens]
+    width = max(per) + 1
+    order = torch.randperm(sum(per), generator=torch.Generator().manual_seed(n)).tolist()
+    k, v = (torch.full((sum(per), bs, Hkv, D), float("nan"), device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    tables, at = torch.zeros(n, width, dtype=torch.int32), 0
+    q = torch.randn(n, H * D + 16, generator=g, device="cuda").bfloat16()[:, :H * D].view(n, H, D)
+    ref, bound = torch.empty(n, H, D, dtype=torch.float64, device="cuda"), torch.empty(n, H, D, dtype=torch.float64, device="cuda")
+    for s, l in enumerate(lens):
+        pages = order[at:at + per[s]]
+        at += per[s]
+        tables[s, :per[s]] = torch.tensor(pages)
+        ks, vs = (torch.randn(l, Hkv, D, generator=g, device="cuda").bfloat16() for _ in range(2))
+        for cache, rows in ((k, ks), (v, vs)):
+            for i, pg in enumerate(pages):
+                part = rows[i * bs:(i + 1) * bs]
+                cache[pg, :part.shape[0]] = part
+        kk, vv = (t.double().repeat_interleave(G, 1) for t in (ks, vs))
+        w = torch.softmax(torch.einsum("hd,khd->hk", q[s].double(), kk) * D ** -0.5, -1)
+        ref[s] = torch.einsum("hk,khd->hd", w, vv)
+        # weights rounded to bf16 (half an ulp, 2^-9, of each), ex2.approx and fp32 scores far below that; result rounded once
+        bound[s] = torch.einsum("hk,khd->hd", w, vv.abs()) * 2.0 ** -8 + ref[s].abs() * 2.0 ** -8 + 1e-5
+    out = torch.empty(n, H, D, device="cuda", dtype=torch.bfloat16)
+    KC.paged_decode(q, k, v, tables.cuda(), torch.tensor(lens, dtype=torch.int32, device="cuda"), out=out, impl="stream")
+    assert ((out.double() - ref).abs() <= bound).all()

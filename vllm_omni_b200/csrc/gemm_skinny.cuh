@@ -79,57 +79,24 @@ __device__ __forceinline__ void skinny_finish(float (&x)[B], int m, int step, in
 }
 
 // ---------------------------------------------------------------------------------------------------- at most 16 rows
-__device__ __forceinline__ uint4 ldg_stream(const __nv_bfloat16* p) {   // read once: past L1
-  uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.L2::256B.v4.u32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-  return v;
-}
-__device__ __forceinline__ void mma_bf16_16x8(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-// NT * 8 rows of A; NW warps, warp w takes the 32-channel chunks w, w + NW, ...  Lane group j of a quad owns channels 8 j .. 8 j + 7 of
-// a chunk for both operands: one 16-byte load per row, and the contraction is permuted alike on both sides.  U chunks are
-// in flight per warp: 16 resident warps x 8 chunks x 1 KB = 128 KB per SM.
+// NT * 8 rows of A; 16 resident warps x 8 chunks x 1 KB = 128 KB of W in flight per SM.
 template <int NT, int NW>
 __global__ void __launch_bounds__(32 * NW, NW == 16 ? 1 : 2)
 gemm_rows_kernel(const __nv_bfloat16* __restrict__ A, int lda, const __nv_bfloat16* __restrict__ W, int ldw, __nv_bfloat16* C, int ldc,
                  int M, int N, int K, const __grid_constant__ GemmEpilogue epi) {
-  constexpr int U = NT == 1 ? 8 : 4;
   __shared__ float part[NW][NT * 8][16];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, j = lane & 3;
   const int n0 = blockIdx.x * 16;
-  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-  const __nv_bfloat16* w0 = W + (size_t)min(n0 + g, N - 1) * ldw;          // columns past N repeat the last one and are not stored
-  const __nv_bfloat16* w1 = W + (size_t)min(n0 + 8 + g, N - 1) * ldw;
+  const __nv_bfloat16* x[NT];
   float acc[NT][4];
 #pragma unroll
-  for (int t = 0; t < NT; ++t)
+  for (int t = 0; t < NT; ++t) {
+    x[t] = t * 8 + g < M ? A + (size_t)(t * 8 + g) * lda : nullptr;
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc[t][i] = 0.f;
-#pragma unroll 1
-  for (int c = warp * 32; c < K; c += 32 * NW * U) {
-    uint4 a[U][2], b[U][NT];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int ch = c + u * 32 * NW + j * 8;                              // K is a multiple of 8
-      const bool in = ch < K;
-      a[u][0] = in ? ldg_stream(w0 + ch) : zero;
-      a[u][1] = in ? ldg_stream(w1 + ch) : zero;
-#pragma unroll
-      for (int t = 0; t < NT; ++t)
-        b[u][t] = in && t * 8 + g < M ? *reinterpret_cast<const uint4*>(A + (size_t)(t * 8 + g) * lda + ch) : zero;
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-#pragma unroll
-      for (int t = 0; t < NT; ++t) {
-        mma_bf16_16x8(acc[t], a[u][0].x, a[u][1].x, a[u][0].y, a[u][1].y, b[u][t].x, b[u][t].y);
-        mma_bf16_16x8(acc[t], a[u][0].z, a[u][1].z, a[u][0].w, a[u][1].w, b[u][t].z, b[u][t].w);
-      }
   }
+  // columns past N repeat the last one and are not stored
+  few_rows_products<NT, NW, NT == 1 ? 8 : 4>(acc, W + (size_t)min(n0 + g, N - 1) * ldw, W + (size_t)min(n0 + 8 + g, N - 1) * ldw, x, K, warp, j);
 #pragma unroll
   for (int t = 0; t < NT; ++t)
 #pragma unroll
@@ -139,10 +106,10 @@ gemm_rows_kernel(const __nv_bfloat16* __restrict__ A, int lda, const __nv_bfloat
     const int n = n0 + (threadIdx.x & 15), m = threadIdx.x >> 4;
     if (n < N && m < M) {
       const float bias = epi.bias ? __bfloat162float(epi.bias[n]) : 0.f;
-      float x[1] = {0.f};
+      float y[1] = {0.f};
 #pragma unroll
-      for (int w = 0; w < NW; ++w) x[0] += part[w][m][threadIdx.x & 15];
-      skinny_finish<1>(x, m, 1, M, n, C, ldc, epi, bias);
+      for (int w = 0; w < NW; ++w) y[0] += part[w][m][threadIdx.x & 15];
+      skinny_finish<1>(y, m, 1, M, n, C, ldc, epi, bias);
     }
   }
 }

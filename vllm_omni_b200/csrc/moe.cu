@@ -5,6 +5,8 @@
 //                      among them, or sigmoid scores divided by their sum, of the best groups of experts (bf16 rows)
 //   omni_moe_topk      the same choice from fp32 logits
 //   omni_moe_pairs_f32 y[p] = act(W[expert of pair p] x[p / per]) in true fp32 (exact mode)
+//   omni_moe_few_plan  few tokens: tiles of at most 16 rows per expert, from router logits (route included) or chosen ids
+//   omni_moe_few_rows  few tokens: y[pair] = act(W[expert] x[pair / per]) with rows gathered in place, SwiGLU included
 //   omni_moe_plan      per-expert counts -> segment offsets padded to 128 rows (the GEMM's M
 //                      tile), the expert of every M tile, and the row of every (token, k) pair
 //   omni_moe_dispatch  copy token rows into the expert-major padded buffer
@@ -30,52 +32,60 @@ struct MoeBounds {
 static MoeBounds g_moe_bounds = {0, nullptr};
 enum { KID_MOE_PLAN = 3, KID_MOE_DISPATCH = 4, KID_MOE_COMBINE = 5 };
 
-// one warp per token; E <= 256 (8 per lane), k <= 16
-__global__ void __launch_bounds__(256)
-moe_route_kernel(const __nv_bfloat16* __restrict__ logits, int ld, int T, int E, int k, int renorm,
-                 int* __restrict__ ids, float* __restrict__ weights) {
-  const int t = blockIdx.x * 8 + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (t >= T) return;
+// Softmax over the logits of one token, its k largest and their weights, by one warp; E <= 256 (8 per lane), k <= 16.  Lane j
+// returns choice j.
+__device__ __forceinline__ void route_token(const __nv_bfloat16* __restrict__ logits, int E, int k, int renorm, int lane, int& id,
+                                            float& weight) {
   float v[8];
   float mx = -INFINITY;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const int e = lane + i * 32;
-    v[i] = e < E ? __bfloat162float(logits[(size_t)t * ld + e]) : -INFINITY;
+    v[i] = i * 32 < E && e < E ? __bfloat162float(logits[e]) : -INFINITY;
     mx = fmaxf(mx, v[i]);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   float sum = 0.f;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) { v[i] = v[i] == -INFINITY ? 0.f : __expf(v[i] - mx); sum += v[i]; }
+  for (int i = 0; i < 8; ++i)
+    if (i * 32 < E) { v[i] = v[i] == -INFINITY ? 0.f : __expf(v[i] - mx); sum += v[i]; }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
   const float inv = 1.0f / sum;
   float picked = 0.f;
+  id = 0;
+  weight = 0.f;
+  // numbers that are not negative compare like their bit patterns, so the best of the warp is one integer reduction
+#pragma unroll 1
   for (int j = 0; j < k; ++j) {
-    float best = -1.f;
-    int bi = 0x7fffffff;
+    int best = -1, bi = 0x7fffffff;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int e = lane + i * 32;
-      if (v[i] > best || (v[i] == best && e < bi)) { best = v[i]; bi = e; }
-    }
+    for (int i = 0; i < 8; ++i)
+      if (i * 32 < E && __float_as_int(v[i]) > best) { best = __float_as_int(v[i]); bi = lane + i * 32; }
+    const int top = __reduce_max_sync(0xffffffffu, best);
+    bi = __reduce_min_sync(0xffffffffu, best == top ? bi : 0x7fffffff);
+    const float w = __int_as_float(top) * inv;
+    if (lane == j) { id = bi; weight = w; }
+    picked += w;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-    }
-    if (lane == 0) { ids[(size_t)t * k + j] = bi; weights[(size_t)t * k + j] = best * inv; }
-    picked += best * inv;
-    if ((bi & 31) == lane) v[bi >> 5] = -1.f;   // remove the winner
+    for (int i = 0; i < 8; ++i)
+      if (bi == lane + i * 32) v[i] = __int_as_float(0x80000000);     // remove the winner: negative as an integer
   }
-  if (renorm && lane == 0) {
-    const float r = 1.0f / fmaxf(picked, 1e-20f);
-    for (int j = 0; j < k; ++j) weights[(size_t)t * k + j] *= r;
-  }
+  if (renorm) weight *= 1.0f / fmaxf(picked, 1e-20f);
+}
+
+// one warp per token
+__global__ void __launch_bounds__(256)
+moe_route_kernel(const __nv_bfloat16* __restrict__ logits, int ld, int T, int E, int k, int renorm,
+                 int* __restrict__ ids, float* __restrict__ weights) {
+  const int t = blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (t >= T) return;
+  int id;
+  float w;
+  route_token(logits + (size_t)t * ld, E, k, renorm, lane, id, w);
+  if (lane < k) { ids[(size_t)t * k + lane] = id; weights[(size_t)t * k + lane] = w; }
 }
 
 // What turns logits into a choice.  sigmoid = 0: softmax among the k largest.  sigmoid = 1: scores 1 / (1 + e^-z); with
@@ -350,59 +360,186 @@ moe_plan_kernel(const int* __restrict__ ids, int n_pairs, int E, int e_lo, int e
   }
 }
 
-// Plan without padding: the rows of expert e are [off[e], off[e] + cnt[e]); expert e owns ceil(cnt[e] / 128)
-// M tiles; tile t = (expert, first row, rows <= 128).  Unused tiles get expert -1.
+// Exclusive sums over the block's 1024 threads of two counts at once; totals in the last two references.
+__device__ __forceinline__ void block_scan2(int& a, int& b, int& total_a, int& total_b) {
+  __shared__ int wa[32], wb[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, a0 = a, b0 = b;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int ua = __shfl_up_sync(0xffffffffu, a, o), ub = __shfl_up_sync(0xffffffffu, b, o);
+    if (lane >= o) { a += ua; b += ub; }
+  }
+  if (lane == 31) { wa[warp] = a; wb[warp] = b; }
+  __syncthreads();
+  int sa = wa[lane], sb = wb[lane];
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int ua = __shfl_up_sync(0xffffffffu, sa, o), ub = __shfl_up_sync(0xffffffffu, sb, o);
+    if (lane >= o) { sa += ua; sb += ub; }
+  }
+  total_a = __shfl_sync(0xffffffffu, sa, 31);
+  total_b = __shfl_sync(0xffffffffu, sb, 31);
+  const int before = (warp + 31) & 31;
+  const int pa = __shfl_sync(0xffffffffu, sa, before), pb = __shfl_sync(0xffffffffu, sb, before);
+  a = a - a0 + (warp ? pa : 0);
+  b = b - b0 + (warp ? pb : 0);
+}
+
+// Plan without padding: the rows of expert e are [off[e], off[e] + cnt[e]); expert e owns ceil(cnt[e] / TILE)
+// M tiles; tile t = (expert, first row, rows <= TILE).  Unused tiles get expert -1.  One block; the place of a pair among its expert's
+// rows is what its atomic add to the expert's count returns (the order inside an expert does not affect results).
 __global__ void __launch_bounds__(1024)
 moe_plan_compact_kernel(const int* __restrict__ ids, int n_pairs, int E, int e_lo, int e_hi, int max_tiles,
                         int* __restrict__ row_of_pair, int* __restrict__ tile_expert, int* __restrict__ tile_row0,
                         int* __restrict__ tile_rows, int* __restrict__ n_rows_out, MoeBounds bd) {
   __shared__ int cnt[1024];
-  __shared__ int off[1025];
-  __shared__ int toff[1025];
-  for (int e = threadIdx.x; e < E; e += blockDim.x) cnt[e] = 0;
+  __shared__ int off[1024];
+  cnt[threadIdx.x] = 0;
   __syncthreads();
-  for (int i = threadIdx.x; i < n_pairs; i += blockDim.x) {
+#pragma unroll 4
+  for (int i = threadIdx.x; i < n_pairs; i += 1024) {
     const int e = ids[i];
-    if (!OMNI_IN_BOUNDS(e >= 0 && e < E, bd.status, KID_MOE_PLAN)) continue;
-    if (e >= e_lo && e < e_hi) atomicAdd(&cnt[e], 1);
+    int r = -1;
+    if (OMNI_IN_BOUNDS(e >= 0 && e < E, bd.status, KID_MOE_PLAN) && e >= e_lo && e < e_hi) r = atomicAdd(&cnt[e], 1);
+    row_of_pair[i] = r;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int acc = 0, tacc = 0;
-    for (int e = 0; e < E; ++e) {
-      off[e] = acc;
-      toff[e] = tacc;
-      acc += cnt[e];
-      tacc += (cnt[e] + MOE_TILE - 1) / MOE_TILE;
-    }
-    off[E] = acc;
-    toff[E] = tacc;
-    *n_rows_out = acc;
+  const int e = threadIdx.x, mine = cnt[e];             // experts past E have none
+  int row = mine, tile = (mine + MOE_TILE - 1) / MOE_TILE, rows, tiles;
+  block_scan2(row, tile, rows, tiles);
+  off[e] = row;
+  if (e == 0) *n_rows_out = rows;
+  for (int i = 0; i * MOE_TILE < mine; ++i) {
+    tile_expert[tile + i] = e;
+    tile_row0[tile + i] = row + i * MOE_TILE;
+    tile_rows[tile + i] = min(MOE_TILE, mine - i * MOE_TILE);
+  }
+  for (int t = tiles + threadIdx.x; t < max_tiles; t += 1024) {
+    tile_expert[t] = -1;
+    tile_row0[t] = 0;
+    tile_rows[t] = 0;
   }
   __syncthreads();
-  for (int tile = threadIdx.x; tile < max_tiles; tile += blockDim.x) {
-    int ex = -1, r0 = 0, nr = 0;
-    if (tile < toff[E]) {
-      int lo = 0, hi = E - 1;            // the last e with toff[e] <= tile that owns tiles
-      while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (toff[mid] <= tile) lo = mid; else hi = mid - 1;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < n_pairs; i += 1024) {
+    const int r = row_of_pair[i];
+    if (r >= 0) row_of_pair[i] = off[ids[i]] + r;
+  }
+}
+
+// ------------------------------------------------------------------------------------------------------ few tokens
+// Up to a few hundred (token, choice) pairs the chain is the streaming of the chosen experts' weights plus launches, so it has three
+// instead of seven: plan (with the choice, from router logits), up projection with SwiGLU, down projection.  Rows are gathered
+// where they are read and results lie at their pair's index, so nothing is copied; a tile is at most 16 rows of one expert.
+constexpr int FEW_TILE = 16, FEW_PAIRS = 2048;
+struct FewPlan {
+  int *ids;                       // [pairs]: read, or written when the choice is made here
+  float* weights;                 // [pairs], written with the choice
+  int *pair_of_row, *row_of_pair; // rows of an expert back to back; row_of_pair is the pair's own index, -1 = not local
+  int *tile_expert, *tile_row0, *tile_rows;
+  int max_tiles;
+};
+
+__global__ void __launch_bounds__(1024)
+moe_few_plan_kernel(const __nv_bfloat16* __restrict__ logits, int ld, int T, int E, int k, int renorm, int e_lo, int e_hi,
+                    const FewPlan p, MoeBounds bd) {
+  __shared__ int sid[FEW_PAIRS];
+  __shared__ int cnt[1024];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_pairs = T * k;
+  cnt[threadIdx.x] = 0;
+  if (logits) {
+    for (int t = warp; t < T; t += 32) {
+      int id;
+      float w;
+      route_token(logits + (size_t)t * ld, E, k, renorm, lane, id, w);
+      if (lane < k) {
+        sid[t * k + lane] = id;
+        p.ids[t * k + lane] = id;
+        p.weights[t * k + lane] = w;
       }
-      ex = lo;
-      const int within = tile - toff[ex];
-      r0 = off[ex] + within * MOE_TILE;
-      nr = min(MOE_TILE, cnt[ex] - within * MOE_TILE);
     }
-    tile_expert[tile] = ex;
-    tile_row0[tile] = r0;
-    tile_rows[tile] = nr;
+  } else {
+    for (int i = threadIdx.x; i < n_pairs; i += 1024) sid[i] = p.ids[i];
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < E; e += blockDim.x) cnt[e] = 0;   // reuse as cursors
+  int place[FEW_PAIRS / 1024];
+#pragma unroll
+  for (int q = 0; q < FEW_PAIRS / 1024; ++q) {
+    const int i = threadIdx.x + q * 1024;
+    place[q] = -1;
+    if (i < n_pairs) {
+      const int e = sid[i];
+      if (OMNI_IN_BOUNDS(e >= 0 && e < E, bd.status, KID_MOE_PLAN) && e >= e_lo && e < e_hi) place[q] = atomicAdd(&cnt[e], 1);
+      p.row_of_pair[i] = place[q] >= 0 ? i : -1;
+    }
+  }
   __syncthreads();
-  for (int i = threadIdx.x; i < n_pairs; i += blockDim.x) {
-    const int e = ids[i];
-    row_of_pair[i] = (e >= e_lo && e < e_hi) ? off[e] + atomicAdd(&cnt[e], 1) : -1;
+  const int e = threadIdx.x, mine = cnt[e];
+  int row = mine, tile = (mine + FEW_TILE - 1) / FEW_TILE, rows, tiles;
+  block_scan2(row, tile, rows, tiles);
+  for (int i = 0; i * FEW_TILE < mine; ++i) {
+    p.tile_expert[tile + i] = e - e_lo;                 // the weights hold the local experts
+    p.tile_row0[tile + i] = row + i * FEW_TILE;
+    p.tile_rows[tile + i] = min(FEW_TILE, mine - i * FEW_TILE);
+  }
+  for (int t = tiles + threadIdx.x; t < p.max_tiles; t += 1024) p.tile_expert[t] = -1;
+  __syncthreads();                                      // everyone has its count: the array becomes the first rows
+  cnt[e] = row;
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < FEW_PAIRS / 1024; ++q) {
+    const int i = threadIdx.x + q * 1024;
+    if (i < n_pairs && place[q] >= 0) p.pair_of_row[cnt[sid[i]] + place[q]] = i;
+  }
+}
+
+// y[pair, n] = act(sum_c W[e, n, c] x[pair / per, c]) for a tile of one expert and 16 columns (GATED: 8 columns n of silu(gate) * lift, rows
+// n and N + n of W are the two halves of the MMA's 16).  The block's NW warps share the contraction.
+template <int NW, bool GATED>
+__global__ void __launch_bounds__(32 * NW, 16 / NW)
+moe_few_rows_kernel(const __nv_bfloat16* __restrict__ x, long ldx, int per, const __nv_bfloat16* __restrict__ w, int N, int K,
+                    const int* __restrict__ tile_expert, const int* __restrict__ tile_row0, const int* __restrict__ tile_rows,
+                    const int* __restrict__ pair_of_row, __nv_bfloat16* __restrict__ y, long ldy, int relu2) {
+  __shared__ float part[NW][FEW_TILE][16];
+  constexpr int COLS = GATED ? 8 : 16;
+  const int e = tile_expert[blockIdx.y];
+  if (e < 0) return;
+  const int row0 = tile_row0[blockIdx.y], rows = tile_rows[blockIdx.y];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, j = lane & 3;
+  const int n0 = blockIdx.x * COLS;
+  const __nv_bfloat16* base = w + (size_t)e * (GATED ? 2 : 1) * N * K;
+  const __nv_bfloat16* w0 = base + (size_t)min(n0 + g, N - 1) * K;
+  const __nv_bfloat16* w1 = base + (size_t)(GATED ? N + min(n0 + g, N - 1) : min(n0 + 8 + g, N - 1)) * K;
+  auto row_of = [&](int r) { return r < rows ? x + (size_t)(pair_of_row[row0 + r] / per) * ldx : nullptr; };
+  float (*mine)[16] = part[warp];
+  if (rows <= 8) {
+    float acc[1][4] = {};
+    const __nv_bfloat16* const xr[1] = {row_of(g)};
+    few_rows_products<1, NW, 8>(acc, w0, w1, xr, K, warp, j);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) mine[j * 2 + (i & 1)][g + 8 * (i >> 1)] = acc[0][i];
+  } else {
+    float acc[2][4] = {};
+    const __nv_bfloat16* const xr[2] = {row_of(g), row_of(8 + g)};
+    few_rows_products<2, NW, 4>(acc, w0, w1, xr, K, warp, j);
+#pragma unroll
+    for (int t = 0; t < 2; ++t)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) mine[t * 8 + j * 2 + (i & 1)][g + 8 * (i >> 1)] = acc[t][i];
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < rows * COLS; i += 32 * NW) {
+    const int m = i / COLS, c = i % COLS;
+    if (n0 + c >= N) continue;
+    float a = 0.f, b = 0.f;
+#pragma unroll
+    for (int q = 0; q < NW; ++q) {
+      a += part[q][m][c];
+      if (GATED) b += part[q][m][8 + c];
+    }
+    if (GATED) a = silu(a) * b;
+    else if (relu2) a = fmaxf(a, 0.f) * fmaxf(a, 0.f);
+    y[(size_t)pair_of_row[row0 + m] * ldy + n0 + c] = __float2bfloat16(a);
   }
 }
 
@@ -423,6 +560,29 @@ moe_dispatch_kernel(const __nv_bfloat16* __restrict__ x, long ldx, const int* __
   }
 }
 
+// acc += sum_j w[j] * y[row(j), c .. c + 7], four rows on their way at a time; pairs with row < 0 contribute nothing.
+__device__ __forceinline__ void add_pairs(float (&acc)[8], const __nv_bfloat16* __restrict__ y, const int* __restrict__ rows,
+                                          const float* __restrict__ w, int k, int D, int c, const MoeBounds& bd) {
+#pragma unroll 1
+  for (int j0 = 0; j0 < k; j0 += 4) {
+    uint4 u[4];
+    float wj[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = j0 + i < k ? rows[j0 + i] : -1;
+      const bool in = r >= 0 && OMNI_IN_BOUNDS(bd.max_rows == 0 || r < bd.max_rows, bd.status, KID_MOE_COMBINE);
+      wj[i] = in ? w[j0 + i] : 0.f;
+      u[i] = in ? *reinterpret_cast<const uint4*>(y + (size_t)r * D + c) : make_uint4(0u, 0u, 0u, 0u);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 a = unpack_bf16(u[i].x), b = unpack_bf16(u[i].y), cc = unpack_bf16(u[i].z), d = unpack_bf16(u[i].w);
+      acc[0] += wj[i] * a.x; acc[1] += wj[i] * a.y; acc[2] += wj[i] * b.x; acc[3] += wj[i] * b.y;
+      acc[4] += wj[i] * cc.x; acc[5] += wj[i] * cc.y; acc[6] += wj[i] * d.x; acc[7] += wj[i] * d.y;
+    }
+  }
+}
+
 // out[t, :] = (residual[t, :]) + sum_j w[t,j] * y[row(t,j), :]; pairs with row < 0 (experts of
 // another rank) contribute nothing.
 __global__ void __launch_bounds__(256)
@@ -440,16 +600,7 @@ moe_combine_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict__ 
       const float2 a = unpack_bf16(u.x), b = unpack_bf16(u.y), cc = unpack_bf16(u.z), d = unpack_bf16(u.w);
       acc[0] = a.x; acc[1] = a.y; acc[2] = b.x; acc[3] = b.y; acc[4] = cc.x; acc[5] = cc.y; acc[6] = d.x; acc[7] = d.y;
     }
-    for (int j = 0; j < k; ++j) {
-      const int r = row_of_pair[(size_t)t * k + j];
-      if (r < 0) continue;
-      if (!OMNI_IN_BOUNDS(bd.max_rows == 0 || r < bd.max_rows, bd.status, KID_MOE_COMBINE)) continue;
-      const float w = weights[(size_t)t * k + j];
-      const uint4 u = *reinterpret_cast<const uint4*>(y + (size_t)r * D + c);
-      const float2 a = unpack_bf16(u.x), b = unpack_bf16(u.y), cc = unpack_bf16(u.z), d = unpack_bf16(u.w);
-      acc[0] += w * a.x; acc[1] += w * a.y; acc[2] += w * b.x; acc[3] += w * b.y;
-      acc[4] += w * cc.x; acc[5] += w * cc.y; acc[6] += w * d.x; acc[7] += w * d.y;
-    }
+    add_pairs(acc, y, row_of_pair + (size_t)t * k, weights + (size_t)t * k, k, D, c, bd);
     uint4 o;
     o.x = pack_bf16(acc[0], acc[1]); o.y = pack_bf16(acc[2], acc[3]);
     o.z = pack_bf16(acc[4], acc[5]); o.w = pack_bf16(acc[6], acc[7]);
@@ -474,16 +625,7 @@ moe_combine_scatter_kernel(const __nv_bfloat16* __restrict__ y, const int* __res
     const int t = (int)(i / chunks);
     const int c = (int)(i % chunks) * 8;
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int j = 0; j < k; ++j) {
-      const int r = row_of_pair[(size_t)t * k + j];
-      if (r < 0) continue;
-      if (!OMNI_IN_BOUNDS(bd.max_rows == 0 || r < bd.max_rows, bd.status, KID_MOE_COMBINE)) continue;
-      const float w = weights[(size_t)t * k + j];
-      const uint4 u = *reinterpret_cast<const uint4*>(y + (size_t)r * D + c);
-      const float2 a = unpack_bf16(u.x), b = unpack_bf16(u.y), cc = unpack_bf16(u.z), d = unpack_bf16(u.w);
-      acc[0] += w * a.x; acc[1] += w * a.y; acc[2] += w * b.x; acc[3] += w * b.y;
-      acc[4] += w * cc.x; acc[5] += w * cc.y; acc[6] += w * d.x; acc[7] += w * d.y;
-    }
+    add_pairs(acc, y, row_of_pair + (size_t)t * k, weights + (size_t)t * k, k, D, c, bd);
     uint4 o;
     o.x = pack_bf16(acc[0], acc[1]); o.y = pack_bf16(acc[2], acc[3]);
     o.z = pack_bf16(acc[4], acc[5]); o.w = pack_bf16(acc[6], acc[7]);
@@ -594,6 +736,41 @@ extern "C" int omni_moe_plan_compact(const int* ids, int n_pairs, int E, int e_l
   if (E > 1024) return RC_BAD_ARG;
   moe_plan_compact_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>(ids, n_pairs, E, e_lo, e_hi, max_tiles, row_of_pair, tile_expert,
                                                                 tile_row0, tile_rows, n_rows_out, g_moe_bounds);
+  return (int)cudaGetLastError();
+}
+
+// Plan of at most FEW_PAIRS pairs.  `logits` bf16 [T, E] (E <= 256, k <= 16): the choice is made here, ids and weights are outputs; null:
+// ids [T * k] are given, E <= 1024.
+extern "C" int omni_moe_few_plan(const void* logits, int ld, int T, int E, int k, int renorm, int e_lo, int e_hi, int* ids, float* weights,
+                                 int* pair_of_row, int* row_of_pair, int* tile_expert, int* tile_row0, int* tile_rows, int max_tiles,
+                                 void* stream) {
+  if (T <= 0) return RC_OK;
+  if (E > (logits ? 256 : 1024) || (logits && (k > 16 || k > E)) || T * k > FEW_PAIRS) return RC_BAD_ARG;
+  const FewPlan p = {ids, weights, pair_of_row, row_of_pair, tile_expert, tile_row0, tile_rows, max_tiles};
+  moe_few_plan_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>((const bf16*)logits, ld, T, E, k, renorm, e_lo, e_hi, p, g_moe_bounds);
+  return (int)cudaGetLastError();
+}
+
+// Pair p reads row p / per of x [.., K] and writes row p of y; w [experts, N or 2 N (gated), K].  act: 0 none, 3 relu2, 5 SwiGLU.
+extern "C" int omni_moe_few_rows(const void* x, long ldx, int per, const void* w, int N, int K, const int* tile_expert,
+                                 const int* tile_row0, const int* tile_rows, int max_tiles, const int* pair_of_row, void* y, long ldy,
+                                 int act, void* stream) {
+  if (max_tiles <= 0 || N <= 0) return RC_OK;
+  if (per < 1 || K <= 0 || (K & 7) || (ldx & 7) || max_tiles > 65535 || (act != 0 && act != 3 && act != 5)) return RC_BAD_ARG;
+  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) return RC_BAD_ARG;
+  const bool gated = act == 5;
+  const dim3 grid((unsigned)((N + (gated ? 7 : 15)) / (gated ? 8 : 16)), (unsigned)max_tiles);
+  cudaStream_t st = (cudaStream_t)stream;
+#define OMNI_FEW(NW, G)                                                                                                             \
+  moe_few_rows_kernel<NW, G><<<grid, 32 * NW, 0, st>>>((const bf16*)x, ldx, per, (const bf16*)w, N, K, tile_expert, tile_row0, tile_rows, \
+                                                      pair_of_row, (bf16*)y, ldy, act == 3)
+  // 8 warps have up to 2048 channels in flight at once; short contractions keep more blocks per SM instead
+  if (K > 1024) {
+    if (gated) OMNI_FEW(8, true); else OMNI_FEW(8, false);
+  } else {
+    if (gated) OMNI_FEW(4, true); else OMNI_FEW(4, false);
+  }
+#undef OMNI_FEW
   return (int)cudaGetLastError();
 }
 

@@ -350,6 +350,48 @@ __device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&v
       : "memory");
 }
 
+// ------------------------------------------------- few rows against streamed weights (mma.sync)
+__device__ __forceinline__ uint4 ldg_stream(const __nv_bfloat16* p) {   // read once: past L1
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.L2::256B.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ void mma_bf16_16x8(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// acc[t] += W x^T over this warp's share of the K channels, for 16 rows of W and NT * 8 rows of x.  Lane (g, j) of the warp holds row
+// pointers of W rows g and g + 8 and of x rows t * 8 + g (null: zeros); warp w of NW takes the 32-channel chunks w, w + NW, ...  Lane
+// group j of a quad owns channels 8 j .. 8 j + 7 of a chunk for both operands: one 16-byte load per row, and the contraction is
+// permuted alike on both sides.  U chunks are in flight per warp.  K is a multiple of 8.
+template <int NT, int NW, int U>
+__device__ __forceinline__ void few_rows_products(float (&acc)[NT][4], const __nv_bfloat16* w0, const __nv_bfloat16* w1,
+                                                  const __nv_bfloat16* const (&x)[NT], int K, int warp, int j) {
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll 1
+  for (int c = warp * 32; c < K; c += 32 * NW * U) {
+    uint4 a[U][2], b[U][NT];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int ch = c + u * 32 * NW + j * 8;
+      const bool in = ch < K;
+      a[u][0] = in ? ldg_stream(w0 + ch) : zero;
+      a[u][1] = in ? ldg_stream(w1 + ch) : zero;
+#pragma unroll
+      for (int t = 0; t < NT; ++t) b[u][t] = in && x[t] ? *reinterpret_cast<const uint4*>(x[t] + ch) : zero;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        mma_bf16_16x8(acc[t], a[u][0].x, a[u][1].x, a[u][0].y, a[u][1].y, b[u][t].x, b[u][t].y);
+        mma_bf16_16x8(acc[t], a[u][0].z, a[u][1].z, a[u][0].w, a[u][1].w, b[u][t].z, b[u][t].w);
+      }
+  }
+}
+
 // ----------------------------------------------------------- UMMA descriptors
 // Shared-memory matrix descriptor, 128-byte swizzle.
 //   bits [0,14)  start address >> 4       bits [16,30) leading byte offset >> 4

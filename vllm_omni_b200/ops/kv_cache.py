@@ -104,7 +104,8 @@ def _attn_paged(q, q_rs, q_hs, q_bs, k_cache, v_cache, block_tables, kv_lens, ou
 def paged_decode(q, k_cache, v_cache, block_tables, seq_lens, scale=None, num_splits=None, out=None, impl=None):
     """q: [num_seqs, H, D] (one new token per sequence) -> [num_seqs, H, D].
 
-    ``impl``: "tc" (tcgen05 kernel; default whenever the page shape allows) or "simt"."""
+    ``impl``: "stream" (csrc/decode_attn.cu; default for head size 128, pages of a multiple of 8 tokens and up to 16 query heads
+    per KV head), "tc" (tcgen05 kernel; default for larger groups where the page shape allows, or with ``num_splits``) or "simt"."""
     n, H, D = q.shape
     nb, bs, Hkv, _ = k_cache.shape
     scale = scale if scale is not None else 1.0 / math.sqrt(D)
@@ -120,7 +121,19 @@ def paged_decode(q, k_cache, v_cache, block_tables, seq_lens, scale=None, num_sp
     assert q.stride(-1) == 1 and q.stride(1) == D and block_tables.dtype == torch.int32 and seq_lens.dtype == torch.int32
     G = H // Hkv
     if impl is None:
-        impl = "tc" if tma_pages_ok(bs, D) and G <= 128 else "simt"
+        impl = "stream" if D == 128 and bs % 8 == 0 and G <= 16 and num_splits is None and q.stride(0) % 8 == 0 and out.stride(0) % 8 == 0 \
+            else "tc" if tma_pages_ok(bs, D) and G <= 128 else "simt"
+    if impl == "stream":
+        assert out.stride(-1) == 1 and out.stride(1) == D and q.dtype == torch.bfloat16
+        lib, max_kv = nv.lib("decode_attn"), block_tables.shape[1] * bs
+        shares = lib.omni_paged_decode_shares(c_int(n), c_int(Hkv), c_int(max_kv))
+        part = torch.empty(n * H * shares * (D + 2), dtype=torch.float32, device=q.device) if shares > 1 else None
+        rc = lib.omni_paged_decode_attn(
+            nv.ptr(q), c_long(q.stride(0)), nv.ptr(k_cache), nv.ptr(v_cache), nv.ptr(block_tables), c_int(block_tables.stride(0)), c_int(bs),
+            nv.ptr(seq_lens), c_int(n), c_int(H), c_int(Hkv), c_int(max_kv), c_float(scale), nv.ptr(part),
+            nv.ptr(None if part is None else part[n * H * shares * D:]), nv.ptr(out), c_long(out.stride(0)), nv.stream_ptr())
+        nv.check_rc(rc, "omni_paged_decode_attn")
+        return out
     if impl == "tc":
         # the G heads of a group are the rows of the query tile: row pitch = one head (D),
         # "head" pitch = one group (G * D), batch pitch = one token

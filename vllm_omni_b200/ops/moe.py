@@ -65,6 +65,8 @@ class _MoEBuffers:
         i32 = lambda *s: torch.zeros(*s, dtype=torch.int32, device=device)
         t = dict(ids=i32(cap, k), row_of_pair=i32(n_pairs), tile_expert=i32(tiles), tile_row0=i32(tiles), tile_rows=i32(tiles),
                  offsets=i32(E + 1), n_rows=i32(1), weights=torch.empty(cap, k, dtype=torch.float32, device=device),
+                 few_expert=i32(_few_tiles(cap, k, E)), few_row0=i32(_few_tiles(cap, k, E)), few_rows=i32(_few_tiles(cap, k, E)),
+                 pair_of_row=i32(n_pairs),
                  xp=torch.zeros(rows, D, dtype=dtype, device=device), h13=torch.empty(rows, 2 * Fd, dtype=dtype, device=device),
                  h=torch.empty(rows, Fd, dtype=dtype, device=device), y=torch.empty(rows, D, dtype=dtype, device=device))
         self.__dict__.update(t)
@@ -78,6 +80,22 @@ def _rows_tiles(T, k, E, pad):
     # rows back to back: every (token, choice) pair is one row; an expert starts a new M tile, so at most one
     # partly filled tile per expert that got rows
     return n_pairs, min(E, n_pairs) + (n_pairs + 127) // 128
+
+
+FEW_TILE, FEW_PAIRS = 16, 2048          # csrc/moe.cu
+
+
+def _few_tiles(T, k, E):
+    n_pairs = T * k
+    return min(E, n_pairs) + n_pairs // FEW_TILE
+
+
+def _few(T, k, E, pad) -> bool:
+    """Whether to stream the chosen experts' weights past gathered rows (csrc/moe.cu, "few tokens"): up to 2 rows per expert on
+    average.  128 experts of 2048 -> 768, top 8, whole layer on cold caches: 1 token 38 us (grouped GEMMs 64), 8 tokens 106 (145), 32
+    tokens 200 (214), 64 tokens 237 (239): from there on every row costs as much again as its share of the weights, and the
+    grouped GEMMs run at memory speed."""
+    return not pad and T * k <= min(FEW_PAIRS, 2 * E)
 
 
 _pool: dict = {}
@@ -106,6 +124,10 @@ class MoEWorkspace:
         self.tile_expert, self.tile_row0, self.tile_rows = (buf.tile_expert[:self.max_tiles], buf.tile_row0[:self.max_tiles],
                                                             buf.tile_rows[:self.max_tiles])
         self.offsets, self.n_rows = buf.offsets, buf.n_rows
+        self.few = _few(T, k, E, pad)
+        n = _few_tiles(T, k, E)
+        self.few_tiles = (buf.few_expert[:n], buf.few_row0[:n], buf.few_rows[:n])
+        self.pair_of_row = buf.pair_of_row[:n_pairs]
         self.xp, self.h13, self.h, self.y = (buf.xp[:self.max_rows], buf.h13[:self.max_rows], buf.h[:self.max_rows],
                                              buf.y[:self.max_rows])
         return self
@@ -153,6 +175,35 @@ def _plan_and_dispatch(ws, x, E, e_lo, e_hi, k):
                     "omni_moe_plan_compact")
     nv.check_rc(lib.omni_moe_dispatch(nv.ptr(x), c_long(x.stride(0)), nv.ptr(ws.row_of_pair), c_int(T * k), c_int(k),
                                       c_int(D), nv.ptr(ws.xp), st), "omni_moe_dispatch")
+
+
+def _route(logits, T, E, k, renorm, ws):
+    nv.check_rc(nv.lib("moe").omni_moe_route(nv.ptr(logits), c_int(logits.stride(0)), c_int(T), c_int(E), c_int(k), c_int(1 if renorm else 0),
+                                             nv.ptr(ws.ids), nv.ptr(ws.weights), nv.stream_ptr()), "omni_moe_route")
+
+
+def _few_plan(ws, T, E, e_lo, e_hi, k, logits=None, renorm=True):
+    """Tiles of few tokens; with ``logits`` the choice (``ws.ids``, ``ws.weights``) is made as well, in the same launch (one block) for
+    up to 16 tokens: 4 us for one token, 12 us for 64 against 3 + 4 us in two launches."""
+    lib, (te, tr, tn) = nv.lib("moe"), ws.few_tiles
+    if logits is not None and T > 16:
+        _route(logits, T, E, k, renorm, ws)
+        logits = None
+    if nv.bounds_check_enabled():
+        lib.omni_moe_set_bounds(c_long(ws.y.shape[0]), nv.ptr(nv.status_word(ws.y.device)))
+    nv.check_rc(lib.omni_moe_few_plan(nv.ptr(logits), c_int(logits.stride(0) if logits is not None else 0), c_int(T), c_int(E), c_int(k),
+                                      c_int(1 if renorm else 0), c_int(e_lo), c_int(e_hi), nv.ptr(ws.ids), nv.ptr(ws.weights),
+                                      nv.ptr(ws.pair_of_row), nv.ptr(ws.row_of_pair), nv.ptr(te), nv.ptr(tr), nv.ptr(tn),
+                                      c_int(te.shape[0]), nv.stream_ptr()), "omni_moe_few_plan")
+
+
+def _few_rows(ws, x, per, w, out, act):
+    """out[pair] = act(w[expert of the pair] x[pair // per]); act "swiglu": w holds gate and lift rows."""
+    te, tr, tn = ws.few_tiles
+    nv.check_rc(nv.lib("moe").omni_moe_few_rows(nv.ptr(x), c_long(x.stride(0)), c_int(per), nv.ptr(w), c_int(out.shape[1]), c_int(w.shape[2]),
+                                                nv.ptr(te), nv.ptr(tr), nv.ptr(tn), c_int(te.shape[0]), nv.ptr(ws.pair_of_row), nv.ptr(out),
+                                                c_long(out.stride(0)), c_int({None: 0, "relu2": 3, "swiglu": 5}[act]), nv.stream_ptr()),
+                "omni_moe_few_rows")
 
 
 class _RouterRule(ctypes.Structure):
@@ -245,6 +296,11 @@ def expert_rows(x, router_w, router_b, router: Router, up, down, act: str, ws: M
     nv.check_rc(lib.omni_moe_router(nv.ptr(x), c_long(x.stride(0)), nv.ptr(router_w), c_long(router_w.stride(0)), nv.ptr(router_b),
                                     c_int(T), c_int(D), c_int(experts), c_int(router_w.shape[0]), c_int(k), ctypes.byref(rule),
                                     nv.ptr(ws.ids), nv.ptr(ws.weights), st), "omni_moe_router")
+    if ws.few:
+        _few_plan(ws, T, experts, 0, experts, k)
+        _few_rows(ws, x, k, up, ws.h, act)
+        _few_rows(ws, ws.h, 1, down, ws.y, None)
+        return ExpertRows(ws.y, ws.row_of_pair, ws.weights)
     _plan_and_dispatch(ws, x, experts, 0, experts, k)
     if act == "swiglu":
         _grouped(ws, ws.xp, D, up, ws.h13, 2 * Fd, 2 * Fd, D, ws.tile_expert)
@@ -288,17 +344,20 @@ def moe_forward(x, router_logits, w13, w2, k, renorm=True, e_lo=0, e_hi=None, ws
     ws = (ws or MoEWorkspace()).get(T, k, E, D, Fd, x.device, x.dtype)
     lib, st = nv.lib("moe"), nv.stream_ptr()
     assert router_logits.dtype == torch.bfloat16 and router_logits.stride(1) == 1
-    nv.check_rc(lib.omni_moe_route(nv.ptr(router_logits), c_int(router_logits.stride(0)), c_int(T), c_int(E), c_int(k),
-                                   c_int(1 if renorm else 0), nv.ptr(ws.ids), nv.ptr(ws.weights), st), "omni_moe_route")
-    _plan_and_dispatch(ws, x, E, e_lo, e_hi, k)
-    # tile_expert holds GLOBAL expert ids; the local weight tensors start at e_lo
-    te = ws.tile_expert
-    if e_lo:
-        te = torch.where(te >= 0, te - e_lo, te)
-
-    _grouped(ws, ws.xp, D, w13, ws.h13, 2 * Fd, 2 * Fd, D, te)
-    fused.silu_mul(ws.h13, out=ws.h)
-    _grouped(ws, ws.h, Fd, w2, ws.y, D, D, Fd, te)
+    if ws.few and x.stride(1) == 1:
+        _few_plan(ws, T, E, e_lo, e_hi, k, router_logits, renorm)
+        _few_rows(ws, x, k, w13, ws.h, "swiglu")
+        _few_rows(ws, ws.h, 1, w2, ws.y, None)
+    else:
+        _route(router_logits, T, E, k, renorm, ws)
+        _plan_and_dispatch(ws, x, E, e_lo, e_hi, k)
+        # tile_expert holds GLOBAL expert ids; the local weight tensors start at e_lo
+        te = ws.tile_expert
+        if e_lo:
+            te = torch.where(te >= 0, te - e_lo, te)
+        _grouped(ws, ws.xp, D, w13, ws.h13, 2 * Fd, 2 * Fd, D, te)
+        fused.silu_mul(ws.h13, out=ws.h)
+        _grouped(ws, ws.h, Fd, w2, ws.y, D, D, Fd, te)
     if scatter is not None:
         per, ptrs = scatter
         arr = (ctypes.c_void_p * len(ptrs))(*ptrs)
