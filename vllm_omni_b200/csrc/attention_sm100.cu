@@ -153,6 +153,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 PeerSignal sig, int* status) {
   constexpr int ATT_TILE_BYTES = AttCfg<HD>::TILE_BYTES;
   constexpr int KV_STAGES = AttCfg<HD>::STAGES;
+  pdl_wait();                        // key lengths and page ids are read from here on
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t q_full, k_full[4], k_empty[4], v_full[4], v_empty[4];
   __shared__ __align__(8) uint64_t s_full[2], p_full[2][4], o_done[2];   // p_full: per 32-key chunk of P
@@ -206,6 +207,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = tmem_base_s;
+  pdl_trigger();
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -691,7 +693,7 @@ static int launch_attn(const CUtensorMap& tq, const CUtensorMap& tk, const CUten
   PeerSignal sig;
   PeerWait unused;
   unpack_sync(sync, sig, unused);
-  fns[di]<<<grid, ATT_THREADS, di == 0 ? AttCfg<64>::SMEM : AttCfg<128>::SMEM, stream>>>(
+  launch_with(!sync, 1, fns[di], grid, ATT_THREADS, di == 0 ? AttCfg<64>::SMEM : AttCfg<128>::SMEM, stream,
       tq, tk, tv, out, Sq, Skv, H, Hkv, kv_lens, scale_log2, causal, q_offset, pg, sig, status);
   return (int)cudaGetLastError();
 }

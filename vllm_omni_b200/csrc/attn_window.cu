@@ -175,6 +175,7 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], const uint32_t (&a)[4],
 template <int KS, int VS, bool UP, bool PAIR>
 __global__ void __launch_bounds__(128, KS <= 8 && !PAIR ? 3 : 1)
 attn_window_decode_kernel(WinAttn p) {
+  pdl_begin();
   constexpr int HB = PAIR ? 8 : 16;                         // heads per block
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ float s_m[4][16], s_l[4][16];
@@ -430,6 +431,7 @@ attn_window_decode_kernel(WinAttn p) {
 
 __global__ void __launch_bounds__(256)
 attn_window_merge_kernel(WinAttn p) {
+  pdl_begin();
   const int seq = min(max(p.seq_list[blockIdx.x], 0), p.num_seqs - 1), h = blockIdx.y;
   const int row = p.q_start[seq];
   const int maps = p.maps == 2 ? 2 : 1;
@@ -491,7 +493,7 @@ static int launch_decode_as(const WinAttn& p, cudaStream_t st) {
   if (smem > cap) return RC_BAD_ARG;
   static unsigned long long prep = 0;
   if (int e = ensure_dynamic_smem((const void*)attn_window_decode_kernel<KS, VS, UP, PAIR>, cap, prep)) return e;
-  attn_window_decode_kernel<KS, VS, UP, PAIR><<<dim3(p.n_list, p.G * ((R + hb - 1) / hb), p.splits), 128, smem, st>>>(p);
+  launch_overlapped(attn_window_decode_kernel<KS, VS, UP, PAIR>, dim3(p.n_list, p.G * ((R + hb - 1) / hb), p.splits), 128, smem, st, p);
   return (int)cudaGetLastError();
 }
 
@@ -538,7 +540,7 @@ extern "C" int omni_attn_window_decode(const WinAttn* args, void* stream) {
     rc = mx <= 64 ? launch_decode<4, 4>(p, st) : (mx <= 128 ? launch_decode<8, 8>(p, st) : launch_decode<16, 16>(p, st));
   if (rc) return rc;
   if (p.splits > 1) {
-    attn_window_merge_kernel<<<dim3(p.n_list, p.H), p.vp <= 64 ? 64 : (p.vp <= 128 ? 128 : 256), 0, st>>>(p);
+    launch_overlapped(attn_window_merge_kernel, dim3(p.n_list, p.H), p.vp <= 64 ? 64 : (p.vp <= 128 ? 128 : 256), 0, st, p);
     rc = (int)cudaGetLastError();
   }
   return rc;

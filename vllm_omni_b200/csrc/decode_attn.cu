@@ -45,6 +45,7 @@ struct DecodeAttn {
 template <bool UP>
 __global__ void __launch_bounds__(32 * DA_WARPS, UP ? 2 : 3)
 paged_decode_kernel(const __grid_constant__ DecodeAttn p) {
+  pdl_begin();
   constexpr int NH = UP ? 2 : 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, j = lane & 3;
   const int seq = blockIdx.y, split = blockIdx.x;
@@ -211,6 +212,7 @@ paged_decode_kernel(const __grid_constant__ DecodeAttn p) {
 __global__ void __launch_bounds__(128)
 paged_decode_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml, int parts, int H,
                           __nv_bfloat16* __restrict__ out, long o_rs) {
+  pdl_begin();
   __shared__ float4 part[4][32];
   const long r = blockIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -306,10 +308,10 @@ extern "C" int omni_paged_decode_attn(const void* q, long q_rs, const void* k, c
   p.part_o = part_o; p.part_ml = part_ml; p.out = (__nv_bfloat16*)out; p.o_rs = o_rs;
   const dim3 grid((unsigned)p.splits, (unsigned)n, (unsigned)((Hkv + DA_WARPS - 1) / DA_WARPS));
   cudaStream_t st = (cudaStream_t)stream;
-  if (H / Hkv > 8) paged_decode_kernel<true><<<grid, 32 * DA_WARPS, 0, st>>>(p);
-  else paged_decode_kernel<false><<<grid, 32 * DA_WARPS, 0, st>>>(p);
+  if (H / Hkv > 8) launch_overlapped(paged_decode_kernel<true>, grid, 32 * DA_WARPS, 0, st, p);
+  else launch_overlapped(paged_decode_kernel<false>, grid, 32 * DA_WARPS, 0, st, p);
   if (parts == 1) return (int)cudaGetLastError();
   if (cudaError_t e = cudaGetLastError()) return (int)e;
-  paged_decode_merge_kernel<<<(unsigned)n * H, 128, 0, st>>>(part_o, part_ml, parts, H, (__nv_bfloat16*)out, o_rs);
+  launch_overlapped(paged_decode_merge_kernel, (unsigned)n * H, 128, 0, st, part_o, part_ml, parts, H, (__nv_bfloat16*)out, o_rs);
   return (int)cudaGetLastError();
 }

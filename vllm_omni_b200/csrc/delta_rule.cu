@@ -17,6 +17,7 @@ constexpr int DS_THREADS = 256;
 template <typename T, bool CHANNEL, int NR>
 __global__ void __launch_bounds__(DS_THREADS)
 delta_steps_kernel(const DeltaRule p, const int cw) {
+  pdl_begin();
   extern __shared__ __align__(16) float sm[];
   __shared__ float sh[64];
   const int tid = threadIdx.x;
@@ -274,10 +275,10 @@ static int launch_steps(const DeltaRule& p, int cw, cudaStream_t st) {
   const dim3 grid(p.seq_list ? p.n_list : p.num_seqs, p.H, (p.vp + cw - 1) / cw);
   const int smem = (4 * p.dp + cw + 8 * DS_THREADS) * 4;
   if (smem > 47 * 1024) return RC_TOO_LARGE;
-  if (rows <= 4) delta_steps_kernel<T, CHANNEL, 4><<<grid, DS_THREADS, smem, st>>>(p, cw);
-  else if (rows <= 8) delta_steps_kernel<T, CHANNEL, 8><<<grid, DS_THREADS, smem, st>>>(p, cw);
-  else if (rows <= 16) delta_steps_kernel<T, CHANNEL, 16><<<grid, DS_THREADS, smem, st>>>(p, cw);
-  else if (rows <= 24) delta_steps_kernel<T, CHANNEL, 24><<<grid, DS_THREADS, smem, st>>>(p, cw);
+  if (rows <= 4) launch_overlapped(delta_steps_kernel<T, CHANNEL, 4>, grid, DS_THREADS, smem, st, p, cw);
+  else if (rows <= 8) launch_overlapped(delta_steps_kernel<T, CHANNEL, 8>, grid, DS_THREADS, smem, st, p, cw);
+  else if (rows <= 16) launch_overlapped(delta_steps_kernel<T, CHANNEL, 16>, grid, DS_THREADS, smem, st, p, cw);
+  else if (rows <= 24) launch_overlapped(delta_steps_kernel<T, CHANNEL, 24>, grid, DS_THREADS, smem, st, p, cw);
   else return RC_TOO_LARGE;
   return (int)cudaGetLastError();
 }

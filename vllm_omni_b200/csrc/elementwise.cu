@@ -52,6 +52,7 @@ norm_modulate_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restr
                      const __nv_bfloat16* __restrict__ weight, const __nv_bfloat16* __restrict__ bias,
                      const __nv_bfloat16* __restrict__ shift, const __nv_bfloat16* __restrict__ scale, int mod_stride,
                      int rows_per_batch, int rms, float eps) {
+  pdl_begin();
   __shared__ float2 red[16];
   const int row = blockIdx.x, nchunk = D >> 3, warps = blockDim.x >> 5;
   const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)row * ldx);
@@ -124,6 +125,7 @@ norm_modulate_warp_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __
                           const __nv_bfloat16* __restrict__ bias, const __nv_bfloat16* __restrict__ shift,
                           const __nv_bfloat16* __restrict__ scale, int mod_stride, int rows_per_batch,
                           int rms, float eps) {
+  pdl_begin();
   __shared__ float2 red[8];
   const int warp = threadIdx.x >> 5, row = blockIdx.x * (8 / WPR) + warp / WPR;
   const int lane = (threadIdx.x & 31) + (warp % WPR) * 32;
@@ -291,6 +293,7 @@ __device__ __forceinline__ void store_head(const HeadRows& a, long row, int h, i
 // with one warp per row; 560 rows of 48 heads 12 us (16).
 __global__ void __launch_bounds__(256)
 qk_norm_rope128_kernel(const __grid_constant__ HeadRows a, PeerWait wt, int* status) {
+  pdl_begin();
   if (wt.counter) {
     // fused exchange: the rows come from the peers' QKV GEMM epilogues; wait for their arrivals
     // here instead of in a barrier kernel of its own
@@ -323,6 +326,7 @@ qk_norm_rope128_kernel(const __grid_constant__ HeadRows a, PeerWait wt, int* sta
 // The same for many rows: a warp walks all heads of its row, 8 at a time, and fetches the rotation coefficients once.
 __global__ void __launch_bounds__(256)
 qk_norm_rope128_rows_kernel(const __grid_constant__ HeadRows a, PeerWait wt, int* status) {
+  pdl_begin();
   if (wt.counter) {
     if (threadIdx.x == 0) {
       peer_wait_arrivals(wt, nullptr, status);
@@ -445,6 +449,7 @@ __global__ void __launch_bounds__(256)
 cfg_euler_kernel(const __nv_bfloat16* __restrict__ pos, const __nv_bfloat16* __restrict__ neg,
                  float* __restrict__ lat, __nv_bfloat16* __restrict__ lat_bf16, long rows, int C,
                  float guidance, float dt, int renorm) {
+  pdl_begin();
   const long row = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= rows) return;
@@ -483,6 +488,7 @@ cfg_euler_kernel(const __nv_bfloat16* __restrict__ pos, const __nv_bfloat16* __r
 __global__ void __launch_bounds__(256)
 silu_mul_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, long rows, int N,
                 int ldx, int ldy) {
+  pdl_begin();
   const long nchunk = (long)rows * (N >> 3);
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < nchunk; i += (long)gridDim.x * blockDim.x) {
     const long r = i / (N >> 3);
@@ -590,12 +596,12 @@ extern "C" int omni_norm_modulate(const void* x, void* y, int rows, int D, int l
   auto sh = (const __nv_bfloat16*)shift; auto sc = (const __nv_bfloat16*)scale;
   cudaStream_t st = (cudaStream_t)stream;
   const int nchunk = D >> 3;
-#define OMNI_NM_WARP(V, W) norm_modulate_warp_kernel<V, W><<<(unsigned)((rows + 8 / W - 1) / (8 / W)), 256, 0, st>>>(xx, yy, rows, D, ldx, ldy, w, bb, sh, sc, mod_stride, rows_per_batch, rms, eps)
+#define OMNI_NM_WARP(V, W) launch_overlapped(norm_modulate_warp_kernel<V, W>, (unsigned)((rows + 8 / W - 1) / (8 / W)), 256, 0, st, xx, yy, rows, D, ldx, ldy, w, bb, sh, sc, mod_stride, rows_per_batch, rms, eps)
   if (nchunk <= 64) OMNI_NM_WARP(2, 1);
   else if (nchunk <= 128) OMNI_NM_WARP(4, 1);
   else if (rows < 8 * sm_count() || nchunk > 640)
     // up to 8 rows per SM a block per row is one round of latencies
-    norm_modulate_kernel<2><<<rows, ((nchunk + 1) / 2 + 31) / 32 * 32, 0, st>>>(xx, yy, D, ldx, ldy, w, bb, sh, sc, mod_stride,
+    launch_overlapped(norm_modulate_kernel<2>, rows, ((nchunk + 1) / 2 + 31) / 32 * 32, 0, st, xx, yy, D, ldx, ldy, w, bb, sh, sc, mod_stride,
                                                                                rows_per_batch, rms, eps);
   else if (nchunk <= 256) OMNI_NM_WARP(4, 2);
   else if (nchunk <= 384) OMNI_NM_WARP(6, 2);
@@ -634,11 +640,12 @@ extern "C" int omni_qk_norm_rope_pages(void* qkv, int B, int S, int H, int Hkv, 
                         {(__nv_bfloat16*)kc, (__nv_bfloat16*)vc, slots}};
     const int all = H + Hkv + (kc ? Hkv : 0);
     const long pairs = rows * ((all + 1) / 2);
+    // (a launch that waits for peers starts when its own predecessor has ended)
     // two heads to a warp up to about 600 rows of 48 heads; from there on a warp per row, which loads the coefficients once
     if (pairs <= 2L * 64 * sm_count())
-      qk_norm_rope128_kernel<<<(unsigned)((pairs + 7) / 8), 256, 0, st>>>(r, wt, status);
+      launch_with(!wt.counter, 1, qk_norm_rope128_kernel, (unsigned)((pairs + 7) / 8), 256, 0, st, r, wt, status);
     else
-      qk_norm_rope128_rows_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(r, wt, status);
+      launch_with(!wt.counter, 1, qk_norm_rope128_rows_kernel, (unsigned)((rows + 7) / 8), 256, 0, st, r, wt, status);
   } else if (D == 128)
     qk_norm_rope_kernel<128><<<grid, wpb * 32, 0, st>>>(q, B, S, H, Hkv, ld, a, b, c, d, s_alt, cosb, sinb, interleaved, eps, positions);
   else if (D == 64)
@@ -669,8 +676,7 @@ extern "C" int omni_cfg_euler_step(const void* pos, const void* neg, float* lat,
   if (rows <= 0) return RC_OK;
   const int wpb = 8;
   const unsigned grid = (unsigned)((rows + wpb - 1) / wpb);
-  cfg_euler_kernel<<<grid, wpb * 32, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)pos, (const __nv_bfloat16*)neg, lat, (__nv_bfloat16*)lat_bf16, rows, C, guidance, dt, renorm);
+  launch_overlapped(cfg_euler_kernel, grid, wpb * 32, 0, (cudaStream_t)stream, (const __nv_bfloat16*)pos, (const __nv_bfloat16*)neg, lat, (__nv_bfloat16*)lat_bf16, rows, C, guidance, dt, renorm);
   return (int)cudaGetLastError();
 }
 
@@ -680,7 +686,7 @@ extern "C" int omni_silu_mul(const void* x, void* y, long rows, int N, int ldx, 
   const long nchunk = rows * (N >> 3);
   long blocks = (nchunk + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
-  silu_mul_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)x, (__nv_bfloat16*)y, rows, N, ldx, ldy);
+  launch_overlapped(silu_mul_kernel, (unsigned)blocks, 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)x, (__nv_bfloat16*)y, rows, N, ldx, ldy);
   return (int)cudaGetLastError();
 }
 

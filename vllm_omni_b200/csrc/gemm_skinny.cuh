@@ -87,6 +87,11 @@ gemm_rows_kernel(const __nv_bfloat16* __restrict__ A, int lda, const __nv_bfloat
   __shared__ float part[NW][NT * 8][16];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, j = lane & 3;
   const int n0 = blockIdx.x * 16;
+  if (blockIdx.x < 2 * 148) {              // W does not come from the kernel before: the first blocks' share is on its way to L2 meanwhile
+    const __nv_bfloat16* w = W + (size_t)min(n0 + (int)(threadIdx.x & 15), N - 1) * ldw;
+    for (int c = (threadIdx.x >> 4) * 64; c < K; c += 2 * NW * 64) prefetch_l2(w + c);
+  }
+  pdl_begin();
   const __nv_bfloat16* x[NT];
   float acc[NT][4];
 #pragma unroll
@@ -122,11 +127,11 @@ static int launch_rows(const void* A, int lda, const void* W, int ldw, __nv_bflo
   // one block per SM: 16 warps, so that a long contraction still is one or two rounds of loads; else two blocks of 8
   const bool wide = tiles <= sm_count() && K > 1024;
   if (M <= 8) {
-    if (wide) gemm_rows_kernel<1, 16><<<tiles, 512, 0, stream>>>(a, lda, w, ldw, C, ldc, M, N, K, epi);
-    else gemm_rows_kernel<1, 8><<<tiles, 256, 0, stream>>>(a, lda, w, ldw, C, ldc, M, N, K, epi);
+    if (wide) launch_overlapped(gemm_rows_kernel<1, 16>, tiles, 512, 0, stream, a, lda, w, ldw, C, ldc, M, N, K, epi);
+    else launch_overlapped(gemm_rows_kernel<1, 8>, tiles, 256, 0, stream, a, lda, w, ldw, C, ldc, M, N, K, epi);
   } else {
-    if (wide) gemm_rows_kernel<2, 16><<<tiles, 512, 0, stream>>>(a, lda, w, ldw, C, ldc, M, N, K, epi);
-    else gemm_rows_kernel<2, 8><<<tiles, 256, 0, stream>>>(a, lda, w, ldw, C, ldc, M, N, K, epi);
+    if (wide) launch_overlapped(gemm_rows_kernel<2, 16>, tiles, 512, 0, stream, a, lda, w, ldw, C, ldc, M, N, K, epi);
+    else launch_overlapped(gemm_rows_kernel<2, 8>, tiles, 256, 0, stream, a, lda, w, ldw, C, ldc, M, N, K, epi);
   }
   return (int)cudaGetLastError();
 }
@@ -171,6 +176,9 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = tmem_base_s;
+  if (threadIdx.x == 0)
+    for (int kb = kb0; kb < kb1 && kb < kb0 + 16; ++kb) tma_prefetch_2d(&tmW, kb * 64, n0);
+  pdl_begin();
 
   if (warp == 0) {
     if (elect_one()) {
@@ -274,17 +282,9 @@ static int launch_skinny_s(const CUtensorMap& tmX, const CUtensorMap& tmW, __nv_
                            const GemmEpilogue& epi, int* status, cudaStream_t stream) {
   static unsigned long long prepared = 0;
   if (int e = ensure_dynamic_smem((const void*)gemm_skinny_kernel<MT, S, ALONE>, SkinnyCfg<MT, ALONE>::SMEM_BYTES, prepared)) return e;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)((N + 127) / 128 * S));
-  cfg.blockDim = dim3(SKINNY_THREADS);
-  cfg.dynamicSmemBytes = SkinnyCfg<MT, ALONE>::SMEM_BYTES;
-  cfg.stream = stream;
-  cudaLaunchAttribute at;
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = S; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = S > 1 ? 1 : 0;
-  return (int)cudaLaunchKernelEx(&cfg, gemm_skinny_kernel<MT, S, ALONE>, tmX, tmW, C, ldc, M, N, K, epi, status);
+  launch_with(true, S, gemm_skinny_kernel<MT, S, ALONE>, (unsigned)((N + 127) / 128 * S), SKINNY_THREADS, SkinnyCfg<MT, ALONE>::SMEM_BYTES, stream,
+              tmX, tmW, C, ldc, M, N, K, epi, status);
+  return (int)cudaGetLastError();
 }
 
 // CTAs per tile: up to about 200 in all (two share an SM), each with at least two K blocks

@@ -307,6 +307,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = tmem_base_s;
+  pdl_begin();
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -568,6 +569,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ PairArgs args, int* status) {
   cluster_sync_all();   // both CTAs' barriers are initialised before either touches the other's
   tc_fence_after_sync();
   const uint32_t tmem_base = tmem_base_s;
+  pdl_begin();
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
@@ -753,6 +755,7 @@ gemm_bf16_multi_kernel(const __grid_constant__ PairArgs args, int* status) {
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = tmem_base_s;
+  pdl_begin();
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -896,7 +899,7 @@ static int launch_gemm_pair(const PairArgs& args, int* status, int max_pairs, cu
   int num_tiles = 0;
   for (int i = 0; i < args.n_problems; ++i) num_tiles += ((args.p[i].M + 2 * BM - 1) / (2 * BM)) * num_n;
   const int pairs = num_tiles < max_pairs ? num_tiles : max_pairs;
-  gemm_bf16_pair_kernel<TN><<<2 * pairs, GEMM_THREADS, Cfg::SMEM_BYTES, stream>>>(args, status);
+  launch_with(!args.wt.counter && !args.sig.n, 1, gemm_bf16_pair_kernel<TN>, 2 * pairs, GEMM_THREADS, Cfg::SMEM_BYTES, stream, args, status);
   return (int)cudaGetLastError();
 }
 
@@ -969,7 +972,8 @@ static int launch_gemm(const CUtensorMap& tmA, const void* W, __nv_bfloat16* C, 
   PeerSignal sig;
   PeerWait wt;
   unpack_sync(sync, sig, wt);
-  gemm_bf16_kernel<BN><<<grid, GEMM_THREADS, Cfg::SMEM_BYTES, stream>>>(tmA, tmB, C, ldc, M, N, K, epi, tile_expert, gt, geom, sig, wt, status);
+  launch_with(!sync, 1, gemm_bf16_kernel<BN>, grid, GEMM_THREADS, Cfg::SMEM_BYTES, stream, tmA, tmB, C, ldc, M, N, K, epi, tile_expert, gt, geom, sig,
+              wt, status);
   return (int)cudaGetLastError();
 }
 
@@ -983,7 +987,7 @@ static int launch_gemm_multi(const PairArgs& args, int* status, int max_ctas, cu
   int num_tiles = 0;
   for (int i = 0; i < args.n_problems; ++i) num_tiles += ((args.p[i].M + BM - 1) / BM) * num_n;
   const int grid = num_tiles < max_ctas ? num_tiles : max_ctas;
-  gemm_bf16_multi_kernel<BN><<<grid, GEMM_THREADS, Cfg::SMEM_BYTES, stream>>>(args, status);
+  launch_with(!args.wt.counter && !args.sig.n, 1, gemm_bf16_multi_kernel<BN>, grid, GEMM_THREADS, Cfg::SMEM_BYTES, stream, args, status);
   return (int)cudaGetLastError();
 }
 

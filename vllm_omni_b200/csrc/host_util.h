@@ -90,6 +90,36 @@ inline int ensure_dynamic_smem(const void* fn, int bytes, unsigned long long& ma
   return 0;
 }
 
+// Launch of a kernel that begins with pdl_trigger / pdl_wait (ptx_sm100.cuh): its blocks may become resident and set themselves up
+// while the kernel before it in the stream runs out.  `cluster` > 1: blocks per cluster along x, for kernels without __cluster_dims__.
+// overlap = false: an ordinary launch.
+template <typename... Params, typename... Args>
+inline int launch_with(bool overlap, int cluster, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                       Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[2];
+  int n = 0;
+  if (overlap) {
+    at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster > 1) {
+    at[n].id = cudaLaunchAttributeClusterDimension;
+    at[n].val.clusterDim.x = cluster; at[n].val.clusterDim.y = 1; at[n++].val.clusterDim.z = 1;
+  }
+  cfg.attrs = at;
+  cfg.numAttrs = n;
+  return (int)cudaLaunchKernelEx(&cfg, kernel, Params(args)...);      // also left for cudaGetLastError
+}
+template <typename... Params, typename... Args>
+inline int launch_overlapped(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+  return launch_with(true, 1, kernel, grid, block, smem, stream, args...);
+}
+
 inline int sm_count() {
   static int n = 0;
   if (n == 0) {

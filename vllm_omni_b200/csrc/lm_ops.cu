@@ -563,6 +563,7 @@ struct RotaryHeads {
 template <typename T, int NV>
 __global__ void __launch_bounds__(256)
 rotary_heads_kernel(const RotaryHeads p) {
+  pdl_begin();
   extern __shared__ float s_v[];                            // sums of squares of the value vectors
   __shared__ float sh[64];
   const long row = blockIdx.x;
@@ -651,6 +652,7 @@ rotary_heads_kernel(const RotaryHeads p) {
 template <typename T>
 __global__ void __launch_bounds__(256)
 tanh_cols_kernel(const T* __restrict__ in, long ldi, T* __restrict__ out, long rows, int n) {
+  pdl_begin();
   const int vec = n / 8;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < rows * vec; i += (long)gridDim.x * blockDim.x) {
     const long r = i / vec;
@@ -667,6 +669,7 @@ tanh_cols_kernel(const T* __restrict__ in, long ldi, T* __restrict__ out, long r
 template <typename T>
 __global__ void __launch_bounds__(256)
 logit_softcap_kernel(const T* __restrict__ in, long ldi, float* __restrict__ out, long ldo, long rows, int V, float cap, float mult) {
+  pdl_begin();
   const long total = rows * V;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
     const long r = i / V;
@@ -797,10 +800,10 @@ extern "C" int omni_rotary_heads(const RotaryHeads* args, int is_bf16, void* str
   cudaStream_t st = (cudaStream_t)stream;
 #define OMNI_ROTARY(ELT)                                                              \
   do {                                                                                \
-    if (nv == 1) rotary_heads_kernel<ELT, 1><<<p.T, threads, smem, st>>>(p);          \
-    else if (nv == 2) rotary_heads_kernel<ELT, 2><<<p.T, threads, smem, st>>>(p);     \
-    else if (nv == 4) rotary_heads_kernel<ELT, 4><<<p.T, threads, smem, st>>>(p);     \
-    else rotary_heads_kernel<ELT, 16><<<p.T, threads, smem, st>>>(p);                 \
+    if (nv == 1) launch_overlapped(rotary_heads_kernel<ELT, 1>, p.T, threads, smem, st, p);          \
+    else if (nv == 2) launch_overlapped(rotary_heads_kernel<ELT, 2>, p.T, threads, smem, st, p);     \
+    else if (nv == 4) launch_overlapped(rotary_heads_kernel<ELT, 4>, p.T, threads, smem, st, p);     \
+    else launch_overlapped(rotary_heads_kernel<ELT, 16>, p.T, threads, smem, st, p);                 \
   } while (0)
   if (is_bf16) OMNI_ROTARY(bf16); else OMNI_ROTARY(float);
 #undef OMNI_ROTARY
@@ -813,8 +816,8 @@ extern "C" int omni_tanh_cols(const void* in, long ldi, void* out, long rows, in
   long blocks = (rows * (n / 8) + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
   cudaStream_t st = (cudaStream_t)stream;
-  if (is_bf16) tanh_cols_kernel<bf16><<<(unsigned)blocks, 256, 0, st>>>((const bf16*)in, ldi, (bf16*)out, rows, n);
-  else tanh_cols_kernel<float><<<(unsigned)blocks, 256, 0, st>>>((const float*)in, ldi, (float*)out, rows, n);
+  if (is_bf16) launch_overlapped(tanh_cols_kernel<bf16>, (unsigned)blocks, 256, 0, st, (const bf16*)in, ldi, (bf16*)out, rows, n);
+  else launch_overlapped(tanh_cols_kernel<float>, (unsigned)blocks, 256, 0, st, (const float*)in, ldi, (float*)out, rows, n);
   return (int)cudaGetLastError();
 }
 
@@ -824,7 +827,7 @@ extern "C" int omni_logit_softcap(const void* in, long ldi, float* out, long ldo
   long blocks = (rows * V + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
   cudaStream_t st = (cudaStream_t)stream;
-  if (is_bf16) logit_softcap_kernel<bf16><<<(unsigned)blocks, 256, 0, st>>>((const bf16*)in, ldi, out, ldo, rows, V, cap, mult);
-  else logit_softcap_kernel<float><<<(unsigned)blocks, 256, 0, st>>>((const float*)in, ldi, out, ldo, rows, V, cap, mult);
+  if (is_bf16) launch_overlapped(logit_softcap_kernel<bf16>, (unsigned)blocks, 256, 0, st, (const bf16*)in, ldi, out, ldo, rows, V, cap, mult);
+  else launch_overlapped(logit_softcap_kernel<float>, (unsigned)blocks, 256, 0, st, (const float*)in, ldi, out, ldo, rows, V, cap, mult);
   return (int)cudaGetLastError();
 }

@@ -79,6 +79,7 @@ __device__ __forceinline__ void route_token(const __nv_bfloat16* __restrict__ lo
 __global__ void __launch_bounds__(256)
 moe_route_kernel(const __nv_bfloat16* __restrict__ logits, int ld, int T, int E, int k, int renorm,
                  int* __restrict__ ids, float* __restrict__ weights) {
+  pdl_begin();
   const int t = blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (t >= T) return;
@@ -210,6 +211,7 @@ __global__ void __launch_bounds__(32 * NW)
 moe_router_kernel(const __nv_bfloat16* __restrict__ x, long ldx, const __nv_bfloat16* __restrict__ w, long ldw,
                   const float* __restrict__ bias, int T, int D, int E, int Ep, int k, RouterRule rule,
                   int* __restrict__ ids, float* __restrict__ weights) {
+  pdl_begin();
   extern __shared__ float sm[];
   float* part = sm;                            // [NW][MT * 16][64]
   float* logit = sm + NW * MT * 16 * 64;        // [MT * 16][256]
@@ -392,6 +394,7 @@ __global__ void __launch_bounds__(1024)
 moe_plan_compact_kernel(const int* __restrict__ ids, int n_pairs, int E, int e_lo, int e_hi, int max_tiles,
                         int* __restrict__ row_of_pair, int* __restrict__ tile_expert, int* __restrict__ tile_row0,
                         int* __restrict__ tile_rows, int* __restrict__ n_rows_out, MoeBounds bd) {
+  pdl_begin();
   __shared__ int cnt[1024];
   __shared__ int off[1024];
   cnt[threadIdx.x] = 0;
@@ -443,6 +446,7 @@ struct FewPlan {
 __global__ void __launch_bounds__(1024)
 moe_few_plan_kernel(const __nv_bfloat16* __restrict__ logits, int ld, int T, int E, int k, int renorm, int e_lo, int e_hi,
                     const FewPlan p, MoeBounds bd) {
+  pdl_begin();
   __shared__ int sid[FEW_PAIRS];
   __shared__ int cnt[1024];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_pairs = T * k;
@@ -500,6 +504,7 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW)
 moe_few_rows_kernel(const __nv_bfloat16* __restrict__ x, long ldx, int per, const __nv_bfloat16* __restrict__ w, int N, int K,
                     const int* __restrict__ tile_expert, const int* __restrict__ tile_row0, const int* __restrict__ tile_rows,
                     const int* __restrict__ pair_of_row, __nv_bfloat16* __restrict__ y, long ldy, int relu2) {
+  pdl_begin();
   __shared__ float part[NW][FEW_TILE][16];
   constexpr int COLS = GATED ? 8 : 16;
   const int e = tile_expert[blockIdx.y];
@@ -548,6 +553,7 @@ moe_few_rows_kernel(const __nv_bfloat16* __restrict__ x, long ldx, int per, cons
 __global__ void __launch_bounds__(256)
 moe_dispatch_kernel(const __nv_bfloat16* __restrict__ x, long ldx, const int* __restrict__ row_of_pair, int n_pairs,
                     int k, int D, __nv_bfloat16* __restrict__ xp, MoeBounds bd) {
+  pdl_begin();
   const int chunks = D >> 3;
   const long total = (long)n_pairs * chunks;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
@@ -589,6 +595,7 @@ __global__ void __launch_bounds__(256)
 moe_combine_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict__ row_of_pair,
                    const float* __restrict__ weights, int T, int k, int D, const __nv_bfloat16* __restrict__ residual,
                    long ldr, __nv_bfloat16* __restrict__ out, long ldo, MoeBounds bd) {
+  pdl_begin();
   const int chunks = D >> 3;
   const long total = (long)T * chunks;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
@@ -672,7 +679,7 @@ extern "C" int omni_moe_route(const void* logits, int ld, int T, int E, int k, i
                               void* stream) {
   if (T <= 0) return RC_OK;
   if (E > 256 || k > 16 || k > E) return RC_BAD_ARG;
-  moe_route_kernel<<<(T + 7) / 8, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)logits, ld, T, E, k, renorm, ids, weights);
+  launch_overlapped(moe_route_kernel, (T + 7) / 8, 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)logits, ld, T, E, k, renorm, ids, weights);
   return (int)cudaGetLastError();
 }
 
@@ -701,11 +708,11 @@ extern "C" int omni_moe_router(const void* x, long ldx, const void* w, long ldw,
   if (T > 148 * 16) {
     const int smem = (8 * 32 * 64 + 32 * 256) * 4;
     if (int e = ensure_dynamic_smem((const void*)moe_router_kernel<2, 8>, smem, prep[0])) return e;
-    moe_router_kernel<2, 8><<<(T + 31) / 32, 256, smem, st>>>(xb, ldx, wb, ldw, bias, T, D, E, Ep, k, *rule, ids, weights);
+    launch_overlapped(moe_router_kernel<2, 8>, (T + 31) / 32, 256, smem, st, xb, ldx, wb, ldw, bias, T, D, E, Ep, k, *rule, ids, weights);
   } else {
     const int smem = (16 * 16 * 64 + 16 * 256) * 4;
     if (int e = ensure_dynamic_smem((const void*)moe_router_kernel<1, 16>, smem, prep[1])) return e;
-    moe_router_kernel<1, 16><<<(T + 15) / 16, 512, smem, st>>>(xb, ldx, wb, ldw, bias, T, D, E, Ep, k, *rule, ids, weights);
+    launch_overlapped(moe_router_kernel<1, 16>, (T + 15) / 16, 512, smem, st, xb, ldx, wb, ldw, bias, T, D, E, Ep, k, *rule, ids, weights);
   }
   return (int)cudaGetLastError();
 }
@@ -734,7 +741,7 @@ extern "C" int omni_moe_plan(const int* ids, int n_pairs, int E, int e_lo, int e
 extern "C" int omni_moe_plan_compact(const int* ids, int n_pairs, int E, int e_lo, int e_hi, int max_tiles, int* row_of_pair,
                                      int* tile_expert, int* tile_row0, int* tile_rows, int* n_rows_out, void* stream) {
   if (E > 1024) return RC_BAD_ARG;
-  moe_plan_compact_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>(ids, n_pairs, E, e_lo, e_hi, max_tiles, row_of_pair, tile_expert,
+  launch_overlapped(moe_plan_compact_kernel, 1, 1024, 0, (cudaStream_t)stream, ids, n_pairs, E, e_lo, e_hi, max_tiles, row_of_pair, tile_expert,
                                                                 tile_row0, tile_rows, n_rows_out, g_moe_bounds);
   return (int)cudaGetLastError();
 }
@@ -747,7 +754,7 @@ extern "C" int omni_moe_few_plan(const void* logits, int ld, int T, int E, int k
   if (T <= 0) return RC_OK;
   if (E > (logits ? 256 : 1024) || (logits && (k > 16 || k > E)) || T * k > FEW_PAIRS) return RC_BAD_ARG;
   const FewPlan p = {ids, weights, pair_of_row, row_of_pair, tile_expert, tile_row0, tile_rows, max_tiles};
-  moe_few_plan_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>((const bf16*)logits, ld, T, E, k, renorm, e_lo, e_hi, p, g_moe_bounds);
+  launch_overlapped(moe_few_plan_kernel, 1, 1024, 0, (cudaStream_t)stream, (const bf16*)logits, ld, T, E, k, renorm, e_lo, e_hi, p, g_moe_bounds);
   return (int)cudaGetLastError();
 }
 
@@ -762,7 +769,7 @@ extern "C" int omni_moe_few_rows(const void* x, long ldx, int per, const void* w
   const dim3 grid((unsigned)((N + (gated ? 7 : 15)) / (gated ? 8 : 16)), (unsigned)max_tiles);
   cudaStream_t st = (cudaStream_t)stream;
 #define OMNI_FEW(NW, G)                                                                                                             \
-  moe_few_rows_kernel<NW, G><<<grid, 32 * NW, 0, st>>>((const bf16*)x, ldx, per, (const bf16*)w, N, K, tile_expert, tile_row0, tile_rows, \
+  launch_overlapped(moe_few_rows_kernel<NW, G>, grid, 32 * NW, 0, st, (const bf16*)x, ldx, per, (const bf16*)w, N, K, tile_expert, tile_row0, tile_rows, \
                                                       pair_of_row, (bf16*)y, ldy, act == 3)
   // 8 warps have up to 2048 channels in flight at once; short contractions keep more blocks per SM instead
   if (K > 1024) {
@@ -780,7 +787,7 @@ extern "C" int omni_moe_dispatch(const void* x, long ldx, const int* row_of_pair
   if (D & 7) return RC_BAD_ARG;
   long blocks = ((long)n_pairs * (D >> 3) + 255) / 256;
   if (blocks > 148 * 8) blocks = 148 * 8;
-  moe_dispatch_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)x, ldx, row_of_pair, n_pairs, k, D, (__nv_bfloat16*)xp,
+  launch_overlapped(moe_dispatch_kernel, (unsigned)blocks, 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)x, ldx, row_of_pair, n_pairs, k, D, (__nv_bfloat16*)xp,
                                                                           g_moe_bounds);
   return (int)cudaGetLastError();
 }
@@ -791,8 +798,7 @@ extern "C" int omni_moe_combine(const void* y, const int* row_of_pair, const flo
   if (D & 7) return RC_BAD_ARG;
   long blocks = ((long)T * (D >> 3) + 255) / 256;
   if (blocks > 148 * 8) blocks = 148 * 8;
-  moe_combine_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)y, row_of_pair, weights, T, k, D, (const __nv_bfloat16*)residual, ldr, (__nv_bfloat16*)out, ldo,
+  launch_overlapped(moe_combine_kernel, (unsigned)blocks, 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)y, row_of_pair, weights, T, k, D, (const __nv_bfloat16*)residual, ldr, (__nv_bfloat16*)out, ldo,
       g_moe_bounds);
   return (int)cudaGetLastError();
 }

@@ -87,6 +87,21 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// ------------------------------------------- launches that overlap their predecessor's end
+// A kernel launched by launch_overlapped (host_util.h) may start once every block of the kernel before it has called pdl_trigger or has
+// ended.  pdl_wait returns when that kernel has ended and its writes are visible: only constants of the launch (parameters, tensor
+// maps) may be read, only shared and tensor memory written, and only L2 prefetches issued before it.  Every thread calls it, so
+// that a kernel never ends before its predecessor has.  pdl_trigger comes after the wait, so that no more than two kernels of a
+// stream are under way and what a kernel reads was complete when its last-but-one predecessor ended; and after an allocation of
+// tensor memory, because a successor on the same SM could otherwise hold the columns the kernel waits for.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_begin() {
+  pdl_wait();
+  pdl_trigger();
+}
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // ----------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
@@ -165,6 +180,11 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* tma
       : "r"(dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar), "r"(c0), "r"(c1), "r"(c2),
         "r"(c3)
       : "memory");
+}
+// the same box into L2 only
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* tmap, int c0, int c1) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(reinterpret_cast<uint64_t>(tmap)), "r"(c0), "r"(c1)
+               : "memory");
 }
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* tmap) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(tmap)) : "memory");

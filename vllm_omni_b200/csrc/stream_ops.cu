@@ -46,6 +46,7 @@ template <> __device__ __forceinline__ float tanh_for<__nv_bfloat16>(float z) { 
 template <typename T, int SRC, int NV>
 __global__ void __launch_bounds__(1024)
 stream_step_kernel(const StreamStep p) {
+  pdl_begin();
   constexpr bool EXPERTS = SRC == SRC_EXPERTS || SRC == SRC_EXPERTS_NORMED;
   constexpr bool NORMED = SRC == SRC_NORMED || SRC == SRC_EXPERTS_NORMED;
   __shared__ float sh[32];
@@ -153,6 +154,7 @@ stream_step_kernel(const StreamStep p) {
 __global__ void __launch_bounds__(256)
 rotary_rows_kernel(const long* __restrict__ pos, const double* __restrict__ freq, float mag, float2* __restrict__ out, int T,
                    int half) {
+  pdl_begin();
   const long n = (long)T * half;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
     const double two_pi = 6.283185307179586476925;
@@ -181,9 +183,9 @@ gelu_lookup_kernel(T* __restrict__ z, long ldz, const T* __restrict__ table, lon
 
 template <typename T, int SRC>
 static int launch_step(const StreamStep& p, int threads, int nv, cudaStream_t st) {
-  if (nv == 1) stream_step_kernel<T, SRC, 1><<<p.rows, threads, 0, st>>>(p);
-  else if (nv == 2) stream_step_kernel<T, SRC, 2><<<p.rows, threads, 0, st>>>(p);
-  else stream_step_kernel<T, SRC, 4><<<p.rows, threads, 0, st>>>(p);
+  if (nv == 1) launch_overlapped(stream_step_kernel<T, SRC, 1>, p.rows, threads, 0, st, p);
+  else if (nv == 2) launch_overlapped(stream_step_kernel<T, SRC, 2>, p.rows, threads, 0, st, p);
+  else launch_overlapped(stream_step_kernel<T, SRC, 4>, p.rows, threads, 0, st, p);
   return (int)cudaGetLastError();
 }
 
@@ -221,7 +223,7 @@ extern "C" int omni_rotary_rows(const long* pos, const double* freq, float mag, 
   if (T <= 0 || half <= 0) return RC_OK;
   long blocks = ((long)T * half + 255) / 256;
   if (blocks > 148 * 8) blocks = 148 * 8;
-  rotary_rows_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(pos, freq, mag, reinterpret_cast<float2*>(out), T, half);
+  launch_overlapped(rotary_rows_kernel, (unsigned)blocks, 256, 0, (cudaStream_t)stream, pos, freq, mag, reinterpret_cast<float2*>(out), T, half);
   return (int)cudaGetLastError();
 }
 
