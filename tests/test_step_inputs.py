@@ -1,0 +1,71 @@
+"""One-launch step inputs (csrc/step_inputs.cu) against the PyTorch forms they stand for."""
+import pytest
+import torch
+
+from vllm_omni_b200.engine.graph_runner import DecodeGraphRunner
+from vllm_omni_b200.models.qwen_decoder import DecoderConfig, ModelBatch, QwenDecoderModel
+from vllm_omni_b200.models.seq_table import SeqTable
+
+pytestmark = pytest.mark.gpu
+
+
+def _decoder(mrope, interleaved=False):
+    cfg = DecoderConfig(vocab_size=100, hidden_size=136, num_hidden_layers=1, num_attention_heads=2, num_key_value_heads=1, head_dim=128,
+                        intermediate_size=64, mrope_section=(24, 20, 20) if mrope else None, mrope_interleaved=interleaved)
+    return QwenDecoderModel(cfg, torch.bfloat16, "cuda")
+
+
+@pytest.mark.parametrize("T", [1, 5, 300])
+@pytest.mark.parametrize("axes", ["one", "sections", "interleaved", "one position for all"])
+@pytest.mark.parametrize("overlay", [None, "mask", "all"])
+def test_rows_and_rotation(T, axes, overlay):
+    m = _decoder(axes != "one", axes == "interleaved")
+    g = torch.Generator(device="cuda").manual_seed(T)
+    ids = torch.randint(-3, 110, (T,), generator=g, device="cuda")              # outside the table too: held inside
+    pos = torch.randint(0, 40000, (3, T) if axes in ("sections", "interleaved") else (T,), generator=g, device="cuda")
+    kw = {}
+    if overlay:
+        kw["input_embeds"] = torch.randn(T, 136, generator=g, device="cuda").bfloat16()
+        kw["embeds_mask"] = torch.rand(T, generator=g, device="cuda") < 0.5 if overlay == "mask" else None
+    b = ModelBatch(ids, pos, None, **kw)
+    x, cos, sin = m.rows_and_rotation(b)
+    c, s = m.rope.cos_sin_for(pos, m.cfg.mrope_section, m.cfg.mrope_interleaved)
+    assert torch.equal(x, m.embed(b))
+    # the same fp32 angle; two correct cosines of it differ by an ulp of 1 at most
+    assert (cos - c).abs().max() <= 2.0 ** -23 and (sin - s).abs().max() <= 2.0 ** -23 and cos.is_contiguous() and sin.is_contiguous()
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 7])
+@pytest.mark.parametrize("mrope,overlay,seqs", [(False, False, False), (True, True, False), (False, True, True), (True, False, True)])
+def test_fill(n, mrope, overlay, seqs, monkeypatch):
+    m = _decoder(mrope)
+    m.uses_seq_table = seqs
+    kv = [tuple(torch.zeros(8, 16, 1, 128, device="cuda", dtype=torch.bfloat16) for _ in range(2)) + ((torch.zeros(1, device="cuda"),) if seqs else ())]
+    runners = [DecodeGraphRunner(m, kv, max_blocks=5, buckets=(1, 4, 8)) for _ in range(2)]
+    g = torch.Generator(device="cuda").manual_seed(n)
+    i32 = lambda *s: torch.randint(0, 50, s, generator=g, device="cuda", dtype=torch.int32)
+    pos = torch.randint(0, 99, (3, n) if mrope and n != 3 else (n,), generator=g, device="cuda")
+    b = ModelBatch(torch.randint(0, 99, (n,), generator=g, device="cuda"), pos, i32(n), [],
+                   decode_rows=torch.randperm(n, generator=g, device="cuda"), decode_block_tables=i32(n, 6)[:, :3], decode_seq_lens=i32(n))
+    if overlay:
+        b.input_embeds, b.embeds_mask = torch.randn(n, 136, generator=g, device="cuda").bfloat16(), torch.rand(n, generator=g, device="cuda") < 0.5
+    if seqs:
+        b.seqs = SeqTable(None, i32(n), None, None, None, n, n, 0, i32(n), i32(n))
+    states = []
+    for r, once in zip(runners, (True, False)):
+        if not once:
+            monkeypatch.setattr(DecodeGraphRunner, "_fill_once", lambda *a: False)
+        st = r._bucket(n)
+        for name in ("ids", "pos", "slots", "tables", "lens"):
+            getattr(st, name).fill_(77)                      # what an earlier step left
+        st.emask.fill_(True)
+        if once:
+            assert r._fill_once(st, b)
+        else:
+            r._fill(st, b)
+        states.append(st)
+    a, c = states
+    for name in ("ids", "pos", "slots", "tables", "lens", "emask") + (("embeds",) if overlay else ()) + (("ctx",) if seqs else ()):
+        assert torch.equal(getattr(a, name), getattr(c, name)), name
+    if seqs:
+        assert torch.equal(a.seqs.state_in, c.seqs.state_in) and torch.equal(a.seqs.state_out, c.seqs.state_out)

@@ -20,6 +20,7 @@ import torch
 
 from ..models.qwen_decoder import ModelBatch
 from ..models.seq_table import SeqTable
+from ..ops.step_inputs import StepFill
 
 DEFAULT_BUCKETS = (1, 2, 4, 8, 16, 32, 64, 128, 256)
 
@@ -88,8 +89,37 @@ class DecodeGraphRunner:
             self._state[size] = st
         return st
 
+    def _fill_once(self, st: _Bucket, b: ModelBatch) -> bool:
+        """``_fill`` as one launch; False where a tensor of the batch is not of a form it takes."""
+        order = b.decode_rows
+        if not (order.is_cuda and order.dtype == torch.int64 and order.is_contiguous()):
+            return False
+        f, pos = StepFill(order.numel(), st.n), b.positions
+        ok = f.put(st.ids, b.input_ids, True)
+        if st.pos.dim() == 2:
+            for ax in range(st.pos.shape[0]):
+                ok = ok and f.put(st.pos[ax], pos if pos.dim() == 1 else pos[ax], True)
+        else:
+            ok = ok and f.put(st.pos, pos, True)
+        ok = ok and f.put(st.slots, b.slot_mapping, True, pad_ones=True) and f.put(st.tables, b.decode_block_tables, False) \
+            and f.put(st.lens, b.decode_seq_lens, False)
+        if st.seqs is not None:
+            ok = ok and f.put(st.ctx, b.seqs.context, True)
+            if st.seqs.state_in is not None:
+                ok = ok and f.put(st.seqs.state_in, b.seqs.state_in, True) and f.put(st.seqs.state_out, b.seqs.state_out, False, pad_ones=True)
+        if b.input_embeds is not None:
+            mask = b.embeds_mask if b.embeds_mask is not None else torch.ones(order.numel(), dtype=torch.bool, device=order.device)
+            ok = ok and f.put(st.embeds, b.input_embeds, True) and f.put(st.emask, mask, True)
+        else:
+            ok = ok and f.put(st.emask, None, False)
+        if ok:
+            f.run(order)
+        return ok
+
     def _fill(self, st: _Bucket, b: ModelBatch) -> int:
         n = int(b.decode_rows.numel())
+        if st.ids.is_cuda and self._fill_once(st, b):
+            return n
         order = b.decode_rows                      # rows of the step's batch in decode order (identity here)
         pad = st.n - n
 

@@ -9,7 +9,7 @@ from .decoder import FikizenDecoder
 
 # libraries under csrc/ that serving this model loads on a GPU
 NATIVE_LIBS = ("gemm_sm100", "gemm_f32", "lm_ops", "stream_ops", "attn_window", "attn_window_sm100", "short_conv", "delta_rule",
-               "delta_chunks", "sampler", "rt_host", "io_host")
+               "delta_chunks", "sampler", "rt_host", "io_host", "step_inputs")
 
 
 class FikizenForCausalLM(StageModel):

@@ -9,7 +9,7 @@ from .decoder import MilivikDecoder
 
 # libraries under csrc/ that serving this model loads on a GPU
 NATIVE_LIBS = ("gemm_sm100", "gemm_f32", "lm_ops", "stream_ops", "elementwise", "moe", "latent_attn", "attn_window",
-               "attn_window_sm100", "sampler", "rt_host", "io_host")
+               "attn_window_sm100", "sampler", "rt_host", "io_host", "step_inputs")
 
 
 class MilivikForCausalLM(StageModel):

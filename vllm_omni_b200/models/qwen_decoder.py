@@ -23,6 +23,7 @@ from ..diffusion.layers.linear import FusedLinear
 from ..ops import fused, kv_cache as KC
 from ..ops.attention import attention
 from ..ops.moe import MoEWorkspace, moe_forward
+from ..ops.step_inputs import token_rows
 
 
 @dataclass
@@ -102,12 +103,28 @@ class RotaryTable:
         self.inv_freq = 1.0 / (theta ** (torch.arange(0, head_dim, 2, dtype=torch.float32) / head_dim))
         self._dev = {}
 
+    def freq_on(self, device) -> torch.Tensor:
+        inv = self._dev.get(device)
+        if inv is None:
+            inv = self._dev[device] = self.inv_freq.to(device)
+        return inv
+
+    def axis_on(self, device, mrope_section, interleaved) -> torch.Tensor:
+        """int32 [head_dim/2]: the position axis every frequency takes (see ``cos_sin_for``)."""
+        key = (device, tuple(mrope_section), interleaved)
+        if key not in self._dev:
+            axis = torch.zeros(self.head_dim // 2, dtype=torch.int32)
+            if interleaved:
+                for ax, off in ((1, 1), (2, 2)):
+                    axis[off:mrope_section[ax] * 3:3] = ax
+            else:
+                axis = torch.repeat_interleave(torch.arange(3, dtype=torch.int32), torch.tensor(mrope_section))
+            self._dev[key] = axis.to(device)
+        return self._dev[key]
+
     def cos_sin_for(self, positions: torch.Tensor, mrope_section=None, interleaved=False):
         """Per-token tables [T, head_dim/2] (fp32).  positions: [T] or [3, T]."""
-        inv = self._dev.get(positions.device)
-        if inv is None:
-            inv = self.inv_freq.to(positions.device)
-            self._dev[positions.device] = inv
+        inv = self.freq_on(positions.device)
         if positions.dim() == 1:
             ang = positions.float()[:, None] * inv[None, :]
         else:
@@ -286,6 +303,19 @@ class QwenDecoderModel(nn.Module):
             x = torch.where(m[:, None], batch.input_embeds.to(x.dtype), x) if m is not None else batch.input_embeds.to(x.dtype)
         return x.contiguous()
 
+    def rows_and_rotation(self, batch: ModelBatch):
+        """(x [T, D], cos, sin): ``embed`` and the rotation tables, on a GPU in one launch where the operands allow."""
+        cfg, pos, got = self.cfg, batch.positions, None
+        if self.embed_tokens.is_cuda and (pos.dim() == 1 or cfg.mrope_section is not None):
+            dev = pos.device
+            axis = self.rope.axis_on(dev, cfg.mrope_section, cfg.mrope_interleaved) if pos.dim() > 1 else None
+            if axis is None or (axis.numel() == self.rope.head_dim // 2 and pos.shape[0] == 3):
+                got = token_rows(batch.input_ids, self.embed_tokens, pos, self.rope.freq_on(dev), axis, batch.input_embeds,
+                                 batch.embeds_mask)
+        if got is not None:
+            return got
+        return (self.embed(batch), *self.rope.cos_sin_for(pos, cfg.mrope_section, cfg.mrope_interleaved))
+
     def attention_block(self, layer: DecoderLayer, qkv: torch.Tensor, batch: ModelBatch, k_cache, v_cache, out):
         cfg = self.cfg
         (H, Hkv), Dh = self.local_heads, cfg.head_dim
@@ -325,9 +355,8 @@ class QwenDecoderModel(nn.Module):
         vision tower's intermediate blocks, zero on the other rows)."""
         cfg = self.cfg
         (H, Hkv), Dh = self.local_heads, cfg.head_dim        # this rank's heads under tensor parallelism
-        x = self.embed(batch)
+        x, cos, sin = self.rows_and_rotation(batch)
         T = x.shape[0]
-        cos, sin = self.rope.cos_sin_for(batch.positions, cfg.mrope_section, cfg.mrope_interleaved)
         captured = {}
         if 0 in capture_layers:
             captured[0] = x.clone()
