@@ -1,0 +1,49 @@
+"""3 x 3 convolutions on CTA pairs (csrc/conv_pair.cuh): ragged images, odd numbers of pixel tiles, channel counts that end inside a
+block of 64 or a step of 16, output widths of every tile, epilogues; against 64-bit sums."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+from vllm_omni_b200.ops import _native as nv, conv as C
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,h,w", [(1, 64, 80), (3, 47, 61), (2, 16, 200), (5, 33, 41), (40, 7, 9)])
+@pytest.mark.parametrize("cin,cout", [(16, 384), (96, 96), (96, 3), (72, 200), (192, 192), (128, 256), (8, 40)])
+@pytest.mark.parametrize("epilogue", [None, "silu", "residual"])
+def test_against_64_bits(n, h, w, cin, cout, epilogue):
+    if epilogue and (cin, cout) not in ((96, 96), (72, 200), (128, 256)):
+        pytest.skip("epilogues at three widths")
+    g = torch.Generator(device="cuda").manual_seed(n * h + w + cin)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    wide = rnd(n, h, w, cin + 8)                                       # channels past cin are not part of the input
+    wt, b = rnd(cout, cin, 3, 3) * (9 * cin) ** -0.5, rnd(cout)
+    pw, pb = C.pack_conv_weight(wt, b)
+    res = rnd(n, h, w, pw.shape[0]) if epilogue == "residual" else None
+    out = C.conv2d_nhwc(wide, pw, pb, 3, cin, act="silu" if epilogue == "silu" else None, residual=res)
+    x64, w64 = wide[..., :cin].double().permute(0, 3, 1, 2), wt.double()
+    ref = F.conv2d(x64, w64, b.double(), padding=1)
+    mass = F.conv2d(x64.abs(), w64.abs(), padding=1)
+    err = 0.0
+    if epilogue == "silu":
+        err, ref = ref.abs() * 2.0 ** -11, F.silu(ref)                 # tanh.approx
+    if res is not None:
+        ref = ref + res[..., :cout].double().permute(0, 3, 1, 2)
+    # result rounded to bf16; fp32 sums of at most 9 * cin / 16 MMA steps
+    bound = 1.2 * (ref.abs() * 2.0 ** -8 + mass * (9 * cin / 16 + 1) * 2.0 ** -23) + err + 1e-6
+    got = out[..., :cout].double().permute(0, 3, 1, 2)
+    assert torch.isfinite(out).all() and ((got - ref).abs() <= bound).all()
+    nv.check_status()
+
+
+@pytest.mark.parametrize("channels", [8, 32, 40, 64, 96, 128, 136, 192, 256, 264, 384, 512, 520, 1024])
+@pytest.mark.parametrize("pixels", [1, 77, 4099])
+def test_rmsnorm_silu(channels, pixels):
+    g = torch.Generator(device="cuda").manual_seed(channels + pixels)
+    x, gamma = torch.randn(pixels, channels, generator=g, device="cuda").bfloat16(), torch.randn(channels, generator=g, device="cuda").bfloat16()
+    z = x.double() * torch.rsqrt(x.double().pow(2).mean(-1, keepdim=True)) * gamma.double()
+    for silu in (False, True):
+        y, ref = C.rmsnorm_silu_nhwc(x, gamma, silu=silu), F.silu(z) if silu else z
+        # one rounding to bf16 of fp32 arithmetic; tanh.approx in silu
+        assert ((y.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + z.abs() * 2.0 ** -11 * silu + 1e-5).all()

@@ -1,0 +1,257 @@
+// 3 x 3 convolution, stride 1, zero padding, channels-last, as an implicit GEMM on CTA pairs (cta_group::2).
+//
+// What bounds the one-CTA kernel (gemm_bf16_kernel) here is the way from L2 to shared memory: it fetches the pixels of a tile once per tap
+// and the weights once per 128 pixels, 32 to 40 KB per 64 channels and tap, 1.6 to 2 times what an SM takes in while its MMAs run.  This
+// kernel fetches both less often:
+//   pixels   a tile is 16 x 8 pixels per CTA; one TMA box of 18 x 8 pixels (one column offset dx, 64 channels) serves the three taps (dy, dx):
+//            a group of 8 rows of the MMA operand is the 8 pixels of one image row, so tap dy is the box from its (dy + 1)-th group on
+//   weights  each CTA of a pair holds half of the TN output channels' weights and the pair's MMA reads both
+// A channel block of which only some channels exist (96 = 64 + 32) issues the K steps that hold any.  Per 64 channels and three taps
+// a CTA takes in 18 KB + 3 * 64 * TN bytes, 0.35 of the one-CTA kernel's 2 * 3 * (16 KB + 128 * TN) / 2 at TN = 96.
+// With residual, one-CTA kernel before: 1024 x 1024 pixels, 96 -> 96 channels 268 us (461), 192 -> 96 317 us (662), 96 -> 8 145 us (743);
+// 512 x 512, 192 -> 192 160 us (193), 384 -> 192 221 us (350); 256 x 256, 384 -> 384 119 us (180).
+#pragma once
+
+namespace omni {
+
+constexpr int C3_W = 8, C3_H = 16;                       // pixels of a CTA's tile
+constexpr int C3_A_BYTES = (C3_H + 2) * C3_W * 128;      // 18 groups of 8 pixels x 64 channels
+
+template <int TN>
+struct Conv3Cfg {
+  static constexpr int B_BYTES = (TN / 2) * 128;         // one tap's weights of this CTA's half
+  static constexpr int STAGE_BYTES = C3_A_BYTES + 3 * B_BYTES;
+  static constexpr int STAGES = 220 * 1024 / STAGE_BYTES < 6 ? 220 * 1024 / STAGE_BYTES : 6;
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024;
+  static constexpr int ACC_STRIDE = TN <= 32 ? 32 : (TN <= 64 ? 64 : (TN <= 128 ? 128 : 256));
+  static constexpr int TMEM_COLS = 2 * ACC_STRIDE;
+};
+
+struct Conv3Args {
+  CUtensorMap tmX, tmW;
+  __nv_bfloat16* y;
+  int ldy;
+  int H, W, n_img, tiles_x, tiles_y;      // tiles of 16 x 8 pixels
+  int Cout, cin, cin_blocks;
+  GemmEpilogue epi;
+};
+
+__device__ __forceinline__ void add8(float (&f)[8], const uint4& u) {
+  const float2 a = unpack_bf16(u.x), b = unpack_bf16(u.y), c = unpack_bf16(u.z), d = unpack_bf16(u.w);
+  f[0] += a.x; f[1] += a.y; f[2] += b.x; f[3] += b.y;
+  f[4] += c.x; f[5] += c.y; f[6] += d.x; f[7] += d.y;
+}
+
+template <int TN>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
+conv3x3_pair_kernel(const __grid_constant__ Conv3Args a, int* status) {
+  using Cfg = Conv3Cfg<TN>;
+  constexpr int STAGES = Cfg::STAGES;
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ __align__(8) uint64_t full_bar[STAGES];
+  __shared__ __align__(8) uint64_t empty_bar[STAGES];
+  __shared__ __align__(8) uint64_t tfull_bar[2];
+  __shared__ __align__(8) uint64_t tempty_bar[2];
+  __shared__ uint32_t tmem_base_s;
+  __shared__ int s_abort;
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_ctarank();
+  const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
+  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  const int per_img = a.tiles_x * a.tiles_y, m_tiles = a.n_img * per_img;
+  const int num_m = (m_tiles + 1) / 2, num_n = (a.Cout + TN - 1) / TN, num_tiles = num_m * num_n;
+  const int num_st = 3 * a.cin_blocks;                    // stages per tile: (channel block, dx)
+
+  if (threadIdx.x == 0) {
+    s_abort = 0;
+    for (int i = 0; i < STAGES; ++i) {
+      mbar_init(smem_u32(&full_bar[i]), 1);
+      mbar_init(smem_u32(&empty_bar[i]), 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(smem_u32(&tfull_bar[i]), 1);
+      mbar_init(smem_u32(&tempty_bar[i]), 16);
+    }
+    fence_mbar_init();
+    tma_prefetch_desc(&a.tmX);
+    tma_prefetch_desc(&a.tmW);
+  }
+  if (warp == 1) {
+    tmem_alloc_pair(smem_u32(&tmem_base_s), Cfg::TMEM_COLS);
+    tmem_relinquish_pair();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  cluster_sync_all();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = tmem_base_s;
+  pdl_begin();
+
+  // the pair's two pixel tiles are neighbours in the tile list; a tile past the end (odd counts) lies below the last image's rows
+  auto place = [&](int t, int& nb, int& img, int& y0, int& x0) {
+    const int mb = (t / num_n) * 2 + (int)rank;
+    nb = t % num_n;
+    img = min(mb / per_img, a.n_img - 1);
+    const int rem = mb - img * per_img;
+    y0 = rem / a.tiles_x * C3_H;
+    x0 = rem % a.tiles_x * C3_W;
+  };
+
+  if (warp == 0) {
+    if (elect_one()) {
+      int stage = 0;
+      uint32_t phase = 0;
+      for (int t = pair; t < num_tiles; t += num_pairs) {
+        int nb, img, y0, x0;
+        place(t, nb, img, y0, x0);
+        for (int s = 0; s < num_st; ++s) {
+          const int cb = s / 3, dx = s - cb * 3;
+          mbar_wait(smem_u32(&empty_bar[stage]), phase ^ 1, &s_abort, status, ERR_WAIT_EMPTY);
+          if (rank == 0) mbar_expect_tx(smem_u32(&full_bar[stage]), 2 * Cfg::STAGE_BYTES);
+          const uint32_t fb = mapa_shared(smem_u32(&full_bar[stage]), 0);
+          const uint32_t sa = smem_base + stage * Cfg::STAGE_BYTES;
+          tma_load_4d_pair(sa, &a.tmX, fb, cb * 64, x0 + dx - 1, y0 - 1, img);
+#pragma unroll
+          for (int dy = 0; dy < 3; ++dy)
+            tma_load_2d_pair(sa + C3_A_BYTES + dy * Cfg::B_BYTES, &a.tmW, fb, ((dy * 3 + dx) * a.cin_blocks + cb) * 64,
+                             nb * TN + (int)rank * (TN / 2));
+          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (rank == 0 && elect_one()) {
+      constexpr uint32_t idesc = umma_idesc(256, TN, 1, 1, 0, 0);
+      int stage = 0, acc = 0;
+      uint32_t phase = 0, acc_phase = 0;
+      for (int t = pair; t < num_tiles; t += num_pairs) {
+        mbar_wait(smem_u32(&tempty_bar[acc]), acc_phase ^ 1, &s_abort, status, ERR_WAIT_TMEM_EMPTY);
+        tc_fence_after_sync();
+        const uint32_t d_tmem = tmem_base + acc * Cfg::ACC_STRIDE;
+        for (int s = 0; s < num_st; ++s) {
+          const int steps = min(4, (a.cin - s / 3 * 64 + 15) / 16);          // 16 channels each
+          mbar_wait(smem_u32(&full_bar[stage]), phase, &s_abort, status, ERR_WAIT_FULL);
+          tc_fence_after_sync();
+          const uint32_t sa = smem_base + stage * Cfg::STAGE_BYTES;
+          const uint64_t a_desc = umma_desc_kmajor_sw128(sa), b_desc = umma_desc_kmajor_sw128(sa + C3_A_BYTES);
+#pragma unroll
+          for (int dy = 0; dy < 3; ++dy)
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              if (k < steps)
+                mma_f16_ss_pair(d_tmem, a_desc + dy * (C3_W * 128 / 16) + 2 * k, b_desc + dy * (Cfg::B_BYTES / 16) + 2 * k, idesc,
+                                (s | dy | k) != 0);
+          tc_commit_pair(mapa_shared(smem_u32(&empty_bar[stage]), 0));
+          tc_commit_pair(mapa_shared(smem_u32(&empty_bar[stage]), 1));
+          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+        }
+        tc_commit_pair(mapa_shared(smem_u32(&tfull_bar[acc]), 0));
+        tc_commit_pair(mapa_shared(smem_u32(&tfull_bar[acc]), 1));
+        acc ^= 1;
+        if (acc == 0) acc_phase ^= 1;
+      }
+    }
+  } else {
+    // A tile of few channels is over in 2 us, less than an epilogue that waits for its residual and writes it takes: the residual is
+    // requested while the MMAs of the tile run.
+    constexpr int CH = TN / 32;                             // 16-column chunks per warp: half of the tile's columns
+    const int q = warp & 3, first = ((warp - 2) >> 2) * (TN / 2);
+    int acc = 0;
+    uint32_t acc_phase = 0;
+    for (int t = pair; t < num_tiles; t += num_pairs) {
+      int nb, img, y0, x0;
+      place(t, nb, img, y0, x0);
+      const int r = q * 32 + lane, y = y0 + r / C3_W, x = x0 + r % C3_W;
+      const bool row_ok = y < a.H && x < a.W;
+      const long row = ((long)img * a.H + y) * a.W + x;
+      const int col = nb * TN + first;
+      uint4 res[CH][2];
+      if (a.epi.residual) {
+#pragma unroll
+        for (int c = 0; c < CH; ++c)
+#pragma unroll
+          for (int g = 0; g < 2; ++g)
+            res[c][g] = row_ok && col + c * 16 + g * 8 < a.Cout
+                            ? *reinterpret_cast<const uint4*>(a.epi.residual + row * a.epi.ldr + col + c * 16 + g * 8)
+                            : make_uint4(0u, 0u, 0u, 0u);
+      }
+      mbar_wait(smem_u32(&tfull_bar[acc]), acc_phase, &s_abort, status, ERR_WAIT_TMEM_FULL);
+      tc_fence_after_sync();
+#pragma unroll
+      for (int c = 0; c < CH; ++c) {
+        uint32_t v[16];
+        tmem_ld_32x16(tmem_base + ((uint32_t)(q * 32) << 16) + acc * Cfg::ACC_STRIDE + first + c * 16, v);
+        tmem_wait_ld();
+        if (c == CH - 1) {                                  // the accumulator is read: the next but one tile may have it
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&tempty_bar[acc]), 0));
+        }
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+          const int cc = col + c * 16 + g * 8;
+          if (!row_ok || cc >= a.Cout) continue;
+          float f[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(v[g * 8 + e]);
+          if (a.epi.bias) add8(f, *reinterpret_cast<const uint4*>(a.epi.bias + cc));
+          if (a.epi.act == ACT_GELU_TANH) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) f[e] = gelu_tanh(f[e]);
+          } else if (a.epi.act == ACT_SILU) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) f[e] = silu(f[e]);
+          } else if (a.epi.act == ACT_RELU2) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) f[e] = fmaxf(f[e], 0.f) * fmaxf(f[e], 0.f);
+          }
+          if (a.epi.residual) add8(f, res[c][g]);
+          *reinterpret_cast<uint4*>(a.y + row * a.ldy + cc) =
+              make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
+        }
+      }
+      acc ^= 1;
+      if (acc == 0) acc_phase ^= 1;
+    }
+  }
+
+  tc_fence_before_sync();
+  __syncthreads();
+  if (s_abort) {
+    const unsigned long long t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 200000ull) {
+    }
+  }
+  cluster_sync_all();
+  if (warp == 1) tmem_dealloc_pair(tmem_base, Cfg::TMEM_COLS);
+}
+
+template <int TN>
+static int launch_conv3(Conv3Args& a, const void* w, int pairs, int* status, cudaStream_t stream) {
+  using Cfg = Conv3Cfg<TN>;
+  const uint64_t K = 9ull * a.cin_blocks * 64;
+  if (int rc = make_tmap_2d(&a.tmW, w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)a.Cout, K, K * 2, TN / 2, 64)) return rc;
+  static unsigned long long prepared = 0;
+  if (int e = ensure_dynamic_smem((const void*)conv3x3_pair_kernel<TN>, Cfg::SMEM_BYTES, prepared)) return e;
+  const long tiles = (long)((a.n_img * a.tiles_x * a.tiles_y + 1) / 2) * ((a.Cout + TN - 1) / TN);
+  const int grid = tiles < pairs ? (int)tiles : pairs;
+  launch_overlapped(conv3x3_pair_kernel<TN>, 2 * grid, GEMM_THREADS, Cfg::SMEM_BYTES, stream, a, status);
+  return (int)cudaGetLastError();
+}
+
+// Widths that leave the fewest columns empty, then the fewest waves; the narrowest for outputs of a few channels (an image).
+static int pick_conv3_tn(long m_pairs, int Cout, int pairs) {
+  const int cand[5] = {256, 192, 128, 96, 32};
+  int best = 256;
+  long best_cost = -1;
+  for (int i = 0; i < 5; ++i) {
+    const int tn = cand[i];
+    const long waves = (m_pairs * ((Cout + tn - 1) / tn) + pairs - 1) / pairs;
+    const long cost = waves * (tn + 24);                  // a tile's pixels are fetched whatever its width
+    if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = tn; }
+  }
+  return best;
+}
+
+}  // namespace omni

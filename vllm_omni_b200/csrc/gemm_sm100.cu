@@ -1048,6 +1048,7 @@ static int pick_bn(int M, int N, int ctas) {
 }  // namespace omni
 
 #include "gemm_skinny.cuh"
+#include "conv_pair.cuh"
 
 // C ABI.  All pointers are device pointers; `status` is a device int32 that receives the
 // first timeout code (0 = none).  Strides are in elements.  force_bn = 0 lets the launcher
@@ -1365,6 +1366,36 @@ extern "C" int omni_conv2d_nhwc_bf16(const void* x, long ldx, const void* w, voi
   EncodeTiledFn enc = get_encode_tiled();
   if (!enc) return RC_NO_DRIVER;
   if (reinterpret_cast<uintptr_t>(x) & 15) return RC_BAD_ARG;
+  const int pairs = ksize == 3 ? max_resident_pairs() : 0;
+  const long m_pairs = ((long)Nimg * ((W + C3_W - 1) / C3_W) * ((H + C3_H - 1) / C3_H) + 1) / 2;
+  // below a quarter of a wave of pixel tiles the one-CTA kernel spreads a problem over more SMs
+  if (ksize == 3 && m_pairs * 4 >= pairs && m_pairs < (1L << 24)) {
+    Conv3Args a = {};
+    a.y = static_cast<__nv_bfloat16*>(y);
+    a.ldy = ldy; a.H = H; a.W = W; a.n_img = Nimg;
+    a.tiles_x = (W + C3_W - 1) / C3_W; a.tiles_y = (H + C3_H - 1) / C3_H;
+    a.Cout = Cout; a.cin = Cin; a.cin_blocks = (Cin + BK - 1) / BK;
+    cuuint64_t gdim[4] = {(cuuint64_t)Cin, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)Nimg};
+    cuuint64_t gstr[3] = {(cuuint64_t)ldx * 2, (cuuint64_t)ldx * 2 * W, (cuuint64_t)ldx * 2 * W * H};
+    cuuint32_t box[4] = {BK, C3_W, C3_H + 2, 1};
+    cuuint32_t estr[4] = {1, 1, 1, 1};
+    if (enc(&a.tmX, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(x), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+      return RC_TMAP;
+    a.epi.bias = static_cast<const __nv_bfloat16*>(bias);
+    a.epi.residual = static_cast<const __nv_bfloat16*>(residual);
+    a.epi.ldr = ldr;
+    a.epi.rows_per_batch = 1;
+    a.epi.act = act;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    switch (pick_conv3_tn(m_pairs, Cout, pairs)) {
+      case 256: return launch_conv3<256>(a, w, pairs, status, st);
+      case 192: return launch_conv3<192>(a, w, pairs, status, st);
+      case 128: return launch_conv3<128>(a, w, pairs, status, st);
+      case 96: return launch_conv3<96>(a, w, pairs, status, st);
+      default: return launch_conv3<32>(a, w, pairs, status, st);
+    }
+  }
   ConvGeom g = {};
   g.taps = ksize * ksize;
   g.H = H; g.W = W;
