@@ -1,4 +1,4 @@
-// K10: mixture-of-experts routing, dispatch and combine around the grouped tcgen05 GEMM.
+// K10: mixture-of-experts routing, dispatch and combine around the tcgen05 expert GEMM.
 //
 //   omni_moe_route     softmax over expert logits, top-k, optional renormalisation
 //   omni_moe_router    router product and choice in one launch: fp32 logits with a bias, the top-k largest, softmax
@@ -7,14 +7,13 @@
 //   omni_moe_pairs_f32 y[p] = act(W[expert of pair p] x[p / per]) in true fp32 (exact mode)
 //   omni_moe_few_plan  few tokens: tiles of at most 16 rows per expert, from router logits (route included) or chosen ids
 //   omni_moe_few_rows  few tokens: y[pair] = act(W[expert] x[pair / per]) with rows gathered in place, SwiGLU included
-//   omni_moe_plan      per-expert counts -> segment offsets padded to 128 rows (the GEMM's M
-//                      tile), the expert of every M tile, and the row of every (token, k) pair
-//   omni_moe_dispatch  copy token rows into the expert-major padded buffer
+//   omni_moe_plan_tiles  rows of every expert back to back, its tiles of rows, and the row of every (token, k) pair
+//   omni_moe_plan      the same with segments padded to 128 rows
+//   omni_moe_dispatch  copy token rows into the expert-major buffer
 //   omni_moe_combine   out[t] = sum_k w[t,k] * y[row(t,k)]  (+ optional residual / shared expert)
 //
-// Padding each expert segment to the 128-row MMA tile keeps every GEMM tile inside one expert,
-// so the expert GEMMs are ONE launch of the grouped kernel (gemm_sm100.cu) with a per-tile
-// expert index.  The reference reaches vLLM's Triton fused_moe or a Python loop over experts
+// Every tile of rows lies inside one expert, so the GEMM of all experts is ONE launch with a per-tile expert index (moe_gemm.cuh;
+// gemm_sm100.cu for padded segments).  The reference reaches vLLM's Triton fused_moe or a Python loop over experts
 // (vllm_omni/model_executor/models/qwen3_omni/qwen3_moe.py).
 #include "host_util.h"
 #include "ptx_sm100.cuh"
@@ -387,11 +386,12 @@ __device__ __forceinline__ void block_scan2(int& a, int& b, int& total_a, int& t
   b = b - b0 + (warp ? pb : 0);
 }
 
-// Plan without padding: the rows of expert e are [off[e], off[e] + cnt[e]); expert e owns ceil(cnt[e] / TILE)
-// M tiles; tile t = (expert, first row, rows <= TILE).  Unused tiles get expert -1.  One block; the place of a pair among its expert's
+// Plan without padding: the rows of expert e are [off[e], off[e] + cnt[e]); expert e owns c = ceil(cnt[e] / tile)
+// tiles of about cnt[e] / c rows (rounded up to 16); tile t = (expert, first row, rows).  Unused tiles get expert -1.  With global_ids
+// tiles are full but for an expert's last, and name experts as `ids` does; else as the local weights do, from 0.  One block; the place of a pair among its expert's
 // rows is what its atomic add to the expert's count returns (the order inside an expert does not affect results).
 __global__ void __launch_bounds__(1024)
-moe_plan_compact_kernel(const int* __restrict__ ids, int n_pairs, int E, int e_lo, int e_hi, int max_tiles,
+moe_plan_compact_kernel(const int* __restrict__ ids, int n_pairs, int E, int e_lo, int e_hi, int tile_cap, int global_ids, int max_tiles,
                         int* __restrict__ row_of_pair, int* __restrict__ tile_expert, int* __restrict__ tile_row0,
                         int* __restrict__ tile_rows, int* __restrict__ n_rows_out, MoeBounds bd) {
   pdl_begin();
@@ -408,14 +408,15 @@ moe_plan_compact_kernel(const int* __restrict__ ids, int n_pairs, int E, int e_l
   }
   __syncthreads();
   const int e = threadIdx.x, mine = cnt[e];             // experts past E have none
-  int row = mine, tile = (mine + MOE_TILE - 1) / MOE_TILE, rows, tiles;
+  const int own = (mine + tile_cap - 1) / tile_cap, size = global_ids ? tile_cap : own ? ((mine + own - 1) / own + 15) / 16 * 16 : 0;
+  int row = mine, tile = own, rows, tiles;
   block_scan2(row, tile, rows, tiles);
   off[e] = row;
   if (e == 0) *n_rows_out = rows;
-  for (int i = 0; i * MOE_TILE < mine; ++i) {
-    tile_expert[tile + i] = e;
-    tile_row0[tile + i] = row + i * MOE_TILE;
-    tile_rows[tile + i] = min(MOE_TILE, mine - i * MOE_TILE);
+  for (int i = 0; i < own; ++i) {                       // never empty: (own - 1) * size < mine, as tile_cap is a multiple of 64
+    tile_expert[tile + i] = global_ids ? e : e - e_lo;
+    tile_row0[tile + i] = row + i * size;
+    tile_rows[tile + i] = min(size, mine - i * size);
   }
   for (int t = tiles + threadIdx.x; t < max_tiles; t += 1024) {
     tile_expert[t] = -1;
@@ -738,12 +739,25 @@ extern "C" int omni_moe_plan(const int* ids, int n_pairs, int E, int e_lo, int e
   return (int)cudaGetLastError();
 }
 
+static int plan_tiles_as(const int* ids, int n_pairs, int E, int e_lo, int e_hi, int tile_cap, int global_ids, int max_tiles,
+                         int* row_of_pair, int* tile_expert, int* tile_row0, int* tile_rows, int* n_rows_out, void* stream) {
+  if (E > 1024) return RC_BAD_ARG;
+  launch_overlapped(moe_plan_compact_kernel, 1, 1024, 0, (cudaStream_t)stream, ids, n_pairs, E, e_lo, e_hi, tile_cap, global_ids, max_tiles,
+                    row_of_pair, tile_expert, tile_row0, tile_rows, n_rows_out, g_moe_bounds);
+  return (int)cudaGetLastError();
+}
+
+// Tiles of 128 rows; max_tiles: at least min(E, n_pairs) + n_pairs / 128.
 extern "C" int omni_moe_plan_compact(const int* ids, int n_pairs, int E, int e_lo, int e_hi, int max_tiles, int* row_of_pair,
                                      int* tile_expert, int* tile_row0, int* tile_rows, int* n_rows_out, void* stream) {
-  if (E > 1024) return RC_BAD_ARG;
-  launch_overlapped(moe_plan_compact_kernel, 1, 1024, 0, (cudaStream_t)stream, ids, n_pairs, E, e_lo, e_hi, max_tiles, row_of_pair, tile_expert,
-                                                                tile_row0, tile_rows, n_rows_out, g_moe_bounds);
-  return (int)cudaGetLastError();
+  return plan_tiles_as(ids, n_pairs, E, e_lo, e_hi, MOE_TILE, 1, max_tiles, row_of_pair, tile_expert, tile_row0, tile_rows, n_rows_out, stream);
+}
+
+// Even tiles of at most tile_cap (64, 128 or 256) rows for omni_gemm_bf16_experts; max_tiles: at least min(E, n_pairs) + n_pairs / tile_cap.
+extern "C" int omni_moe_plan_tiles(const int* ids, int n_pairs, int E, int e_lo, int e_hi, int tile_cap, int max_tiles, int* row_of_pair,
+                                   int* tile_expert, int* tile_row0, int* tile_rows, int* n_rows_out, void* stream) {
+  if (tile_cap != 64 && tile_cap != 128 && tile_cap != 256) return RC_BAD_ARG;
+  return plan_tiles_as(ids, n_pairs, E, e_lo, e_hi, tile_cap, 0, max_tiles, row_of_pair, tile_expert, tile_row0, tile_rows, n_rows_out, stream);
 }
 
 // Plan of at most FEW_PAIRS pairs.  `logits` bf16 [T, E] (E <= 256, k <= 16): the choice is made here, ids and weights are outputs; null:

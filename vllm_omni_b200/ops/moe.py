@@ -1,8 +1,7 @@
-"""K10 — mixture-of-experts forward on the grouped tcgen05 GEMM (csrc/moe.cu, gemm_sm100.cu).
+"""K10 — mixture-of-experts forward on the tcgen05 expert GEMM (csrc/moe.cu, moe_gemm.cuh).
 
-``moe_forward`` = route (softmax, top-k, renorm) -> plan (expert segments padded to the
-128-row MMA tile) -> dispatch (gather rows expert-major) -> grouped GEMM w13 -> SwiGLU ->
-grouped GEMM w2 -> weighted combine.  With expert parallelism a rank passes its local expert
+``moe_forward`` = route (softmax, top-k, renorm) -> plan (tiles of an expert's rows) -> dispatch (gather rows
+expert-major) -> expert GEMM w13 with SwiGLU -> expert GEMM w2 -> weighted combine; few tokens skip the dispatch.  With expert parallelism a rank passes its local expert
 range; pairs routed to other ranks contribute nothing locally and the caller sums the
 partial outputs across ranks.  ``moe_reference`` is the dense per-token restatement (the
 semantics of vllm_omni/model_executor/models/qwen3_omni/qwen3_moe.py).
@@ -61,13 +60,14 @@ class _MoEBuffers:
 
     def __init__(self, cap, k, E, D, Fd, device, dtype, pad):
         n_pairs = cap * k
-        rows, tiles = _rows_tiles(cap, k, E, pad)
+        # the tile size grows with the number of tokens, so a smaller batch of the bucket can need more tiles
+        rows, tiles = _rows_tiles(cap, k, E, pad)[0], max(_rows_tiles(t, k, E, pad)[1] for t in (cap, min(cap, 32 * E // k), min(cap, 64 * E // k)))
         i32 = lambda *s: torch.zeros(*s, dtype=torch.int32, device=device)
         t = dict(ids=i32(cap, k), row_of_pair=i32(n_pairs), tile_expert=i32(tiles), tile_row0=i32(tiles), tile_rows=i32(tiles),
                  offsets=i32(E + 1), n_rows=i32(1), weights=torch.empty(cap, k, dtype=torch.float32, device=device),
                  few_expert=i32(_few_tiles(cap, k, E)), few_row0=i32(_few_tiles(cap, k, E)), few_rows=i32(_few_tiles(cap, k, E)),
                  pair_of_row=i32(n_pairs),
-                 xp=torch.zeros(rows, D, dtype=dtype, device=device), h13=torch.empty(rows, 2 * Fd, dtype=dtype, device=device),
+                 xp=torch.zeros(rows, D, dtype=dtype, device=device), h13=torch.empty(rows if pad else 0, 2 * Fd, dtype=dtype, device=device),
                  h=torch.empty(rows, Fd, dtype=dtype, device=device), y=torch.empty(rows, D, dtype=dtype, device=device))
         self.__dict__.update(t)
 
@@ -77,9 +77,15 @@ def _rows_tiles(T, k, E, pad):
     if pad:
         rows = ((n_pairs + E * 127) + 127) // 128 * 128
         return rows, rows // 128
-    # rows back to back: every (token, choice) pair is one row; an expert starts a new M tile, so at most one
+    # rows back to back: every (token, choice) pair is one row; an expert starts a new tile, so at most one
     # partly filled tile per expert that got rows
-    return n_pairs, min(E, n_pairs) + (n_pairs + 127) // 128
+    return n_pairs, min(E, n_pairs) + n_pairs // _tile_rows(T, k, E)
+
+
+def _tile_rows(T, k, E) -> int:
+    """Most rows of an expert tile (csrc/moe_gemm.cuh): twice the average, so that most experts are one tile.  Small tiles leave more of
+    the shared memory to the weights."""
+    return 64 if T * k <= 32 * E else 128 if T * k <= 64 * E else 256
 
 
 FEW_TILE, FEW_PAIRS = 16, 2048          # csrc/moe.cu
@@ -91,11 +97,10 @@ def _few_tiles(T, k, E):
 
 
 def _few(T, k, E, pad) -> bool:
-    """Whether to stream the chosen experts' weights past gathered rows (csrc/moe.cu, "few tokens"): up to 2 rows per expert on
-    average.  128 experts of 2048 -> 768, top 8, whole layer on cold caches: 1 token 38 us (grouped GEMMs 64), 8 tokens 106 (145), 32
-    tokens 200 (214), 64 tokens 237 (239): from there on every row costs as much again as its share of the weights, and the
-    grouped GEMMs run at memory speed."""
-    return not pad and T * k <= min(FEW_PAIRS, 2 * E)
+    """Whether to stream the chosen experts' weights past gathered rows (csrc/moe.cu, "few tokens"): up to one row per expert on
+    average.  128 experts of 2048 -> 768, top 8, whole layer on cold caches, against the expert GEMMs (csrc/moe_gemm.cuh): 1 token
+    28 us (35), 8 tokens 94 (99), 32 tokens 189 (172): from there on every row costs as much again as its share of the weights."""
+    return not pad and T * k <= min(FEW_PAIRS, E)
 
 
 _pool: dict = {}
@@ -119,6 +124,7 @@ class MoEWorkspace:
             buf = _pool[key] = _MoEBuffers(cap, k, E, D, Fd, device, dtype, pad)
         self.key, self.padded = (T,) + key, pad
         self.max_rows, self.max_tiles = _rows_tiles(T, k, E, pad)
+        self.tile_cap = _tile_rows(T, k, E)
         n_pairs = T * k
         self.ids, self.weights, self.row_of_pair = buf.ids[:T], buf.weights[:T], buf.row_of_pair[:n_pairs]
         self.tile_expert, self.tile_row0, self.tile_rows = (buf.tile_expert[:self.max_tiles], buf.tile_row0[:self.max_tiles],
@@ -142,19 +148,22 @@ class ExpertRows:
     weights: torch.Tensor
 
 
-def _grouped(ws, a, lda, w, c, ldc, n, kk, tile_expert, act=0):
-    """c = act(a @ w[e].T) over the workspace's expert tiles."""
+def _grouped(ws, a, w, c, tile_expert, act=None):
+    """c = act(a @ w[e].T) over the workspace's expert tiles; act "swiglu": w holds gate and lift rows."""
     g, st, status = nv.lib("gemm_sm100"), nv.stream_ptr(), nv.status_word(a.device)
+    n, kk = c.shape[1], w.shape[2]
     if ws.padded:
-        nv.check_rc(g.omni_gemm_bf16_grouped(nv.ptr(a), c_int(lda), nv.ptr(w), c_int(w.shape[0]), nv.ptr(c), c_int(ldc),
-                                             c_int(ws.max_rows), c_int(n), c_int(kk), nv.ptr(tile_expert), c_int(act), c_int(0),
-                                             nv.ptr(status), st), "omni_gemm_bf16_grouped")
+        full = ws.h13 if act == "swiglu" else c
+        nv.check_rc(g.omni_gemm_bf16_grouped(nv.ptr(a), c_int(a.stride(0)), nv.ptr(w), c_int(w.shape[0]), nv.ptr(full), c_int(full.stride(0)),
+                                             c_int(ws.max_rows), c_int(full.shape[1]), c_int(kk), nv.ptr(tile_expert),
+                                             c_int(gemm.ACT.get(act, 0)), c_int(0), nv.ptr(status), st), "omni_gemm_bf16_grouped")
+        if act == "swiglu":
+            fused.silu_mul(full, out=c)
     else:
-        nv.check_rc(g.omni_gemm_bf16_grouped_compact(nv.ptr(a), c_int(lda), nv.ptr(w), c_int(w.shape[0]), nv.ptr(c), c_int(ldc),
-                                                     c_int(ws.max_rows), c_int(n), c_int(kk), nv.ptr(tile_expert),
-                                                     nv.ptr(ws.tile_row0), nv.ptr(ws.tile_rows), c_int(ws.max_tiles),
-                                                     c_int(act), c_int(0), nv.ptr(status), st),
-                    "omni_gemm_bf16_grouped_compact")
+        nv.check_rc(g.omni_gemm_bf16_experts(nv.ptr(a), c_int(a.stride(0)), nv.ptr(w), c_int(w.shape[0]), nv.ptr(c), c_int(c.stride(0)),
+                                             c_int(ws.max_rows), c_int(n), c_int(kk), nv.ptr(tile_expert), nv.ptr(ws.tile_row0),
+                                             nv.ptr(ws.tile_rows), c_int(ws.max_tiles), c_int(ws.tile_cap),
+                                             c_int({None: 0, "relu2": 3, "swiglu": 5}[act]), nv.ptr(status), st), "omni_gemm_bf16_experts")
 
 
 def _plan_and_dispatch(ws, x, E, e_lo, e_hi, k):
@@ -169,10 +178,10 @@ def _plan_and_dispatch(ws, x, E, e_lo, e_hi, k):
                                       c_int(ws.max_tiles), nv.ptr(ws.row_of_pair), nv.ptr(ws.tile_expert),
                                       nv.ptr(ws.offsets), nv.ptr(ws.n_rows), st), "omni_moe_plan")
     else:
-        nv.check_rc(lib.omni_moe_plan_compact(nv.ptr(ws.ids), c_int(T * k), c_int(E), c_int(e_lo), c_int(e_hi),
-                                              c_int(ws.max_tiles), nv.ptr(ws.row_of_pair), nv.ptr(ws.tile_expert),
+        nv.check_rc(lib.omni_moe_plan_tiles(nv.ptr(ws.ids), c_int(T * k), c_int(E), c_int(e_lo), c_int(e_hi),
+                                              c_int(ws.tile_cap), c_int(ws.max_tiles), nv.ptr(ws.row_of_pair), nv.ptr(ws.tile_expert),
                                               nv.ptr(ws.tile_row0), nv.ptr(ws.tile_rows), nv.ptr(ws.n_rows), st),
-                    "omni_moe_plan_compact")
+                    "omni_moe_plan_tiles")
     nv.check_rc(lib.omni_moe_dispatch(nv.ptr(x), c_long(x.stride(0)), nv.ptr(ws.row_of_pair), c_int(T * k), c_int(k),
                                       c_int(D), nv.ptr(ws.xp), st), "omni_moe_dispatch")
 
@@ -302,12 +311,8 @@ def expert_rows(x, router_w, router_b, router: Router, up, down, act: str, ws: M
         _few_rows(ws, ws.h, 1, down, ws.y, None)
         return ExpertRows(ws.y, ws.row_of_pair, ws.weights)
     _plan_and_dispatch(ws, x, experts, 0, experts, k)
-    if act == "swiglu":
-        _grouped(ws, ws.xp, D, up, ws.h13, 2 * Fd, 2 * Fd, D, ws.tile_expert)
-        fused.silu_mul(ws.h13, out=ws.h)
-    else:
-        _grouped(ws, ws.xp, D, up, ws.h, Fd, Fd, D, ws.tile_expert, gemm.ACT[act])
-    _grouped(ws, ws.h, Fd, down, ws.y, D, D, Fd, ws.tile_expert)
+    _grouped(ws, ws.xp, up, ws.h, ws.tile_expert, act)
+    _grouped(ws, ws.h, down, ws.y, ws.tile_expert)
     return ExpertRows(ws.y, ws.row_of_pair, ws.weights)
 
 
@@ -351,13 +356,11 @@ def moe_forward(x, router_logits, w13, w2, k, renorm=True, e_lo=0, e_hi=None, ws
     else:
         _route(router_logits, T, E, k, renorm, ws)
         _plan_and_dispatch(ws, x, E, e_lo, e_hi, k)
-        # tile_expert holds GLOBAL expert ids; the local weight tensors start at e_lo
         te = ws.tile_expert
-        if e_lo:
+        if e_lo and ws.padded:                             # GLOBAL expert ids; the local weight tensors start at e_lo
             te = torch.where(te >= 0, te - e_lo, te)
-        _grouped(ws, ws.xp, D, w13, ws.h13, 2 * Fd, 2 * Fd, D, te)
-        fused.silu_mul(ws.h13, out=ws.h)
-        _grouped(ws, ws.h, Fd, w2, ws.y, D, D, Fd, te)
+        _grouped(ws, ws.xp, w13, ws.h, te, "swiglu")
+        _grouped(ws, ws.h, w2, ws.y, te)
     if scatter is not None:
         per, ptrs = scatter
         arr = (ctypes.c_void_p * len(ptrs))(*ptrs)
