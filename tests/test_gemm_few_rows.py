@@ -56,3 +56,18 @@ def test_epilogue(rows, act):
                 out_batch_stride=joint.stride(0))
     assert torch.equal(joint[:, 1:1 + rows // 2].reshape(rows, n), out) and (joint[:, 0] == 0).all() and (joint[:, 1 + rows // 2:] == 0).all()
     nv.check_status()
+
+
+@pytest.mark.parametrize("rows", [1, 8, 9, 16])
+@pytest.mark.parametrize("per_sm", [1, 2, 3, 3.5, 4, 4.5, 6, 8])
+def test_splits_of_at_most_16_rows(rows, per_sm):
+    """Every split of csrc/gemm_skinny.cuh's launch_rows, at and just past its limits in 16-column tiles per SM."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for n in (int(per_sm * sms) * 16, int(per_sm * sms) * 16 + 8):
+        for k in (72, 1032):
+            g = torch.Generator(device="cuda").manual_seed(rows + n + k)
+            rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+            x, w, b, res = rnd(rows, k), rnd(n, k), rnd(n), rnd(rows, n)
+            y = gemm.linear(x, w, b, residual=res)
+            _check(y, x.double() @ w.double().T + b.double() + res.double(), x.double().abs() @ w.double().abs().T)
+    nv.check_status()

@@ -79,15 +79,15 @@ __device__ __forceinline__ void skinny_finish(float (&x)[B], int m, int step, in
 }
 
 // ---------------------------------------------------------------------------------------------------- at most 16 rows
-// NT * 8 rows of A; 16 resident warps x 8 chunks x 1 KB = 128 KB of W in flight per SM.
-template <int NT, int NW>
-__global__ void __launch_bounds__(32 * NW, NW == 16 ? 1 : 2)
+// NT * 8 rows of A; 16 resident warps x U chunks x 1 KB = up to 128 KB of W in flight per SM.
+template <int NT, int NW, int U, int BLOCKS>
+__global__ void __launch_bounds__(32 * NW, BLOCKS)
 gemm_rows_kernel(const __nv_bfloat16* __restrict__ A, int lda, const __nv_bfloat16* __restrict__ W, int ldw, __nv_bfloat16* C, int ldc,
                  int M, int N, int K, const __grid_constant__ GemmEpilogue epi) {
   __shared__ float part[NW][NT * 8][16];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, j = lane & 3;
   const int n0 = blockIdx.x * 16;
-  if (blockIdx.x < 2 * 148) {              // W does not come from the kernel before: the first blocks' share is on its way to L2 meanwhile
+  if (blockIdx.x < BLOCKS * 148) {              // W does not come from the kernel before: the first blocks' share is on its way to L2 meanwhile
     const __nv_bfloat16* w = W + (size_t)min(n0 + (int)(threadIdx.x & 15), N - 1) * ldw;
     for (int c = (threadIdx.x >> 4) * 64; c < K; c += 2 * NW * 64) prefetch_l2(w + c);
   }
@@ -101,22 +101,46 @@ gemm_rows_kernel(const __nv_bfloat16* __restrict__ A, int lda, const __nv_bfloat
     for (int i = 0; i < 4; ++i) acc[t][i] = 0.f;
   }
   // columns past N repeat the last one and are not stored
-  few_rows_products<NT, NW, NT == 1 ? 8 : 4>(acc, W + (size_t)min(n0 + g, N - 1) * ldw, W + (size_t)min(n0 + 8 + g, N - 1) * ldw, x, K, warp, j);
+  few_rows_products<NT, NW, U>(acc, W + (size_t)min(n0 + g, N - 1) * ldw, W + (size_t)min(n0 + 8 + g, N - 1) * ldw, x, K, warp, j);
 #pragma unroll
   for (int t = 0; t < NT; ++t)
 #pragma unroll
     for (int i = 0; i < 4; ++i) part[warp][t * 8 + j * 2 + (i & 1)][g + 8 * (i >> 1)] = acc[t][i];
   __syncthreads();
-  if (threadIdx.x < NT * 128) {
-    const int n = n0 + (threadIdx.x & 15), m = threadIdx.x >> 4;
+#pragma unroll
+  for (int e = threadIdx.x; e < NT * 128; e += 32 * NW) {
+    const int n = n0 + (e & 15), m = e >> 4;
     if (n < N && m < M) {
       const float bias = epi.bias ? __bfloat162float(epi.bias[n]) : 0.f;
       float y[1] = {0.f};
 #pragma unroll
-      for (int w = 0; w < NW; ++w) y[0] += part[w][m][threadIdx.x & 15];
+      for (int w = 0; w < NW; ++w) y[0] += part[w][m][e & 15];
       skinny_finish<1>(y, m, 1, M, n, C, ldc, epi, bias);
     }
   }
+}
+
+// How a tile's contraction is split over warps (NW), loads in flight per warp (U) and blocks on an SM, by the number of 16-column
+// tiles per SM.  Measured with 8 and 16 rows in us, streaming the weights from memory:
+//   up to one    a block of 16 warps, so that a long contraction still is one or two rounds of loads: 2048 x 9216 12.7 / 15.2 with
+//                8 warps, 9.8 / 11.0 with 16; a contraction of at most 1024 is one round with 8 warps, 2.6 / 2.6 against 2.9 / 2.9
+//   two to three three blocks of 8 with half the loads, since two blocks would leave a second round that is nearly empty:
+//                6144 x 4096 14.0 / 17.4 with two blocks, 11.4 / 14.3 with three; 5120 x 2048 7.0 / 9.7 and 6.2 / 7.4
+//   more, 9 rows and up: four blocks of 4 warps where their last round is at least half full (24576 x 4096 46.1 with two blocks
+//                of 8, 42.1 with four of 4; 9216 x 2048 10.2 and 9.2), not where it is emptier (12288 x 4096 25.3 and 27.8)
+//   else         two blocks of 8 (8 rows, 32768 x 4096: 46.2; four of 4 48.0, three of 8 47.9; the copy rate would be 40.4)
+template <int NT>
+static void launch_rows(int tiles, const __nv_bfloat16* A, int lda, const __nv_bfloat16* W, int ldw, __nv_bfloat16* C, int ldc, int M,
+                        int N, int K, const GemmEpilogue& epi, cudaStream_t stream) {
+  constexpr int U = NT == 1 ? 8 : 4;
+  const int sms = sm_count(), last = tiles % (4 * sms);
+  const auto go = [&](auto kernel, int warps) {
+    launch_overlapped(kernel, tiles, 32 * warps, 0, stream, A, lda, W, ldw, C, ldc, M, N, K, epi);
+  };
+  if (tiles <= sms && K > 1024) go(gemm_rows_kernel<NT, 16, U, 1>, 16);
+  else if (tiles > 2 * sms && tiles <= 3 * sms) go(gemm_rows_kernel<NT, 8, U / 2, 3>, 8);
+  else if (NT == 2 && tiles > 3 * sms && (last == 0 || last >= 2 * sms)) go(gemm_rows_kernel<NT, 4, U, 4>, 4);
+  else go(gemm_rows_kernel<NT, 8, U, 2>, 8);
 }
 
 static int launch_rows(const void* A, int lda, const void* W, int ldw, __nv_bfloat16* C, int ldc, int M, int N, int K,
@@ -124,15 +148,8 @@ static int launch_rows(const void* A, int lda, const void* W, int ldw, __nv_bflo
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15) return RC_BAD_ARG;
   const auto a = static_cast<const __nv_bfloat16*>(A), w = static_cast<const __nv_bfloat16*>(W);
   const int tiles = (N + 15) / 16;
-  // one block per SM: 16 warps, so that a long contraction still is one or two rounds of loads; else two blocks of 8
-  const bool wide = tiles <= sm_count() && K > 1024;
-  if (M <= 8) {
-    if (wide) launch_overlapped(gemm_rows_kernel<1, 16>, tiles, 512, 0, stream, a, lda, w, ldw, C, ldc, M, N, K, epi);
-    else launch_overlapped(gemm_rows_kernel<1, 8>, tiles, 256, 0, stream, a, lda, w, ldw, C, ldc, M, N, K, epi);
-  } else {
-    if (wide) launch_overlapped(gemm_rows_kernel<2, 16>, tiles, 512, 0, stream, a, lda, w, ldw, C, ldc, M, N, K, epi);
-    else launch_overlapped(gemm_rows_kernel<2, 8>, tiles, 256, 0, stream, a, lda, w, ldw, C, ldc, M, N, K, epi);
-  }
+  if (M <= 8) launch_rows<1>(tiles, a, lda, w, ldw, C, ldc, M, N, K, epi, stream);
+  else launch_rows<2>(tiles, a, lda, w, ldw, C, ldc, M, N, K, epi, stream);
   return (int)cudaGetLastError();
 }
 
