@@ -8,8 +8,11 @@
 //   weights  each CTA of a pair holds half of the TN output channels' weights and the pair's MMA reads both
 // A channel block of which only some channels exist (96 = 64 + 32) issues the K steps that hold any.  Per 64 channels and three taps
 // a CTA takes in 18 KB + 3 * 64 * TN bytes, 0.35 of the one-CTA kernel's 2 * 3 * (16 KB + 128 * TN) / 2 at TN = 96.
-// With residual, one-CTA kernel before: 1024 x 1024 pixels, 96 -> 96 channels 268 us (461), 192 -> 96 317 us (662), 96 -> 8 145 us (743);
+// With residual, one-CTA kernel before: 1024 x 1024 pixels, 96 -> 96 channels 211 us (461), 192 -> 96 257 us (662), 96 -> 8 127 us (743);
 // 512 x 512, 192 -> 192 160 us (193), 384 -> 192 221 us (350); 256 x 256, 384 -> 384 119 us (180).
+// Up to 96 output channels the epilogue was what a tile waited for (16 -> 96 took as long as 96 -> 96): a lane's 16 bytes at the pitch of a
+// pixel fill half a sector.  Results and residuals therefore move as boxes by TMA: 268 -> 211 us, 317 -> 257 us, 145 -> 127 us in the order
+// above.  Wider outputs have MMAs enough to hide it behind and no shared memory to spare.
 #pragma once
 
 namespace omni {
@@ -21,14 +24,16 @@ template <int TN>
 struct Conv3Cfg {
   static constexpr int B_BYTES = (TN / 2) * 128;         // one tap's weights of this CTA's half
   static constexpr int STAGE_BYTES = C3_A_BYTES + 3 * B_BYTES;
-  static constexpr int STAGES = 220 * 1024 / STAGE_BYTES < 6 ? 220 * 1024 / STAGE_BYTES : 6;
-  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024;
+  static constexpr bool STAGED = TN <= 96;               // results leave, and the residual arrives, by TMA through shared memory
+  static constexpr int OUT_BYTES = STAGED ? TN * 2 * C3_W * C3_H : 0;        // a tile's outputs, two of them
+  static constexpr int FIT = (220 * 1024 - 2 * OUT_BYTES) / STAGE_BYTES, STAGES = FIT < 6 ? FIT : 6;
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 2 * OUT_BYTES + 1024;
   static constexpr int ACC_STRIDE = TN <= 32 ? 32 : (TN <= 64 ? 64 : (TN <= 128 ? 128 : 256));
   static constexpr int TMEM_COLS = 2 * ACC_STRIDE;
 };
 
 struct Conv3Args {
-  CUtensorMap tmX, tmW;
+  CUtensorMap tmX, tmW, tmY, tmR;         // Y, residual: 32 channels of a tile
   __nv_bfloat16* y;
   int ldy;
   int H, W, n_img, tiles_x, tiles_y;      // tiles of 16 x 8 pixels
@@ -42,6 +47,38 @@ __device__ __forceinline__ void add8(float (&f)[8], const uint4& u) {
   f[4] += c.x; f[5] += c.y; f[6] += d.x; f[7] += d.y;
 }
 
+__device__ __forceinline__ void conv3_finish(float (&f)[8], const GemmEpilogue& epi, int col) {
+  if (epi.bias) add8(f, *reinterpret_cast<const uint4*>(epi.bias + col));
+  if (epi.act == ACT_GELU_TANH) {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) f[e] = gelu_tanh(f[e]);
+  } else if (epi.act == ACT_SILU) {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) f[e] = silu(f[e]);
+  } else if (epi.act == ACT_RELU2) {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) f[e] = fmaxf(f[e], 0.f) * fmaxf(f[e], 0.f);
+  }
+}
+
+__device__ __forceinline__ uint4 lds128(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ void sts128(uint32_t addr, const uint4& v) {
+  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+__device__ __forceinline__ void tma_store_4d(const CUtensorMap* tmap, uint32_t src, int c0, int c1, int c2, int c3) {
+  asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
+               :
+               : "l"(reinterpret_cast<uint64_t>(tmap)), "r"(src), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+               : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
 template <int TN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
 conv3x3_pair_kernel(const __grid_constant__ Conv3Args a, int* status) {
@@ -52,6 +89,7 @@ conv3x3_pair_kernel(const __grid_constant__ Conv3Args a, int* status) {
   __shared__ __align__(8) uint64_t empty_bar[STAGES];
   __shared__ __align__(8) uint64_t tfull_bar[2];
   __shared__ __align__(8) uint64_t tempty_bar[2];
+  __shared__ __align__(8) uint64_t res_bar[2];
   __shared__ uint32_t tmem_base_s;
   __shared__ int s_abort;
 
@@ -71,7 +109,8 @@ conv3x3_pair_kernel(const __grid_constant__ Conv3Args a, int* status) {
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&tfull_bar[i]), 1);
-      mbar_init(smem_u32(&tempty_bar[i]), 16);
+      mbar_init(smem_u32(&tempty_bar[i]), Cfg::STAGED ? 8 : 16);
+      mbar_init(smem_u32(&res_bar[i]), 1);
     }
     fence_mbar_init();
     tma_prefetch_desc(&a.tmX);
@@ -152,9 +191,71 @@ conv3x3_pair_kernel(const __grid_constant__ Conv3Args a, int* status) {
         if (acc == 0) acc_phase ^= 1;
       }
     }
+  } else if constexpr (Cfg::STAGED) {
+    // A tile of few channels is over in 1 to 3 us, less than one epilogue takes from the accumulator to memory: four warps have the even
+    // tiles and four the odd ones.  A pixel's channels are a row of their own in memory, so each group of 32 channels goes out, and its
+    // residual comes in a tile ahead, as one box through shared memory (64 bytes per pixel, swizzled: no bank conflicts).
+    constexpr int GROUPS = TN / 32;
+    const int q = warp & 3, mine = (warp - 2) >> 2, r = q * 32 + lane;
+    const uint32_t buf = smem_base + STAGES * Cfg::STAGE_BYTES + mine * Cfg::OUT_BYTES;
+    const bool leader = q == 2 && lane == 0;                // warps 2 and 6
+    const uint32_t swizzle = (r >> 1) & 3;
+    auto fetch_residual = [&](int t) {
+      int nb, img, y0, x0;
+      place(t, nb, img, y0, x0);
+      const int groups = min(GROUPS, (a.Cout - nb * TN + 31) / 32);
+      mbar_expect_tx(smem_u32(&res_bar[mine]), groups * (Cfg::OUT_BYTES / GROUPS));
+      for (int g = 0; g < groups; ++g)
+        tma_load_4d(buf + g * (Cfg::OUT_BYTES / GROUPS), &a.tmR, smem_u32(&res_bar[mine]), nb * TN + g * 32, x0, y0, img);
+    };
+    uint32_t phase = 0;
+    int t = pair + mine * num_pairs;
+    if (leader && a.epi.residual && t < num_tiles) fetch_residual(t);
+    for (; t < num_tiles; t += 2 * num_pairs, phase ^= 1) {
+      int nb, img, y0, x0;
+      place(t, nb, img, y0, x0);
+      if (a.epi.residual) mbar_wait(smem_u32(&res_bar[mine]), phase, &s_abort, status, ERR_WAIT_FULL);
+      mbar_wait(smem_u32(&tfull_bar[mine]), phase, &s_abort, status, ERR_WAIT_TMEM_FULL);
+      tc_fence_after_sync();
+#pragma unroll
+      for (int g = 0; g < GROUPS; ++g) {
+        uint32_t v[32];
+        tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + mine * Cfg::ACC_STRIDE + g * 32, v);
+        tmem_wait_ld();
+        if (g == GROUPS - 1) {                              // the accumulator is read: the next but one tile may have it
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&tempty_bar[mine]), 0));
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const int col = nb * TN + g * 32 + c * 8;
+          if (col >= a.Cout) break;
+          const uint32_t at = buf + g * (Cfg::OUT_BYTES / GROUPS) + r * 64 + ((c ^ swizzle) << 4);
+          float f[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(v[c * 8 + e]);
+          conv3_finish(f, a.epi, col);
+          if (a.epi.residual) add8(f, lds128(at));
+          sts128(at, make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7])));
+        }
+      }
+      fence_proxy_async_smem();
+      asm volatile("bar.sync %0, 128;" ::"r"(1 + mine) : "memory");
+      if (leader) {
+        if ((t / num_n) * 2 + (int)rank < m_tiles)
+          for (int g = 0; g < GROUPS && nb * TN + g * 32 < a.Cout; ++g)
+            tma_store_4d(&a.tmY, buf + g * (Cfg::OUT_BYTES / GROUPS), nb * TN + g * 32, x0, y0, img);
+        bulk_commit();
+        bulk_wait_read();
+        if (a.epi.residual && t + 2 * num_pairs < num_tiles) fetch_residual(t + 2 * num_pairs);
+      }
+      __syncwarp();
+      asm volatile("bar.sync %0, 128;" ::"r"(1 + mine) : "memory");          // the buffer is free
+    }
+    if (leader) bulk_wait_all();
   } else {
-    // A tile of few channels is over in 2 us, less than an epilogue that waits for its residual and writes it takes: the residual is
-    // requested while the MMAs of the tile run.
+    // the residual is requested while the MMAs of the tile run
     constexpr int CH = TN / 32;                             // 16-column chunks per warp: half of the tile's columns
     const int q = warp & 3, first = ((warp - 2) >> 2) * (TN / 2);
     int acc = 0;
@@ -195,17 +296,7 @@ conv3x3_pair_kernel(const __grid_constant__ Conv3Args a, int* status) {
           float f[8];
 #pragma unroll
           for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(v[g * 8 + e]);
-          if (a.epi.bias) add8(f, *reinterpret_cast<const uint4*>(a.epi.bias + cc));
-          if (a.epi.act == ACT_GELU_TANH) {
-#pragma unroll
-            for (int e = 0; e < 8; ++e) f[e] = gelu_tanh(f[e]);
-          } else if (a.epi.act == ACT_SILU) {
-#pragma unroll
-            for (int e = 0; e < 8; ++e) f[e] = silu(f[e]);
-          } else if (a.epi.act == ACT_RELU2) {
-#pragma unroll
-            for (int e = 0; e < 8; ++e) f[e] = fmaxf(f[e], 0.f) * fmaxf(f[e], 0.f);
-          }
+          conv3_finish(f, a.epi, cc);
           if (a.epi.residual) add8(f, res[c][g]);
           *reinterpret_cast<uint4*>(a.y + row * a.ldy + cc) =
               make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
@@ -227,11 +318,27 @@ conv3x3_pair_kernel(const __grid_constant__ Conv3Args a, int* status) {
   if (warp == 1) tmem_dealloc_pair(tmem_base, Cfg::TMEM_COLS);
 }
 
+static int conv3_out_map(CUtensorMap* map, const Conv3Args& a, const void* p, int ld) {
+  EncodeTiledFn enc = get_encode_tiled();
+  if (!enc) return RC_NO_DRIVER;
+  if (reinterpret_cast<uintptr_t>(p) & 15) return RC_BAD_ARG;
+  const cuuint64_t px = (cuuint64_t)ld * 2;
+  cuuint64_t gdim[4] = {(cuuint64_t)a.Cout, (cuuint64_t)a.W, (cuuint64_t)a.H, (cuuint64_t)a.n_img}, gstr[3] = {px, px * a.W, px * a.W * a.H};
+  cuuint32_t box[4] = {32, C3_W, C3_H, 1}, estr[4] = {1, 1, 1, 1};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(p), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? RC_OK : RC_TMAP;
+}
+
 template <int TN>
 static int launch_conv3(Conv3Args& a, const void* w, int pairs, int* status, cudaStream_t stream) {
   using Cfg = Conv3Cfg<TN>;
   const uint64_t K = 9ull * a.cin_blocks * 64;
   if (int rc = make_tmap_2d(&a.tmW, w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)a.Cout, K, K * 2, TN / 2, 64)) return rc;
+  if (Cfg::STAGED) {
+    if (int rc = conv3_out_map(&a.tmY, a, a.y, a.ldy)) return rc;
+    if (a.epi.residual)
+      if (int rc = conv3_out_map(&a.tmR, a, a.epi.residual, a.epi.ldr)) return rc;
+  }
   static unsigned long long prepared = 0;
   if (int e = ensure_dynamic_smem((const void*)conv3x3_pair_kernel<TN>, Cfg::SMEM_BYTES, prepared)) return e;
   const long tiles = (long)((a.n_img * a.tiles_x * a.tiles_y + 1) / 2) * ((a.Cout + TN - 1) / TN);
