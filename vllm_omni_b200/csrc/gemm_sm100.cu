@@ -13,6 +13,10 @@
 //                            the M=256 MMAs.  Used whenever the problem fills a wave of such tiles;
 //                            one launch can carry two problems of the same (N, K).
 //
+// Beside them, in headers of their own: linear layers of at most 128 rows (gemm_skinny.cuh), 3 x 3
+// convolutions on CTA pairs (conv_pair.cuh) and the GEMM of all experts over rows that sit back to
+// back (moe_gemm.cuh).
+//
 // Roles inside a CTA (both kernels):
 //   warp 0    TMA producer: cp.async.bulk.tensor loads of the A / W k-blocks (128-byte
 //             swizzle) into a multi-stage shared-memory ring, completion on mbarriers
