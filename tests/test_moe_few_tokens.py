@@ -136,3 +136,20 @@ def test_even_plan(n_pairs, E, lo, hi, tile):
             assert r0 == at and 1 <= rn <= tile and (of_row[r0:r0 + rn] == e).all()
             at += rn
     assert at == of_row.numel() == int(n)
+
+
+@pytest.mark.parametrize("T,D", [(1, 2048), (3, 72), (70, 264), (5, 8192), (2, 8184)])
+def test_norm_of_the_result(T, D):
+    """The combining launch with the next norm: the same rows, and their norm against 64 bits."""
+    from vllm_omni_b200.ops import fused
+    E, k, Fd = 8, 2, 40
+    x, logits, w13, w2 = _problem(T, E, k, D, Fd, False)
+    res, gain = torch.randn(T, D, device="cuda").bfloat16(), torch.randn(D, device="cuda").bfloat16()
+    plain = moe_forward(x, logits, w13, w2, k, residual=res)
+    xn = x.clone()
+    y = moe_forward(xn, logits, w13, w2, k, residual=res, norm=(gain, 1e-6, xn))         # into its own input
+    assert torch.equal(y, plain)
+    ref = y.double() * torch.rsqrt(y.double().pow(2).mean(-1, keepdim=True) + 1e-6) * gain.double()
+    # one rounding to bf16; fp32 sums of at most 8192 squares and rsqrtf (2 ulp)
+    assert ((xn.double() - ref).abs() <= ref.abs() * (2.0 ** -8 + 1e-4) + 1e-30).all()
+    nv.check_status()

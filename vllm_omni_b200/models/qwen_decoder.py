@@ -363,8 +363,11 @@ class QwenDecoderModel(nn.Module):
         xn = torch.empty_like(x)
         attn = torch.empty(T, H * Dh, dtype=x.dtype, device=x.device)
         tp_cap = max(64, 1 << (T - 1).bit_length())          # peer-buffer bucket of the row-parallel reduces
+        normed = False                                       # xn already holds the norm that comes next
         for li, layer in enumerate(self.layers):
-            fused.norm_modulate(x, weight=layer.input_layernorm, rms=True, eps=cfg.rms_norm_eps, out=xn)
+            if not normed:
+                fused.norm_modulate(x, weight=layer.input_layernorm, rms=True, eps=cfg.rms_norm_eps, out=xn)
+            normed = False
             qkv = layer.qkv_proj(xn)
             kc, vc = kv_caches[li] if kv_caches is not None else (None, None)
             fused.qk_norm_rope_(qkv.view(1, T, -1), H, Hkv, Dh, wq=layer.q_norm, wk=layer.k_norm, cos=cos, sin=sin,
@@ -385,8 +388,11 @@ class QwenDecoderModel(nn.Module):
                     g = torch.sigmoid(xn.float() @ layer.shared_expert_gate.float().t())
                     shared = layer.shared_down(fused.silu_mul(layer.shared_gate_up(xn))).float().mul_(g)
                 if self.ep_group is None or self.ep_group.world_size == 1:
+                    # where nothing else is added to the rows, the next norm leaves the combining launch with them
+                    normed = shared is None and (deepstack is None or li >= len(deepstack))
+                    gain = self.layers[li + 1].input_layernorm if li + 1 < len(self.layers) else self.norm
                     moe_forward(xn, logits, layer.w13, layer.w2, cfg.num_experts_per_tok, cfg.norm_topk_prob,
-                                ws=layer.moe_ws, residual=x, out=x)
+                                ws=layer.moe_ws, residual=x, out=x, norm=(gain, cfg.rms_norm_eps, xn) if normed else None)
                 elif self.ep_reduce is not None and self.ep_reduce.mode == "peer" and x.is_cuda:
                     # combine stores each token's partial sum into its row owner's peer slot; the
                     # owners reduce locally, add the residual and push the rows to every rank
@@ -414,7 +420,7 @@ class QwenDecoderModel(nn.Module):
                 x.add_(deepstack[li].to(x.dtype))
             if (li + 1) in capture_layers:
                 captured[li + 1] = x.clone()
-        hidden = fused.norm_modulate(x, weight=self.norm, rms=True, eps=cfg.rms_norm_eps)
+        hidden = xn if normed else fused.norm_modulate(x, weight=self.norm, rms=True, eps=cfg.rms_norm_eps)
         return hidden, captured
 
     def compute_logits(self, hidden: torch.Tensor) -> torch.Tensor:

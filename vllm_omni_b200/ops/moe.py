@@ -17,7 +17,7 @@ import torch.nn.functional as F
 from . import _native as nv
 from . import fused, gemm
 
-c_int, c_long = ctypes.c_int, ctypes.c_long
+c_int, c_long, c_float = ctypes.c_int, ctypes.c_long, ctypes.c_float
 
 
 def moe_route_reference(logits, k, renorm=True):
@@ -317,14 +317,16 @@ def expert_rows(x, router_w, router_b, router: Router, up, down, act: str, ws: M
 
 
 def moe_forward(x, router_logits, w13, w2, k, renorm=True, e_lo=0, e_hi=None, ws: MoEWorkspace | None = None,
-                residual=None, out=None, scatter=None):
+                residual=None, out=None, scatter=None, norm=None):
     """x [T, D] bf16, router_logits [T, E] bf16, w13 [E_local, 2F, D], w2 [E_local, D, F] (the
     local experts [e_lo, e_hi) of E = router_logits.shape[1]).
 
     ``scatter = (rows_per_owner, ptrs)`` (GPU, expert parallel): instead of returning the partial
     sum of the local experts, store token t's partial into ``ptrs[t // rows_per_owner]`` (peer
     memory of the rank that owns that block of rows) at local row ``t % rows_per_owner``; the
-    cross-rank sum is finished by ``parallel.tensor_parallel.RowParallelReduce.reduce_from``."""
+    cross-rank sum is finished by ``parallel.tensor_parallel.RowParallelReduce.reduce_from``.
+
+    ``norm = (gain, eps, normed)``: the RMS norm of the result as well, into ``normed`` [T, D] (which may be ``x``)."""
     T, D = x.shape
     E = router_logits.shape[1]
     e_hi = E if e_hi is None else e_hi
@@ -343,8 +345,9 @@ def moe_forward(x, router_logits, w13, w2, k, renorm=True, e_lo=0, e_hi=None, ws
             y += residual.float()
         y = y.to(x.dtype)
         if out is not None:
-            out.copy_(y)
-            return out
+            y = out.copy_(y)
+        if norm is not None:
+            fused.norm_modulate(y, weight=norm[0], rms=True, eps=norm[1], out=norm[2])
         return y
     ws = (ws or MoEWorkspace()).get(T, k, E, D, Fd, x.device, x.dtype)
     lib, st = nv.lib("moe"), nv.stream_ptr()
@@ -369,7 +372,13 @@ def moe_forward(x, router_logits, w13, w2, k, renorm=True, e_lo=0, e_hi=None, ws
         return None
     if out is None:
         out = torch.empty_like(x)
+    ldr = c_long(residual.stride(0) if residual is not None else 0)
+    if norm is not None:
+        gain, eps, normed = norm
+        nv.check_rc(lib.omni_moe_combine_norm(nv.ptr(ws.y), nv.ptr(ws.row_of_pair), nv.ptr(ws.weights), c_int(T), c_int(k), c_int(D),
+                                              nv.ptr(residual), ldr, nv.ptr(out), c_long(out.stride(0)), nv.ptr(gain), c_float(eps),
+                                              nv.ptr(normed), c_long(normed.stride(0)), st), "omni_moe_combine_norm")
+        return out
     nv.check_rc(lib.omni_moe_combine(nv.ptr(ws.y), nv.ptr(ws.row_of_pair), nv.ptr(ws.weights), c_int(T), c_int(k),
-                                     c_int(D), nv.ptr(residual), c_long(residual.stride(0) if residual is not None else 0),
-                                     nv.ptr(out), c_long(out.stride(0)), st), "omni_moe_combine")
+                                     c_int(D), nv.ptr(residual), ldr, nv.ptr(out), c_long(out.stride(0)), st), "omni_moe_combine")
     return out
