@@ -1,4 +1,4 @@
-"""Row kernels at the sizes where their layout changes: norms of more than 1024 channels (one block per row, or rings of rows), head
+"""Row kernels at the sizes where their layout changes: norms of more than 1024 channels (a block per row, or some warps per row), head
 norms with rotation of few and of many rows, with and without pages."""
 import pytest
 import torch
@@ -41,12 +41,22 @@ def test_norm_modulate(width, rows, rms):
 @pytest.mark.parametrize("heads,kv", [(32, 4), (3, 1), (24, 24)])
 @pytest.mark.parametrize("interleaved", [False, True])
 def test_head_norm_rotation_and_pages(rows, heads, kv, interleaved):
-    if rows == 1300 and heads == 3:
-        pytest.skip("the same path as the other head counts")
+    _heads_and_pages(rows, heads, kv, interleaved)
+
+
+# rows enough for a warp per row with every count: heads and pages that leave 0, 1, 2 and 6 of a step of 8 over (without pages
+# heads + kv, with them heads + 2 kv)
+@pytest.mark.parametrize("heads,kv", [(7, 1), (8, 1), (3, 1), (4, 2), (32, 1)])
+@pytest.mark.parametrize("interleaved,gains", [(False, True), (True, False)])
+def test_many_rows_and_head_counts_within_a_step(heads, kv, interleaved, gains):
+    _heads_and_pages(9501, heads, kv, interleaved, gains)
+
+
+def _heads_and_pages(rows, heads, kv, interleaved, gains=True):
     D, g = 128, _gen(rows + heads)
     rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
     qkv = rnd(1, rows, (heads + 2 * kv) * D).bfloat16()
-    wq, wk = (1 + 0.1 * rnd(2, D)).bfloat16()
+    wq, wk = (1 + 0.1 * rnd(2, D)).bfloat16() if gains else (None, None)
     ang = rnd(rows * 64 + 1) * 3
     cos, sin = ang[1:].cos().view(rows, 64), ang[:-1].sin().view(rows, 64).clone()
     if not interleaved:                                     # tables at an offset that no 16-byte load can take

@@ -349,17 +349,18 @@ qk_norm_rope128_rows_kernel(const __grid_constant__ HeadRows a, PeerWait wt, int
   rope_coefficients(a, row, s, l16, cs, sn);
   const int page = a.pages.k ? a.pages.slots[row] : -1;
   constexpr int U = 4;
+  // both halves of the warp take every step, whether or not their last heads exist: head_norm_rope exchanges values over the whole warp
 #pragma unroll 1
-  for (int h0 = hsel; h0 < all; h0 += 2 * U) {
+  for (int h0 = 0; h0 < all; h0 += 2 * U) {
     uint4 v[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int h = h0 + 2 * u;
+      const int h = h0 + 2 * u + hsel;
       v[u] = h < all ? *reinterpret_cast<const uint4*>(a.qkv + (size_t)row * a.ld + (size_t)h * 128 + l16 * 8) : make_uint4(0u, 0u, 0u, 0u);
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int h = h0 + 2 * u;
+      const int h = h0 + 2 * u + hsel;
       const uint4 o = head_norm_rope(v[u], a.wq != nullptr, h < a.H ? gq : gk, a.cosb != nullptr, a.interleaved, cs, sn, a.eps);
       if (h < all) store_head(a, row, h, l16, page, v[u], o);
     }
