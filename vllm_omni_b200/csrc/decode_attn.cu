@@ -94,16 +94,16 @@ paged_decode_kernel(const __grid_constant__ DecodeAttn p) {
     const __nv_bfloat16* k1 = p.k + (long)(b + row_in_half(t, 1, g)) * row + (long)hk * DA_D + j * 8;
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-      kr[0][c] = ldg_stream(k0 + c * 32);
-      kr[1][c] = ldg_stream(k1 + c * 32);
+      kr[0][c] = ld_stream(k0 + c * 32);
+      kr[1][c] = ld_stream(k1 + c * 32);
     }
   };
   auto load_v = [&](int t, int a, int b) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const __nv_bfloat16* v = p.v + (long)((i < 2 ? a : b) + row_in_half(t, i >> 1, 2 * j + (i & 1))) * row + (long)hk * DA_D + g * 8;
-      vr[i][0] = ldg_stream(v);
-      vr[i][1] = ldg_stream(v + 64);
+      vr[i][0] = ld_stream(v);
+      vr[i][1] = ld_stream(v + 64);
     }
   };
   int t = split * per + sub, pa = 0, pb = 0, na = 0, nb = 0;

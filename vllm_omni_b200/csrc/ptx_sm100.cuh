@@ -380,9 +380,11 @@ __device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&v
 }
 
 // ------------------------------------------------- few rows against streamed weights (mma.sync)
-__device__ __forceinline__ uint4 ldg_stream(const __nv_bfloat16* p) {   // read once: past L1
+// read once: past L1.  Not ld.global.nc, whose memory nothing may write while the kernel is resident: the kernel before may still be
+// writing it (keys in their pages, a W that is an activation) when this one waits in pdl_wait.
+__device__ __forceinline__ uint4 ld_stream(const __nv_bfloat16* p) {
   uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.L2::256B.v4.u32 {%0, %1, %2, %3}, [%4];"
+  asm volatile("ld.global.L1::no_allocate.L2::256B.v4.u32 {%0, %1, %2, %3}, [%4];"
                : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
   return v;
 }
@@ -406,8 +408,8 @@ __device__ __forceinline__ void few_rows_products(float (&acc)[NT][4], const __n
     for (int u = 0; u < U; ++u) {
       const int ch = c + u * 32 * NW + j * 8;
       const bool in = ch < K;
-      a[u][0] = in ? ldg_stream(w0 + ch) : zero;
-      a[u][1] = in ? ldg_stream(w1 + ch) : zero;
+      a[u][0] = in ? ld_stream(w0 + ch) : zero;
+      a[u][1] = in ? ld_stream(w1 + ch) : zero;
 #pragma unroll
       for (int t = 0; t < NT; ++t) b[u][t] = in && x[t] ? *reinterpret_cast<const uint4*>(x[t] + ch) : zero;
     }
