@@ -38,3 +38,23 @@ def test_against_64_bits(H, Hkv, bs, lens):
     out = torch.empty(n, H, D, device="cuda", dtype=torch.bfloat16)
     KC.paged_decode(q, k, v, tables.cuda(), torch.tensor(lens, dtype=torch.int32, device="cuda"), out=out, impl="stream")
     assert ((out.double() - ref).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("H,Hkv", [(8, 1), (16, 1)])
+@pytest.mark.parametrize("dead", [1, 16, 40, 99])
+def test_scores_of_minus_infinity(H, Hkv, dead):
+    """Keys whose scores are -inf at the head of a sequence, whole tiles and shares of them too, weigh nothing."""
+    D, n, L = 128, 3, 100
+    g = torch.Generator(device="cuda").manual_seed(dead)
+    q = torch.randn(n, H, D, generator=g, device="cuda").bfloat16()
+    q[..., 0] = q[..., 0].abs() + 0.25
+    k, v = (torch.randn(n * 7, 16, Hkv, D, generator=g, device="cuda").bfloat16() for _ in range(2))
+    k.view(n, 112, Hkv, D)[:, :dead, :, 0] = float("-inf")
+    tables = torch.arange(n * 7, dtype=torch.int32, device="cuda").view(n, 7)
+    out = KC.paged_decode(q, k, v, tables, torch.full((n,), L, dtype=torch.int32, device="cuda"))
+    kk, vv = (t.view(n, 112, Hkv, D)[:, :L].double().repeat_interleave(H // Hkv, 2) for t in (k, v))
+    w = torch.softmax(torch.einsum("nhd,nkhd->nhk", q.double(), kk) * D ** -0.5, -1)
+    ref = torch.einsum("nhk,nkhd->nhd", w, vv)
+    # as above: weights and result rounded to bf16
+    bound = torch.einsum("nhk,nkhd->nhd", w, vv.abs()) * 2.0 ** -8 + ref.abs() * 2.0 ** -8 + 1e-5
+    assert ((out.double() - ref).abs() <= bound).all()

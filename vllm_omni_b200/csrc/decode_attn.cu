@@ -129,6 +129,7 @@ paged_decode_kernel(const __grid_constant__ DecodeAttn p) {
     uint32_t pw[NH][2];
 #pragma unroll
     for (int u = 0; u < NH; ++u) {
+      const float before = m[u];
       float mx = -INFINITY;
 #pragma unroll
       for (int n = 0; n < 2; ++n)
@@ -140,9 +141,9 @@ paged_decode_kernel(const __grid_constant__ DecodeAttn p) {
         }
       mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
       mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-      const float top = fmaxf(m[u], mx);                       // finite: a tile holds at least one key
-      const float alpha = da_ex2(m[u] - top);
-      m[u] = top;
+      m[u] = fmaxf(m[u], mx);
+      const float top = m[u] == -INFINITY ? 0.f : m[u];        // only scores of -inf so far: all weights are zero
+      const float alpha = da_ex2(before - top);
       l[u] *= alpha;
 #pragma unroll
       for (int n = 0; n < 2; ++n) {
