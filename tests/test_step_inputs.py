@@ -69,3 +69,20 @@ def test_fill(n, mrope, overlay, seqs, monkeypatch):
         assert torch.equal(getattr(a, name), getattr(c, name)), name
     if seqs:
         assert torch.equal(a.seqs.state_in, c.seqs.state_in) and torch.equal(a.seqs.state_out, c.seqs.state_out)
+
+
+
+def 
+
+def test_rows_on_another_device_are_left_to_the_general_form():
+    """Given rows, their mask or positions in host memory: refused by the general form, never read by the kernel."""
+    from vllm_omni_b200.ops.step_inputs import token_rows
+    m, T = _decoder(False), 3
+    ids = pos = torch.arange(T, device="cuda")
+    given, mask, freq = torch.zeros(T, 136, dtype=torch.bfloat16), torch.ones(T, dtype=torch.bool), m.rope.freq_on(ids.device)
+    assert token_rows(ids, m.embed_tokens, pos, freq, None, given.cuda(), mask.cuda()) is not None
+    for kw in (dict(given=given), dict(given=given, mask=mask.cuda()), dict(given=given.cuda(), mask=mask)):
+        assert token_rows(ids, m.embed_tokens, pos, freq, None, **kw) is None
+    assert token_rows(ids, m.embed_tokens, pos.cpu(), freq) is None and token_rows(ids, m.embed_tokens, pos, freq.cpu()) is None
+    with pytest.raises(RuntimeError):
+        m.rows_and_rotation(ModelBatch(ids, pos, None, input_embeds=given, embeds_mask=mask))

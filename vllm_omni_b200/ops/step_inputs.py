@@ -64,7 +64,9 @@ def token_rows(ids, table, positions, freq, axis=None, given=None, mask=None):
     inside the table; angles positions * freq in fp32, frequency i by the position on axis[i] of ``positions`` [axes, T] (or [T]).
     None when an operand is not of a form the kernel takes."""
     T, (vocab, D) = ids.numel(), table.shape
-    if not (table.is_cuda and ids.is_cuda and positions.is_cuda and T and ids.dtype == positions.dtype == torch.int64 and ids.is_contiguous()
+    if not table.is_cuda or any(t is not None and t.device != table.device for t in (ids, positions, freq, axis, given, mask)):
+        return None
+    if not (T and ids.dtype == positions.dtype == torch.int64 and ids.is_contiguous()
             and table.is_contiguous() and positions.stride(-1) == 1 and positions.shape[-1] == T and (axis is None) == (positions.dim() == 1)
             and D * table.element_size() % 16 == 0 and table.data_ptr() % 16 == 0):
         return None
