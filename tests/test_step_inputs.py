@@ -86,3 +86,15 @@ def test_rows_on_another_device_are_left_to_the_general_form():
     assert token_rows(ids, m.embed_tokens, pos.cpu(), freq) is None and token_rows(ids, m.embed_tokens, pos, freq.cpu()) is None
     with pytest.raises(RuntimeError):
         m.rows_and_rotation(ModelBatch(ids, pos, None, input_embeds=given, embeds_mask=mask))
+
+
+
+def test_rotation_tables_are_fp32_whatever_the_default_type():
+    m, pos = _decoder(False), torch.arange(5, device="cuda")
+    want = m.rows_and_rotation(ModelBatch(pos, pos, None))
+    torch.set_default_dtype(torch.bfloat16)
+    try:
+        got = m.rows_and_rotation(ModelBatch(pos, pos, None))
+    finally:
+        torch.set_default_dtype(torch.float32)
+    assert all(a.dtype == b.dtype and torch.equal(a, b) for a, b in zip(want, got)) and got[1].dtype == torch.float32

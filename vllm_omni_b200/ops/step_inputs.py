@@ -75,7 +75,7 @@ def token_rows(ids, table, positions, freq, axis=None, given=None, mask=None):
         return None
     half = freq.numel()
     x = torch.empty(T, D, dtype=table.dtype, device=table.device)
-    cos, sin = torch.empty(2, T, half, device=table.device)
+    cos, sin = torch.empty(2, T, half, dtype=torch.float32, device=table.device)
     a, P = _Tokens(), lambda t: None if t is None else t.data_ptr()
     a.ids, a.table, a.given, a.mask, a.out, a.pos, a.freq, a.axis = P(ids), P(table), P(given), P(mask if given is not None else None), P(x), \
         P(positions), P(freq), P(axis)
