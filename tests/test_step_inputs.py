@@ -98,3 +98,19 @@ def test_rotation_tables_are_fp32_whatever_the_default_type():
     finally:
         torch.set_default_dtype(torch.float32)
     assert all(a.dtype == b.dtype and torch.equal(a, b) for a, b in zip(want, got)) and got[1].dtype == torch.float32
+
+
+
+def test_fill_takes_whole_rows_only():
+    """Only block tables may be narrower than the static tensor; narrower embeddings are refused as before."""
+    m, n = _decoder(False), 2
+    r = DecodeGraphRunner(m, [tuple(torch.zeros(8, 16, 1, 128, device="cuda", dtype=torch.bfloat16) for _ in range(2))], max_blocks=5, buckets=(2,))
+    i32 = lambda *s: torch.zeros(s, device="cuda", dtype=torch.int32)
+    b = ModelBatch(torch.zeros(n, device="cuda", dtype=torch.long), torch.zeros(n, device="cuda", dtype=torch.long), i32(n), [],
+                   decode_rows=torch.arange(n, device="cuda"), decode_block_tables=i32(n, 3), decode_seq_lens=i32(n))
+    st = r._bucket(n)
+    assert r._fill_once(st, b)
+    b.input_embeds = torch.zeros(n, 72, device="cuda", dtype=torch.bfloat16)
+    assert not r._fill_once(st, b)
+    with pytest.raises(RuntimeError):
+        r._fill(st, b)

@@ -92,7 +92,7 @@ class DecodeGraphRunner:
     def _fill_once(self, st: _Bucket, b: ModelBatch) -> bool:
         """``_fill`` as one launch; False where a tensor of the batch is not of a form it takes."""
         order = b.decode_rows
-        if not (order.is_cuda and order.dtype == torch.int64 and order.is_contiguous()):
+        if not (order.device == st.ids.device and order.dtype == torch.int64 and order.is_contiguous()):
             return False
         f, pos = StepFill(order.numel(), st.n), b.positions
         ok = f.put(st.ids, b.input_ids, True)
@@ -101,7 +101,7 @@ class DecodeGraphRunner:
                 ok = ok and f.put(st.pos[ax], pos if pos.dim() == 1 else pos[ax], True)
         else:
             ok = ok and f.put(st.pos, pos, True)
-        ok = ok and f.put(st.slots, b.slot_mapping, True, pad_ones=True) and f.put(st.tables, b.decode_block_tables, False) \
+        ok = ok and f.put(st.slots, b.slot_mapping, True, pad_ones=True) and f.put(st.tables, b.decode_block_tables, False, narrow=True) \
             and f.put(st.lens, b.decode_seq_lens, False)
         if st.seqs is not None:
             ok = ok and f.put(st.ctx, b.seqs.context, True)

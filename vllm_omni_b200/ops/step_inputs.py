@@ -34,8 +34,8 @@ class StepFill:
     def __init__(self, n: int, rows: int):
         self.a, self.n, self.rows, self.count, self.keep = _Fill(), n, rows, 0, []
 
-    def put(self, dst: torch.Tensor, src: torch.Tensor | None, ordered: bool, pad_ones: bool = False) -> bool:
-        """dst [rows] or [rows, c]; src the same with n rows and at most c columns (the rest of a row is zeroed)."""
+    def put(self, dst: torch.Tensor, src: torch.Tensor | None, ordered: bool, pad_ones: bool = False, narrow: bool = False) -> bool:
+        """dst [rows] or [rows, c]; src the same with n rows and c columns, or with ``narrow`` fewer (the rest of a row is zeroed)."""
         if self.count == _JOBS:
             return False
         j = self.a.jobs[self.count]
@@ -45,7 +45,7 @@ class StepFill:
             j.src, j.src_pitch, j.src_bytes = None, 0, 0
         else:
             if src.dtype != dst.dtype or src.device != dst.device or src.dim() != dst.dim() or src.shape[0] != self.n \
-                    or (src.dim() == 2 and (src.stride(1) != 1 or src.shape[1] > dst.shape[1])):
+                    or (src.dim() == 2 and (src.stride(1) != 1 or src.shape[1] > dst.shape[1] or (src.shape[1] < dst.shape[1] and not narrow))):
                 return False
             j.src, j.src_pitch, j.src_bytes = src.data_ptr(), src.stride(0) * size, (src.shape[1] if src.dim() == 2 else 1) * size
             self.keep.append(src)
