@@ -71,9 +71,6 @@ def test_fill(n, mrope, overlay, seqs, monkeypatch):
         assert torch.equal(a.seqs.state_in, c.seqs.state_in) and torch.equal(a.seqs.state_out, c.seqs.state_out)
 
 
-
-def 
-
 def test_rows_on_another_device_are_left_to_the_general_form():
     """Given rows, their mask or positions in host memory: refused by the general form, never read by the kernel."""
     from vllm_omni_b200.ops.step_inputs import token_rows
@@ -88,7 +85,6 @@ def test_rows_on_another_device_are_left_to_the_general_form():
         m.rows_and_rotation(ModelBatch(ids, pos, None, input_embeds=given, embeds_mask=mask))
 
 
-
 def test_rotation_tables_are_fp32_whatever_the_default_type():
     m, pos = _decoder(False), torch.arange(5, device="cuda")
     want = m.rows_and_rotation(ModelBatch(pos, pos, None))
@@ -98,7 +94,6 @@ def test_rotation_tables_are_fp32_whatever_the_default_type():
     finally:
         torch.set_default_dtype(torch.float32)
     assert all(a.dtype == b.dtype and torch.equal(a, b) for a, b in zip(want, got)) and got[1].dtype == torch.float32
-
 
 
 def test_fill_takes_whole_rows_only():
