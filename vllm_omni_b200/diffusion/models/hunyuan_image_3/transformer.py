@@ -37,7 +37,7 @@ from torch import nn
 from ....ops import conv as C
 from ....ops import fused
 from ....ops.attention import attention
-from ....ops.moe import MoEWorkspace, moe_forward
+from ....ops.moe import MoEScratch, MoEWorkspace, moe_forward
 from ...layers.linear import FusedLinear
 
 
@@ -243,7 +243,7 @@ class UNetUp(nn.Module):
 # decoder
 # ------------------------------------------------------------------------------------------------
 class HunyuanDecoderLayer(nn.Module):
-    def __init__(self, cfg: HunyuanImage3Config, li: int, dtype, device):
+    def __init__(self, cfg: HunyuanImage3Config, li: int, dtype, device, moe_scratch: MoEScratch):
         super().__init__()
         D, H, Hkv, Dh = cfg.hidden_size, cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim
         P = lambda *s: nn.Parameter(torch.ones(*s, dtype=dtype, device=device), requires_grad=False)
@@ -260,7 +260,7 @@ class HunyuanDecoderLayer(nn.Module):
             self.router = FusedLinear(D, E, bias=False, dtype=dtype, device=device)
             self.w13 = nn.Parameter(torch.empty(E, 2 * Fm, D, dtype=dtype, device=device).normal_(0, 0.02), requires_grad=False)
             self.w2 = nn.Parameter(torch.empty(E, D, Fm, dtype=dtype, device=device).normal_(0, 0.02), requires_grad=False)
-            self.moe_ws = MoEWorkspace()
+            self.moe_ws = MoEWorkspace(moe_scratch)
             Fs = cfg.intermediate_size * int(cfg.per_layer("num_shared_expert", li)) if cfg.use_mixed_mlp_moe else 0
         else:
             self.router = None
@@ -288,7 +288,8 @@ class HunyuanImage3Model(nn.Module):
         self.cfg, self.dtype_ = cfg, dtype
         self.wte = nn.Parameter(torch.empty(cfg.vocab_size, cfg.hidden_size, dtype=dtype, device=device).normal_(0, 0.02),
                                 requires_grad=False)
-        self.layers = nn.ModuleList([HunyuanDecoderLayer(cfg, i, dtype, device) for i in range(cfg.num_hidden_layers)])
+        moe_scratch = MoEScratch()
+        self.layers = nn.ModuleList([HunyuanDecoderLayer(cfg, i, dtype, device, moe_scratch) for i in range(cfg.num_hidden_layers)])
         self.ln_f = nn.Parameter(torch.ones(cfg.hidden_size, dtype=dtype, device=device), requires_grad=False)
         self.tp_group = None
         self.tp_reduce = None

@@ -180,7 +180,7 @@ class _Gated(nn.Module):
 
 
 class _Experts(nn.Module):
-    def __init__(self, cfg: MilivikConfig, m: ExpertsConfig, dtype, device):
+    def __init__(self, cfg: MilivikConfig, m: ExpertsConfig, dtype, device, scratch: moe.MoEScratch):
         super().__init__()
         self.m = m
         D, E, self.ff_p = cfg.padded_width, m.router.experts, round_up(m.ff, 8)
@@ -188,7 +188,7 @@ class _Experts(nn.Module):
         self.up = _zeros(E, 2 * self.ff_p, D, dtype=dtype, device=device)
         self.down = _zeros(E, D, self.ff_p, dtype=dtype, device=device)
         self.shared = _Gated(cfg, m.shared_ff, dtype, device, extra=True) if m.shared_ff else None
-        self.ws = moe.MoEWorkspace()
+        self.ws = moe.MoEWorkspace(scratch)
 
     def targets(self, p: str, D: int) -> dict:
         m = self.m
@@ -208,7 +208,7 @@ class _Experts(nn.Module):
 
 
 class MilivikLayer(nn.Module):
-    def __init__(self, cfg: MilivikConfig, lc: LayerConfig, dtype, device):
+    def __init__(self, cfg: MilivikConfig, lc: LayerConfig, dtype, device, scratch: moe.MoEScratch):
         super().__init__()
         D, Dp = cfg.hidden_size, cfg.padded_width
         self.norm1 = _Gain(D, Dp, device)
@@ -218,7 +218,7 @@ class MilivikLayer(nn.Module):
         if isinstance(lc.mlp, DenseConfig):
             self.mlp = _Gated(cfg, lc.mlp.ff, dtype, device)
         elif lc.mlp is not None:
-            self.mlp = _Experts(cfg, lc.mlp, dtype, device)
+            self.mlp = _Experts(cfg, lc.mlp, dtype, device, scratch)
 
     def targets(self, p: str, D: int) -> dict:
         t = {**self.norm1.targets(p + "norm1"), **self.mix.targets(p + "mix.", D)}
@@ -234,7 +234,8 @@ class MilivikDecoder(PackedDecoder):
         self.cfg, self.dtype_ = cfg, dtype
         # also the output projection, hence whole rows of eight
         self.embed_tokens = _zeros(round_up(cfg.vocab_size, 8), cfg.padded_width, dtype=dtype, device=device)
-        self.layers = nn.ModuleList([MilivikLayer(cfg, l, dtype, device) for l in cfg.layers])
+        scratch = moe.MoEScratch()
+        self.layers = nn.ModuleList([MilivikLayer(cfg, l, dtype, device, scratch) for l in cfg.layers])
         self.final_norm = _Gain(cfg.hidden_size, cfg.padded_width, device)
 
     # ------------------------------------------------------------------ forward

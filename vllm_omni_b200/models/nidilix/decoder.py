@@ -132,7 +132,7 @@ class _Scan(nn.Module):
 
 
 class _Experts(nn.Module):
-    def __init__(self, cfg: NidilixConfig, m: ExpertsConfig, dtype, device):
+    def __init__(self, cfg: NidilixConfig, m: ExpertsConfig, dtype, device, scratch: moe.MoEScratch):
         super().__init__()
         self.m = m
         D, ff = cfg.padded_width, round_up(m.ff, 8)
@@ -143,7 +143,7 @@ class _Experts(nn.Module):
         if m.shared_ff:
             self.shared_up = _linear(cfg.hidden_size, m.shared_ff, dtype, device)
             self.shared_down = _linear(m.shared_ff, cfg.hidden_size, dtype, device)
-        self.ws = moe.MoEWorkspace()
+        self.ws = moe.MoEWorkspace(scratch)
 
     def targets(self, p: str, D: int) -> dict:
         m = self.m
@@ -163,13 +163,13 @@ class _Experts(nn.Module):
 
 
 class NidilixLayer(nn.Module):
-    def __init__(self, cfg: NidilixConfig, lc: LayerConfig, dtype, device):
+    def __init__(self, cfg: NidilixConfig, lc: LayerConfig, dtype, device, scratch: moe.MoEScratch):
         super().__init__()
         Dp = cfg.padded_width
         self.norm1 = _TanhNorm(Dp, device)
         self.mix = (_Latent if isinstance(lc.mixer, LatentMixer) else _Scan)(cfg, lc.mixer, dtype, device)
         self.norm2 = _TanhNorm(Dp, device) if lc.mlp is not None else None
-        self.mlp = _Experts(cfg, lc.mlp, dtype, device) if lc.mlp is not None else None
+        self.mlp = _Experts(cfg, lc.mlp, dtype, device, scratch) if lc.mlp is not None else None
         self.side_gate = self.side_proj = None
         if cfg.side_dim:
             self.side_gate, self.side_proj = _linear(cfg.hidden_size, cfg.side_dim, dtype, device), \
@@ -196,7 +196,8 @@ class NidilixDecoder(PackedDecoder):
         self.embed_tokens = _zeros(cfg.vocab_size, cfg.padded_width, dtype=dtype, device=device)
         self.side_table = _zeros(cfg.vocab_size, cfg.side_dim * len(cfg.layers), dtype=dtype, device=device) \
             if cfg.side_dim else None
-        self.layers = nn.ModuleList([NidilixLayer(cfg, l, dtype, device) for l in cfg.layers])
+        scratch = moe.MoEScratch()
+        self.layers = nn.ModuleList([NidilixLayer(cfg, l, dtype, device, scratch) for l in cfg.layers])
         self.final_norm = _TanhNorm(cfg.padded_width, device)
         self.lm_head = _linear(cfg.hidden_size, cfg.vocab_size, dtype, device)
 

@@ -22,7 +22,7 @@ from torch import nn
 from ..diffusion.layers.linear import FusedLinear
 from ..ops import fused, kv_cache as KC
 from ..ops.attention import attention
-from ..ops.moe import MoEWorkspace, moe_forward
+from ..ops.moe import MoEScratch, MoEWorkspace, moe_forward
 from ..ops.step_inputs import token_rows
 
 
@@ -145,7 +145,7 @@ class RotaryTable:
 
 
 class DecoderLayer(nn.Module):
-    def __init__(self, cfg: DecoderConfig, dtype, device):
+    def __init__(self, cfg: DecoderConfig, dtype, device, moe_scratch: MoEScratch):
         super().__init__()
         D, H, Hkv, Dh = cfg.hidden_size, cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim
         P = lambda *s: nn.Parameter(torch.ones(*s, dtype=dtype, device=device), requires_grad=False)
@@ -162,7 +162,7 @@ class DecoderLayer(nn.Module):
                                     requires_grad=False)
             self.w2 = nn.Parameter(torch.empty(E, D, F_, dtype=dtype, device=device).normal_(0, 0.02),
                                    requires_grad=False)
-            self.moe_ws = MoEWorkspace()
+            self.moe_ws = MoEWorkspace(moe_scratch)
             Fs = cfg.shared_expert_intermediate_size
             if Fs:
                 self.shared_gate_up = FusedLinear(D, 2 * Fs, bias=False, dtype=dtype, device=device)
@@ -180,7 +180,8 @@ class QwenDecoderModel(nn.Module):
         self.cfg, self.dtype_ = cfg, dtype
         self.embed_tokens = nn.Parameter(torch.empty(cfg.vocab_size, cfg.hidden_size, dtype=dtype, device=device)
                                          .normal_(0, 0.02), requires_grad=False)
-        self.layers = nn.ModuleList([DecoderLayer(cfg, dtype, device) for _ in range(cfg.num_hidden_layers)])
+        moe_scratch = MoEScratch()
+        self.layers = nn.ModuleList([DecoderLayer(cfg, dtype, device, moe_scratch) for _ in range(cfg.num_hidden_layers)])
         self.norm = nn.Parameter(torch.ones(cfg.hidden_size, dtype=dtype, device=device), requires_grad=False)
         self.lm_head = None
         if with_lm_head and not cfg.tie_word_embeddings:

@@ -103,25 +103,32 @@ def _few(T, k, E, pad) -> bool:
     return not pad and T * k <= min(FEW_PAIRS, E)
 
 
-_pool: dict = {}
+class MoEScratch:
+    """Scratch buffers of one decoder: its layers run one after the other and share them; they go when the decoder goes.  Two
+    decoders never share any: their steps run in threads and on streams of their own.  Token counts are rounded up to powers of two and
+    a bucket keeps its buffers: a CUDA graph captured at one batch size keeps pointing at live memory when a larger prefill comes
+    along, and a 48-layer model holds one set of scratch, not 48."""
+
+    def __init__(self):
+        self.buckets: dict = {}
+
+    def __deepcopy__(self, memo):
+        return memo.setdefault(id(self), MoEScratch())      # a copied decoder starts with scratch of its own
 
 
 class MoEWorkspace:
-    """Handle a layer keeps for its MoE scratch.  The buffers themselves are shared by every layer of
-    the process (layers run one after the other on a stream) and sized by power-of-two token buckets
-    that are never freed: a CUDA graph captured at one batch size keeps pointing at live memory when a
-    larger prefill comes along, and a 48-layer model holds one set of scratch, not 48."""
+    """Handle a layer keeps for its MoE scratch, in the buffers of ``scratch`` (its decoder's) or in its own."""
 
-    def __init__(self):
-        self.key = None
+    def __init__(self, scratch: MoEScratch | None = None):
+        self.key, self.scratch = None, scratch if scratch is not None else MoEScratch()
 
     def get(self, T, k, E, D, Fd, device, dtype):
         pad = padded_rows()
         cap = max(64, 1 << (max(T, 1) - 1).bit_length())
         key = (cap, k, E, D, Fd, str(device), dtype, pad)
-        buf = _pool.get(key)
+        buf = self.scratch.buckets.get(key)
         if buf is None:
-            buf = _pool[key] = _MoEBuffers(cap, k, E, D, Fd, device, dtype, pad)
+            buf = self.scratch.buckets[key] = _MoEBuffers(cap, k, E, D, Fd, device, dtype, pad)
         self.key, self.padded = (T,) + key, pad
         self.max_rows, self.max_tiles = _rows_tiles(T, k, E, pad)
         self.tile_cap = _tile_rows(T, k, E)
