@@ -67,17 +67,9 @@ def rows_gather(k_cache, block_table, T):
     return k_cache.view(-1, *k_cache.shape[2:])[block_table.long()[j // bs] * bs + j % bs]
 
 
-_scratch: dict = {}
-
-
 def _scratch_for(device, n_part: int, D: int):
-    key = (device.index, n_part)
-    sc = _scratch.get(key)
-    if sc is None:
-        sc = (torch.empty(n_part * D, dtype=torch.float32, device=device),
-              torch.empty(n_part * 2, dtype=torch.float32, device=device))
-        _scratch[key] = sc
-    return sc
+    """Partial sums and their maxima and weights of a split call, its own: other threads and streams run calls of the same size."""
+    return (torch.empty(n_part * D, dtype=torch.float32, device=device), torch.empty(n_part * 2, dtype=torch.float32, device=device))
 
 
 def tma_pages_ok(block_size: int, D: int) -> bool:
