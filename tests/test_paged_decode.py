@@ -58,3 +58,22 @@ def test_scores_of_minus_infinity(H, Hkv, dead):
     # as above: weights and result rounded to bf16
     bound = torch.einsum("nhk,nkhd->nhd", w, vv.abs()) * 2.0 ** -8 + ref.abs() * 2.0 ** -8 + 1e-5
     assert ((out.double() - ref).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("bs", [24, 48, 256])
+@pytest.mark.parametrize("H,Hkv", [(8, 1), (8, 4)])
+def test_pages_of_other_sizes_keep_fp32_weights(bs, H, Hkv):
+    """Pages the tensor-core kernel does not take are decoded with weights in fp32."""
+    D, n, L = 128, 3, 500
+    g = torch.Generator(device="cuda").manual_seed(bs)
+    per = -(-L // bs)
+    q = torch.randn(n, H, D, generator=g, device="cuda").bfloat16()
+    k, v = (torch.randn(n * per, bs, Hkv, D, generator=g, device="cuda").bfloat16() for _ in range(2))
+    tables = torch.arange(n * per, dtype=torch.int32, device="cuda").view(n, per)
+    out = KC.paged_decode(q, k, v, tables, torch.full((n,), L, dtype=torch.int32, device="cuda"))
+    kk, vv = (t.view(n, per * bs, Hkv, D)[:, :L].double().repeat_interleave(H // Hkv, 2) for t in (k, v))
+    w = torch.softmax(torch.einsum("nhd,nkhd->nhk", q.double(), kk) * D ** -0.5, -1)
+    ref = torch.einsum("nhk,nkhd->nhd", w, vv)
+    # the result's rounding to bf16 alone; fp32 scores, weights and sums are 2^-14 and below
+    bound = ref.abs() * 2.0 ** -8 + torch.einsum("nhk,nkhd->nhd", w, vv.abs()) * 2.0 ** -14
+    assert ((out.double() - ref).abs() <= bound).all()

@@ -93,11 +93,20 @@ def _attn_paged(q, q_rs, q_hs, q_bs, k_cache, v_cache, block_tables, kv_lens, ou
     nv.check_rc(rc, "omni_attn_fwd_paged")
 
 
+def decode_impl(n: int, H: int, Hkv: int, D: int, block_size: int, num_splits, q_stride: int, out_stride: int) -> str:
+    """The kernel that decodes ``n`` sequences.  Pages that the tensor-core kernel does not take: "simt", which keeps the weights in fp32
+    where the others round them to bf16 ("stream" for group sizes it does not have).  Else "tc" where a number of splits is asked for or
+    more than 16 heads share a KV head, and "stream" for the rest."""
+    G = H // Hkv
+    if not tma_pages_ok(block_size, D) or G > 128:
+        return "stream" if D == 128 and block_size % 8 == 0 and G <= 16 and G not in (1, 2, 4, 8) and num_splits is None else "simt"
+    return "tc" if G > 16 or num_splits is not None or q_stride % 8 or out_stride % 8 else "stream"
+
+
 def paged_decode(q, k_cache, v_cache, block_tables, seq_lens, scale=None, num_splits=None, out=None, impl=None):
     """q: [num_seqs, H, D] (one new token per sequence) -> [num_seqs, H, D].
 
-    ``impl``: "stream" (csrc/decode_attn.cu; default for head size 128, pages of a multiple of 8 tokens and up to 16 query heads
-    per KV head), "tc" (tcgen05 kernel; default for larger groups where the page shape allows, or with ``num_splits``) or "simt"."""
+    ``impl``: "stream" (csrc/decode_attn.cu), "tc" (tcgen05 kernel) or "simt"; by default as ``decode_impl`` says."""
     n, H, D = q.shape
     nb, bs, Hkv, _ = k_cache.shape
     scale = scale if scale is not None else 1.0 / math.sqrt(D)
@@ -113,8 +122,7 @@ def paged_decode(q, k_cache, v_cache, block_tables, seq_lens, scale=None, num_sp
     assert q.stride(-1) == 1 and q.stride(1) == D and block_tables.dtype == torch.int32 and seq_lens.dtype == torch.int32
     G = H // Hkv
     if impl is None:
-        impl = "stream" if D == 128 and bs % 8 == 0 and G <= 16 and num_splits is None and q.stride(0) % 8 == 0 and out.stride(0) % 8 == 0 \
-            else "tc" if tma_pages_ok(bs, D) and G <= 128 else "simt"
+        impl = decode_impl(n, H, Hkv, D, bs, num_splits, q.stride(0), out.stride(0))
     if impl == "stream":
         assert out.stride(-1) == 1 and out.stride(1) == D and q.dtype == torch.bfloat16
         lib, max_kv = nv.lib("decode_attn"), block_tables.shape[1] * bs
