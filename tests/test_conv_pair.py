@@ -9,7 +9,7 @@ from vllm_omni_b200.ops import _native as nv, conv as C
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n,h,w", [(1, 64, 80), (3, 47, 61), (2, 16, 200), (5, 33, 41), (40, 7, 9)])
+@pytest.mark.parametrize("n,h,w", [(1, 64, 80), (3, 47, 61), (2, 16, 200), (5, 33, 41), (40, 7, 9), (20, 8, 130), (9, 3, 401)])
 @pytest.mark.parametrize("cin,cout", [(16, 384), (96, 96), (96, 3), (72, 200), (192, 192), (128, 256), (8, 40)])
 @pytest.mark.parametrize("epilogue", [None, "silu", "residual"])
 def test_against_64_bits(n, h, w, cin, cout, epilogue):

@@ -1358,21 +1358,21 @@ extern "C" int omni_conv2d_nhwc_bf16(const void* x, long ldx, const void* w, voi
   if (!enc) return RC_NO_DRIVER;
   if (reinterpret_cast<uintptr_t>(x) & 15) return RC_BAD_ARG;
   const int pairs = ksize == 3 ? max_resident_pairs() : 0;
-  const long m_pairs = ((long)Nimg * ((W + C3_W - 1) / C3_W) * ((H + C3_H - 1) / C3_H) + 1) / 2;
-  // below a quarter of a wave of pixel tiles the one-CTA kernel spreads a problem over more SMs
+  const bool flat = ksize == 3 && conv3_flat(Nimg, H, W, Cout, pairs);
+  const long m_pairs = ((flat ? conv3_tiles(Nimg, W, H) : conv3_tiles(Nimg, H, W)) + 1) / 2;
+  // The line at a quarter of a wave of pixel tiles was drawn for the one-CTA kernel's larger number of blocks and does not show in the times: below
+  // it the pair kernel is the faster one too (us, one-CTA kernel in brackets: 48 x 48 pixels, 384 -> 384 channels 14.7 (29.1), 96 -> 96
+  // 6.6 (13.7); 32 x 32, 16 -> 384 6.5 (11.0); just above it 64 x 80, 384 -> 384 16.7 (29.7)).
   if (ksize == 3 && m_pairs * 4 >= pairs && m_pairs < (1L << 24)) {
     Conv3Args a = {};
     a.y = static_cast<__nv_bfloat16*>(y);
-    a.ldy = ldy; a.H = H; a.W = W; a.n_img = Nimg;
-    a.tiles_x = (W + C3_W - 1) / C3_W; a.tiles_y = (H + C3_H - 1) / C3_H;
+    a.ldy = ldy; a.n_img = Nimg;
+    a.H = flat ? W : H; a.W = flat ? H : W;
+    a.tap_y = flat ? 1 : 3; a.tap_x = flat ? 3 : 1;
+    a.px_y = flat ? 1 : W; a.px_x = flat ? W : 1;
+    a.tiles_x = (a.W + C3_W - 1) / C3_W; a.tiles_y = (a.H + C3_H - 1) / C3_H;
     a.Cout = Cout; a.cin = Cin; a.cin_blocks = (Cin + BK - 1) / BK;
-    cuuint64_t gdim[4] = {(cuuint64_t)Cin, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)Nimg};
-    cuuint64_t gstr[3] = {(cuuint64_t)ldx * 2, (cuuint64_t)ldx * 2 * W, (cuuint64_t)ldx * 2 * W * H};
-    cuuint32_t box[4] = {BK, C3_W, C3_H + 2, 1};
-    cuuint32_t estr[4] = {1, 1, 1, 1};
-    if (enc(&a.tmX, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(x), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-      return RC_TMAP;
+    if (int rc = conv3_map(&a.tmX, a, x, ldx, Cin, BK, C3_H + 2, CU_TENSOR_MAP_SWIZZLE_128B)) return rc;
     a.epi.bias = static_cast<const __nv_bfloat16*>(bias);
     a.epi.residual = static_cast<const __nv_bfloat16*>(residual);
     a.epi.ldr = ldr;
