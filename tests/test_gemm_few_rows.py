@@ -71,3 +71,17 @@ def test_splits_of_at_most_16_rows(rows, per_sm):
             y = gemm.linear(x, w, b, residual=res)
             _check(y, x.double() @ w.double().T + b.double() + res.double(), x.double().abs() @ w.double().abs().T)
     nv.check_status()
+
+
+@pytest.mark.parametrize("rows,n,k", [(8, 14400, 8192), (9, 14208, 6912), (9, 14216, 6912), (16, 14216, 3840), (16, 14216, 3912), (16, 14208, 4096),
+                                      (16, 9480, 12288), (16, 9472, 12288), (17, 9480, 136), (32, 12808, 1032), (32, 18944, 200), (32, 18952, 200), (48, 4736, 520), (64, 4608, 1024), (64, 9472, 72), (64, 9480, 72),
+                                      (65, 2048, 1016), (65, 2048, 960), (65, 2056, 1024), (128, 2688, 1032), (128, 2824, 1024), (128, 2824, 1096),
+                                      (128, 6272, 2304), (128, 6272, 2240), (128, 6280, 3200)])
+def test_edges_of_the_rules(rows, n, k):
+    """Both sides of every limit of few_rows() and of the widest layout that is one cluster short of a round (37 tiles)."""
+    g = torch.Generator(device="cuda").manual_seed(rows + n + k)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    x, w, b, res = rnd(rows, k), rnd(n, k), rnd(n), rnd(rows, n)
+    y = gemm.linear(x, w, b, residual=res)
+    _check(y, x.double() @ w.double().T + b.double() + res.double(), x.double().abs() @ w.double().abs().T)
+    nv.check_status()

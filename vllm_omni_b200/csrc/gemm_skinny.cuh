@@ -304,7 +304,33 @@ static int launch_skinny_s(const CUtensorMap& tmX, const CUtensorMap& tmW, __nv_
   return (int)cudaGetLastError();
 }
 
-// CTAs per tile: up to about 200 in all (two share an SM), each with at least two K blocks
+// CTAs that one SM holds one of (ALONE) all run at once up to as many clusters as the device places; whole clusters do not use every SM of
+// a group of SMs, so that is less than the SMs divided by S: 37 tiles of 4 CTAs would be one cluster short of a round (48 rows 4736 x 2048
+// took 15.5 us, the general kernel 12.1).
+template <int MT, int S>
+static int clusters_alone() {
+  static int cached = 0;
+  if (cached) return cached;
+  int n = 0;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(sm_count() / S * S);
+  cfg.blockDim = dim3(SKINNY_THREADS);
+  cfg.dynamicSmemBytes = SkinnyCfg<MT, true>::SMEM_BYTES;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = S; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  static unsigned long long prepared = 0;
+  if (ensure_dynamic_smem((const void*)gemm_skinny_kernel<MT, S, true>, SkinnyCfg<MT, true>::SMEM_BYTES, prepared) ||
+      cudaOccupancyMaxActiveClusters(&n, gemm_skinny_kernel<MT, S, true>, &cfg) != cudaSuccess)
+    n = 0;
+  (void)cudaGetLastError();
+  return cached = n > 0 ? n : 1;
+}
+
+// CTAs per tile: up to about 200 in all (two share an SM), each with at least two K blocks.
+// us with a limit of 148, 200, 296: 64 rows 3072 x 4096 9.9, 9.5, 9.4; 6144 x 4096 15.5, 16.9, 16.9; 9216 x 2048 12.7, 12.7, 18.7.
 static int skinny_split(int N, int K) {
   const int tiles = (N + 127) / 128, num_kb = (K + 63) / 64;
   for (int s = 8; s > 1; s >>= 1)
@@ -317,27 +343,40 @@ static int launch_skinny_mt(const CUtensorMap& tmW, const void* A, int lda, __nv
                             const GemmEpilogue& epi, int split, int* status, cudaStream_t stream) {
   CUtensorMap tmX;
   if (int rc = make_tmap_2d(&tmX, A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)M, (uint64_t)K, (uint64_t)lda * 2, MT, 64)) return rc;
-  const bool alone = split <= 4 && (N + 127) / 128 * split <= sm_count();   // clusters of 8 CTAs do not fit every GPC's SMs one by one
-#define OMNI_SKINNY(S)                                                                                       \
-  return alone ? launch_skinny_s<MT, S, true>(tmX, tmW, C, ldc, M, N, K, epi, status, stream)                \
-               : launch_skinny_s<MT, S, false>(tmX, tmW, C, ldc, M, N, K, epi, status, stream)
-  switch (split) {
-    case 8: OMNI_SKINNY(8);
-    case 4: OMNI_SKINNY(4);
-    case 2: OMNI_SKINNY(2);
-    default: OMNI_SKINNY(1);
+  const int tiles = (N + 127) / 128;
+#define OMNI_SKINNY(S)                                                                                                           \
+  return tiles <= clusters_alone<MT, S>() ? launch_skinny_s<MT, S, true>(tmX, tmW, C, ldc, M, N, K, epi, status, stream)         \
+                                          : launch_skinny_s<MT, S, false>(tmX, tmW, C, ldc, M, N, K, epi, status, stream)
+  // clusters of 8 CTAs do not fit every GPC's SMs one by one
+  if (split == 8) return launch_skinny_s<MT, 8, false>(tmX, tmW, C, ldc, M, N, K, epi, status, stream);
+  if constexpr (MT < 128) {                // few_rows() leaves 128 rows 49 tiles at most, of 16 K blocks at least
+    if (split == 2) OMNI_SKINNY(2);
+    if (split == 1) OMNI_SKINNY(1);
   }
+  OMNI_SKINNY(4);
 #undef OMNI_SKINNY
 }
 
-// Which problems leave the general kernels (tiles of 128 or 256 rows).  M <= 16: all.  Above, the split needs room: with half as
-// many tiles as SMs or more the general kernels stream W as fast, and their wider tiles read A less often.
+// Which problems leave the general kernels (tiles of 128 or 256 rows).
+//   up to 16 rows    all but those whose rows of A do not stay in L1 (120 KB) between the blocks of an SM: every block reads them all, and past six
+//                    blocks per SM, or four of very long rows, that costs more than it saves.  us, general kernel in brackets: 13 rows 16384 x 4096 30.0
+//                    (37.3), 16 rows 16384 x 3584 28.3 (33.9), 16384 x 4096 31.5 (28.7), 13824 x 4096 24.4 (25.7), 12288 x 12288 1.05 times
+//                    as long, 8192 x 4096 18.1 (20.5).  Up to 8 rows the products are half as many and it pays at any length.
+//   17 to 32         up to as many tiles as SMs: 17 rows 10240 x 2048 12.5 (17.1), 12288 x 1024 8.0 (11.6), 32 rows 18432 x 2048 15.4 (16.7)
+//   33 to 64         up to half as many; above, the general kernels stream W as fast and read A less often: 64 rows 9216 x 2048 12.7 (13.8),
+//                    10240 x 2048 14.4 (13.2)
+//   65 to 128        up to a third, and contractions long enough for the split: exchange and epilogue of 128 rows take 4 us, which a split
+//                    wins back from 16 K blocks on and, with less to split by, from three quarters of the number of tiles: 128 rows 1536 x 768
+//                    9.8 (9.2), 1536 x 1024 8.1 (10.0), 4096 x 1024 11.2 (10.0), 4096 x 2048 12.9 (13.0); 65 rows 4096 x 1536 10.3 (10.7)
 enum class FewRows { no, rows, skinny };
-static FewRows few_rows(int M, int N) {
-  const int tiles = (N + 127) / 128;
-  if (M <= 16) return FewRows::rows;
-  if ((M <= 64 && tiles * 2 <= sm_count()) || (M <= 128 && tiles * 3 <= sm_count())) return FewRows::skinny;
-  return FewRows::no;
+static FewRows few_rows(int M, int N, int K) {
+  const int tiles = (N + 127) / 128, num_kb = (K + 63) / 64;
+  if (M <= 16) {
+    const long a_kb = (long)M * K * 2 / 1024, blocks = (N + 15) / 16;
+    return M > 8 && ((a_kb > 120 && blocks > 6L * sm_count()) || (a_kb >= 384 && blocks > 4L * sm_count())) ? FewRows::no : FewRows::rows;
+  }
+  if (M <= 64) return tiles * (M <= 32 ? 1 : 2) <= sm_count() ? FewRows::skinny : FewRows::no;
+  return M <= 128 && tiles * 3 <= sm_count() && num_kb >= 16 && num_kb * 4 >= tiles * 3 ? FewRows::skinny : FewRows::no;
 }
 
 static int launch_skinny(const void* A, int lda, const void* W, int ldw, __nv_bfloat16* C, int ldc, int M, int N, int K,

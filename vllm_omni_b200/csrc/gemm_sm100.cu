@@ -1088,7 +1088,7 @@ extern "C" int omni_gemm_bf16_coef(const void* A, int lda, const void* W, int ld
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   __nv_bfloat16* c = static_cast<__nv_bfloat16*>(C);
   if (force_bn == 0 && !sync && epi.scatter_P == 0 && epi.scatter_rows == 0) {
-    switch (few_rows(M, N)) {
+    switch (few_rows(M, N, K)) {
       case FewRows::rows: return launch_rows(A, lda, W, ldw, c, ldc, M, N, K, epi, s);
       case FewRows::skinny: return launch_skinny(A, lda, W, ldw, c, ldc, M, N, K, epi, status, s);
       default: break;
