@@ -25,3 +25,10 @@ def test_route(H, Hkv, bs):
         assert impl != "tc" or (tiles and G <= 128)
         assert KC.decode_impl(n, H, Hkv, 128, bs, 4, H * 128, H * 128) == ("tc" if tiles and G <= 128 else "simt")
     assert KC.decode_impl(4, H, Hkv, 64, bs, None, H * 64, H * 64) == "simt"
+
+
+@pytest.mark.parametrize("H,Hkv,n,impl", [(64, 4, 4, "stream"), (64, 4, 5, "tc"), (64, 4, 37, "tc"), (64, 4, 38, "stream"), (64, 4, 66, "stream"),
+                                          (64, 4, 67, "tc"), (64, 4, 74, "tc"), (64, 4, 75, "stream"), (32, 2, 8, "stream"), (32, 2, 9, "tc"),
+                                          (16, 1, 148, "tc"), (16, 1, 149, "stream"), (36, 3, 2, "tc"), (36, 3, 200, "tc"), (32, 4, 40, "stream")])
+def test_groups_of_9_to_16_heads(H, Hkv, n, impl):
+    assert KC.decode_impl(n, H, Hkv, 128, 16, None, H * 128, H * 128) == impl

@@ -56,6 +56,14 @@ paged_decode_kernel(const __grid_constant__ DecodeAttn p) {
   const int len = min(p.lens[seq], p.max_keys);
   const int tiles = (len + DA_KEYS - 1) / DA_KEYS, per = (tiles + p.splits - 1) / p.splits;
   const int t1 = min(tiles, (split + 1) * per);
+  if (split * per + sub >= t1) {      // no keys (a table wider than the sequence): weight zero, and no sum for the merge to read
+    if (parts > 1 && lane < G) {
+      float* ml = p.part_ml + (((long)seq * p.H + h0 + lane) * parts + split * p.subs + sub) * 2;
+      ml[0] = -INFINITY;
+      ml[1] = 0.f;
+    }
+    if (parts > 1) return;
+  }
   const int* bt = p.block_tables + (long)seq * p.bt_stride;
   const long row = (long)p.Hkv * DA_D;
 
@@ -237,7 +245,7 @@ paged_decode_merge_kernel(const float* __restrict__ part_o, const float* __restr
     for (int i = 0; i < 8; ++i) {
       const int s = s0 + 4 * i;                                // below 64 + 32: a lane of a or b, or past the end
       w[i] = __shfl_sync(0xffffffffu, s < 32 ? wa : wb, s & 31);
-      // a share without keys has written nothing
+      // a share without keys has written no sum
       x[i] = s < parts && w[i] != 0.f ? po[(long)s * (DA_D / 4)] : make_float4(0.f, 0.f, 0.f, 0.f);
     }
 #pragma unroll
@@ -264,10 +272,14 @@ paged_decode_merge_kernel(const float* __restrict__ part_o, const float* __restr
 
 constexpr int DA_MAX_PARTS = 64;
 
-// Shares of a sequence's keys: about `target` warps in all, at least two tiles of 16 keys each.
+// Shares of a sequence's keys: about `target` warps in all, at least two tiles of 16 keys each.  Twelve warps fit an SM; up to two rounds
+// of them even out lengths, but every share costs a sum to write and to read.  20 per SM, 16 to 16 heads of 1 to 16 KV heads, 1 to 256
+// sequences of 64 to 32768 keys: 1.5 % below 24 and 2 % below 16 in the mean, and nowhere above the tensor-core kernel (24: up to 1.11
+// of it for 72 sequences of 1024 keys in tables of 4096; 16 rounds off a whole one for few sequences).  A single sequence has at most
+// 64 shares: 131072 keys of 4 KV heads take 148 us, the tensor-core kernel 246 (the copy rate would be 41; more shares would reach more SMs).
 static void plan_shares(int n, int Hkv, int max_keys, int& splits, int& subs) {
   subs = Hkv < DA_WARPS ? DA_WARPS / Hkv : 1;
-  const long warps = (long)n * Hkv, target = 2L * 12 * sm_count();
+  const long warps = (long)n * Hkv, target = 20L * sm_count();
   const int tiles = (max_keys + DA_KEYS - 1) / DA_KEYS;
   long parts = (target + warps - 1) / warps;
   if (parts > tiles / 2) parts = tiles / 2;

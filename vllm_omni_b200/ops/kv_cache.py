@@ -96,11 +96,20 @@ def _attn_paged(q, q_rs, q_hs, q_bs, k_cache, v_cache, block_tables, kv_lens, ou
 def decode_impl(n: int, H: int, Hkv: int, D: int, block_size: int, num_splits, q_stride: int, out_stride: int) -> str:
     """The kernel that decodes ``n`` sequences.  Pages that the tensor-core kernel does not take: "simt", which keeps the weights in fp32
     where the others round them to bf16 ("stream" for group sizes it does not have).  Else "tc" where a number of splits is asked for or
-    more than 16 heads share a KV head, and "stream" for the rest."""
-    G = H // Hkv
+    more than 16 heads share a KV head, and "stream" for up to 8 of them.  Groups of 9 to 16 heads fill both halves of its products and
+    leave room for fewer loads in flight: it wins where the tensor-core kernel, a block per sequence and KV head, has very few blocks or
+    a last round that is less than nine tenths full, and loses where it has nearly one or two rounds of them.  Of "tc"'s time, 64 / 4 and
+    32 / 2 heads at 64 to 32768 keys: 16 groups 0.57 to 0.84, 32 groups 0.77 to 1.12, 128 groups 0.95 to 1.34, 160 groups 0.36 to 0.95,
+    256 groups 0.45 to 1.06, 288 groups 0.88 to 1.17, 320 groups 0.33 to 0.86."""
+    G, groups, sms = H // Hkv, n * Hkv, 148
     if not tma_pages_ok(block_size, D) or G > 128:
         return "stream" if D == 128 and block_size % 8 == 0 and G <= 16 and G not in (1, 2, 4, 8) and num_splits is None else "simt"
-    return "tc" if G > 16 or num_splits is not None or q_stride % 8 or out_stride % 8 else "stream"
+    if G > 16 or num_splits is not None or q_stride % 8 or out_stride % 8:
+        return "tc"
+    if G <= 8:
+        return "stream"
+    whole = Hkv % 4 == 0 or Hkv <= 2                   # all four warps of a block have heads: 36 / 3 heads, 576 groups, 1.10 of "tc"'s time
+    return "stream" if whole and (groups <= 16 or (groups > sms and not 1.8 * sms <= groups <= 2 * sms)) else "tc"
 
 
 def paged_decode(q, k_cache, v_cache, block_tables, seq_lens, scale=None, num_splits=None, out=None, impl=None):
