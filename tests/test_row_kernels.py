@@ -16,6 +16,19 @@ def _gen(seed):
 @pytest.mark.parametrize("rows", [1, 6, 1183, 1184, 5002])
 @pytest.mark.parametrize("rms", [True, False])
 def test_norm_modulate(width, rows, rms):
+    _norm(width, rows, rms)
+
+
+@pytest.mark.parametrize("width", [1032, 2048, 2056, 2560, 2568, 3072, 3080, 4096, 4104, 5120, 5128, 6144, 6152, 8192])
+@pytest.mark.parametrize("per_sm", [1, 2, 4, 5, 12, 16])
+def test_norm_layouts(width, per_sm):
+    """Both sides of every limit, in rows per SM, at which the number of warps per row changes, at the widths where the chunks per lane do."""
+    rows = per_sm * torch.cuda.get_device_properties(0).multi_processor_count
+    for r in (rows, rows + 1):
+        _norm(width, r, r % 2 == 0)
+
+
+def _norm(width, rows, rms):
     g = _gen(width + rows)
     rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
     b = 1 if rows % 2 else 2

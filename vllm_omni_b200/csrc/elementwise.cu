@@ -42,10 +42,10 @@ __device__ __forceinline__ float warp_sum(float v) {
 }
 
 // ---------------------------------------------------------------- norm + modulate
-// Few rows of more than 1024 channels: one block per row, CPT 16-byte chunks per thread.  Gains and modulation are fetched
+// Up to a row per SM of more than 1024 channels: one block per row, CPT 16-byte chunks per thread.  Gains and modulation are fetched
 // together with the row, so a launch is one round trip to memory and one reduction; short code matters as much, because a
 // launch of a few rows spends its time fetching instructions.  Caches cold, launch included: 8 rows of 4096 8 us (one
-// warp per row with all chunks unrolled: 18), 512 rows of 3072 10 us (14).
+// warp per row with all chunks unrolled: 18).
 template <int CPT>
 __global__ void __launch_bounds__(512)
 norm_modulate_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, int D, int ldx, int ldy,
@@ -114,9 +114,9 @@ norm_modulate_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restr
   }
 }
 
-// Many rows, or rows of up to 1024 channels: WPR warps per row, the row packed (bf16) in VPL 16-byte registers per lane.  All loads of a
-// row are in flight at once and 40 to 60 registers leave room for 32 warps and more per SM.  8192 rows of 4096 (134 MB): 39 us, with one
-// warp per row and 16 chunks per lane 53 us; keeping rows in flight through shared memory instead (bulk copies,
+// More rows, or rows of up to 1024 channels: WPR warps per row, the row packed (bf16) in VPL 16-byte registers per lane.  All loads of a
+// row are in flight at once and 40 to 60 registers leave room for 32 warps and more per SM.  8192 rows of 4096 (134 MB): 34 us, with one
+// warp per row and 16 chunks per lane 48 us; keeping rows in flight through shared memory instead (bulk copies,
 // 200 KB per SM) did not help: 16 warps issue too little.
 template <int VPL, int WPR>
 __global__ void __launch_bounds__(256)
@@ -600,14 +600,33 @@ extern "C" int omni_norm_modulate(const void* x, void* y, int rows, int D, int l
 #define OMNI_NM_WARP(V, W) launch_overlapped(norm_modulate_warp_kernel<V, W>, (unsigned)((rows + 8 / W - 1) / (8 / W)), 256, 0, st, xx, yy, rows, D, ldx, ldy, w, bb, sh, sc, mod_stride, rows_per_batch, rms, eps)
   if (nchunk <= 64) OMNI_NM_WARP(2, 1);
   else if (nchunk <= 128) OMNI_NM_WARP(4, 1);
-  else if (rows < 8 * sm_count() || nchunk > 640)
-    // up to 8 rows per SM a block per row is one round of latencies
+  else if (rows <= (nchunk <= 256 ? 5 : nchunk <= 640 ? 2 : 1) * sms)
+  // Rows of more than 1024 channels, by the rows per SM, RMS norm in us on cold operands:
+  //   up to 2, or 5 of up   a block per row, two chunks per thread: one round of latencies (64 rows of 5120: 2.5, 4 warps per row 3.4; 740 rows of
+  //   to 2048 channels      2048: 3.3 and 3.4).  Above, the blocks of a second round cost more than they save (592 rows of 3072: 5.1, 4 warps 3.9)
+  //   more than 5120        from the second row per SM on 8 warps per row, since blocks of 512 threads fit an SM twice at most: 592 rows of 6144
+  //                         6.2 (block per row 9.7, 4 warps 6.5), 8192 rows of 8192 60.6 (127, 62.5); 4 warps where they need at most 6
+  //                         chunks per lane and rows are many: 8192 rows of 6144 46.5 (8 warps 48.2)
+  //   many, of up to 3072   2 warps per row: fewer warps that wait for one another (8192 rows of 2048: 16.1, 4 warps 18.1, one warp 17.5; 4096 rows of
+  //                         3072: 12.6 and 13.1; below the limits 4 warps: 2048 rows of 3072 8.6, 2 warps 9.7)
+  //   else                  4 warps per row (1183 rows of 4096: 6.7, block per row 10.0)
+  const long sms = sm_count();
     launch_overlapped(norm_modulate_kernel<2>, rows, ((nchunk + 1) / 2 + 31) / 32 * 32, 0, st, xx, yy, D, ldx, ldy, w, bb, sh, sc, mod_stride,
                                                                                rows_per_batch, rms, eps);
-  else if (nchunk <= 256) OMNI_NM_WARP(4, 2);
-  else if (nchunk <= 384) OMNI_NM_WARP(6, 2);
-  else if (nchunk <= 512) OMNI_NM_WARP(8, 2);
-  else OMNI_NM_WARP(5, 4);
+  else if (nchunk > 768) OMNI_NM_WARP(4, 8);
+  else if (nchunk > 640) {
+    if (rows <= 4 * sms) OMNI_NM_WARP(3, 8);
+    else OMNI_NM_WARP(6, 4);
+  } else if (nchunk <= 384 && rows > (nchunk <= 256 ? 12 : 16) * sms) {
+    if (nchunk <= 256) OMNI_NM_WARP(4, 2);
+    else if (nchunk <= 320) OMNI_NM_WARP(5, 2);
+    else OMNI_NM_WARP(6, 2);
+  } else {
+    if (nchunk <= 256) OMNI_NM_WARP(2, 4);
+    else if (nchunk <= 384) OMNI_NM_WARP(3, 4);
+    else if (nchunk <= 512) OMNI_NM_WARP(4, 4);
+    else OMNI_NM_WARP(5, 4);
+  }
 #undef OMNI_NM_WARP
   return (int)cudaGetLastError();
 }
