@@ -207,7 +207,7 @@ struct HeadPages {
 
 // Norm and rotation of one head held by half a warp, 8 consecutive elements per lane (D = 128).  c, s: this lane's rotation
 // coefficients, 4 pairs of neighbours (interleaved) or the 8 frequencies of its elements (halves, the sign already on s).
-__device__ __forceinline__ uint4 head_norm_rope(const uint4& v, bool norm, const uint4& gain, bool rope, int interleaved, const float (&c)[8],
+__device__ __forceinline__ uint4 head_norm_rope(const uint4& v, bool norm, const float (&gain)[8], bool rope, int interleaved, const float (&c)[8],
                                                 const float (&s)[8], float eps) {
   const uint32_t w[4] = {v.x, v.y, v.z, v.w};
   float x[8];
@@ -222,13 +222,8 @@ __device__ __forceinline__ uint4 head_norm_rope(const uint4& v, bool norm, const
 #pragma unroll
     for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     const float r = rsqrtf(ss * (1.0f / 128) + eps);
-    const uint32_t g[4] = {gain.x, gain.y, gain.z, gain.w};
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float2 f = unpack_bf16(g[j]);
-      x[2 * j] = x[2 * j] * r * f.x;
-      x[2 * j + 1] = x[2 * j + 1] * r * f.y;
-    }
+    for (int e = 0; e < 8; ++e) x[e] = x[e] * r * gain[e];
   }
   if (rope) {
     if (interleaved) {
@@ -309,13 +304,14 @@ qk_norm_rope128_kernel(const __grid_constant__ HeadRows a, PeerWait wt, int* sta
   if (row >= a.rows) return;
   const int lane = threadIdx.x & 31, l16 = lane & 15;
   const int h = (int)(unit - row * pairs) * 2 + (lane >> 4);
-  uint4 v = make_uint4(0u, 0u, 0u, 0u), gain = v;
+  uint4 v = make_uint4(0u, 0u, 0u, 0u);
+  float gain[8];
   if (h < all) v = *reinterpret_cast<const uint4*>(a.qkv + (size_t)row * a.ld + (size_t)h * 128 + l16 * 8);
   const int s = (int)(row % a.S);
   const bool alt = s >= a.s_alt;
   if (a.wq) {
     const __nv_bfloat16* g = h < a.H ? ((alt && a.wq_alt) ? a.wq_alt : a.wq) : ((alt && a.wk_alt) ? a.wk_alt : a.wk);
-    gain = *reinterpret_cast<const uint4*>(g + l16 * 8);
+    load8(g + l16 * 8, gain);
   }
   float cs[8], sn[8];
   rope_coefficients(a, row, s, l16, cs, sn);
@@ -323,7 +319,9 @@ qk_norm_rope128_kernel(const __grid_constant__ HeadRows a, PeerWait wt, int* sta
   if (h < all) store_head(a, row, h, l16, a.pages.k ? a.pages.slots[row] : -1, v, o);
 }
 
-// The same for many rows: a warp walks all heads of its row, 8 at a time, and fetches the rotation coefficients once.
+// The same for many rows: a warp walks the query heads of its row, 8 at a time, then key and value heads, and fetches gains and rotation
+// coefficients once.  After the projection that makes the rows, both together in us: 2000 rows of 32 / 4 heads, 2048 wide, 44.9; gains kept
+// as bf16 and chosen per head 45.7, two heads to a warp 50.0; 8192 rows of 32 / 8 180.2, 182.7 and 206.1.
 __global__ void __launch_bounds__(256)
 qk_norm_rope128_rows_kernel(const __grid_constant__ HeadRows a, PeerWait wt, int* status) {
   pdl_begin();
@@ -340,31 +338,37 @@ qk_norm_rope128_rows_kernel(const __grid_constant__ HeadRows a, PeerWait wt, int
   const int lane = threadIdx.x & 31, l16 = lane & 15, hsel = lane >> 4;
   const int s = (int)(row % a.S);
   const bool alt = s >= a.s_alt;
-  uint4 gq = make_uint4(0u, 0u, 0u, 0u), gk = gq;
+  float gq[8], gk[8];
   if (a.wq) {
-    gq = *reinterpret_cast<const uint4*>(((alt && a.wq_alt) ? a.wq_alt : a.wq) + l16 * 8);
-    gk = *reinterpret_cast<const uint4*>(((alt && a.wk_alt) ? a.wk_alt : a.wk) + l16 * 8);
+    load8(((alt && a.wq_alt) ? a.wq_alt : a.wq) + l16 * 8, gq);
+    load8(((alt && a.wk_alt) ? a.wk_alt : a.wk) + l16 * 8, gk);
   }
   float cs[8], sn[8];
   rope_coefficients(a, row, s, l16, cs, sn);
   const int page = a.pages.k ? a.pages.slots[row] : -1;
   constexpr int U = 4;
-  // both halves of the warp take every step, whether or not their last heads exist: head_norm_rope exchanges values over the whole warp
+  // heads lo .. hi - 1; both halves of the warp take every step, whether or not their last heads exist: head_norm_rope exchanges values
+  // over the whole warp
+  const auto span = [&](int lo, int hi, const float (&gain)[8], bool queries) {
 #pragma unroll 1
-  for (int h0 = 0; h0 < all; h0 += 2 * U) {
-    uint4 v[U];
+    for (int h0 = lo; h0 < hi; h0 += 2 * U) {
+      uint4 v[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int h = h0 + 2 * u + hsel;
-      v[u] = h < all ? *reinterpret_cast<const uint4*>(a.qkv + (size_t)row * a.ld + (size_t)h * 128 + l16 * 8) : make_uint4(0u, 0u, 0u, 0u);
-    }
+      for (int u = 0; u < U; ++u) {
+        const int h = h0 + 2 * u + hsel;
+        v[u] = h < hi ? *reinterpret_cast<const uint4*>(a.qkv + (size_t)row * a.ld + (size_t)h * 128 + l16 * 8) : make_uint4(0u, 0u, 0u, 0u);
+      }
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int h = h0 + 2 * u + hsel;
-      const uint4 o = head_norm_rope(v[u], a.wq != nullptr, h < a.H ? gq : gk, a.cosb != nullptr, a.interleaved, cs, sn, a.eps);
-      if (h < all) store_head(a, row, h, l16, page, v[u], o);
+      for (int u = 0; u < U; ++u) {
+        const int h = h0 + 2 * u + hsel;
+        const uint4 o = head_norm_rope(v[u], a.wq != nullptr, gain, a.cosb != nullptr, a.interleaved, cs, sn, a.eps);
+        if (h < hi && queries) *reinterpret_cast<uint4*>(a.qkv + (size_t)row * a.ld + (size_t)h * 128 + l16 * 8) = o;
+        else if (h < hi) store_head(a, row, h, l16, page, v[u], o);
+      }
     }
-  }
+  };
+  span(0, a.H, gq, true);
+  span(a.H, all, gk, false);
 }
 
 // ------------------------------------------------------------------ qk norm + rope
@@ -598,9 +602,6 @@ extern "C" int omni_norm_modulate(const void* x, void* y, int rows, int D, int l
   cudaStream_t st = (cudaStream_t)stream;
   const int nchunk = D >> 3;
 #define OMNI_NM_WARP(V, W) launch_overlapped(norm_modulate_warp_kernel<V, W>, (unsigned)((rows + 8 / W - 1) / (8 / W)), 256, 0, st, xx, yy, rows, D, ldx, ldy, w, bb, sh, sc, mod_stride, rows_per_batch, rms, eps)
-  if (nchunk <= 64) OMNI_NM_WARP(2, 1);
-  else if (nchunk <= 128) OMNI_NM_WARP(4, 1);
-  else if (rows <= (nchunk <= 256 ? 5 : nchunk <= 640 ? 2 : 1) * sms)
   // Rows of more than 1024 channels, by the rows per SM, RMS norm in us on cold operands:
   //   up to 2, or 5 of up   a block per row, two chunks per thread: one round of latencies (64 rows of 5120: 2.5, 4 warps per row 3.4; 740 rows of
   //   to 2048 channels      2048: 3.3 and 3.4).  Above, the blocks of a second round cost more than they save (592 rows of 3072: 5.1, 4 warps 3.9)
@@ -611,6 +612,9 @@ extern "C" int omni_norm_modulate(const void* x, void* y, int rows, int D, int l
   //                         3072: 12.6 and 13.1; below the limits 4 warps: 2048 rows of 3072 8.6, 2 warps 9.7)
   //   else                  4 warps per row (1183 rows of 4096: 6.7, block per row 10.0)
   const long sms = sm_count();
+  if (nchunk <= 64) OMNI_NM_WARP(2, 1);
+  else if (nchunk <= 128) OMNI_NM_WARP(4, 1);
+  else if (rows <= (nchunk <= 256 ? 5 : nchunk <= 640 ? 2 : 1) * sms)
     launch_overlapped(norm_modulate_kernel<2>, rows, ((nchunk + 1) / 2 + 31) / 32 * 32, 0, st, xx, yy, D, ldx, ldy, w, bb, sh, sc, mod_stride,
                                                                                rows_per_batch, rms, eps);
   else if (nchunk > 768) OMNI_NM_WARP(4, 8);
@@ -665,7 +669,9 @@ extern "C" int omni_qk_norm_rope_pages(void* qkv, int B, int S, int H, int Hkv, 
     if (pairs <= 2L * 64 * sm_count())
       launch_with(!wt.counter, 1, qk_norm_rope128_kernel, (unsigned)((pairs + 7) / 8), 256, 0, st, r, wt, status);
     else
-      launch_with(!wt.counter, 1, qk_norm_rope128_rows_kernel, (unsigned)((rows + 7) / 8), 256, 0, st, r, wt, status);
+      // An ordinary launch: with many blocks, those that start while the last of a GEMM still hold their SMs are dealt out unevenly
+      // (projection and this kernel, overlapped: 2000 rows of 32 / 4 heads 46.5 us, 8192 of 32 / 8 184.7)
+      launch_with(false, 1, qk_norm_rope128_rows_kernel, (unsigned)((rows + 7) / 8), 256, 0, st, r, wt, status);
   } else if (D == 128)
     qk_norm_rope_kernel<128><<<grid, wpb * 32, 0, st>>>(q, B, S, H, Hkv, ld, a, b, c, d, s_alt, cosb, sinb, interleaved, eps, positions);
   else if (D == 64)
