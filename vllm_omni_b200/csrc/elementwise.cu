@@ -711,8 +711,11 @@ extern "C" int omni_silu_mul(const void* x, void* y, long rows, int N, int ldx, 
   if ((N & 7) || (ldx & 7) || (ldy & 7)) return RC_BAD_ARG;
   const long nchunk = rows * (N >> 3);
   long blocks = (nchunk + 255) / 256;
-  if (blocks > 148 * 16) blocks = 148 * 16;
-  launch_overlapped(silu_mul_kernel, (unsigned)blocks, 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)x, (__nv_bfloat16*)y, rows, N, ldx, ldy);
+  const bool full = blocks > 148 * 16;
+  if (full) blocks = 148 * 16;
+  // More blocks than the device holds at once: an ordinary launch, because blocks that start while a GEMM's last ones hold their SMs are dealt out
+  // unevenly (norm, 2048 -> 2 x 6144, this, 6144 -> 2048, 4096 rows: 258 us, overlapped 266; 600 rows 70.5 and 70.0)
+  launch_with(!full, 1, silu_mul_kernel, (unsigned)blocks, 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)x, (__nv_bfloat16*)y, rows, N, ldx, ldy);
   return (int)cudaGetLastError();
 }
 
