@@ -38,7 +38,7 @@ def test_against_64_bits(n, h, w, cin, cout, epilogue):
 
 
 @pytest.mark.parametrize("channels", [8, 32, 40, 64, 96, 128, 136, 192, 256, 264, 384, 512, 520, 1024])
-@pytest.mark.parametrize("pixels", [1, 77, 4099])
+@pytest.mark.parametrize("pixels", [1, 77, 2369, 4099, 4736, 9472, 9473, 18944, 18945, 37889])     # lanes per pixel change at 256 * SMs / lanes
 def test_rmsnorm_silu(channels, pixels):
     g = torch.Generator(device="cuda").manual_seed(channels + pixels)
     x, gamma = torch.randn(pixels, channels, generator=g, device="cuda").bfloat16(), torch.randn(channels, generator=g, device="cuda").bfloat16()

@@ -16,8 +16,8 @@
 
 namespace omni {
 
-// C % 8 == 0, C <= 1024.  LANES lanes per pixel with up to 4 chunks of 8 channels each, so that every lane has work at the decoders' widths (96 channels are
-// 12 chunks: with a warp per pixel 20 of 32 lanes idle).  1024 x 1024 pixels of 96 channels (403 MB): 73 us, with a warp per pixel 322 us.
+// C % 8 == 0, C <= 1024.  LANES lanes per pixel with up to 4 chunks of 8 channels each: of many pixels every lane has work at the decoders' widths (96
+// channels are 12 chunks: with a warp per pixel 20 of 32 lanes idle).  1024 x 1024 pixels of 96 channels (403 MB): 73 us, with a warp per pixel 322 us.
 template <int LANES>
 __global__ void __launch_bounds__(256)
 rmsnorm_silu_nhwc_kernel(const __nv_bfloat16* __restrict__ x, long ldx, const __nv_bfloat16* __restrict__ gamma,
@@ -276,12 +276,18 @@ extern "C" int omni_rmsnorm_silu_nhwc(const void* x, long ldx, const void* gamma
   launch_overlapped(rmsnorm_silu_nhwc_kernel<L>, (unsigned)((pixels * L + 255) / 256), 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)x, ldx, \
                     (const __nv_bfloat16*)gamma, (__nv_bfloat16*)y, ldy, pixels, C, apply_silu)
   const int chunks = C >> 3;
-  if (chunks <= 4) OMNI_RMS(1);
-  else if (chunks <= 8) OMNI_RMS(2);
-  else if (chunks <= 16) OMNI_RMS(4);
-  else if (chunks <= 32) OMNI_RMS(8);
-  else if (chunks <= 64) OMNI_RMS(16);
-  else OMNI_RMS(32);
+  // as few lanes as hold a pixel, or, where those would be less than a block per SM, up to a lane per chunk (us, fewest lanes in brackets:
+  // 256 pixels of 64 channels 2.0 (3.0), of 256 2.1 (2.9), 4096 of 64 2.3 (3.1); two blocks per SM: 8192 of 64 2.9, one 2.3)
+  int lanes = 1;
+  while (lanes < 32 && (lanes * 4 < chunks || (lanes < chunks && pixels * lanes < 256L * sm_count()))) lanes *= 2;
+  switch (lanes) {
+    case 1: OMNI_RMS(1); break;
+    case 2: OMNI_RMS(2); break;
+    case 4: OMNI_RMS(4); break;
+    case 8: OMNI_RMS(8); break;
+    case 16: OMNI_RMS(16); break;
+    default: OMNI_RMS(32);
+  }
 #undef OMNI_RMS
   return (int)cudaGetLastError();
 }
