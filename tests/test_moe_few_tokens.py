@@ -93,30 +93,8 @@ def test_expert_rows(act, T):
     assert same.sum() >= T - 4 and ((y - ref).abs() <= bound + 0.01 * ref.abs())[same].all()
 
 
-@pytest.mark.parametrize("n_pairs,E,lo,hi", [(1, 1, 0, 1), (5000, 128, 0, 128), (3000, 7, 2, 5), (2048, 1024, 0, 1024), (70001, 64, 0, 64)])
-def test_compact_plan(n_pairs, E, lo, hi):
-    g = torch.Generator(device="cuda").manual_seed(n_pairs)
-    ids = (torch.rand(n_pairs, generator=g, device="cuda") ** 2 * E).int().clamp(max=E - 1)
-    tiles = E + n_pairs // 128 + 1
-    row, te, t0, tn, n = (torch.full((m,), -7, dtype=torch.int32, device="cuda") for m in (n_pairs, tiles, tiles, tiles, 1))
-    from ctypes import c_int
-    nv.check_rc(nv.lib("moe").omni_moe_plan_compact(nv.ptr(ids), c_int(n_pairs), c_int(E), c_int(lo), c_int(hi), c_int(tiles), nv.ptr(row),
-                                                    nv.ptr(te), nv.ptr(t0), nv.ptr(tn), nv.ptr(n), nv.stream_ptr()), "plan")
-    local = (ids >= lo) & (ids < hi)
-    assert int(n) == int(local.sum()) and (row[~local] == -1).all()
-    assert torch.equal(row[local].sort().values, torch.arange(int(n), device="cuda", dtype=torch.int32))
-    of_row = torch.empty(int(n), dtype=torch.int32, device="cuda")
-    of_row[row[local].long()] = ids[local]
-    assert torch.equal(of_row, of_row.sort().values)                            # experts in order, rows back to back
-    at = 0
-    for e, r0, rn in zip(te.tolist(), t0.tolist(), tn.tolist()):
-        if e >= 0:
-            assert r0 == at and 1 <= rn <= 128 and (of_row[r0:r0 + rn] == e).all()
-            at += rn
-    assert at == int(n)
-
-
-@pytest.mark.parametrize("n_pairs,E,lo,hi,tile", [(1, 1, 0, 1, 64), (5000, 128, 0, 128, 64), (3000, 7, 2, 5, 128), (70001, 64, 0, 64, 256), (1300, 4, 1, 4, 256)])
+@pytest.mark.parametrize("n_pairs,E,lo,hi,tile", [(1, 1, 0, 1, 64), (5000, 128, 0, 128, 64), (5000, 128, 0, 128, 128), (3000, 7, 2, 5, 128), (2048, 1024, 0, 1024, 128),
+                                                     (70001, 64, 0, 64, 256), (70001, 64, 0, 64, 128), (1300, 4, 1, 4, 256)])
 def test_even_plan(n_pairs, E, lo, hi, tile):
     g = torch.Generator(device="cuda").manual_seed(n_pairs)
     ids = (torch.rand(n_pairs, generator=g, device="cuda") ** 2 * E).int().clamp(max=E - 1)
@@ -126,8 +104,11 @@ def test_even_plan(n_pairs, E, lo, hi, tile):
     nv.check_rc(nv.lib("moe").omni_moe_plan_tiles(nv.ptr(ids), c_int(n_pairs), c_int(E), c_int(lo), c_int(hi), c_int(tile), c_int(tiles), nv.ptr(row),
                                                   nv.ptr(te), nv.ptr(t0), nv.ptr(tn), nv.ptr(n), nv.stream_ptr()), "plan")
     local = (ids >= lo) & (ids < hi)
+    assert int(n) == int(local.sum()) and (row[~local] == -1).all()
+    assert torch.equal(row[local].sort().values, torch.arange(int(n), device="cuda", dtype=torch.int32))
     of_row = torch.empty(int(local.sum()), dtype=torch.int32, device="cuda")
     of_row[row[local].long()] = ids[local] - lo
+    assert torch.equal(of_row, of_row.sort().values)                            # experts in order, rows back to back
     at, used = 0, True
     for e, r0, rn in zip(te.tolist(), t0.tolist(), tn.tolist()):
         used = used and e >= 0

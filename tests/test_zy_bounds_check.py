@@ -79,12 +79,21 @@ ids = torch.tensor([0, 1, 2, 9, 3, 3, 7, 0], dtype=torch.int32, device=dev)
 rop = torch.empty(8, dtype=torch.int32, device=dev)
 te, t0, tr = (torch.empty(16, dtype=torch.int32, device=dev) for _ in range(3))
 nr = torch.zeros(1, dtype=torch.int32, device=dev)
-nv.check_rc(lib.omni_moe_plan_compact(nv.ptr(ids), c_int(8), c_int(E), c_int(0), c_int(E), c_int(16), nv.ptr(rop),
-                                      nv.ptr(te), nv.ptr(t0), nv.ptr(tr), nv.ptr(nr), nv.stream_ptr()), "plan")
+nv.check_rc(lib.omni_moe_plan_tiles(nv.ptr(ids), c_int(8), c_int(E), c_int(0), c_int(E), c_int(128), c_int(16), nv.ptr(rop),
+                                    nv.ptr(te), nv.ptr(t0), nv.ptr(tr), nv.ptr(nr), nv.stream_ptr()), "plan")
 torch.cuda.synchronize()
 code = int(st.item())
 assert code & 0xff == 9 and (code >> 8) & 0xff == 3, hex(code)
 assert int(nr.item()) == 7 and int(rop[3].item()) == -1
+st.zero_()
+# the same in the plan of few tokens, with ids given
+por = torch.full((8,), -5, dtype=torch.int32, device=dev)
+nv.check_rc(lib.omni_moe_few_plan(None, c_int(0), c_int(4), c_int(E), c_int(2), c_int(1), c_int(0), c_int(E), nv.ptr(ids), None, nv.ptr(por),
+                                  nv.ptr(rop), nv.ptr(te), nv.ptr(t0), nv.ptr(tr), c_int(8), nv.stream_ptr()), "few plan")
+torch.cuda.synchronize()
+code = int(st.item())
+assert code & 0xff == 9 and (code >> 8) & 0xff == 3, hex(code)
+assert rop.tolist() == [0, 1, 2, -1, 4, 5, 6, 7] and sorted(por[:7].tolist()) == [0, 1, 2, 4, 5, 6, 7] and int(por[7].item()) == -5
 st.zero_()
 print("BOUNDS-OK")
 """

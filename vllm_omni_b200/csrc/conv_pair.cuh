@@ -28,7 +28,7 @@ struct Conv3Cfg {
   static constexpr int OUT_BYTES = STAGED ? TN * 2 * C3_W * C3_H : 0;        // a tile's outputs, two of them
   static constexpr int FIT = (220 * 1024 - 2 * OUT_BYTES) / STAGE_BYTES, STAGES = FIT < 6 ? FIT : 6;
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 2 * OUT_BYTES + 1024;
-  static constexpr int ACC_STRIDE = TN <= 32 ? 32 : (TN <= 64 ? 64 : (TN <= 128 ? 128 : 256));
+  static constexpr int ACC_STRIDE = TN <= 32 ? 32 : (TN <= 128 ? 128 : 256);
   static constexpr int TMEM_COLS = 2 * ACC_STRIDE;
 };
 

@@ -387,11 +387,11 @@ __device__ __forceinline__ void block_scan2(int& a, int& b, int& total_a, int& t
 }
 
 // Plan without padding: the rows of expert e are [off[e], off[e] + cnt[e]); expert e owns c = ceil(cnt[e] / tile)
-// tiles of about cnt[e] / c rows (rounded up to 16); tile t = (expert, first row, rows).  Unused tiles get expert -1.  With global_ids
-// tiles are full but for an expert's last, and name experts as `ids` does; else as the local weights do, from 0.  One block; the place of a pair among its expert's
-// rows is what its atomic add to the expert's count returns (the order inside an expert does not affect results).
+// tiles of about cnt[e] / c rows (rounded up to 16); tile t = (expert as the local weights number them, first row, rows).  Unused tiles get
+// expert -1.  One block; the place of a pair among its expert's rows is what its atomic add to the expert's count returns (the order
+// inside an expert does not affect results).
 __global__ void __launch_bounds__(1024)
-moe_plan_compact_kernel(const int* __restrict__ ids, int n_pairs, int E, int e_lo, int e_hi, int tile_cap, int global_ids, int max_tiles,
+moe_plan_tiles_kernel(const int* __restrict__ ids, int n_pairs, int E, int e_lo, int e_hi, int tile_cap, int max_tiles,
                         int* __restrict__ row_of_pair, int* __restrict__ tile_expert, int* __restrict__ tile_row0,
                         int* __restrict__ tile_rows, int* __restrict__ n_rows_out, MoeBounds bd) {
   pdl_begin();
@@ -408,13 +408,13 @@ moe_plan_compact_kernel(const int* __restrict__ ids, int n_pairs, int E, int e_l
   }
   __syncthreads();
   const int e = threadIdx.x, mine = cnt[e];             // experts past E have none
-  const int own = (mine + tile_cap - 1) / tile_cap, size = global_ids ? tile_cap : own ? ((mine + own - 1) / own + 15) / 16 * 16 : 0;
+  const int own = (mine + tile_cap - 1) / tile_cap, size = own ? ((mine + own - 1) / own + 15) / 16 * 16 : 0;
   int row = mine, tile = own, rows, tiles;
   block_scan2(row, tile, rows, tiles);
   off[e] = row;
   if (e == 0) *n_rows_out = rows;
   for (int i = 0; i < own; ++i) {                       // never empty: (own - 1) * size < mine, as tile_cap is a multiple of 64
-    tile_expert[tile + i] = global_ids ? e : e - e_lo;
+    tile_expert[tile + i] = e - e_lo;
     tile_row0[tile + i] = row + i * size;
     tile_rows[tile + i] = min(size, mine - i * size);
   }
@@ -435,7 +435,7 @@ moe_plan_compact_kernel(const int* __restrict__ ids, int n_pairs, int E, int e_l
 // Up to a few hundred (token, choice) pairs the chain is the streaming of the chosen experts' weights plus launches, so it has three
 // instead of seven: plan (with the choice, from router logits), up projection with SwiGLU, down projection.  Rows are gathered
 // where they are read and results lie at their pair's index, so nothing is copied; a tile is at most 16 rows of one expert.
-constexpr int FEW_TILE = 16, FEW_PAIRS = 2048;
+constexpr int FEW_TILE = 16, FEW_PAIRS = 1024;          // no more pairs than experts (ops/moe.py), of which the plan takes 1024
 struct FewPlan {
   int *ids;                       // [pairs]: read, or written when the choice is made here
   float* weights;                 // [pairs], written with the choice
@@ -463,39 +463,31 @@ moe_few_plan_kernel(const __nv_bfloat16* __restrict__ logits, int ld, int T, int
         p.weights[t * k + lane] = w;
       }
     }
-  } else {
-    for (int i = threadIdx.x; i < n_pairs; i += 1024) sid[i] = p.ids[i];
+  } else if (threadIdx.x < n_pairs) {
+    sid[threadIdx.x] = p.ids[threadIdx.x];
   }
   __syncthreads();
-  int place[FEW_PAIRS / 1024];
-#pragma unroll
-  for (int q = 0; q < FEW_PAIRS / 1024; ++q) {
-    const int i = threadIdx.x + q * 1024;
-    place[q] = -1;
-    if (i < n_pairs) {
-      const int e = sid[i];
-      if (OMNI_IN_BOUNDS(e >= 0 && e < E, bd.status, KID_MOE_PLAN) && e >= e_lo && e < e_hi) place[q] = atomicAdd(&cnt[e], 1);
-      p.row_of_pair[i] = place[q] >= 0 ? i : -1;
-    }
+  const int i = threadIdx.x;
+  int place = -1;
+  if (i < n_pairs) {
+    const int e = sid[i];
+    if (OMNI_IN_BOUNDS(e >= 0 && e < E, bd.status, KID_MOE_PLAN) && e >= e_lo && e < e_hi) place = atomicAdd(&cnt[e], 1);
+    p.row_of_pair[i] = place >= 0 ? i : -1;
   }
   __syncthreads();
   const int e = threadIdx.x, mine = cnt[e];
   int row = mine, tile = (mine + FEW_TILE - 1) / FEW_TILE, rows, tiles;
   block_scan2(row, tile, rows, tiles);
-  for (int i = 0; i * FEW_TILE < mine; ++i) {
-    p.tile_expert[tile + i] = e - e_lo;                 // the weights hold the local experts
-    p.tile_row0[tile + i] = row + i * FEW_TILE;
-    p.tile_rows[tile + i] = min(FEW_TILE, mine - i * FEW_TILE);
+  for (int q = 0; q * FEW_TILE < mine; ++q) {
+    p.tile_expert[tile + q] = e - e_lo;                 // the weights hold the local experts
+    p.tile_row0[tile + q] = row + q * FEW_TILE;
+    p.tile_rows[tile + q] = min(FEW_TILE, mine - q * FEW_TILE);
   }
   for (int t = tiles + threadIdx.x; t < p.max_tiles; t += 1024) p.tile_expert[t] = -1;
   __syncthreads();                                      // everyone has its count: the array becomes the first rows
   cnt[e] = row;
   __syncthreads();
-#pragma unroll
-  for (int q = 0; q < FEW_PAIRS / 1024; ++q) {
-    const int i = threadIdx.x + q * 1024;
-    if (i < n_pairs && place[q] >= 0) p.pair_of_row[cnt[sid[i]] + place[q]] = i;
-  }
+  if (place >= 0) p.pair_of_row[cnt[sid[i]] + place] = i;
 }
 
 // y[pair, n] = act(sum_c W[e, n, c] x[pair / per, c]) for a tile of one expert and 16 columns (GATED: 8 columns n of silu(gate) * lift, rows
@@ -788,25 +780,13 @@ extern "C" int omni_moe_plan(const int* ids, int n_pairs, int E, int e_lo, int e
   return (int)cudaGetLastError();
 }
 
-static int plan_tiles_as(const int* ids, int n_pairs, int E, int e_lo, int e_hi, int tile_cap, int global_ids, int max_tiles,
-                         int* row_of_pair, int* tile_expert, int* tile_row0, int* tile_rows, int* n_rows_out, void* stream) {
-  if (E > 1024) return RC_BAD_ARG;
-  launch_overlapped(moe_plan_compact_kernel, 1, 1024, 0, (cudaStream_t)stream, ids, n_pairs, E, e_lo, e_hi, tile_cap, global_ids, max_tiles,
-                    row_of_pair, tile_expert, tile_row0, tile_rows, n_rows_out, g_moe_bounds);
-  return (int)cudaGetLastError();
-}
-
-// Tiles of 128 rows; max_tiles: at least min(E, n_pairs) + n_pairs / 128.
-extern "C" int omni_moe_plan_compact(const int* ids, int n_pairs, int E, int e_lo, int e_hi, int max_tiles, int* row_of_pair,
-                                     int* tile_expert, int* tile_row0, int* tile_rows, int* n_rows_out, void* stream) {
-  return plan_tiles_as(ids, n_pairs, E, e_lo, e_hi, MOE_TILE, 1, max_tiles, row_of_pair, tile_expert, tile_row0, tile_rows, n_rows_out, stream);
-}
-
 // Even tiles of at most tile_cap (64, 128 or 256) rows for omni_gemm_bf16_experts; max_tiles: at least min(E, n_pairs) + n_pairs / tile_cap.
 extern "C" int omni_moe_plan_tiles(const int* ids, int n_pairs, int E, int e_lo, int e_hi, int tile_cap, int max_tiles, int* row_of_pair,
                                    int* tile_expert, int* tile_row0, int* tile_rows, int* n_rows_out, void* stream) {
-  if (tile_cap != 64 && tile_cap != 128 && tile_cap != 256) return RC_BAD_ARG;
-  return plan_tiles_as(ids, n_pairs, E, e_lo, e_hi, tile_cap, 0, max_tiles, row_of_pair, tile_expert, tile_row0, tile_rows, n_rows_out, stream);
+  if (E > 1024 || (tile_cap != 64 && tile_cap != 128 && tile_cap != 256)) return RC_BAD_ARG;
+  launch_overlapped(moe_plan_tiles_kernel, 1, 1024, 0, (cudaStream_t)stream, ids, n_pairs, E, e_lo, e_hi, tile_cap, max_tiles, row_of_pair,
+                    tile_expert, tile_row0, tile_rows, n_rows_out, g_moe_bounds);
+  return (int)cudaGetLastError();
 }
 
 // Plan of at most FEW_PAIRS pairs.  `logits` bf16 [T, E] (E <= 256, k <= 16): the choice is made here, ids and weights are outputs; null:

@@ -88,7 +88,7 @@ def _tile_rows(T, k, E) -> int:
     return 64 if T * k <= 32 * E else 128 if T * k <= 64 * E else 256
 
 
-FEW_TILE, FEW_PAIRS = 16, 2048          # csrc/moe.cu
+FEW_TILE, FEW_PAIRS = 16, 1024          # csrc/moe.cu
 
 
 def _few_tiles(T, k, E):
