@@ -7,7 +7,7 @@
 //            a group of 8 rows of the MMA operand is the 8 pixels of one image row, so tap dy is the box from its (dy + 1)-th group on
 //   weights  each CTA of a pair holds half of the TN output channels' weights and the pair's MMA reads both
 // A channel block of which only some channels exist (96 = 64 + 32) issues the K steps that hold any.  Per 64 channels and three taps
-// a CTA takes in 18 KB + 3 * 64 * TN bytes, 0.35 of the one-CTA kernel's 2 * 3 * (16 KB + 128 * TN) / 2 at TN = 96.
+// a CTA takes in 18 KB + 3 * 64 * TN bytes, 36 KB at TN = 96; the one-CTA kernel, whose narrowest tile has 128 columns, 3 * (16 KB + 16 KB).
 // With residual, one-CTA kernel before: 1024 x 1024 pixels, 96 -> 96 channels 211 us (461), 192 -> 96 257 us (662), 96 -> 8 127 us (743);
 // 512 x 512, 192 -> 192 160 us (193), 384 -> 192 221 us (350); 256 x 256, 384 -> 384 119 us (180).
 // Up to 96 output channels the epilogue was what a tile waited for (16 -> 96 took as long as 96 -> 96): a lane's 16 bytes at the pitch of a

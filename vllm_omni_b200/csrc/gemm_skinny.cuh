@@ -83,11 +83,11 @@ __device__ __forceinline__ void skinny_finish(float (&x)[B], int m, int step, in
 template <int NT, int NW, int U, int BLOCKS>
 __global__ void __launch_bounds__(32 * NW, BLOCKS)
 gemm_rows_kernel(const __nv_bfloat16* __restrict__ A, int lda, const __nv_bfloat16* __restrict__ W, int ldw, __nv_bfloat16* C, int ldc,
-                 int M, int N, int K, const __grid_constant__ GemmEpilogue epi) {
+                 int M, int N, int K, const __grid_constant__ GemmEpilogue epi, int resident) {
   __shared__ float part[NW][NT * 8][16];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, j = lane & 3;
   const int n0 = blockIdx.x * 16;
-  if (blockIdx.x < BLOCKS * 148) {              // W does not come from the kernel before: the first blocks' share is on its way to L2 meanwhile
+  if ((int)blockIdx.x < resident) {             // W does not come from the kernel before: the first blocks' share is on its way to L2 meanwhile
     const __nv_bfloat16* w = W + (size_t)min(n0 + (int)(threadIdx.x & 15), N - 1) * ldw;
     for (int c = (threadIdx.x >> 4) * 64; c < K; c += 2 * NW * 64) prefetch_l2(w + c);
   }
@@ -134,13 +134,13 @@ static void launch_rows(int tiles, const __nv_bfloat16* A, int lda, const __nv_b
                         int N, int K, const GemmEpilogue& epi, cudaStream_t stream) {
   constexpr int U = NT == 1 ? 8 : 4;
   const int sms = sm_count(), last = tiles % (4 * sms);
-  const auto go = [&](auto kernel, int warps) {
-    launch_overlapped(kernel, tiles, 32 * warps, 0, stream, A, lda, W, ldw, C, ldc, M, N, K, epi);
+  const auto go = [&](auto kernel, int warps, int blocks) {
+    launch_overlapped(kernel, tiles, 32 * warps, 0, stream, A, lda, W, ldw, C, ldc, M, N, K, epi, blocks * sms);
   };
-  if (tiles <= sms && K > 1024) go(gemm_rows_kernel<NT, 16, U, 1>, 16);
-  else if (tiles > 2 * sms && tiles <= 3 * sms) go(gemm_rows_kernel<NT, 8, U / 2, 3>, 8);
-  else if (NT == 2 && tiles > 3 * sms && (last == 0 || last >= 2 * sms)) go(gemm_rows_kernel<NT, 4, U, 4>, 4);
-  else go(gemm_rows_kernel<NT, 8, U, 2>, 8);
+  if (tiles <= sms && K > 1024) go(gemm_rows_kernel<NT, 16, U, 1>, 16, 1);
+  else if (tiles > 2 * sms && tiles <= 3 * sms) go(gemm_rows_kernel<NT, 8, U / 2, 3>, 8, 3);
+  else if (NT == 2 && tiles > 3 * sms && (last == 0 || last >= 2 * sms)) go(gemm_rows_kernel<NT, 4, U, 4>, 4, 4);
+  else go(gemm_rows_kernel<NT, 8, U, 2>, 8, 2);
 }
 
 static int launch_rows(const void* A, int lda, const void* W, int ldw, __nv_bfloat16* C, int ldc, int M, int N, int K,

@@ -90,7 +90,7 @@ inline int ensure_dynamic_smem(const void* fn, int bytes, unsigned long long& ma
   return 0;
 }
 
-// Launch of a kernel that begins with pdl_trigger / pdl_wait (ptx_sm100.cuh): its blocks may become resident and set themselves up
+// Launch of a kernel that begins with pdl_wait, then pdl_trigger (ptx_sm100.cuh): its blocks may become resident and set themselves up
 // while the kernel before it in the stream runs out.  `cluster` > 1: blocks per cluster along x, for kernels without __cluster_dims__.
 // overlap = false: an ordinary launch.
 template <typename... Params, typename... Args>
