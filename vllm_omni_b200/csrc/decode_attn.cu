@@ -272,14 +272,14 @@ paged_decode_merge_kernel(const float* __restrict__ part_o, const float* __restr
 
 constexpr int DA_MAX_PARTS = 64;
 
-// Shares of a sequence's keys: about `target` warps in all, at least two tiles of 16 keys each.  Twelve warps fit an SM; up to two rounds
-// of them even out lengths, but every share costs a sum to write and to read.  20 per SM, 16 to 16 heads of 1 to 16 KV heads, 1 to 256
-// sequences of 64 to 32768 keys: 1.5 % below 24 and 2 % below 16 in the mean, and nowhere above the tensor-core kernel (24: up to 1.11
-// of it for 72 sequences of 1024 keys in tables of 4096; 16 rounds off a whole one for few sequences).  A single sequence has at most
+// Shares of a sequence's keys: about `target` warps in all, at least two tiles of 16 keys each.  Twelve warps fit an SM; two rounds of them
+// even out lengths (8 sequences of 4096 keys, 8 KV heads: 20 warps per SM 1.05 and 18 1.12 times as long as 24).  Blocks of fewer KV
+// heads hold shares of one sequence, whose sums are many and small: 20, since 24 took 1.11 times the tensor-core kernel's time for 72
+// sequences of 1024 keys in tables of 4096 and 1 KV head, and 20 never more than 1.01 of it.  A single sequence has at most
 // 64 shares: 131072 keys of 4 KV heads take 148 us, the tensor-core kernel 246 (the copy rate would be 41; more shares would reach more SMs).
 static void plan_shares(int n, int Hkv, int max_keys, int& splits, int& subs) {
   subs = Hkv < DA_WARPS ? DA_WARPS / Hkv : 1;
-  const long warps = (long)n * Hkv, target = 20L * sm_count();
+  const long warps = (long)n * Hkv, target = (Hkv < DA_WARPS ? 20L : 24L) * sm_count();
   const int tiles = (max_keys + DA_KEYS - 1) / DA_KEYS;
   long parts = (target + warps - 1) / warps;
   if (parts > tiles / 2) parts = tiles / 2;
