@@ -91,3 +91,16 @@ def _heads_and_pages(rows, heads, kv, interleaved, gains=True):
     r = plain.view(rows, -1)
     KC.kv_write(r[:, heads * D:(heads + kv) * D].view(rows, kv, D), r[:, (heads + kv) * D:].view(rows, kv, D), k2, v2, slots)
     assert torch.equal(kc, k2) and torch.equal(vc, v2)
+
+
+def test_more_slots_than_rows():
+    """A slot mapping may be longer than the batch, as the page-writing kernel takes it."""
+    D, g, rows = 128, _gen(3), 5
+    qkv = torch.randn(1, rows, 4 * D, generator=g, device="cuda").bfloat16()
+    slots = torch.tensor([3, -1, 0, 17, 9, 30, 31], dtype=torch.int32, device="cuda")
+    pages = [torch.full((2, 16, 1, D), 9.0, device="cuda", dtype=torch.bfloat16) for _ in range(2)]
+    fused.qk_norm_rope_(qkv, 2, 1, D, pages=(*pages, slots))
+    want = [torch.full((2, 16, 1, D), 9.0, device="cuda", dtype=torch.bfloat16) for _ in range(2)]
+    r = qkv.view(rows, 4, D)
+    KC.kv_write(r[:, 2:3], r[:, 3:], *want, slots)
+    assert torch.equal(pages[0], want[0]) and torch.equal(pages[1], want[1])

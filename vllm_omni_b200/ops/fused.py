@@ -137,7 +137,7 @@ def qk_norm_rope_(qkv, H, Hkv, D, wq=None, wk=None, wq_alt=None, wk_alt=None, s_
             rows = qkv.view(B * S, -1)
             kv_write(rows[:, H * D:(H + Hkv) * D].view(B * S, Hkv, D), rows[:, (H + Hkv) * D:].view(B * S, Hkv, D), kc, vc, slots)
             return qkv
-        assert slots.dtype == torch.int32 and slots.is_contiguous() and slots.numel() == B * S
+        assert slots.dtype == torch.int32 and slots.is_contiguous() and slots.numel() >= B * S        # as kv_write: the rows' come first
         assert kc.is_contiguous() and vc.is_contiguous() and kc.shape[2:] == (Hkv, D) == vc.shape[2:] and kc.dtype == vc.dtype == qkv.dtype
     if not qkv.is_cuda:
         qkv.copy_(qk_norm_rope_reference(qkv, H, Hkv, D, wq, wk, wq_alt, wk_alt, s_alt, cos, sin, interleaved, eps, positions))
