@@ -319,9 +319,8 @@ qk_norm_rope128_kernel(const __grid_constant__ HeadRows a, PeerWait wt, int* sta
   if (h < all) store_head(a, row, h, l16, a.pages.k ? a.pages.slots[row] : -1, v, o);
 }
 
-// The same for many rows: a warp walks the query heads of its row, 8 at a time, then key and value heads, and fetches gains and rotation
-// coefficients once.  After the projection that makes the rows, both together in us: 2000 rows of 32 / 4 heads, 2048 wide, 44.9; gains kept
-// as bf16 and chosen per head 45.7, two heads to a warp 50.0; 8192 rows of 32 / 8 180.2, 182.7 and 206.1.
+// The same for many rows: a warp walks all heads of its row, 8 at a time, and fetches gains and rotation coefficients once; steps of
+// query heads alone neither choose a gain nor look for a page.
 __global__ void __launch_bounds__(256)
 qk_norm_rope128_rows_kernel(const __grid_constant__ HeadRows a, PeerWait wt, int* status) {
   pdl_begin();
@@ -347,28 +346,35 @@ qk_norm_rope128_rows_kernel(const __grid_constant__ HeadRows a, PeerWait wt, int
   rope_coefficients(a, row, s, l16, cs, sn);
   const int page = a.pages.k ? a.pages.slots[row] : -1;
   constexpr int U = 4;
-  // heads lo .. hi - 1; both halves of the warp take every step, whether or not their last heads exist: head_norm_rope exchanges values
-  // over the whole warp
-  const auto span = [&](int lo, int hi, const float (&gain)[8], bool queries) {
+  // Both halves of the warp take every step, whether or not their last heads exist: head_norm_rope exchanges values over the whole warp.
+  uint4 v[U];
+  int h0 = 0;
 #pragma unroll 1
-    for (int h0 = lo; h0 < hi; h0 += 2 * U) {
-      uint4 v[U];
+  for (; h0 + 2 * U <= a.H; h0 += 2 * U) {                 // query heads alone
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int h = h0 + 2 * u + hsel;
-        v[u] = h < hi ? *reinterpret_cast<const uint4*>(a.qkv + (size_t)row * a.ld + (size_t)h * 128 + l16 * 8) : make_uint4(0u, 0u, 0u, 0u);
-      }
+    for (int u = 0; u < U; ++u) v[u] = *reinterpret_cast<const uint4*>(a.qkv + (size_t)row * a.ld + (size_t)(h0 + 2 * u + hsel) * 128 + l16 * 8);
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int h = h0 + 2 * u + hsel;
-        const uint4 o = head_norm_rope(v[u], a.wq != nullptr, gain, a.cosb != nullptr, a.interleaved, cs, sn, a.eps);
-        if (h < hi && queries) *reinterpret_cast<uint4*>(a.qkv + (size_t)row * a.ld + (size_t)h * 128 + l16 * 8) = o;
-        else if (h < hi) store_head(a, row, h, l16, page, v[u], o);
-      }
+    for (int u = 0; u < U; ++u)
+      *reinterpret_cast<uint4*>(a.qkv + (size_t)row * a.ld + (size_t)(h0 + 2 * u + hsel) * 128 + l16 * 8) =
+          head_norm_rope(v[u], a.wq != nullptr, gq, a.cosb != nullptr, a.interleaved, cs, sn, a.eps);
+  }
+#pragma unroll 1
+  for (; h0 < all; h0 += 2 * U) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int h = h0 + 2 * u + hsel;
+      v[u] = h < all ? *reinterpret_cast<const uint4*>(a.qkv + (size_t)row * a.ld + (size_t)h * 128 + l16 * 8) : make_uint4(0u, 0u, 0u, 0u);
     }
-  };
-  span(0, a.H, gq, true);
-  span(a.H, all, gk, false);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int h = h0 + 2 * u + hsel;
+      float gain[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) gain[e] = h < a.H ? gq[e] : gk[e];
+      const uint4 o = head_norm_rope(v[u], a.wq != nullptr, gain, a.cosb != nullptr, a.interleaved, cs, sn, a.eps);
+      if (h < all) store_head(a, row, h, l16, page, v[u], o);
+    }
+  }
 }
 
 // ------------------------------------------------------------------ qk norm + rope
@@ -670,7 +676,8 @@ extern "C" int omni_qk_norm_rope_pages(void* qkv, int B, int S, int H, int Hkv, 
       launch_with(!wt.counter, 1, qk_norm_rope128_kernel, (unsigned)((pairs + 7) / 8), 256, 0, st, r, wt, status);
     else
       // An ordinary launch: with many blocks, those that start while the last of a GEMM still hold their SMs are dealt out unevenly
-      // (projection and this kernel, overlapped: 2000 rows of 32 / 4 heads 46.5 us, 8192 of 32 / 8 184.7)
+      // (projection and this kernel, in brackets overlapped: 2000 rows of 32 / 4 heads 45.0 us (46.5), 8192 of 32 / 8 181.1 (184.7); two
+      // heads to a warp 50.0 and 206)
       launch_with(false, 1, qk_norm_rope128_rows_kernel, (unsigned)((rows + 7) / 8), 256, 0, st, r, wt, status);
   } else if (D == 128)
     qk_norm_rope_kernel<128><<<grid, wpb * 32, 0, st>>>(q, B, S, H, Hkv, ld, a, b, c, d, s_alt, cosb, sinb, interleaved, eps, positions);
