@@ -109,3 +109,14 @@ def test_fill_takes_whole_rows_only():
     assert not r._fill_once(st, b)
     with pytest.raises(RuntimeError):
         r._fill(st, b)
+
+
+def test_positions_of_two_axes_keep_the_general_form():
+    """Sections of two axes (the one-launch form has three): the tables of the general form, as before there was another."""
+    m = _decoder(False)
+    m.cfg.mrope_section = (40, 24)
+    pos = torch.arange(10, device="cuda").view(2, 5)
+    ids = torch.arange(5, device="cuda")
+    x, cos, sin = m.rows_and_rotation(ModelBatch(ids, pos, None))
+    c, s = m.rope.cos_sin_for(pos, m.cfg.mrope_section, False)
+    assert torch.equal(x, m.embed_tokens[ids]) and torch.equal(cos, c) and torch.equal(sin, s)

@@ -307,10 +307,10 @@ class QwenDecoderModel(nn.Module):
     def rows_and_rotation(self, batch: ModelBatch):
         """(x [T, D], cos, sin): ``embed`` and the rotation tables, on a GPU in one launch where the operands allow."""
         cfg, pos, got = self.cfg, batch.positions, None
-        if self.embed_tokens.is_cuda and (pos.dim() == 1 or cfg.mrope_section is not None):
+        if self.embed_tokens.is_cuda and (pos.dim() == 1 or (pos.shape[0] == 3 and len(cfg.mrope_section or ()) == 3)):
             dev = pos.device
             axis = self.rope.axis_on(dev, cfg.mrope_section, cfg.mrope_interleaved) if pos.dim() > 1 else None
-            if axis is None or (axis.numel() == self.rope.head_dim // 2 and pos.shape[0] == 3):
+            if axis is None or axis.numel() == self.rope.head_dim // 2:
                 got = token_rows(batch.input_ids, self.embed_tokens, pos, self.rope.freq_on(dev), axis, batch.input_embeds,
                                  batch.embeds_mask)
         if got is not None:
