@@ -1,5 +1,6 @@
 """Kernels that are resident while the kernel before them still writes (pdl_wait in csrc/ptx_sm100.cuh) read its results by ordinary
-loads: ld.global.nc is for memory that nothing writes during the kernel's lifetime."""
+loads: ld.global.nc is for memory that nothing writes during the kernel's lifetime.  The compiler chooses it for parameters declared
+const and __restrict__."""
 import re
 
 import pytest
@@ -7,8 +8,24 @@ import pytest
 from vllm_omni_b200.build import CSRC
 
 TEXT = {f.name: re.sub(r"//[^\n]*", "", f.read_text()) for f in sorted([*CSRC.glob("*.cu"), *CSRC.glob("*.cuh")])}
+# parameters and first lines of every kernel
+KERNELS = {f"{n}:{m[1]}": (m[2], m[3]) for n, t in TEXT.items()
+           for m in re.finditer(r"__global__ void[^;{]*?\b(\w+_kernel)\(([^{;]*?)\)\s*\{(.*?)(?=__global__|\Z)", t, re.S)}
+OVERLAPPED = [k for k, (_, body) in KERNELS.items() if "pdl_wait" in body or "pdl_begin" in body]
 
 
 @pytest.mark.parametrize("name", [n for n, t in TEXT.items() if "pdl_wait" in t or "pdl_begin" in t])
 def test_no_read_only_loads(name):
     assert "__ldg" not in TEXT[name] and "ld.global.nc" not in TEXT[name]
+
+
+def test_overlapped_kernels_are_found():
+    launched = {k for t in TEXT.values() for k in re.findall(r"launch_(?:overlapped|with)\([^;]*?\b(\w+_kernel)\b", t)}
+    assert len(OVERLAPPED) > 30 and launched <= {k.split(":")[1] for k in OVERLAPPED} | {"kernel"}
+
+
+@pytest.mark.parametrize("kernel", OVERLAPPED)
+def test_no_parameter_that_may_be_read_that_way(kernel):
+    # the channel norm keeps them: 1024 x 1024 pixels of 96 channels took 69.1 us without and 65.5 with; its loads come after the wait
+    allowed = {"x", "gamma"} if kernel == "vae_ops.cu:rmsnorm_silu_nhwc_kernel" else set()
+    assert set(re.findall(r"\bconst\s+[\w:]+\s*\*\s*(?:const\s+)?__restrict__\s+(\w+)", KERNELS[kernel][0])) <= allowed

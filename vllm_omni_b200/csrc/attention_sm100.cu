@@ -149,7 +149,7 @@ template <int NH, int HD>
 __global__ void __launch_bounds__(ATT_THREADS, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, AttnOut out, int Sq, int Skv, int H, int Hkv,
-                const int* __restrict__ kv_lens, float scale_log2, int causal, int q_offset, AttnPaging pg,
+                const int* kv_lens, float scale_log2, int causal, int q_offset, AttnPaging pg,
                 PeerSignal sig, int* status) {
   constexpr int ATT_TILE_BYTES = AttCfg<HD>::TILE_BYTES;
   constexpr int KV_STAGES = AttCfg<HD>::STAGES;

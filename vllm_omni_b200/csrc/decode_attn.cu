@@ -219,7 +219,7 @@ paged_decode_kernel(const __grid_constant__ DecodeAttn p) {
 // out[seq, h] = sum_s 2^(m_s - m*) O_s / sum_s 2^(m_s - m*) l_s over a row's shares (at most 64): one block per row, its warps take
 // every fourth share, four channels per lane.
 __global__ void __launch_bounds__(128)
-paged_decode_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml, int parts, int H,
+paged_decode_merge_kernel(const float* part_o, const float* part_ml, int parts, int H,
                           __nv_bfloat16* __restrict__ out, long o_rs) {
   pdl_begin();
   __shared__ float4 part[4][32];

@@ -48,9 +48,9 @@ __device__ __forceinline__ float warp_sum(float v) {
 // warp per row with all chunks unrolled: 18).
 template <int CPT>
 __global__ void __launch_bounds__(512)
-norm_modulate_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, int D, int ldx, int ldy,
-                     const __nv_bfloat16* __restrict__ weight, const __nv_bfloat16* __restrict__ bias,
-                     const __nv_bfloat16* __restrict__ shift, const __nv_bfloat16* __restrict__ scale, int mod_stride,
+norm_modulate_kernel(const __nv_bfloat16* x, __nv_bfloat16* __restrict__ y, int D, int ldx, int ldy,
+                     const __nv_bfloat16* weight, const __nv_bfloat16* bias,
+                     const __nv_bfloat16* shift, const __nv_bfloat16* scale, int mod_stride,
                      int rows_per_batch, int rms, float eps) {
   pdl_begin();
   __shared__ float2 red[16];
@@ -120,10 +120,10 @@ norm_modulate_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restr
 // 200 KB per SM) did not help: 16 warps issue too little.
 template <int VPL, int WPR>
 __global__ void __launch_bounds__(256)
-norm_modulate_warp_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, int rows,
-                          int D, int ldx, int ldy, const __nv_bfloat16* __restrict__ weight,
-                          const __nv_bfloat16* __restrict__ bias, const __nv_bfloat16* __restrict__ shift,
-                          const __nv_bfloat16* __restrict__ scale, int mod_stride, int rows_per_batch,
+norm_modulate_warp_kernel(const __nv_bfloat16* x, __nv_bfloat16* __restrict__ y, int rows,
+                          int D, int ldx, int ldy, const __nv_bfloat16* weight,
+                          const __nv_bfloat16* bias, const __nv_bfloat16* shift,
+                          const __nv_bfloat16* scale, int mod_stride, int rows_per_batch,
                           int rms, float eps) {
   pdl_begin();
   __shared__ float2 red[8];
@@ -457,7 +457,7 @@ qk_norm_rope_kernel(__nv_bfloat16* __restrict__ qkv, int B, int S, int H, int Hk
 // lat_bf16: bf16 copy of the updated latents for the next transformer call.
 // One warp per row.  neg == nullptr means no guidance (v = pos).
 __global__ void __launch_bounds__(256)
-cfg_euler_kernel(const __nv_bfloat16* __restrict__ pos, const __nv_bfloat16* __restrict__ neg,
+cfg_euler_kernel(const __nv_bfloat16* pos, const __nv_bfloat16* neg,
                  float* __restrict__ lat, __nv_bfloat16* __restrict__ lat_bf16, long rows, int C,
                  float guidance, float dt, int renorm) {
   pdl_begin();
@@ -497,7 +497,7 @@ cfg_euler_kernel(const __nv_bfloat16* __restrict__ pos, const __nv_bfloat16* __r
 
 // ------------------------------------------------------------------------ SwiGLU
 __global__ void __launch_bounds__(256)
-silu_mul_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, long rows, int N,
+silu_mul_kernel(const __nv_bfloat16* x, __nv_bfloat16* __restrict__ y, long rows, int N,
                 int ldx, int ldy) {
   pdl_begin();
   const long nchunk = (long)rows * (N >> 3);

@@ -82,7 +82,7 @@ __device__ __forceinline__ void skinny_finish(float (&x)[B], int m, int step, in
 // NT * 8 rows of A; 16 resident warps x U chunks x 1 KB = up to 128 KB of W in flight per SM.
 template <int NT, int NW, int U, int BLOCKS>
 __global__ void __launch_bounds__(32 * NW, BLOCKS)
-gemm_rows_kernel(const __nv_bfloat16* __restrict__ A, int lda, const __nv_bfloat16* __restrict__ W, int ldw, __nv_bfloat16* C, int ldc,
+gemm_rows_kernel(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W, int ldw, __nv_bfloat16* C, int ldc,
                  int M, int N, int K, const __grid_constant__ GemmEpilogue epi, int resident) {
   __shared__ float part[NW][NT * 8][16];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, j = lane & 3;

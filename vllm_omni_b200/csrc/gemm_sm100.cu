@@ -257,7 +257,7 @@ template <int BN>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  __nv_bfloat16* __restrict__ C, int ldc, int M, int N, int K, GemmEpilogue epi,
-                 const int* __restrict__ tile_expert, ConvGeom conv, PeerSignal sig, PeerWait wt, int* status) {
+                 const int* tile_expert, ConvGeom conv, PeerSignal sig, PeerWait wt, int* status) {
   using Cfg = GemmCfg<BN>;
   constexpr int STAGES = Cfg::STAGES;
 

@@ -651,7 +651,7 @@ rotary_heads_kernel(const RotaryHeads p) {
 // ------------------------------------------------------------------------------ tanh of columns
 template <typename T>
 __global__ void __launch_bounds__(256)
-tanh_cols_kernel(const T* __restrict__ in, long ldi, T* __restrict__ out, long rows, int n) {
+tanh_cols_kernel(const T* in, long ldi, T* __restrict__ out, long rows, int n) {
   pdl_begin();
   const int vec = n / 8;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < rows * vec; i += (long)gridDim.x * blockDim.x) {
@@ -668,7 +668,7 @@ tanh_cols_kernel(const T* __restrict__ in, long ldi, T* __restrict__ out, long r
 // ------------------------------------------------------------------------------ logit cap
 template <typename T>
 __global__ void __launch_bounds__(256)
-logit_softcap_kernel(const T* __restrict__ in, long ldi, float* __restrict__ out, long ldo, long rows, int V, float cap, float mult) {
+logit_softcap_kernel(const T* in, long ldi, float* __restrict__ out, long ldo, long rows, int V, float cap, float mult) {
   pdl_begin();
   const long total = rows * V;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {

@@ -76,7 +76,7 @@ __device__ __forceinline__ void route_token(const __nv_bfloat16* __restrict__ lo
 
 // one warp per token
 __global__ void __launch_bounds__(256)
-moe_route_kernel(const __nv_bfloat16* __restrict__ logits, int ld, int T, int E, int k, int renorm,
+moe_route_kernel(const __nv_bfloat16* logits, int ld, int T, int E, int k, int renorm,
                  int* __restrict__ ids, float* __restrict__ weights) {
   pdl_begin();
   const int t = blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -207,8 +207,8 @@ moe_topk_kernel(const float* __restrict__ logits, long ld, int T, int E, int k, 
 // sides.
 template <int MT, int NW>
 __global__ void __launch_bounds__(32 * NW)
-moe_router_kernel(const __nv_bfloat16* __restrict__ x, long ldx, const __nv_bfloat16* __restrict__ w, long ldw,
-                  const float* __restrict__ bias, int T, int D, int E, int Ep, int k, RouterRule rule,
+moe_router_kernel(const __nv_bfloat16* x, long ldx, const __nv_bfloat16* w, long ldw,
+                  const float* bias, int T, int D, int E, int Ep, int k, RouterRule rule,
                   int* __restrict__ ids, float* __restrict__ weights) {
   pdl_begin();
   extern __shared__ float sm[];
@@ -391,7 +391,7 @@ __device__ __forceinline__ void block_scan2(int& a, int& b, int& total_a, int& t
 // expert -1.  One block; the place of a pair among its expert's rows is what its atomic add to the expert's count returns (the order
 // inside an expert does not affect results).
 __global__ void __launch_bounds__(1024)
-moe_plan_tiles_kernel(const int* __restrict__ ids, int n_pairs, int E, int e_lo, int e_hi, int tile_cap, int max_tiles,
+moe_plan_tiles_kernel(const int* ids, int n_pairs, int E, int e_lo, int e_hi, int tile_cap, int max_tiles,
                         int* __restrict__ row_of_pair, int* __restrict__ tile_expert, int* __restrict__ tile_row0,
                         int* __restrict__ tile_rows, int* __restrict__ n_rows_out, MoeBounds bd) {
   pdl_begin();
@@ -445,7 +445,7 @@ struct FewPlan {
 };
 
 __global__ void __launch_bounds__(1024)
-moe_few_plan_kernel(const __nv_bfloat16* __restrict__ logits, int ld, int T, int E, int k, int renorm, int e_lo, int e_hi,
+moe_few_plan_kernel(const __nv_bfloat16* logits, int ld, int T, int E, int k, int renorm, int e_lo, int e_hi,
                     const FewPlan p, MoeBounds bd) {
   pdl_begin();
   __shared__ int sid[FEW_PAIRS];
@@ -494,9 +494,9 @@ moe_few_plan_kernel(const __nv_bfloat16* __restrict__ logits, int ld, int T, int
 // n and N + n of W are the two halves of the MMA's 16).  The block's NW warps share the contraction.
 template <int NW, bool GATED>
 __global__ void __launch_bounds__(32 * NW, 16 / NW)
-moe_few_rows_kernel(const __nv_bfloat16* __restrict__ x, long ldx, int per, const __nv_bfloat16* __restrict__ w, int N, int K,
-                    const int* __restrict__ tile_expert, const int* __restrict__ tile_row0, const int* __restrict__ tile_rows,
-                    const int* __restrict__ pair_of_row, __nv_bfloat16* __restrict__ y, long ldy, int relu2) {
+moe_few_rows_kernel(const __nv_bfloat16* x, long ldx, int per, const __nv_bfloat16* w, int N, int K,
+                    const int* tile_expert, const int* tile_row0, const int* tile_rows,
+                    const int* pair_of_row, __nv_bfloat16* __restrict__ y, long ldy, int relu2) {
   pdl_begin();
   __shared__ float part[NW][FEW_TILE][16];
   constexpr int COLS = GATED ? 8 : 16;
@@ -544,7 +544,7 @@ moe_few_rows_kernel(const __nv_bfloat16* __restrict__ x, long ldx, int per, cons
 // x: [T, D] (pitch ldx) -> xp[row_of_pair[t*k+j], :] ; rows not written stay as they are (the GEMM
 // output rows of padding are never read back)
 __global__ void __launch_bounds__(256)
-moe_dispatch_kernel(const __nv_bfloat16* __restrict__ x, long ldx, const int* __restrict__ row_of_pair, int n_pairs,
+moe_dispatch_kernel(const __nv_bfloat16* x, long ldx, const int* row_of_pair, int n_pairs,
                     int k, int D, __nv_bfloat16* __restrict__ xp, MoeBounds bd) {
   pdl_begin();
   const int chunks = D >> 3;
@@ -571,7 +571,7 @@ __device__ __forceinline__ void add_pairs(float (&acc)[8], const __nv_bfloat16* 
       const int r = j0 + i < k ? rows[j0 + i] : -1;
       const bool in = r >= 0 && OMNI_IN_BOUNDS(bd.max_rows == 0 || r < bd.max_rows, bd.status, KID_MOE_COMBINE);
       wj[i] = in ? w[j0 + i] : 0.f;
-      u[i] = in ? *reinterpret_cast<const uint4*>(y + (size_t)r * D + c) : make_uint4(0u, 0u, 0u, 0u);
+      u[i] = in ? ld_stream(y + (size_t)r * D + c) : make_uint4(0u, 0u, 0u, 0u);
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -585,8 +585,8 @@ __device__ __forceinline__ void add_pairs(float (&acc)[8], const __nv_bfloat16* 
 // out[t, :] = (residual[t, :]) + sum_j w[t,j] * y[row(t,j), :]; pairs with row < 0 (experts of
 // another rank) contribute nothing.
 __global__ void __launch_bounds__(256)
-moe_combine_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict__ row_of_pair,
-                   const float* __restrict__ weights, int T, int k, int D, const __nv_bfloat16* __restrict__ residual,
+moe_combine_kernel(const __nv_bfloat16* y, const int* row_of_pair,
+                   const float* weights, int T, int k, int D, const __nv_bfloat16* residual,
                    long ldr, __nv_bfloat16* __restrict__ out, long ldo, MoeBounds bd) {
   pdl_begin();
   const int chunks = D >> 3;
@@ -613,9 +613,9 @@ moe_combine_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict__ 
 // rows again for many.  Four layers of 128 experts (2048 -> 768, top 8) and their attention: one sequence 249 -> 239 us per step, 64 sequences
 // 1190 -> 1159 us.
 __global__ void __launch_bounds__(1024)
-moe_combine_norm_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict__ row_of_pair, const float* __restrict__ weights, int k, int D,
-                        const __nv_bfloat16* __restrict__ residual, long ldr, __nv_bfloat16* __restrict__ out, long ldo,
-                        const __nv_bfloat16* __restrict__ gain, float eps, __nv_bfloat16* __restrict__ normed, long ldn, MoeBounds bd) {
+moe_combine_norm_kernel(const __nv_bfloat16* y, const int* row_of_pair, const float* weights, int k, int D,
+                        const __nv_bfloat16* residual, long ldr, __nv_bfloat16* __restrict__ out, long ldo,
+                        const __nv_bfloat16* gain, float eps, __nv_bfloat16* __restrict__ normed, long ldn, MoeBounds bd) {
   pdl_begin();
   __shared__ float red[32];
   const int t = blockIdx.x, c = threadIdx.x * 8, warps = blockDim.x >> 5;

@@ -152,7 +152,7 @@ stream_step_kernel(const StreamStep p) {
 
 // out[t, i] = mag (cos, sin) of pos[t] * freq[i]
 __global__ void __launch_bounds__(256)
-rotary_rows_kernel(const long* __restrict__ pos, const double* __restrict__ freq, float mag, float2* __restrict__ out, int T,
+rotary_rows_kernel(const long* pos, const double* freq, float mag, float2* __restrict__ out, int T,
                    int half) {
   pdl_begin();
   const long n = (long)T * half;
