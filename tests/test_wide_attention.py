@@ -1,0 +1,55 @@
+"""Attention of one 384-channel head (csrc/attn_wide_sm100.cu) against softmax(q k^T) v in 64 bits."""
+import pytest
+import torch
+
+from vllm_omni_b200.ops import _native as nv
+from vllm_omni_b200.ops import conv as C
+
+pytestmark = pytest.mark.gpu
+
+
+def _exact(q, k, v):
+    q, k, v = q.double(), k.double(), v.double()
+    return torch.softmax(q @ k.transpose(1, 2) * q.shape[2] ** -0.5, -1) @ v
+
+
+# rows below, at and past a tile of 256 and a step of 128 keys; runs of work that begin and end inside tiles (workers not a multiple of the tiles)
+@pytest.mark.parametrize("B,N,workers", [(1, 1, 0), (1, 63, 0), (1, 64, 0), (1, 127, 0), (1, 128, 0), (1, 129, 2), (2, 256, 0), (2, 257, 7), (1, 1000, 0), (1, 1024, 5),
+                                         (3, 700, 33), (1, 4099, 74), (1, 4099, 17), (1, 4099, 0), (2, 9999, 0)])
+def test_wide_attention(B, N, workers):
+    g = torch.Generator(device="cuda").manual_seed(N)
+    t = torch.randn(B, N, 3, 384, device="cuda", generator=g).bfloat16()
+    t[..., :2, :] *= 3.0                                   # scores of several units: row maxima grow, weights are uneven
+    q, k, v = t[:, :, 0], t[:, :, 1], t[:, :, 2]
+    out = C._wide_head_flash(q, k, v, 384 ** -0.5, workers)
+    torch.cuda.synchronize()
+    nv.check_status(q.device)
+    ref = _exact(q, k, v)
+    # probabilities and results are bf16 (2^-9 each, at worst aligned), the exponentials 2^-22
+    assert (out.double() - ref).norm() <= 2 ** -8 * ref.norm()
+    assert (out.double() - ref).abs().max() <= 2 ** -7 * v.abs().max()
+
+
+def test_wide_attention_growing_maxima():
+    """Keys sorted by their score: every step raises the maximum by more than the kernel lets pass without rescaling."""
+    N = 640
+    g = torch.Generator(device="cuda").manual_seed(1)
+    d = torch.randn(384, device="cuda", generator=g)
+    q = (d + 0.1 * torch.randn(1, N, 384, device="cuda", generator=g)).bfloat16()
+    k = (torch.linspace(-6, 6, N, device="cuda")[None, :, None] * d).bfloat16()
+    v = torch.randn(1, N, 384, device="cuda", generator=g).bfloat16()
+    ref = _exact(q, k, v)
+    for workers in (0, 11):
+        out = C._wide_head_flash(q, k, v, 384 ** -0.5, workers)
+        torch.cuda.synchronize()
+        nv.check_status(q.device)
+        assert (out.double() - ref).norm() <= 2 ** -8 * ref.norm()
+
+
+def test_wide_attention_width_outside_the_kernel():
+    """512 channels stay with the two GEMMs around the row softmax, whose scores pass through bf16 as well."""
+    g = torch.Generator(device="cuda").manual_seed(2)
+    q, k, v = (torch.randn(1, 520, 512, device="cuda", generator=g).bfloat16() for _ in range(3))
+    out, ref = C.wide_head_attention(q, k, v, chunk_rows=256), _exact(q, k, v)
+    nv.check_status(q.device)
+    assert (out.double() - ref).norm() <= 2 ** -7 * ref.norm()

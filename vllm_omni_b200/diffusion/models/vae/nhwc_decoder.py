@@ -3,8 +3,8 @@
 Built from a ``Decoder2d`` (same parameters, repacked once): every convolution is an implicit
 GEMM on the tcgen05 kernel with bias / residual in its epilogue, RMS-norm + SiLU is one fused
 kernel per pixel row, activations stay NHWC bf16 from the latent to the image.  The single
-mid-block attention (one head of width C, outside the flash kernel's head sizes) is two GEMMs on the
-same kernel around a row-softmax kernel (``ops.conv.wide_head_attention``).  Replaces the cuDNN path the
+mid-block attention (one head of width C, outside the flash kernel's head sizes) is one launch at 384 channels and two GEMMs
+around a row-softmax kernel at other widths (``ops.conv.wide_head_attention``).  Replaces the cuDNN path the
 reference takes through diffusers (vllm_omni/diffusion/models/qwen_image/
 autoencoder_kl_qwenimage.py).
 """

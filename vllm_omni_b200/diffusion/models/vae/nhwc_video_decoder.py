@@ -6,7 +6,7 @@ launches of the 2-D implicit-GEMM kernel: tap ``j`` convolves the frames shifted
 past with the weight slice ``W[:, :, j]`` and accumulates into the same output through the kernel's residual
 operand (the block's skip connection rides on the first tap), so the whole convolution is tensor-core GEMM
 work with K = k*k*Cin per launch and no im2col.  RMS-norm + SiLU is one fused kernel per pixel row, the
-per-frame mid-block attention is two GEMMs around a row softmax (``ops.conv.wide_head_attention``), nearest
+per-frame mid-block attention is ``ops.conv.wide_head_attention``, nearest
 up-sampling and the layout changes are this library's element-wise kernels.
 
 Latent frames are decoded in chunks exactly like the PyTorch module does: every causal convolution keeps the

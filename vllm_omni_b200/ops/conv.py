@@ -310,15 +310,38 @@ def softmax_rows_(x: torch.Tensor, scale: float = 1.0) -> torch.Tensor:
     return x
 
 
+WIDE_HEAD = 384          # csrc/attn_wide_sm100.cu
+
+
+def _wide_head_flash(q, k, v, scale, workers: int = 0):
+    """Scores, softmax and P v in one launch (csrc/attn_wide_sm100.cu); ``workers``: CTA pairs that share the work (0: by size)."""
+    B, N, C = q.shape
+    lib = nv.lib("attn_wide_sm100")
+    need = c_long(0)
+    if not workers:
+        workers = lib.omni_attn_wide_workers(c_int(B), c_int(N), ctypes.byref(need))
+    else:
+        need = c_long(workers * 4 * 128 * (C + 2))
+    out = torch.empty(B, N, C, dtype=q.dtype, device=q.device)
+    scratch = torch.empty(need.value, dtype=torch.float32, device=q.device) if need.value else None
+    ops = [a for t in (q, k, v, out) for a in (nv.ptr(t), c_long(t.stride(1)), c_long(t.stride(0) if B > 1 else N * t.stride(1)))]
+    nv.check_rc(lib.omni_attn_wide(*ops, c_int(B), c_int(N), c_int(C), ctypes.c_float(scale), c_int(workers), nv.ptr(scratch),
+                                   nv.ptr(nv.status_word(q.device)), nv.stream_ptr()), "omni_attn_wide")
+    return out
+
+
 def wide_head_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, chunk_rows: int = 4096) -> torch.Tensor:
     """One attention head whose width is the channel count (the VAE mid block: 384 or 512), which the flash
-    kernel's head sizes do not cover.  q, k, v: [B, N, C] bf16 views with the last dim contiguous.  On a GPU:
-    scores = q k^T on the tcgen05 GEMM for ``chunk_rows`` queries at a time, row softmax in place, P v on the
-    GEMM again against v transposed once; the score block (chunk_rows x N bf16) is the only scratch."""
+    kernel's head sizes do not cover.  q, k, v: [B, N, C] bf16 views with the last dim contiguous.  On a GPU: 384 channels in
+    one launch (csrc/attn_wide_sm100.cu); otherwise scores = q k^T on the tcgen05 GEMM for ``chunk_rows`` queries at a time, row softmax
+    in place, P v on the GEMM again against v transposed once; the score block (chunk_rows x N bf16) is the only scratch."""
     B, N, C = q.shape
     scale = C ** -0.5
     if not q.is_cuda or q.dtype != torch.bfloat16 or N % 8 or C % 8:
         return F.scaled_dot_product_attention(q[:, None], k[:, None], v[:, None])[:, 0]
+    if C == WIDE_HEAD and all(t.stride(2) == 1 and t.stride(1) % 8 == 0 and (B == 1 or t.stride(0) % 8 == 0) and t.data_ptr() % 16 == 0
+                              for t in (q, k, v)):
+        return _wide_head_flash(q, k, v, scale)
     from .gemm import linear
     out = torch.empty(B, N, C, dtype=q.dtype, device=q.device)
     rows = min(chunk_rows, N)
