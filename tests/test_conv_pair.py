@@ -47,3 +47,30 @@ def test_rmsnorm_silu(channels, pixels):
         y, ref = C.rmsnorm_silu_nhwc(x, gamma, silu=silu), F.silu(z) if silu else z
         # one rounding to bf16 of fp32 arithmetic; tanh.approx in silu
         assert ((y.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + z.abs() * 2.0 ** -11 * silu + 1e-5).all()
+
+
+# both places where the epilogue makes the norm (a thread has all channels of a pixel; two threads share them), widths that leave columns of a tile empty, a
+# width whose channels span tiles (norm of its own); one image that is doubled in place, several and flat ones that are not
+@pytest.mark.parametrize("cin,cout", [(96, 96), (16, 24), (192, 96), (40, 192), (192, 136), (64, 384), (72, 3)])
+@pytest.mark.parametrize("n,h,w,up", [(1, 64, 80, False), (1, 33, 41, True), (1, 16, 8, True), (2, 33, 41, False), (2, 20, 24, True), (1, 5, 400, True)])
+@pytest.mark.parametrize("residual", [False, True])
+def test_norm_and_doubling_in_the_launch(n, h, w, up, cin, cout, residual):
+    g = torch.Generator(device="cuda").manual_seed(n * h + w + cin)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    x, wt = rnd(n, h, w, (cin + 7) // 8 * 8), rnd(cout, cin, 3, 3) * (9 * cin) ** -0.5
+    pw, pb = C.pack_conv_weight(wt, rnd(cout))
+    gamma = rnd(pw.shape[0])
+    s = 2 if up else 1
+    res = rnd(n, s * h, s * w, pw.shape[0]) if residual else None
+    want = C.conv2d_nhwc(x.repeat_interleave(s, 1).repeat_interleave(s, 2), pw, pb, 3, cin, residual=res)       # the same products in the same order
+    for silu in (True, False):
+        norm = C.rmsnorm_silu_nhwc(want, gamma, silu=silu).double()
+        for keep in (True, False):
+            y, z = C.conv3x3_norm_nhwc(x, pw, pb, cin, residual=res, up=up, gamma=gamma, silu=silu, keep=keep)
+            nv.check_status()
+            assert torch.equal(y, want) if keep else y is None or torch.equal(y, want)
+            # sums of squares in another order may round the other way: one unit in the last place of bf16
+            assert ((z.double() - norm).abs() <= norm.abs() * 2.0 ** -7 + 1e-6).all()
+    y, z = C.conv3x3_norm_nhwc(x, pw, pb, cin, residual=res, up=up)
+    assert z is None and torch.equal(y, want)
+    assert torch.equal(want[..., cout:], torch.zeros_like(want[..., cout:]) if res is None else res[..., cout:])

@@ -1,46 +1,55 @@
 // 3 x 3 convolution, stride 1, zero padding, channels-last, as an implicit GEMM on CTA pairs (cta_group::2).
 //
 // What bounds the one-CTA kernel (gemm_bf16_kernel) here is the way from L2 to shared memory: it fetches the pixels of a tile once per tap
-// and the weights once per 128 pixels, 32 to 40 KB per 64 channels and tap, 1.6 to 2 times what an SM takes in while its MMAs run.  This
-// kernel fetches both less often:
-//   pixels   a tile is 16 x 8 pixels per CTA; one TMA box of 18 x 8 pixels (one column offset dx, 64 channels) serves the three taps (dy, dx):
-//            a group of 8 rows of the MMA operand is the 8 pixels of one image row, so tap dy is the box from its (dy + 1)-th group on
-//   weights  each CTA of a pair holds half of the TN output channels' weights and the pair's MMA reads both
-// A channel block of which only some channels exist (96 = 64 + 32) issues the K steps that hold any.  Per 64 channels and three taps
-// a CTA takes in 18 KB + 3 * 64 * TN bytes, 36 KB at TN = 96; the one-CTA kernel, whose narrowest tile has 128 columns, 3 * (16 KB + 16 KB).
-// With residual, one-CTA kernel before: 1024 x 1024 pixels, 96 -> 96 channels 211 us (461), 192 -> 96 257 us (662), 96 -> 8 127 us (743);
-// 512 x 512, 192 -> 192 160 us (193), 384 -> 192 221 us (350); 256 x 256, 384 -> 384 119 us (180).
-// Up to 96 output channels the epilogue was what a tile waited for (16 -> 96 took as long as 96 -> 96): a lane's 16 bytes at the pitch of a
-// pixel fill half a sector.  Results and residuals therefore move as boxes by TMA: 268 -> 211 us, 317 -> 257 us, 145 -> 127 us in the order
-// above.  Wider outputs have MMAs enough to hide it behind and no shared memory to spare.
+// and the weights once per 128 pixels.  This kernel fetches both less often:
+//   pixels   a tile is 16 x 8 pixels per CTA; ONE TMA box of 18 x 10 pixels (64 channels) serves all nine taps: a group of 8 rows of the MMA
+//            operand is 8 neighbouring pixels of an image row, 128 bytes each, groups lie one box row (1280 bytes) apart, and a tap is the
+//            operand that begins some rows and pixels further into the box (the swizzle goes by address, not by operand row)
+//   weights  each CTA of a pair holds half of the TN output channels' weights and the pair's MMA reads both; where all of a layer's weights fit
+//            beside the tiles they are fetched once per CTA, otherwise tap by tap through a ring
+// A channel block of which only some channels exist (96 = 64 + 32) issues the K steps that hold any.
+// Results leave, and residuals arrive, as boxes by TMA through shared memory: a lane's 16 bytes at the pitch of a pixel fill half a sector.
+// Where a tile holds all channels of its pixels, the RMS norm (+ SiLU) that follows is made there as well, beside or instead of the result.
+// An image that is to be doubled first (nearest neighbour) is read as it is: output pixels of one parity of (y, x) see, tap by tap, the same
+// shifted box of the small image, so a tile takes 16 x 8 pixels of one parity.
+//
+// us with residual where it says +, in brackets the form before, with a box per dx, weights by the ring and results of wide tiles by plain stores:
+// 1024 x 1024 pixels, 96 -> 96 channels 143 (179), + 176 (206), 192 -> 96 250 (261), 96 -> 8 86 (116); 512 x 512, 192 -> 192 110 (128), + 120 (153),
+// 384 -> 192 205 (220); 256 x 256, 384 -> 384 + 106 (117).  Without epilogue and loads the MMAs of 96 -> 96 take 109.
 #pragma once
+#include <type_traits>
 
 namespace omni {
 
 constexpr int C3_W = 8, C3_H = 16;                       // pixels of a CTA's tile
-constexpr int C3_A_BYTES = (C3_H + 2) * C3_W * 128;      // 18 groups of 8 pixels x 64 channels
+constexpr int C3_BOX_ROW = (C3_W + 2) * 128;             // a box row: 10 pixels x 64 channels
+constexpr int C3_PX_BYTES = (C3_H + 2) * C3_BOX_ROW, C3_PX_STAGE = (C3_PX_BYTES + 1023) / 1024 * 1024;
+constexpr int C3_MAX_PX = 8, C3_MAX_W = 16;              // stages of the pixel and the weight ring
 
 template <int TN>
 struct Conv3Cfg {
-  static constexpr int B_BYTES = (TN / 2) * 128;         // one tap's weights of this CTA's half
-  static constexpr int STAGE_BYTES = C3_A_BYTES + 3 * B_BYTES;
-  static constexpr bool STAGED = TN <= 96;               // results leave, and the residual arrives, by TMA through shared memory
-  static constexpr int OUT_BYTES = STAGED ? TN * 2 * C3_W * C3_H : 0;        // a tile's outputs, two of them
-  static constexpr int FIT = (220 * 1024 - 2 * OUT_BYTES) / STAGE_BYTES, STAGES = FIT < 6 ? FIT : 6;
-  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 2 * OUT_BYTES + 1024;
+  static constexpr int W_BYTES = (TN / 2) * 128;         // one tap's weights of this CTA's half, 64 channels
+  static constexpr int TAPS = TN <= 128 ? 3 : 1;         // per stage of the weight ring: narrow MMAs are over before the next wait is through
+  static constexpr int TEAMS = TN <= 96 ? 2 : 1;         // narrow: four warps have the even tiles and four the odd ones; wide: half of the columns each
+  static constexpr int COLS = TN / (3 - TEAMS);          // columns per epilogue thread
+  static constexpr int OUT_BYTES = TN * 2 * C3_W * C3_H; // a tile's outputs
+  static constexpr int FIXED = TEAMS * OUT_BYTES + (TEAMS == 1 ? 1024 : 0) + 1024;      // + half rows' sums of squares, alignment
+  static constexpr int DYN_MAX = 231424;
   static constexpr int ACC_STRIDE = TN <= 32 ? 32 : (TN <= 128 ? 128 : 256);
   static constexpr int TMEM_COLS = 2 * ACC_STRIDE;
 };
 
 struct Conv3Args {
-  CUtensorMap tmX, tmW, tmY, tmR;         // Y, residual: 32 channels of a tile
-  __nv_bfloat16* y;
-  int ldy;
+  CUtensorMap tmX, tmW, tmY, tmR, tmZ;    // Y, Z (norm), residual: 32 channels of a tile
   // The image as the tiles see it: rows of W pixels, H of them, in tiles of 16 x 8.  An image that is flat (see conv3_flat) is seen with
-  // its columns as rows: the maps swap the two, tap (dy, dx) is weight dy * tap_y + dx and pixel (y, x) is y * px_y + x * px_x.
-  int H, W, n_img, tiles_x, tiles_y;
+  // its columns as rows: the maps swap the two, tap (dy, dx) is weight dy * tap_y + dx * tap_x and pixel (y, x) is y * px_y + x * px_x.
+  // up: H and W are those of the small image, and every tile exists for the four parities of output pixels.
+  int H, W, n_img, tiles_x, tiles_y, up;
   int tap_y, tap_x, px_y, px_x;
   int Cout, cin, cin_blocks;
+  int px_stages, w_stages;
+  int has_y, norm_silu;
+  const __nv_bfloat16* gamma;             // of the norm; null: none
   GemmEpilogue epi;
 };
 
@@ -50,17 +59,17 @@ __device__ __forceinline__ void add8(float (&f)[8], const uint4& u) {
   f[4] += c.x; f[5] += c.y; f[6] += d.x; f[7] += d.y;
 }
 
+// not inlined: few convolutions have one, and its code would crowd the instruction cache
+__device__ __noinline__ float conv3_act(float x, int act) {
+  if (act == ACT_GELU_TANH) return gelu_tanh(x);
+  if (act == ACT_SILU) return silu(x);
+  return act == ACT_RELU2 ? fmaxf(x, 0.f) * fmaxf(x, 0.f) : x;
+}
 __device__ __forceinline__ void conv3_finish(float (&f)[8], const GemmEpilogue& epi, int col) {
   if (epi.bias) add8(f, *reinterpret_cast<const uint4*>(epi.bias + col));
-  if (epi.act == ACT_GELU_TANH) {
-#pragma unroll
-    for (int e = 0; e < 8; ++e) f[e] = gelu_tanh(f[e]);
-  } else if (epi.act == ACT_SILU) {
-#pragma unroll
-    for (int e = 0; e < 8; ++e) f[e] = silu(f[e]);
-  } else if (epi.act == ACT_RELU2) {
-#pragma unroll
-    for (int e = 0; e < 8; ++e) f[e] = fmaxf(f[e], 0.f) * fmaxf(f[e], 0.f);
+  if (epi.act != ACT_NONE) {
+    f[0] = conv3_act(f[0], epi.act); f[1] = conv3_act(f[1], epi.act); f[2] = conv3_act(f[2], epi.act); f[3] = conv3_act(f[3], epi.act);
+    f[4] = conv3_act(f[4], epi.act); f[5] = conv3_act(f[5], epi.act); f[6] = conv3_act(f[6], epi.act); f[7] = conv3_act(f[7], epi.act);
   }
 }
 
@@ -72,47 +81,50 @@ __device__ __forceinline__ uint4 lds128(uint32_t addr) {
 __device__ __forceinline__ void sts128(uint32_t addr, const uint4& v) {
   asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
-__device__ __forceinline__ void tma_store_4d(const CUtensorMap* tmap, uint32_t src, int c0, int c1, int c2, int c3) {
-  asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
+__device__ __forceinline__ void tma_store_5d(const CUtensorMap* tmap, uint32_t src, int c0, int c1, int c2, int c3, int c4) {
+  asm volatile("cp.async.bulk.tensor.5d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5, %6}], [%1];"
                :
-               : "l"(reinterpret_cast<uint64_t>(tmap)), "r"(src), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+               : "l"(reinterpret_cast<uint64_t>(tmap)), "r"(src), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
                : "memory");
 }
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
-template <int TN>
+// RESIDENT: all weights stay in shared memory
+template <int TN, bool RESIDENT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
 conv3x3_pair_kernel(const __grid_constant__ Conv3Args a, int* status) {
   using Cfg = Conv3Cfg<TN>;
-  constexpr int STAGES = Cfg::STAGES;
+  constexpr int TEAMS = Cfg::TEAMS, COLS = Cfg::COLS, GROUP_BYTES = C3_W * C3_H * 64;
   extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t full_bar[STAGES];
-  __shared__ __align__(8) uint64_t empty_bar[STAGES];
-  __shared__ __align__(8) uint64_t tfull_bar[2];
-  __shared__ __align__(8) uint64_t tempty_bar[2];
-  __shared__ __align__(8) uint64_t res_bar[2];
+  __shared__ __align__(8) uint64_t px_full[C3_MAX_PX], px_empty[C3_MAX_PX], w_full[C3_MAX_W], w_empty[C3_MAX_W];
+  __shared__ __align__(8) uint64_t tfull_bar[2], tempty_bar[2], res_bar[2];
   __shared__ uint32_t tmem_base_s;
   __shared__ int s_abort;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
-  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const int per_img = a.tiles_x * a.tiles_y, m_tiles = a.n_img * per_img;
-  const int num_m = (m_tiles + 1) / 2, num_n = (a.Cout + TN - 1) / TN, num_tiles = num_m * num_n;
-  const int num_st = 3 * a.cin_blocks;                    // stages per tile: (channel block, dx)
+  const uint32_t s_px = (smem_u32(smem_raw) + 1023u) & ~1023u, s_w = s_px + a.px_stages * C3_PX_STAGE;
+  const uint32_t s_out = s_w + (RESIDENT ? 9 * a.cin_blocks : a.w_stages * Cfg::TAPS) * Cfg::W_BYTES;
+  float* half_ss = reinterpret_cast<float*>(smem_raw + (s_out - smem_u32(smem_raw)) + TEAMS * Cfg::OUT_BYTES);      // TEAMS == 1: [2][128]
+  const int per_img = a.tiles_x * a.tiles_y, m_tiles = a.n_img * per_img, phases = a.up ? 4 : 1;
+  const int num_m = (m_tiles + 1) / 2 * phases, num_n = (a.Cout + TN - 1) / TN, num_tiles = num_m * num_n;
 
   if (threadIdx.x == 0) {
     s_abort = 0;
-    for (int i = 0; i < STAGES; ++i) {
-      mbar_init(smem_u32(&full_bar[i]), 1);
-      mbar_init(smem_u32(&empty_bar[i]), 1);
+    for (int i = 0; i < C3_MAX_PX; ++i) {
+      mbar_init(smem_u32(&px_full[i]), 1);
+      mbar_init(smem_u32(&px_empty[i]), 1);
+    }
+    for (int i = 0; i < C3_MAX_W; ++i) {
+      mbar_init(smem_u32(&w_full[i]), 1);
+      mbar_init(smem_u32(&w_empty[i]), 1);
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&tfull_bar[i]), 1);
-      mbar_init(smem_u32(&tempty_bar[i]), Cfg::STAGED ? 8 : 16);
+      mbar_init(smem_u32(&tempty_bar[i]), TEAMS == 2 ? 8 : 16);
       mbar_init(smem_u32(&res_bar[i]), 1);
     }
     fence_mbar_init();
@@ -131,9 +143,11 @@ conv3x3_pair_kernel(const __grid_constant__ Conv3Args a, int* status) {
   pdl_begin();
 
   // the pair's two pixel tiles are neighbours in the tile list; a tile past the end (odd counts) lies below the last image's rows
-  auto place = [&](int t, int& nb, int& img, int& y0, int& x0) {
-    const int mb = (t / num_n) * 2 + (int)rank;
-    nb = t % num_n;
+  auto place = [&](int t, int& mb, int& nb, int& phase, int& img, int& y0, int& x0) {
+    const int p = t / num_n;
+    nb = t - p * num_n;
+    phase = a.up ? p & 3 : 0;
+    mb = (a.up ? p >> 2 : p) * 2 + (int)rank;
     img = min(mb / per_img, a.n_img - 1);
     const int rem = mb - img * per_img;
     y0 = rem / a.tiles_x * C3_H;
@@ -142,51 +156,91 @@ conv3x3_pair_kernel(const __grid_constant__ Conv3Args a, int* status) {
 
   if (warp == 0) {
     if (elect_one()) {
-      int stage = 0;
-      uint32_t phase = 0;
+      int ps = 0, ws = 0;
+      uint32_t pphase = 0, wphase = 0;
+      auto load_w = [&](uint32_t dst, uint32_t fb, int cb, int tap, int nb) {
+        const int dx = tap / 3, dy = tap - dx * 3;
+        tma_load_2d_pair(dst, &a.tmW, fb, ((dy * a.tap_y + dx * a.tap_x) * a.cin_blocks + cb) * 64, nb * TN + (int)rank * (TN / 2));
+      };
+      if (RESIDENT && pair < num_tiles) {
+        if (rank == 0) mbar_expect_tx(smem_u32(&w_full[0]), 2 * 9 * a.cin_blocks * Cfg::W_BYTES);
+        const uint32_t fb = mapa_shared(smem_u32(&w_full[0]), 0);
+        for (int i = 0; i < 9 * a.cin_blocks; ++i) load_w(s_w + i * Cfg::W_BYTES, fb, i / 9, i % 9, 0);
+      }
       for (int t = pair; t < num_tiles; t += num_pairs) {
-        int nb, img, y0, x0;
-        place(t, nb, img, y0, x0);
-        for (int s = 0; s < num_st; ++s) {
-          const int cb = s / 3, dx = s - cb * 3;
-          mbar_wait(smem_u32(&empty_bar[stage]), phase ^ 1, &s_abort, status, ERR_WAIT_EMPTY);
-          if (rank == 0) mbar_expect_tx(smem_u32(&full_bar[stage]), 2 * Cfg::STAGE_BYTES);
-          const uint32_t fb = mapa_shared(smem_u32(&full_bar[stage]), 0);
-          const uint32_t sa = smem_base + stage * Cfg::STAGE_BYTES;
-          tma_load_4d_pair(sa, &a.tmX, fb, cb * 64, x0 + dx - 1, y0 - 1, img);
-#pragma unroll
-          for (int dy = 0; dy < 3; ++dy)
-            tma_load_2d_pair(sa + C3_A_BYTES + dy * Cfg::B_BYTES, &a.tmW, fb, ((dy * a.tap_y + dx * a.tap_x) * a.cin_blocks + cb) * 64,
-                             nb * TN + (int)rank * (TN / 2));
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+        int mb, nb, phase, img, y0, x0;
+        place(t, mb, nb, phase, img, y0, x0);
+        for (int cb = 0; cb < a.cin_blocks; ++cb) {
+          mbar_wait(smem_u32(&px_empty[ps]), pphase ^ 1, &s_abort, status, ERR_WAIT_EMPTY);
+          if (rank == 0) mbar_expect_tx(smem_u32(&px_full[ps]), 2 * C3_PX_BYTES);
+          tma_load_4d_pair(s_px + ps * C3_PX_STAGE, &a.tmX, mapa_shared(smem_u32(&px_full[ps]), 0), cb * 64, x0 - 1, y0 - 1, img);
+          if (++ps == a.px_stages) { ps = 0; pphase ^= 1; }
+          if (RESIDENT) continue;
+          for (int tap = 0; tap < 9; tap += Cfg::TAPS) {
+            mbar_wait(smem_u32(&w_empty[ws]), wphase ^ 1, &s_abort, status, ERR_WAIT_EMPTY);
+            if (rank == 0) mbar_expect_tx(smem_u32(&w_full[ws]), 2 * Cfg::TAPS * Cfg::W_BYTES);
+            const uint32_t fb = mapa_shared(smem_u32(&w_full[ws]), 0);
+            for (int i = 0; i < Cfg::TAPS; ++i) load_w(s_w + (ws * Cfg::TAPS + i) * Cfg::W_BYTES, fb, cb, tap + i, nb);
+            if (++ws == a.w_stages) { ws = 0; wphase ^= 1; }
+          }
         }
       }
     }
   } else if (warp == 1) {
     if (rank == 0 && elect_one()) {
       constexpr uint32_t idesc = umma_idesc(256, TN, 1, 1, 0, 0);
-      int stage = 0, acc = 0;
-      uint32_t phase = 0, acc_phase = 0;
+      // One thread issues everything and the tensor cores wait for it where MMAs are narrow: no test between the MMAs of a block of channels (with one
+      // per K step 96 -> 96 took 40 us more), and the loop over dx stays a loop for the instruction cache.
+      int ps = 0, ws = 0, acc = 0;
+      uint32_t pphase = 0, wphase = 0, acc_phase = 0;
+      const uint32_t w_free0 = mapa_shared(smem_u32(w_empty), 0), w_free1 = mapa_shared(smem_u32(w_empty), 1);
+      const uint32_t px_free0 = mapa_shared(smem_u32(px_empty), 0), px_free1 = mapa_shared(smem_u32(px_empty), 1);
+      if (RESIDENT && pair < num_tiles) mbar_wait(smem_u32(&w_full[0]), 0, &s_abort, status, ERR_WAIT_FULL);
       for (int t = pair; t < num_tiles; t += num_pairs) {
+        const int phase = a.up ? (t / num_n) & 3 : 0;
+        uint32_t y_at[3];                                    // where the pixels of a tap's row begin in the box
+#pragma unroll
+        for (int d = 0; d < 3; ++d) y_at[d] = (a.up ? (((phase >> 1) + d - 1) >> 1) + 1 : d) * (C3_BOX_ROW / 16);
         mbar_wait(smem_u32(&tempty_bar[acc]), acc_phase ^ 1, &s_abort, status, ERR_WAIT_TMEM_EMPTY);
         tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + acc * Cfg::ACC_STRIDE;
-        for (int s = 0; s < num_st; ++s) {
-          const int steps = min(4, (a.cin - s / 3 * 64 + 15) / 16);          // 16 channels each
-          mbar_wait(smem_u32(&full_bar[stage]), phase, &s_abort, status, ERR_WAIT_FULL);
+        for (int cb = 0; cb < a.cin_blocks; ++cb) {
+          mbar_wait(smem_u32(&px_full[ps]), pphase, &s_abort, status, ERR_WAIT_FULL);
           tc_fence_after_sync();
-          const uint32_t sa = smem_base + stage * Cfg::STAGE_BYTES;
-          const uint64_t a_desc = umma_desc_kmajor_sw128(sa), b_desc = umma_desc_kmajor_sw128(sa + C3_A_BYTES);
+          const uint64_t a_desc = umma_desc_sw128(s_px + ps * C3_PX_STAGE, 0, C3_BOX_ROW);
+          uint64_t b_desc = umma_desc_kmajor_sw128(s_w + cb * 9 * Cfg::W_BYTES);
+          auto products = [&](auto steps) {                  // K steps of 16 channels
+#pragma unroll 1
+            for (int dx = 0; dx < 3; ++dx) {
+              const uint64_t col = a_desc + (uint32_t)((a.up ? (((phase & 1) + dx - 1) >> 1) + 1 : dx) * (128 / 16));
 #pragma unroll
-          for (int dy = 0; dy < 3; ++dy)
+              for (int dy = 0; dy < 3; ++dy) {
+                if (!RESIDENT && (Cfg::TAPS == 1 || dy == 0)) {
+                  mbar_wait(smem_u32(&w_full[ws]), wphase, &s_abort, status, ERR_WAIT_FULL);
+                  tc_fence_after_sync();
+                  b_desc = umma_desc_kmajor_sw128(s_w + ws * Cfg::TAPS * Cfg::W_BYTES);
+                }
+                const uint64_t at = col + y_at[dy];
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
-              if (k < steps)
-                mma_f16_ss_pair(d_tmem, a_desc + dy * (C3_W * 128 / 16) + 2 * k, b_desc + dy * (Cfg::B_BYTES / 16) + 2 * k, idesc,
-                                (s | dy | k) != 0);
-          tc_commit_pair(mapa_shared(smem_u32(&empty_bar[stage]), 0));
-          tc_commit_pair(mapa_shared(smem_u32(&empty_bar[stage]), 1));
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+                for (int k = 0; k < decltype(steps)::value; ++k) mma_f16_ss_pair(d_tmem, at + 2 * k, b_desc + 2 * k, idesc, (cb | dx | dy | k) != 0);
+                b_desc += Cfg::W_BYTES / 16;
+                if (!RESIDENT && (Cfg::TAPS == 1 || dy == 2)) {
+                  tc_commit_pair(w_free0 + ws * 8);
+                  tc_commit_pair(w_free1 + ws * 8);
+                  if (++ws == a.w_stages) { ws = 0; wphase ^= 1; }
+                }
+              }
+            }
+          };
+          switch (min(4, (a.cin - cb * 64 + 15) / 16)) {
+            case 4: products(std::integral_constant<int, 4>()); break;
+            case 3: products(std::integral_constant<int, 3>()); break;
+            case 2: products(std::integral_constant<int, 2>()); break;
+            default: products(std::integral_constant<int, 1>()); break;
+          }
+          tc_commit_pair(px_free0 + ps * 8);
+          tc_commit_pair(px_free1 + ps * 8);
+          if (++ps == a.px_stages) { ps = 0; pphase ^= 1; }
         }
         tc_commit_pair(mapa_shared(smem_u32(&tfull_bar[acc]), 0));
         tc_commit_pair(mapa_shared(smem_u32(&tfull_bar[acc]), 1));
@@ -194,120 +248,111 @@ conv3x3_pair_kernel(const __grid_constant__ Conv3Args a, int* status) {
         if (acc == 0) acc_phase ^= 1;
       }
     }
-  } else if constexpr (Cfg::STAGED) {
-    // A tile of few channels is over in 1 to 3 us, less than one epilogue takes from the accumulator to memory: four warps have the even
-    // tiles and four the odd ones.  A pixel's channels are a row of their own in memory, so each group of 32 channels goes out, and its
-    // residual comes in a tile ahead, as one box through shared memory (64 bytes per pixel, swizzled: no bank conflicts).
-    constexpr int GROUPS = TN / 32;
-    const int q = warp & 3, mine = (warp - 2) >> 2, r = q * 32 + lane;
-    const uint32_t buf = smem_base + STAGES * Cfg::STAGE_BYTES + mine * Cfg::OUT_BYTES;
-    const bool leader = q == 2 && lane == 0;                // warps 2 and 6
-    const uint32_t swizzle = (r >> 1) & 3;
-    auto fetch_residual = [&](int t) {
-      int nb, img, y0, x0;
-      place(t, nb, img, y0, x0);
-      const int groups = min(GROUPS, (a.Cout - nb * TN + 31) / 32);
-      mbar_expect_tx(smem_u32(&res_bar[mine]), groups * (Cfg::OUT_BYTES / GROUPS));
-      for (int g = 0; g < groups; ++g)
-        tma_load_4d(buf + g * (Cfg::OUT_BYTES / GROUPS), &a.tmR, smem_u32(&res_bar[mine]), nb * TN + g * 32, x0, y0, img);
-    };
-    uint32_t phase = 0;
-    int t = pair + mine * num_pairs;
-    if (leader && a.epi.residual && t < num_tiles) fetch_residual(t);
-    for (; t < num_tiles; t += 2 * num_pairs, phase ^= 1) {
-      int nb, img, y0, x0;
-      place(t, nb, img, y0, x0);
-      if (a.epi.residual) mbar_wait(smem_u32(&res_bar[mine]), phase, &s_abort, status, ERR_WAIT_FULL);
-      mbar_wait(smem_u32(&tfull_bar[mine]), phase, &s_abort, status, ERR_WAIT_TMEM_FULL);
-      tc_fence_after_sync();
-#pragma unroll
-      for (int g = 0; g < GROUPS; ++g) {
-        uint32_t v[32];
-        tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + mine * Cfg::ACC_STRIDE + g * 32, v);
-        tmem_wait_ld();
-        if (g == GROUPS - 1) {                              // the accumulator is read: the next but one tile may have it
-          tc_fence_before_sync();
-          __syncwarp();
-          if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&tempty_bar[mine]), 0));
-        }
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const int col = nb * TN + g * 32 + c * 8;
-          if (col >= a.Cout) break;
-          const uint32_t at = buf + g * (Cfg::OUT_BYTES / GROUPS) + r * 64 + ((c ^ swizzle) << 4);
-          float f[8];
-#pragma unroll
-          for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(v[c * 8 + e]);
-          conv3_finish(f, a.epi, col);
-          if (a.epi.residual) add8(f, lds128(at));
-          sts128(at, make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7])));
-        }
-      }
-      fence_proxy_async_smem();
-      asm volatile("bar.sync %0, 128;" ::"r"(1 + mine) : "memory");
-      if (leader) {
-        if ((t / num_n) * 2 + (int)rank < m_tiles)
-          for (int g = 0; g < GROUPS && nb * TN + g * 32 < a.Cout; ++g)
-            tma_store_4d(&a.tmY, buf + g * (Cfg::OUT_BYTES / GROUPS), nb * TN + g * 32, x0, y0, img);
-        bulk_commit();
-        bulk_wait_read();
-        if (a.epi.residual && t + 2 * num_pairs < num_tiles) fetch_residual(t + 2 * num_pairs);
-      }
-      __syncwarp();
-      asm volatile("bar.sync %0, 128;" ::"r"(1 + mine) : "memory");          // the buffer is free
-    }
-    if (leader) bulk_wait_all();
   } else {
-    // the residual is requested while the MMAs of the tile run
-    constexpr int CH = TN / 32;                             // 16-column chunks per warp: half of the tile's columns
-    const int q = warp & 3, first = ((warp - 2) >> 2) * (TN / 2);
-    int acc = 0;
-    uint32_t acc_phase = 0;
-    for (int t = pair; t < num_tiles; t += num_pairs) {
-      int nb, img, y0, x0;
-      place(t, nb, img, y0, x0);
-      const int r = q * 32 + lane, y = y0 + r / C3_W, x = x0 + r % C3_W;
-      const bool row_ok = y < a.H && x < a.W;
-      const long row = (long)img * a.H * a.W + (long)y * a.px_y + (long)x * a.px_x;
-      const int col = nb * TN + first;
-      uint4 res[CH][2];
-      if (a.epi.residual) {
-#pragma unroll
-        for (int c = 0; c < CH; ++c)
-#pragma unroll
-          for (int g = 0; g < 2; ++g)
-            res[c][g] = row_ok && col + c * 16 + g * 8 < a.Cout
-                            ? *reinterpret_cast<const uint4*>(a.epi.residual + row * a.epi.ldr + col + c * 16 + g * 8)
-                            : make_uint4(0u, 0u, 0u, 0u);
-      }
+    // one thread per pixel and COLS channels; a team shares a buffer of 32-channel boxes (64 bytes per pixel, swizzled: no bank conflicts)
+    const int q = warp & 3, hi = (warp - 2) >> 2, team = TEAMS == 2 ? hi : 0, half = TEAMS == 1 ? hi : 0, r = q * 32 + lane;
+    const uint32_t buf = s_out + team * Cfg::OUT_BYTES, swizzle = (r >> 1) & 3;
+    const bool leader = q == 2 && half == 0 && lane == 0, norm = a.gamma != nullptr;
+    auto team_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "n"(TEAMS == 2 ? 128 : 256) : "memory"); };
+    auto fetch_residual = [&](int t) {
+      int mb, nb, phase, img, y0, x0;
+      place(t, mb, nb, phase, img, y0, x0);
+      const int groups = min(TN / 32, (a.Cout - nb * TN + 31) / 32);
+      mbar_expect_tx(smem_u32(&res_bar[team]), groups * GROUP_BYTES);
+      for (int g = 0; g < groups; ++g) tma_load_4d(buf + g * GROUP_BYTES, &a.tmR, smem_u32(&res_bar[team]), nb * TN + g * 32, x0, y0, img);
+    };
+    int t = pair + team * num_pairs;
+    if (leader && a.epi.residual && t < num_tiles) fetch_residual(t);
+#pragma unroll 1
+    for (int i = 0; t < num_tiles; t += TEAMS * num_pairs, ++i) {
+      int mb, nb, phase, img, y0, x0;
+      place(t, mb, nb, phase, img, y0, x0);
+      const int acc = TEAMS == 2 ? team : i & 1, acc_phase = TEAMS == 2 ? i & 1 : (i >> 1) & 1;
+      auto at = [&](int c) { return buf + (half * (COLS / 32) + (c >> 2)) * GROUP_BYTES + r * 64 + (((c & 3) ^ swizzle) << 4); };   // 8 channels
+      auto store = [&](const CUtensorMap* tm) {
+        if (mb < m_tiles)
+          for (int g = 0; g < TN / 32 && nb * TN + g * 32 < a.Cout; ++g)
+            tma_store_5d(tm, buf + g * GROUP_BYTES, nb * TN + g * 32, x0, y0, a.up ? phase & 1 : img, phase >> 1);
+        bulk_commit();
+      };
+      if (a.epi.residual) mbar_wait(smem_u32(&res_bar[team]), i & 1, &s_abort, status, ERR_WAIT_FULL);
       mbar_wait(smem_u32(&tfull_bar[acc]), acc_phase, &s_abort, status, ERR_WAIT_TMEM_FULL);
       tc_fence_after_sync();
-#pragma unroll
-      for (int c = 0; c < CH; ++c) {
-        uint32_t v[16];
-        tmem_ld_32x16(tmem_base + ((uint32_t)(q * 32) << 16) + acc * Cfg::ACC_STRIDE + first + c * 16, v);
+      // Both passes are rolled and a pixel's channels wait in the buffer for the second: unrolled, with the channels in registers, the code outgrew the
+      // instruction cache (96 -> 96: 306 us)
+      float ss = 0.f;
+#pragma unroll 1
+      for (int g = 0; g < COLS / 32; ++g) {
+        uint32_t v[32];
+        tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + acc * Cfg::ACC_STRIDE + half * COLS + g * 32, v);
         tmem_wait_ld();
-        if (c == CH - 1) {                                  // the accumulator is read: the next but one tile may have it
+        if (g == COLS / 32 - 1) {                           // the accumulator is read: the next but one tile may have it
           tc_fence_before_sync();
           __syncwarp();
           if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&tempty_bar[acc]), 0));
         }
 #pragma unroll
-        for (int g = 0; g < 2; ++g) {
-          const int cc = col + c * 16 + g * 8;
-          if (!row_ok || cc >= a.Cout) continue;
+        for (int c = 0; c < 4; ++c) {
+          const int col = nb * TN + half * COLS + g * 32 + c * 8;
+          if (col >= a.Cout) break;
           float f[8];
 #pragma unroll
-          for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(v[g * 8 + e]);
-          conv3_finish(f, a.epi, cc);
-          if (a.epi.residual) add8(f, res[c][g]);
-          *reinterpret_cast<uint4*>(a.y + row * a.ldy + cc) =
-              make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
+          for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(v[c * 8 + e]);
+          conv3_finish(f, a.epi, col);
+          if (a.epi.residual) add8(f, lds128(at(g * 4 + c)));
+          const uint4 w = make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
+          sts128(at(g * 4 + c), w);
+          if (norm) {                                       // of the rounded values
+            const float2 p0 = unpack_bf16(w.x), p1 = unpack_bf16(w.y), p2 = unpack_bf16(w.z), p3 = unpack_bf16(w.w);
+            ss += (p0.x * p0.x + p0.y * p0.y + p1.x * p1.x + p1.y * p1.y) + (p2.x * p2.x + p2.y * p2.y + p3.x * p3.x + p3.y * p3.y);
+          }
         }
       }
-      acc ^= 1;
-      if (acc == 0) acc_phase ^= 1;
+      if (norm && TEAMS == 1) half_ss[half * 128 + r] = ss;
+      if (a.has_y) {
+        fence_proxy_async_smem();
+        team_sync();
+        if (leader) {
+          store(&a.tmY);
+          if (norm) bulk_wait_read();
+        }
+        if (norm) {
+          __syncwarp();
+          team_sync();
+        }
+      } else if (TEAMS == 1) {
+        team_sync();
+      }
+      if (norm) {
+        if (TEAMS == 1) ss += half_ss[(half ^ 1) * 128 + r];
+        const float inv = rsqrtf(fmaxf(ss / (float)a.Cout, 1e-24f));
+#pragma unroll 2
+        for (int c = 0; c < COLS / 8; ++c) {
+          const int col = half * COLS + c * 8;
+          if (col >= a.Cout) break;
+          const uint4 u = lds128(at(c)), gm = *reinterpret_cast<const uint4*>(a.gamma + col);
+          const uint32_t uw[4] = {u.x, u.y, u.z, u.w}, gw[4] = {gm.x, gm.y, gm.z, gm.w};
+          uint32_t o[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float2 p = unpack_bf16(uw[e]), g2 = unpack_bf16(gw[e]);
+            const float x = p.x * inv * g2.x, y = p.y * inv * g2.y;
+            o[e] = a.norm_silu ? pack_bf16(silu(x), silu(y)) : pack_bf16(x, y);
+          }
+          sts128(at(c), make_uint4(o[0], o[1], o[2], o[3]));
+        }
+        fence_proxy_async_smem();
+        team_sync();
+        if (leader) store(&a.tmZ);
+      }
+      if (leader) {
+        bulk_wait_read();
+        if (a.epi.residual && t + TEAMS * num_pairs < num_tiles) fetch_residual(t + TEAMS * num_pairs);
+      }
+      __syncwarp();
+      team_sync();                                          // the buffer is free
     }
+    if (leader) bulk_wait_all();
   }
 
   tc_fence_before_sync();
@@ -321,37 +366,61 @@ conv3x3_pair_kernel(const __grid_constant__ Conv3Args a, int* status) {
   if (warp == 1) tmem_dealloc_pair(tmem_base, Cfg::TMEM_COLS);
 }
 
-// Boxes of `chans` channels x 8 pixels x `rows` rows of an image of C channels, `ld` elements per pixel.
-static int conv3_map(CUtensorMap* map, const Conv3Args& a, const void* p, long ld, int C, int chans, int rows, CUtensorMapSwizzle swizzle) {
+// Boxes of `chans` channels x `cols` x `rows` pixels of an image of C channels, `ld` elements per pixel, that is read.
+static int conv3_map(CUtensorMap* map, const Conv3Args& a, const void* p, long ld, int C, int chans, int cols, int rows, CUtensorMapSwizzle swizzle) {
   EncodeTiledFn enc = get_encode_tiled();
   if (!enc) return RC_NO_DRIVER;
   if (reinterpret_cast<uintptr_t>(p) & 15) return RC_BAD_ARG;
   const cuuint64_t px = (cuuint64_t)ld * 2;
   cuuint64_t gdim[4] = {(cuuint64_t)C, (cuuint64_t)a.W, (cuuint64_t)a.H, (cuuint64_t)a.n_img};
   cuuint64_t gstr[3] = {px * a.px_x, px * a.px_y, px * a.W * a.H};
-  cuuint32_t box[4] = {(cuuint32_t)chans, C3_W, (cuuint32_t)rows, 1}, estr[4] = {1, 1, 1, 1};
+  cuuint32_t box[4] = {(cuuint32_t)chans, (cuuint32_t)cols, (cuuint32_t)rows, 1}, estr[4] = {1, 1, 1, 1};
   return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(p), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? RC_OK : RC_TMAP;
+}
+// The same of an image that is written: 32 channels of a tile; the fourth and fifth coordinates are the image and 0, or the parities of x and y.
+static int conv3_out_map(CUtensorMap* map, const Conv3Args& a, const void* p, long ld) {
+  EncodeTiledFn enc = get_encode_tiled();
+  if (!enc) return RC_NO_DRIVER;
+  if (reinterpret_cast<uintptr_t>(p) & 15) return RC_BAD_ARG;
+  const cuuint64_t px = (cuuint64_t)ld * 2, image = px * a.W * a.H;
+  cuuint64_t gdim[5] = {(cuuint64_t)a.Cout, (cuuint64_t)a.W, (cuuint64_t)a.H, (cuuint64_t)(a.up ? 2 : a.n_img), (cuuint64_t)(a.up ? 2 : 1)};
+  cuuint64_t gstr[4] = {px * a.px_x, px * a.px_y, image, image * a.n_img};
+  if (a.up) { gstr[0] = px * 2; gstr[1] = px * 4 * a.W; gstr[2] = px; gstr[3] = px * 2 * a.W; }
+  cuuint32_t box[5] = {32, C3_W, C3_H, 1, 1}, estr[5] = {1, 1, 1, 1, 1};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(p), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? RC_OK : RC_TMAP;
 }
 
 static long conv3_tiles(long n_img, int H, int W) { return n_img * ((W + C3_W - 1) / C3_W) * ((H + C3_H - 1) / C3_H); }
 
 
 template <int TN>
-static int launch_conv3(Conv3Args& a, const void* w, int pairs, int* status, cudaStream_t stream) {
+static int launch_conv3(Conv3Args& a, const void* w, const void* y, long ldy, const void* z, long ldz, int pairs, int* status, cudaStream_t stream) {
   using Cfg = Conv3Cfg<TN>;
   const uint64_t K = 9ull * a.cin_blocks * 64;
   if (int rc = make_tmap_2d(&a.tmW, w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)a.Cout, K, K * 2, TN / 2, 64)) return rc;
-  if (Cfg::STAGED) {
-    if (int rc = conv3_map(&a.tmY, a, a.y, a.ldy, a.Cout, 32, C3_H, CU_TENSOR_MAP_SWIZZLE_64B)) return rc;
-    if (a.epi.residual)
-      if (int rc = conv3_map(&a.tmR, a, a.epi.residual, a.epi.ldr, a.Cout, 32, C3_H, CU_TENSOR_MAP_SWIZZLE_64B)) return rc;
-  }
-  static unsigned long long prepared = 0;
-  if (int e = ensure_dynamic_smem((const void*)conv3x3_pair_kernel<TN>, Cfg::SMEM_BYTES, prepared)) return e;
-  const long tiles = (long)((a.n_img * a.tiles_x * a.tiles_y + 1) / 2) * ((a.Cout + TN - 1) / TN);
+  if (y)
+    if (int rc = conv3_out_map(&a.tmY, a, y, ldy)) return rc;
+  if (z)
+    if (int rc = conv3_out_map(&a.tmZ, a, z, ldz)) return rc;
+  if (a.epi.residual)
+    if (int rc = conv3_map(&a.tmR, a, a.epi.residual, a.epi.ldr, a.Cout, 32, C3_W, C3_H, CU_TENSOR_MAP_SWIZZLE_64B)) return rc;
+  // weights stay where they leave room for two channel blocks of pixels; otherwise two or more blocks of pixels and the rest for the weights' ring
+  constexpr int ROOM = Cfg::DYN_MAX - Cfg::FIXED, RING = Cfg::TAPS * Cfg::W_BYTES, FIT = (ROOM - 2 * C3_PX_STAGE) / RING;
+  constexpr bool MAY_STAY = Cfg::TEAMS == 2;
+  const int all_w = 9 * a.cin_blocks * Cfg::W_BYTES;
+  const bool stay = MAY_STAY && a.Cout <= TN && all_w + 2 * C3_PX_STAGE <= ROOM;
+  a.w_stages = stay ? 0 : (FIT < C3_MAX_W ? FIT : C3_MAX_W);
+  const int w_bytes = stay ? all_w : a.w_stages * RING;
+  a.px_stages = (ROOM - w_bytes) / C3_PX_STAGE < C3_MAX_PX ? (ROOM - w_bytes) / C3_PX_STAGE : C3_MAX_PX;
+  const int bytes = w_bytes + a.px_stages * C3_PX_STAGE + Cfg::FIXED;
+  const long tiles = (long)((a.n_img * a.tiles_x * a.tiles_y + 1) / 2) * (a.up ? 4 : 1) * ((a.Cout + TN - 1) / TN);
   const int grid = tiles < pairs ? (int)tiles : pairs;
-  launch_overlapped(conv3x3_pair_kernel<TN>, 2 * grid, GEMM_THREADS, Cfg::SMEM_BYTES, stream, a, status);
+  static unsigned long long prepared[2] = {0, 0};
+  const auto kernel = stay ? conv3x3_pair_kernel<TN, MAY_STAY> : conv3x3_pair_kernel<TN, false>;
+  if (int e = ensure_dynamic_smem((const void*)kernel, Cfg::DYN_MAX, prepared[stay])) return e;
+  launch_overlapped(kernel, 2 * grid, GEMM_THREADS, bytes, stream, a, status);
   return (int)cudaGetLastError();
 }
 
@@ -377,6 +446,41 @@ static bool conv3_flat(long n_img, int H, int W, int Cout, int pairs) {
   if (turned * 4 > seen * 3 || turned * 4 < pairs) return false;
   const int tn = pick_conv3_tn(seen, Cout, pairs), num_n = (Cout + tn - 1) / tn;
   return (turned * num_n + pairs - 1) / pairs < (seen * num_n + pairs - 1) / pairs;
+}
+
+static bool conv3_fits(long n_img, int H, int W) { return conv3_tiles(n_img, H, W) < (1L << 22); }
+
+static int conv3_run(const void* x, long ldx, const void* w, void* y, long ldy, void* z, long ldz, int n_img, int H, int W, int Cin, int Cout, bool up,
+                     const void* bias, const void* residual, int ldr, int act, const void* gamma, int norm_silu, int* status, cudaStream_t stream) {
+  const int pairs = max_resident_pairs();
+  const bool flat = conv3_flat(n_img, H, W, Cout, pairs);
+  Conv3Args a = {};
+  a.n_img = n_img;
+  a.H = flat ? W : H; a.W = flat ? H : W;
+  a.tap_y = flat ? 1 : 3; a.tap_x = flat ? 3 : 1;
+  a.px_y = flat ? 1 : W; a.px_x = flat ? W : 1;
+  a.tiles_x = (a.W + C3_W - 1) / C3_W; a.tiles_y = (a.H + C3_H - 1) / C3_H;
+  a.up = up;
+  a.Cout = Cout; a.cin = Cin; a.cin_blocks = (Cin + 63) / 64;
+  if (int rc = conv3_map(&a.tmX, a, x, ldx, Cin, 64, C3_W + 2, C3_H + 2, CU_TENSOR_MAP_SWIZZLE_128B)) return rc;
+  a.epi.bias = static_cast<const __nv_bfloat16*>(bias);
+  a.epi.residual = static_cast<const __nv_bfloat16*>(residual);
+  a.epi.ldr = ldr;
+  a.epi.rows_per_batch = 1;
+  a.epi.act = act;
+  a.has_y = y != nullptr;
+  a.gamma = static_cast<const __nv_bfloat16*>(gamma);
+  a.norm_silu = norm_silu;
+  const long m_pairs = (conv3_tiles(n_img, a.H, a.W) + 1) / 2;
+  const int tn = pick_conv3_tn(m_pairs, Cout, pairs);
+  if ((gamma && tn < Cout) || (up && (flat || n_img != 1 || residual))) return RC_BAD_ARG;
+  switch (tn) {
+    case 256: return launch_conv3<256>(a, w, y, ldy, z, ldz, pairs, status, stream);
+    case 192: return launch_conv3<192>(a, w, y, ldy, z, ldz, pairs, status, stream);
+    case 128: return launch_conv3<128>(a, w, y, ldy, z, ldz, pairs, status, stream);
+    case 96: return launch_conv3<96>(a, w, y, ldy, z, ldz, pairs, status, stream);
+    default: return launch_conv3<32>(a, w, y, ldy, z, ldz, pairs, status, stream);
+  }
 }
 
 }  // namespace omni

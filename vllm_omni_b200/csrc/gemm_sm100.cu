@@ -1343,6 +1343,29 @@ extern "C" int omni_gemm_bf16_experts(const void* A, int lda, const void* W, int
 }
 
 
+// 3 x 3 convolutions on CTA pairs with what may ride along.  omni_conv3x3_fuses: bit 0, the RMS norm of the result can be made in the epilogue; bit 1, the
+// input can be read as its doubled self (up).  omni_conv3x3_nhwc_bf16: as omni_conv2d_nhwc_bf16 with ksize 3; z (pitch ldz) receives
+// rms_norm(result) * gamma, SiLU of it with norm_silu, and y may then be null; up: H and W are the input's, y and z have twice as many rows and columns.
+extern "C" int omni_conv3x3_fuses(int Nimg, int H, int W, int Cout) {
+  using namespace omni;
+  if (Nimg <= 0 || H <= 0 || W <= 0 || Cout <= 0 || !conv3_fits(Nimg, H, W)) return 0;
+  const int pairs = max_resident_pairs();
+  const bool flat = conv3_flat(Nimg, H, W, Cout, pairs);
+  const long m_pairs = ((flat ? conv3_tiles(Nimg, W, H) : conv3_tiles(Nimg, H, W)) + 1) / 2;
+  return (pick_conv3_tn(m_pairs, Cout, pairs) >= Cout ? 1 : 0) | (!flat && Nimg == 1 ? 2 : 0);
+}
+
+extern "C" int omni_conv3x3_nhwc_bf16(const void* x, long ldx, const void* w, void* y, int ldy, void* z, int ldz, int Nimg, int H, int W, int Cin, int Cout,
+                                      int up, const void* bias, const void* residual, int ldr, int act, const void* gamma, int norm_silu, int* status,
+                                      void* stream) {
+  using namespace omni;
+  if (act == ACT_XIELU || (z != nullptr) != (gamma != nullptr) || (y == nullptr && z == nullptr)) return RC_BAD_ARG;
+  if (Nimg <= 0 || H <= 0 || W <= 0 || Cin <= 0 || Cout <= 0) return RC_OK;
+  if ((Cout & 7) || (ldx & 7) || (ldy & 7) || (ldz & 7) || (ldr & 7) || !conv3_fits(Nimg, H, W)) return RC_BAD_ARG;
+  return conv3_run(x, ldx, w, y, ldy, z, ldz, Nimg, H, W, Cin, Cout, up != 0, bias, residual, ldr, act, gamma, norm_silu, status,
+                   static_cast<cudaStream_t>(stream));
+}
+
 // Convolution, stride 1, zero "same" padding, NHWC bf16:  y[n,h,w,:] = act(sum_taps x[n,h+dy,w+dx,:] W_tap^T + bias)
 // (+ residual).  x: [Nimg, H, W, Cin] with pixel pitch ldx (elements, >= Cin, multiple of 8);
 // w: [Cout, taps * cin_pad] with cin_pad = ceil(Cin / 64) * 64, tap-major (tap = ky * 3 + kx for 3x3),
@@ -1357,36 +1380,8 @@ extern "C" int omni_conv2d_nhwc_bf16(const void* x, long ldx, const void* w, voi
   EncodeTiledFn enc = get_encode_tiled();
   if (!enc) return RC_NO_DRIVER;
   if (reinterpret_cast<uintptr_t>(x) & 15) return RC_BAD_ARG;
-  const int pairs = ksize == 3 ? max_resident_pairs() : 0;
-  const bool flat = ksize == 3 && conv3_flat(Nimg, H, W, Cout, pairs);
-  const long m_pairs = ((flat ? conv3_tiles(Nimg, W, H) : conv3_tiles(Nimg, H, W)) + 1) / 2;
-  // The line at a quarter of a wave of pixel tiles was drawn for the one-CTA kernel's larger number of blocks and does not show in the times: below
-  // it the pair kernel is the faster one too (us, one-CTA kernel in brackets: 48 x 48 pixels, 384 -> 384 channels 14.7 (29.1), 96 -> 96
-  // 6.6 (13.7); 32 x 32, 16 -> 384 6.5 (11.0); just above it 64 x 80, 384 -> 384 16.7 (29.7)).
-  if (ksize == 3 && m_pairs * 4 >= pairs && m_pairs < (1L << 24)) {
-    Conv3Args a = {};
-    a.y = static_cast<__nv_bfloat16*>(y);
-    a.ldy = ldy; a.n_img = Nimg;
-    a.H = flat ? W : H; a.W = flat ? H : W;
-    a.tap_y = flat ? 1 : 3; a.tap_x = flat ? 3 : 1;
-    a.px_y = flat ? 1 : W; a.px_x = flat ? W : 1;
-    a.tiles_x = (a.W + C3_W - 1) / C3_W; a.tiles_y = (a.H + C3_H - 1) / C3_H;
-    a.Cout = Cout; a.cin = Cin; a.cin_blocks = (Cin + BK - 1) / BK;
-    if (int rc = conv3_map(&a.tmX, a, x, ldx, Cin, BK, C3_H + 2, CU_TENSOR_MAP_SWIZZLE_128B)) return rc;
-    a.epi.bias = static_cast<const __nv_bfloat16*>(bias);
-    a.epi.residual = static_cast<const __nv_bfloat16*>(residual);
-    a.epi.ldr = ldr;
-    a.epi.rows_per_batch = 1;
-    a.epi.act = act;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    switch (pick_conv3_tn(m_pairs, Cout, pairs)) {
-      case 256: return launch_conv3<256>(a, w, pairs, status, st);
-      case 192: return launch_conv3<192>(a, w, pairs, status, st);
-      case 128: return launch_conv3<128>(a, w, pairs, status, st);
-      case 96: return launch_conv3<96>(a, w, pairs, status, st);
-      default: return launch_conv3<32>(a, w, pairs, status, st);
-    }
-  }
+  if (ksize == 3 && conv3_fits(Nimg, H, W))
+    return conv3_run(x, ldx, w, y, ldy, nullptr, 0, Nimg, H, W, Cin, Cout, false, bias, residual, ldr, act, nullptr, 0, status, static_cast<cudaStream_t>(stream));
   ConvGeom g = {};
   g.taps = ksize * ksize;
   g.H = H; g.W = W;

@@ -95,6 +95,7 @@ class NHWCDecoderKL:
                 o = C.wide_head_attention(t[:, :, 0], t[:, :, 1], t[:, :, 2])
                 x = proj(o.reshape(B, H, W, ch).contiguous(), residual=x)
             else:
-                x = st[1](C.upsample2x_nhwc(x))
+                c = st[1]
+                x = C.conv3x3_norm_nhwc(x, c.w, c.b, c.cin, up=True)[0] if c.k == 3 else c(C.upsample2x_nhwc(x))
         x = self.conv_out(self.norm_out(x))
         return C.nhwc_to_image(x)

@@ -21,7 +21,7 @@ class NativeError(RuntimeError):
 
 
 # kernels launched per exported entry point (default 1); used for the launch counter
-_KERNELS_PER_CALL = {"omni_rel_l1": 2, "omni_rel_l1_parts": 0, "omni_paged_decode": 2, "omni_gemm_set_pair_mode": 0, "omni_attn_wide_workers": 0,
+_KERNELS_PER_CALL = {"omni_rel_l1": 2, "omni_rel_l1_parts": 0, "omni_paged_decode": 2, "omni_gemm_set_pair_mode": 0, "omni_attn_wide_workers": 0, "omni_conv3x3_fuses": 0,
                      "omni_paged_decode_attn": 2, "omni_paged_decode_shares": 0}
 launch_count = 0
 _timing: list | None = None      # (entry point, start event, stop event) while kernel timing is on

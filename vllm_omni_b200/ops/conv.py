@@ -68,6 +68,37 @@ def conv2d_nhwc(x, w_packed, bias, ksize: int, cin: int, act=None, residual=None
     return out
 
 
+def conv3x3_norm_nhwc(x, w_packed, bias, cin: int, residual=None, up: bool = False, gamma=None, silu: bool = True, keep: bool = True):
+    """(y, z): y = the 3 x 3 convolution of x, or with ``up`` of ``upsample2x_nhwc(x)``, plus ``residual``; z = ``rmsnorm_silu_nhwc(y, gamma, silu)``,
+    None without ``gamma``.  ``keep=False``: y is not wanted (None where z leaves the convolution's own launch).  One launch where a tile of the
+    convolution holds all channels of its pixels and one image is doubled (csrc/conv_pair.cuh); otherwise the launches one after the other."""
+    N, H, W, ldx = x.shape
+    C = w_packed.shape[0]
+    fuses = 0
+    if x.is_cuda and (up or gamma is not None) and x.numel():
+        fuses = nv.lib("gemm_sm100").omni_conv3x3_fuses(c_int(N), c_int(H), c_int(W), c_int(C))
+    if up and not (fuses & 2 and residual is None):
+        x, up = upsample2x_nhwc(x), False
+        N, H, W, _ = x.shape
+        fuses = nv.lib("gemm_sm100").omni_conv3x3_fuses(c_int(N), c_int(H), c_int(W), c_int(C)) if fuses else 0
+    make = gamma is not None and fuses & 1 and gamma.dtype == torch.bfloat16 and gamma.numel() == C and gamma.is_contiguous() and gamma.data_ptr() % 16 == 0
+    if not (up or make):
+        y = conv2d_nhwc(x, w_packed, bias, 3, cin, residual=residual)
+        return y, None if gamma is None else rmsnorm_silu_nhwc(y, gamma, silu)
+    assert x.is_contiguous() and x.dtype == torch.bfloat16 and w_packed.dtype == torch.bfloat16
+    s = 2 if up else 1
+    new = lambda: torch.empty(N, s * H, s * W, C, dtype=x.dtype, device=x.device)
+    y, z = new() if keep or not make else None, new() if make else None
+    rc = nv.lib("gemm_sm100").omni_conv3x3_nhwc_bf16(
+        nv.ptr(x), c_long(ldx), nv.ptr(w_packed), nv.ptr(y), c_int(C), nv.ptr(z), c_int(C), c_int(N), c_int(H), c_int(W), c_int(cin), c_int(C),
+        c_int(1 if up else 0), nv.ptr(bias), nv.ptr(residual), c_int(residual.stride(2) if residual is not None else 0), c_int(0),
+        nv.ptr(gamma if make else None), c_int(1 if silu else 0), nv.ptr(nv.status_word(x.device)), nv.stream_ptr())
+    nv.check_rc(rc, "omni_conv3x3_nhwc_bf16")
+    if gamma is not None and not make:
+        z = rmsnorm_silu_nhwc(y, gamma, silu)
+    return y, z
+
+
 def rmsnorm_silu_nhwc(x, gamma, silu: bool = True, out=None):
     """Per pixel: x / sqrt(mean_c x^2) * gamma, then SiLU.  x: [..., C]."""
     C = x.shape[-1]
