@@ -7,15 +7,17 @@
 //            operand that begins some rows and pixels further into the box (the swizzle goes by address, not by operand row)
 //   weights  each CTA of a pair holds half of the TN output channels' weights and the pair's MMA reads both; where all of a layer's weights fit
 //            beside the tiles they are fetched once per CTA, otherwise tap by tap through a ring
-// A channel block of which only some channels exist (96 = 64 + 32) issues the K steps that hold any.
+// A last channel block of at most 32 channels (96 = 64 + 32) is 32 wide: 64-byte rows, swizzled as such, in half the space.
 // Results leave, and residuals arrive, as boxes by TMA through shared memory: a lane's 16 bytes at the pitch of a pixel fill half a sector.
 // Where a tile holds all channels of its pixels, the RMS norm (+ SiLU) that follows is made there as well, beside or instead of the result.
 // An image that is to be doubled first (nearest neighbour) is read as it is: output pixels of one parity of (y, x) see, tap by tap, the same
 // shifted box of the small image, so a tile takes 16 x 8 pixels of one parity.
 //
 // us with residual where it says +, in brackets the form before, with a box per dx, weights by the ring and results of wide tiles by plain stores:
-// 1024 x 1024 pixels, 96 -> 96 channels 143 (179), + 176 (206), 192 -> 96 250 (261), 96 -> 8 86 (116); 512 x 512, 192 -> 192 110 (128), + 120 (153),
-// 384 -> 192 205 (220); 256 x 256, 384 -> 384 + 106 (117).  Without epilogue and loads the MMAs of 96 -> 96 take 109.
+// 1024 x 1024 pixels, 96 -> 96 channels 133 (179), + 166 (206), 192 -> 96 247 (261), 96 -> 8 87 (116); 512 x 512, 192 -> 192 110 (128), + 119 (153),
+// 384 -> 192 205 (220); 256 x 256, 384 -> 384 + 105 (117).  With the norm: 96 -> 96 163 (179 + 72 as its own launch), + beside the result 210 (206 + 72);
+// 192 -> 192 117 (128 + 42), + 143 (153 + 42).  Without epilogue and loads the MMAs of 96 -> 96 take 109.  Four warps per team instead of eight: 198 and 265
+// for 96 -> 96 with the norm, even without.
 #pragma once
 #include <type_traits>
 
@@ -25,30 +27,31 @@ constexpr int C3_W = 8, C3_H = 16;                       // pixels of a CTA's ti
 constexpr int C3_BOX_ROW = (C3_W + 2) * 128;             // a box row: 10 pixels x 64 channels
 constexpr int C3_PX_BYTES = (C3_H + 2) * C3_BOX_ROW, C3_PX_STAGE = (C3_PX_BYTES + 1023) / 1024 * 1024;
 constexpr int C3_MAX_PX = 8, C3_MAX_W = 16;              // stages of the pixel and the weight ring
+constexpr int C3_THREADS = 64 + 512;                     // TMA, MMA, 16 epilogue warps
 
 template <int TN>
 struct Conv3Cfg {
   static constexpr int W_BYTES = (TN / 2) * 128;         // one tap's weights of this CTA's half, 64 channels
   static constexpr int TAPS = TN <= 128 ? 3 : 1;         // per stage of the weight ring: narrow MMAs are over before the next wait is through
-  static constexpr int TEAMS = TN <= 96 ? 2 : 1;         // narrow: four warps have the even tiles and four the odd ones; wide: half of the columns each
-  static constexpr int COLS = TN / (3 - TEAMS);          // columns per epilogue thread
+  static constexpr int TEAMS = TN <= 96 ? 2 : 1;         // narrow: eight warps have the even tiles and eight the odd ones; wide: sixteen share a tile
+  static constexpr int SHARE = 4 / TEAMS, COLS = TN / SHARE;                           // threads per pixel, columns of each
   static constexpr int OUT_BYTES = TN * 2 * C3_W * C3_H; // a tile's outputs
-  static constexpr int FIXED = TEAMS * OUT_BYTES + (TEAMS == 1 ? 1024 : 0) + 1024;      // + half rows' sums of squares, alignment
+  static constexpr int FIXED = TEAMS * OUT_BYTES + 4 * 128 * 4 + 1024;               // + sums of squares of a thread's columns, alignment
   static constexpr int DYN_MAX = 231424;
   static constexpr int ACC_STRIDE = TN <= 32 ? 32 : (TN <= 128 ? 128 : 256);
   static constexpr int TMEM_COLS = 2 * ACC_STRIDE;
 };
 
 struct Conv3Args {
-  CUtensorMap tmX, tmW, tmY, tmR, tmZ;    // Y, Z (norm), residual: 32 channels of a tile
+  CUtensorMap tmX, tmW, tmX32, tmW32, tmY, tmR, tmZ;      // X32, W32: of a last block of 32 channels; Y, Z (norm), residual: 32 channels of a tile
   // The image as the tiles see it: rows of W pixels, H of them, in tiles of 16 x 8.  An image that is flat (see conv3_flat) is seen with
   // its columns as rows: the maps swap the two, tap (dy, dx) is weight dy * tap_y + dx * tap_x and pixel (y, x) is y * px_y + x * px_x.
   // up: H and W are those of the small image, and every tile exists for the four parities of output pixels.
   int H, W, n_img, tiles_x, tiles_y, up;
   int tap_y, tap_x, px_y, px_x;
-  int Cout, cin, cin_blocks;
+  int Cout, cin, cin_blocks, tail32;      // tail32: the last block is 32 channels wide
   int px_stages, w_stages;
-  int has_y, norm_silu;
+  int has_y, norm_silu, z_apart;          // z_apart: the norm has buffers of its own
   const __nv_bfloat16* gamma;             // of the norm; null: none
   GemmEpilogue epi;
 };
@@ -93,10 +96,10 @@ __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wa
 
 // RESIDENT: all weights stay in shared memory
 template <int TN, bool RESIDENT>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(C3_THREADS, 1)
 conv3x3_pair_kernel(const __grid_constant__ Conv3Args a, int* status) {
   using Cfg = Conv3Cfg<TN>;
-  constexpr int TEAMS = Cfg::TEAMS, COLS = Cfg::COLS, GROUP_BYTES = C3_W * C3_H * 64;
+  constexpr int TEAMS = Cfg::TEAMS, SHARE = Cfg::SHARE, COLS = Cfg::COLS, GROUP_BYTES = C3_W * C3_H * 64;
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t px_full[C3_MAX_PX], px_empty[C3_MAX_PX], w_full[C3_MAX_W], w_empty[C3_MAX_W];
   __shared__ __align__(8) uint64_t tfull_bar[2], tempty_bar[2], res_bar[2];
@@ -107,8 +110,8 @@ conv3x3_pair_kernel(const __grid_constant__ Conv3Args a, int* status) {
   const uint32_t rank = cluster_ctarank();
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
   const uint32_t s_px = (smem_u32(smem_raw) + 1023u) & ~1023u, s_w = s_px + a.px_stages * C3_PX_STAGE;
-  const uint32_t s_out = s_w + (RESIDENT ? 9 * a.cin_blocks : a.w_stages * Cfg::TAPS) * Cfg::W_BYTES;
-  float* half_ss = reinterpret_cast<float*>(smem_raw + (s_out - smem_u32(smem_raw)) + TEAMS * Cfg::OUT_BYTES);      // TEAMS == 1: [2][128]
+  const uint32_t s_out = s_w + (RESIDENT ? 18 * a.cin_blocks - 9 * a.tail32 : 2 * a.w_stages * Cfg::TAPS) * (Cfg::W_BYTES / 2);
+  float* part_ss = reinterpret_cast<float*>(smem_raw + (s_out - smem_u32(smem_raw)) + (1 + a.z_apart) * TEAMS * Cfg::OUT_BYTES);      // [team][share][128]
   const int per_img = a.tiles_x * a.tiles_y, m_tiles = a.n_img * per_img, phases = a.up ? 4 : 1;
   const int num_m = (m_tiles + 1) / 2 * phases, num_n = (a.Cout + TN - 1) / TN, num_tiles = num_m * num_n;
 
@@ -124,13 +127,14 @@ conv3x3_pair_kernel(const __grid_constant__ Conv3Args a, int* status) {
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&tfull_bar[i]), 1);
-      mbar_init(smem_u32(&tempty_bar[i]), TEAMS == 2 ? 8 : 16);
+      mbar_init(smem_u32(&tempty_bar[i]), 2 * 4 * SHARE);
       mbar_init(smem_u32(&res_bar[i]), 1);
     }
     fence_mbar_init();
     tma_prefetch_desc(&a.tmX);
     tma_prefetch_desc(&a.tmW);
   }
+  const int full_blocks = a.cin_blocks - a.tail32;
   if (warp == 1) {
     tmem_alloc_pair(smem_u32(&tmem_base_s), Cfg::TMEM_COLS);
     tmem_relinquish_pair();
@@ -160,27 +164,29 @@ conv3x3_pair_kernel(const __grid_constant__ Conv3Args a, int* status) {
       uint32_t pphase = 0, wphase = 0;
       auto load_w = [&](uint32_t dst, uint32_t fb, int cb, int tap, int nb) {
         const int dx = tap / 3, dy = tap - dx * 3;
-        tma_load_2d_pair(dst, &a.tmW, fb, ((dy * a.tap_y + dx * a.tap_x) * a.cin_blocks + cb) * 64, nb * TN + (int)rank * (TN / 2));
+        tma_load_2d_pair(dst, cb < full_blocks ? &a.tmW : &a.tmW32, fb, ((dy * a.tap_y + dx * a.tap_x) * a.cin_blocks + cb) * 64, nb * TN + (int)rank * (TN / 2));
       };
       if (RESIDENT && pair < num_tiles) {
-        if (rank == 0) mbar_expect_tx(smem_u32(&w_full[0]), 2 * 9 * a.cin_blocks * Cfg::W_BYTES);
+        if (rank == 0) mbar_expect_tx(smem_u32(&w_full[0]), (18 * a.cin_blocks - 9 * a.tail32) * Cfg::W_BYTES);
         const uint32_t fb = mapa_shared(smem_u32(&w_full[0]), 0);
-        for (int i = 0; i < 9 * a.cin_blocks; ++i) load_w(s_w + i * Cfg::W_BYTES, fb, i / 9, i % 9, 0);
+        for (int cb = 0; cb < a.cin_blocks; ++cb)
+          for (int tap = 0; tap < 9; ++tap) load_w(s_w + (cb * 18 + (cb < full_blocks ? 2 * tap : tap)) * (Cfg::W_BYTES / 2), fb, cb, tap, 0);
       }
       for (int t = pair; t < num_tiles; t += num_pairs) {
         int mb, nb, phase, img, y0, x0;
         place(t, mb, nb, phase, img, y0, x0);
         for (int cb = 0; cb < a.cin_blocks; ++cb) {
           mbar_wait(smem_u32(&px_empty[ps]), pphase ^ 1, &s_abort, status, ERR_WAIT_EMPTY);
-          if (rank == 0) mbar_expect_tx(smem_u32(&px_full[ps]), 2 * C3_PX_BYTES);
-          tma_load_4d_pair(s_px + ps * C3_PX_STAGE, &a.tmX, mapa_shared(smem_u32(&px_full[ps]), 0), cb * 64, x0 - 1, y0 - 1, img);
+          const bool wide = cb < full_blocks;
+          if (rank == 0) mbar_expect_tx(smem_u32(&px_full[ps]), wide ? 2 * C3_PX_BYTES : C3_PX_BYTES);
+          tma_load_4d_pair(s_px + ps * C3_PX_STAGE, wide ? &a.tmX : &a.tmX32, mapa_shared(smem_u32(&px_full[ps]), 0), cb * 64, x0 - 1, y0 - 1, img);
           if (++ps == a.px_stages) { ps = 0; pphase ^= 1; }
           if (RESIDENT) continue;
           for (int tap = 0; tap < 9; tap += Cfg::TAPS) {
             mbar_wait(smem_u32(&w_empty[ws]), wphase ^ 1, &s_abort, status, ERR_WAIT_EMPTY);
-            if (rank == 0) mbar_expect_tx(smem_u32(&w_full[ws]), 2 * Cfg::TAPS * Cfg::W_BYTES);
+            if (rank == 0) mbar_expect_tx(smem_u32(&w_full[ws]), (wide ? 2 : 1) * Cfg::TAPS * Cfg::W_BYTES);
             const uint32_t fb = mapa_shared(smem_u32(&w_full[ws]), 0);
-            for (int i = 0; i < Cfg::TAPS; ++i) load_w(s_w + (ws * Cfg::TAPS + i) * Cfg::W_BYTES, fb, cb, tap + i, nb);
+            for (int i = 0; i < Cfg::TAPS; ++i) load_w(s_w + (ws * Cfg::TAPS * 2 + (wide ? 2 * i : i)) * (Cfg::W_BYTES / 2), fb, cb, tap + i, nb);
             if (++ws == a.w_stages) { ws = 0; wphase ^= 1; }
           }
         }
@@ -207,23 +213,26 @@ conv3x3_pair_kernel(const __grid_constant__ Conv3Args a, int* status) {
         for (int cb = 0; cb < a.cin_blocks; ++cb) {
           mbar_wait(smem_u32(&px_full[ps]), pphase, &s_abort, status, ERR_WAIT_FULL);
           tc_fence_after_sync();
-          const uint64_t a_desc = umma_desc_sw128(s_px + ps * C3_PX_STAGE, 0, C3_BOX_ROW);
-          uint64_t b_desc = umma_desc_kmajor_sw128(s_w + cb * 9 * Cfg::W_BYTES);
-          auto products = [&](auto steps) {                  // K steps of 16 channels
+          // N K steps of 16 channels from rows of ROW bytes
+          auto products = [&](auto n, auto row) {
+            constexpr int N = decltype(n)::value, ROW = decltype(row)::value;
+            constexpr uint64_t swizzle = ROW == 128 ? 0 : 6ull << 61;          // umma_desc_sw128's 2 becomes 4: 64 bytes
+            const uint64_t a_desc = umma_desc_sw128(s_px + ps * C3_PX_STAGE, 0, C3_BOX_ROW * ROW / 128) ^ swizzle;
+            uint64_t b_desc = umma_desc_sw128(s_w + cb * 9 * Cfg::W_BYTES, 0, 8 * ROW) ^ swizzle;
 #pragma unroll 1
             for (int dx = 0; dx < 3; ++dx) {
-              const uint64_t col = a_desc + (uint32_t)((a.up ? (((phase & 1) + dx - 1) >> 1) + 1 : dx) * (128 / 16));
+              const uint64_t col = a_desc + (uint32_t)((a.up ? (((phase & 1) + dx - 1) >> 1) + 1 : dx) * (ROW / 16));
 #pragma unroll
               for (int dy = 0; dy < 3; ++dy) {
                 if (!RESIDENT && (Cfg::TAPS == 1 || dy == 0)) {
                   mbar_wait(smem_u32(&w_full[ws]), wphase, &s_abort, status, ERR_WAIT_FULL);
                   tc_fence_after_sync();
-                  b_desc = umma_desc_kmajor_sw128(s_w + ws * Cfg::TAPS * Cfg::W_BYTES);
+                  b_desc = umma_desc_sw128(s_w + ws * Cfg::TAPS * Cfg::W_BYTES, 0, 8 * ROW) ^ swizzle;
                 }
-                const uint64_t at = col + y_at[dy];
+                const uint64_t at = col + y_at[dy] * ROW / 128;
 #pragma unroll
-                for (int k = 0; k < decltype(steps)::value; ++k) mma_f16_ss_pair(d_tmem, at + 2 * k, b_desc + 2 * k, idesc, (cb | dx | dy | k) != 0);
-                b_desc += Cfg::W_BYTES / 16;
+                for (int k = 0; k < N; ++k) mma_f16_ss_pair(d_tmem, at + 2 * k, b_desc + 2 * k, idesc, (cb | dx | dy | k) != 0);
+                b_desc += Cfg::W_BYTES * ROW / 128 / 16;
                 if (!RESIDENT && (Cfg::TAPS == 1 || dy == 2)) {
                   tc_commit_pair(w_free0 + ws * 8);
                   tc_commit_pair(w_free1 + ws * 8);
@@ -232,12 +241,11 @@ conv3x3_pair_kernel(const __grid_constant__ Conv3Args a, int* status) {
               }
             }
           };
-          switch (min(4, (a.cin - cb * 64 + 15) / 16)) {
-            case 4: products(std::integral_constant<int, 4>()); break;
-            case 3: products(std::integral_constant<int, 3>()); break;
-            case 2: products(std::integral_constant<int, 2>()); break;
-            default: products(std::integral_constant<int, 1>()); break;
-          }
+          const int steps = (a.cin - cb * 64 + 15) / 16;
+          if (steps >= 4) products(std::integral_constant<int, 4>(), std::integral_constant<int, 128>());
+          else if (steps == 3) products(std::integral_constant<int, 3>(), std::integral_constant<int, 128>());
+          else if (steps == 2) products(std::integral_constant<int, 2>(), std::integral_constant<int, 64>());
+          else products(std::integral_constant<int, 1>(), std::integral_constant<int, 64>());
           tc_commit_pair(px_free0 + ps * 8);
           tc_commit_pair(px_free1 + ps * 8);
           if (++ps == a.px_stages) { ps = 0; pphase ^= 1; }
@@ -249,11 +257,11 @@ conv3x3_pair_kernel(const __grid_constant__ Conv3Args a, int* status) {
       }
     }
   } else {
-    // one thread per pixel and COLS channels; a team shares a buffer of 32-channel boxes (64 bytes per pixel, swizzled: no bank conflicts)
-    const int q = warp & 3, hi = (warp - 2) >> 2, team = TEAMS == 2 ? hi : 0, half = TEAMS == 1 ? hi : 0, r = q * 32 + lane;
-    const uint32_t buf = s_out + team * Cfg::OUT_BYTES, swizzle = (r >> 1) & 3;
-    const bool leader = q == 2 && half == 0 && lane == 0, norm = a.gamma != nullptr;
-    auto team_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "n"(TEAMS == 2 ? 128 : 256) : "memory"); };
+    // SHARE threads per pixel, COLS channels each; a team shares a buffer of 32-channel boxes (64 bytes per pixel, swizzled: no bank conflicts)
+    const int q = warp & 3, team = (warp - 2) / (4 * SHARE), share = ((warp - 2) >> 2) % SHARE, r = q * 32 + lane;
+    const uint32_t buf = s_out + team * Cfg::OUT_BYTES, zbuf = buf + a.z_apart * TEAMS * Cfg::OUT_BYTES, swizzle = (r >> 1) & 3;
+    const bool leader = (warp - 2) % (4 * SHARE) == 0 && lane == 0, norm = a.gamma != nullptr;
+    auto team_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "n"(128 * SHARE) : "memory"); };
     auto fetch_residual = [&](int t) {
       int mb, nb, phase, img, y0, x0;
       place(t, mb, nb, phase, img, y0, x0);
@@ -268,11 +276,11 @@ conv3x3_pair_kernel(const __grid_constant__ Conv3Args a, int* status) {
       int mb, nb, phase, img, y0, x0;
       place(t, mb, nb, phase, img, y0, x0);
       const int acc = TEAMS == 2 ? team : i & 1, acc_phase = TEAMS == 2 ? i & 1 : (i >> 1) & 1;
-      auto at = [&](int c) { return buf + (half * (COLS / 32) + (c >> 2)) * GROUP_BYTES + r * 64 + (((c & 3) ^ swizzle) << 4); };   // 8 channels
-      auto store = [&](const CUtensorMap* tm) {
+      auto at = [&](uint32_t b, int c) { return b + (c >> 5) * GROUP_BYTES + r * 64 + ((((c >> 3) & 3) ^ swizzle) << 4); };       // 8 channels from c on
+      auto store = [&](const CUtensorMap* tm, uint32_t from) {
         if (mb < m_tiles)
           for (int g = 0; g < TN / 32 && nb * TN + g * 32 < a.Cout; ++g)
-            tma_store_5d(tm, buf + g * GROUP_BYTES, nb * TN + g * 32, x0, y0, a.up ? phase & 1 : img, phase >> 1);
+            tma_store_5d(tm, from + g * GROUP_BYTES, nb * TN + g * 32, x0, y0, a.up ? phase & 1 : img, phase >> 1);
         bulk_commit();
       };
       if (a.epi.residual) mbar_wait(smem_u32(&res_bar[team]), i & 1, &s_abort, status, ERR_WAIT_FULL);
@@ -282,55 +290,56 @@ conv3x3_pair_kernel(const __grid_constant__ Conv3Args a, int* status) {
       // instruction cache (96 -> 96: 306 us)
       float ss = 0.f;
 #pragma unroll 1
-      for (int g = 0; g < COLS / 32; ++g) {
-        uint32_t v[32];
-        tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + acc * Cfg::ACC_STRIDE + half * COLS + g * 32, v);
+      for (int g = 0; g < COLS; g += 16) {
+        uint32_t v[16];
+        tmem_ld_32x16(tmem_base + ((uint32_t)(q * 32) << 16) + acc * Cfg::ACC_STRIDE + share * COLS + g, v);
         tmem_wait_ld();
-        if (g == COLS / 32 - 1) {                           // the accumulator is read: the next but one tile may have it
+        if (g == COLS - 16) {                               // the accumulator is read: the next but one tile may have it
           tc_fence_before_sync();
           __syncwarp();
           if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&tempty_bar[acc]), 0));
         }
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const int col = nb * TN + half * COLS + g * 32 + c * 8;
+        for (int c = 0; c < 2; ++c) {
+          const int in_tile = share * COLS + g + c * 8, col = nb * TN + in_tile;
           if (col >= a.Cout) break;
           float f[8];
 #pragma unroll
           for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(v[c * 8 + e]);
           conv3_finish(f, a.epi, col);
-          if (a.epi.residual) add8(f, lds128(at(g * 4 + c)));
+          if (a.epi.residual) add8(f, lds128(at(buf, in_tile)));
           const uint4 w = make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
-          sts128(at(g * 4 + c), w);
+          sts128(at(buf, in_tile), w);
           if (norm) {                                       // of the rounded values
             const float2 p0 = unpack_bf16(w.x), p1 = unpack_bf16(w.y), p2 = unpack_bf16(w.z), p3 = unpack_bf16(w.w);
             ss += (p0.x * p0.x + p0.y * p0.y + p1.x * p1.x + p1.y * p1.y) + (p2.x * p2.x + p2.y * p2.y + p3.x * p3.x + p3.y * p3.y);
           }
         }
       }
-      if (norm && TEAMS == 1) half_ss[half * 128 + r] = ss;
+      if (norm) part_ss[(team * SHARE + share) * 128 + r] = ss;
       if (a.has_y) {
         fence_proxy_async_smem();
         team_sync();
         if (leader) {
-          store(&a.tmY);
-          if (norm) bulk_wait_read();
+          store(&a.tmY, buf);
+          if (norm && !a.z_apart) bulk_wait_read();
         }
-        if (norm) {
+        if (norm && !a.z_apart) {
           __syncwarp();
           team_sync();
         }
-      } else if (TEAMS == 1) {
+      } else {
         team_sync();
       }
       if (norm) {
-        if (TEAMS == 1) ss += half_ss[(half ^ 1) * 128 + r];
+        ss = 0.f;
+#pragma unroll
+        for (int h = 0; h < SHARE; ++h) ss += part_ss[(team * SHARE + h) * 128 + r];
         const float inv = rsqrtf(fmaxf(ss / (float)a.Cout, 1e-24f));
 #pragma unroll 2
-        for (int c = 0; c < COLS / 8; ++c) {
-          const int col = half * COLS + c * 8;
+        for (int col = share * COLS; col < (share + 1) * COLS; col += 8) {
           if (col >= a.Cout) break;
-          const uint4 u = lds128(at(c)), gm = *reinterpret_cast<const uint4*>(a.gamma + col);
+          const uint4 u = lds128(at(buf, col)), gm = *reinterpret_cast<const uint4*>(a.gamma + col);
           const uint32_t uw[4] = {u.x, u.y, u.z, u.w}, gw[4] = {gm.x, gm.y, gm.z, gm.w};
           uint32_t o[4];
 #pragma unroll
@@ -339,11 +348,11 @@ conv3x3_pair_kernel(const __grid_constant__ Conv3Args a, int* status) {
             const float x = p.x * inv * g2.x, y = p.y * inv * g2.y;
             o[e] = a.norm_silu ? pack_bf16(silu(x), silu(y)) : pack_bf16(x, y);
           }
-          sts128(at(c), make_uint4(o[0], o[1], o[2], o[3]));
+          sts128(at(zbuf, col), make_uint4(o[0], o[1], o[2], o[3]));
         }
         fence_proxy_async_smem();
         team_sync();
-        if (leader) store(&a.tmZ);
+        if (leader) store(&a.tmZ, zbuf);
       }
       if (leader) {
         bulk_wait_read();
@@ -400,6 +409,7 @@ static int launch_conv3(Conv3Args& a, const void* w, const void* y, long ldy, co
   using Cfg = Conv3Cfg<TN>;
   const uint64_t K = 9ull * a.cin_blocks * 64;
   if (int rc = make_tmap_2d(&a.tmW, w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)a.Cout, K, K * 2, TN / 2, 64)) return rc;
+  if (int rc = make_tmap_2d(&a.tmW32, w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)a.Cout, K, K * 2, TN / 2, 32, CU_TENSOR_MAP_SWIZZLE_64B)) return rc;
   if (y)
     if (int rc = conv3_out_map(&a.tmY, a, y, ldy)) return rc;
   if (z)
@@ -407,20 +417,26 @@ static int launch_conv3(Conv3Args& a, const void* w, const void* y, long ldy, co
   if (a.epi.residual)
     if (int rc = conv3_map(&a.tmR, a, a.epi.residual, a.epi.ldr, a.Cout, 32, C3_W, C3_H, CU_TENSOR_MAP_SWIZZLE_64B)) return rc;
   // weights stay where they leave room for two channel blocks of pixels; otherwise two or more blocks of pixels and the rest for the weights' ring
-  constexpr int ROOM = Cfg::DYN_MAX - Cfg::FIXED, RING = Cfg::TAPS * Cfg::W_BYTES, FIT = (ROOM - 2 * C3_PX_STAGE) / RING;
+  constexpr int RING = Cfg::TAPS * Cfg::W_BYTES, Z = Cfg::TEAMS * Cfg::OUT_BYTES;
   constexpr bool MAY_STAY = Cfg::TEAMS == 2;
-  const int all_w = 9 * a.cin_blocks * Cfg::W_BYTES;
-  const bool stay = MAY_STAY && a.Cout <= TN && all_w + 2 * C3_PX_STAGE <= ROOM;
-  a.w_stages = stay ? 0 : (FIT < C3_MAX_W ? FIT : C3_MAX_W);
+  const int all_w = (18 * a.cin_blocks - 9 * a.tail32) * (Cfg::W_BYTES / 2);
+  int room = Cfg::DYN_MAX - Cfg::FIXED;
+  const bool stay = MAY_STAY && a.Cout <= TN && all_w + 2 * C3_PX_STAGE <= room;
+  // Result and norm from one buffer wait for each other; apart they cost pixel stages or the weights' ring (not below six stages).  Both of 96 -> 96 at
+  // 1024 x 1024 with residual 210 us (233 from one buffer), 192 -> 192 at 512 x 512 143 (147).
+  a.z_apart = y && z && (stay ? all_w : 6 * RING) + 2 * C3_PX_STAGE + Z <= room;
+  room -= a.z_apart * Z;
+  const int fit = (room - 2 * C3_PX_STAGE) / RING;
+  a.w_stages = stay ? 0 : (fit < C3_MAX_W ? fit : C3_MAX_W);
   const int w_bytes = stay ? all_w : a.w_stages * RING;
-  a.px_stages = (ROOM - w_bytes) / C3_PX_STAGE < C3_MAX_PX ? (ROOM - w_bytes) / C3_PX_STAGE : C3_MAX_PX;
-  const int bytes = w_bytes + a.px_stages * C3_PX_STAGE + Cfg::FIXED;
+  a.px_stages = (room - w_bytes) / C3_PX_STAGE < C3_MAX_PX ? (room - w_bytes) / C3_PX_STAGE : C3_MAX_PX;
+  const int bytes = w_bytes + a.px_stages * C3_PX_STAGE + Cfg::FIXED + a.z_apart * Z;
   const long tiles = (long)((a.n_img * a.tiles_x * a.tiles_y + 1) / 2) * (a.up ? 4 : 1) * ((a.Cout + TN - 1) / TN);
   const int grid = tiles < pairs ? (int)tiles : pairs;
   static unsigned long long prepared[2] = {0, 0};
   const auto kernel = stay ? conv3x3_pair_kernel<TN, MAY_STAY> : conv3x3_pair_kernel<TN, false>;
   if (int e = ensure_dynamic_smem((const void*)kernel, Cfg::DYN_MAX, prepared[stay])) return e;
-  launch_overlapped(kernel, 2 * grid, GEMM_THREADS, bytes, stream, a, status);
+  launch_overlapped(kernel, 2 * grid, C3_THREADS, bytes, stream, a, status);
   return (int)cudaGetLastError();
 }
 
@@ -462,7 +478,9 @@ static int conv3_run(const void* x, long ldx, const void* w, void* y, long ldy, 
   a.tiles_x = (a.W + C3_W - 1) / C3_W; a.tiles_y = (a.H + C3_H - 1) / C3_H;
   a.up = up;
   a.Cout = Cout; a.cin = Cin; a.cin_blocks = (Cin + 63) / 64;
+  a.tail32 = (Cin - 1) % 64 < 32;
   if (int rc = conv3_map(&a.tmX, a, x, ldx, Cin, 64, C3_W + 2, C3_H + 2, CU_TENSOR_MAP_SWIZZLE_128B)) return rc;
+  if (int rc = conv3_map(&a.tmX32, a, x, ldx, Cin, 32, C3_W + 2, C3_H + 2, CU_TENSOR_MAP_SWIZZLE_64B)) return rc;
   a.epi.bias = static_cast<const __nv_bfloat16*>(bias);
   a.epi.residual = static_cast<const __nv_bfloat16*>(residual);
   a.epi.ldr = ldr;
@@ -471,7 +489,7 @@ static int conv3_run(const void* x, long ldx, const void* w, void* y, long ldy, 
   a.has_y = y != nullptr;
   a.gamma = static_cast<const __nv_bfloat16*>(gamma);
   a.norm_silu = norm_silu;
-  const long m_pairs = (conv3_tiles(n_img, a.H, a.W) + 1) / 2;
+  const long m_pairs = (conv3_tiles(n_img, a.H, a.W) + 1) / 2 * (up ? 4 : 1);
   const int tn = pick_conv3_tn(m_pairs, Cout, pairs);
   if ((gamma && tn < Cout) || (up && (flat || n_img != 1 || residual))) return RC_BAD_ARG;
   switch (tn) {

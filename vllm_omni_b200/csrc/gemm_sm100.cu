@@ -1343,16 +1343,17 @@ extern "C" int omni_gemm_bf16_experts(const void* A, int lda, const void* W, int
 }
 
 
-// 3 x 3 convolutions on CTA pairs with what may ride along.  omni_conv3x3_fuses: bit 0, the RMS norm of the result can be made in the epilogue; bit 1, the
-// input can be read as its doubled self (up).  omni_conv3x3_nhwc_bf16: as omni_conv2d_nhwc_bf16 with ksize 3; z (pitch ldz) receives
+// 3 x 3 convolutions on CTA pairs with what may ride along.  omni_conv3x3_fuses, for the input's H and W: bit 0, the RMS norm of the result can be made in
+// the epilogue; bit 1, the input can be read as its doubled self (up); with up, bit 0 is for that case.  omni_conv3x3_nhwc_bf16: as omni_conv2d_nhwc_bf16 with ksize 3; z (pitch ldz) receives
 // rms_norm(result) * gamma, SiLU of it with norm_silu, and y may then be null; up: H and W are the input's, y and z have twice as many rows and columns.
-extern "C" int omni_conv3x3_fuses(int Nimg, int H, int W, int Cout) {
+extern "C" int omni_conv3x3_fuses(int Nimg, int H, int W, int Cout, int up) {
   using namespace omni;
   if (Nimg <= 0 || H <= 0 || W <= 0 || Cout <= 0 || !conv3_fits(Nimg, H, W)) return 0;
   const int pairs = max_resident_pairs();
   const bool flat = conv3_flat(Nimg, H, W, Cout, pairs);
-  const long m_pairs = ((flat ? conv3_tiles(Nimg, W, H) : conv3_tiles(Nimg, H, W)) + 1) / 2;
-  return (pick_conv3_tn(m_pairs, Cout, pairs) >= Cout ? 1 : 0) | (!flat && Nimg == 1 ? 2 : 0);
+  if (up && (flat || Nimg != 1)) return 0;
+  const long m_pairs = ((flat ? conv3_tiles(Nimg, W, H) : conv3_tiles(Nimg, H, W)) + 1) / 2 * (up ? 4 : 1);
+  return (pick_conv3_tn(m_pairs, Cout, pairs) >= Cout ? 1 : 0) | (up ? 2 : 0);
 }
 
 extern "C" int omni_conv3x3_nhwc_bf16(const void* x, long ldx, const void* w, void* y, int ldy, void* z, int ldz, int Nimg, int H, int W, int Cin, int Cout,

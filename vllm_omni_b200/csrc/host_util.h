@@ -39,11 +39,11 @@ inline EncodeTiledFn get_encode_tiled() {
 }
 
 // Row-major 2-D tensor [rows, cols] of `elt_bytes` elements with a row pitch of
-// `pitch_bytes`; box = {box_cols, box_rows}; 128-byte swizzle (box_cols * elt_bytes must
-// be 128).  Out-of-range elements read as zero.
+// `pitch_bytes`; box = {box_cols, box_rows}; 128-byte swizzle unless told otherwise (box_cols * elt_bytes must
+// be the swizzle's width).  Out-of-range elements read as zero.
 inline int make_tmap_2d(CUtensorMap* out, const void* ptr, CUtensorMapDataType dt, int elt_bytes,
                         uint64_t rows, uint64_t cols, uint64_t pitch_bytes, uint32_t box_rows,
-                        uint32_t box_cols) {
+                        uint32_t box_cols, CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B) {
   EncodeTiledFn enc = get_encode_tiled();
   if (!enc) return RC_NO_DRIVER;
   if ((reinterpret_cast<uintptr_t>(ptr) & 15) || (pitch_bytes & 15)) return RC_BAD_ARG;
@@ -52,7 +52,7 @@ inline int make_tmap_2d(CUtensorMap* out, const void* ptr, CUtensorMapDataType d
   cuuint32_t box[2] = {box_cols, box_rows};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = enc(out, dt, 2, const_cast<void*>(ptr), gdim, gstr, box, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   (void)elt_bytes;
   return r == CUDA_SUCCESS ? RC_OK : RC_TMAP;

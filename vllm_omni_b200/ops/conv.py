@@ -74,13 +74,13 @@ def conv3x3_norm_nhwc(x, w_packed, bias, cin: int, residual=None, up: bool = Fal
     convolution holds all channels of its pixels and one image is doubled (csrc/conv_pair.cuh); otherwise the launches one after the other."""
     N, H, W, ldx = x.shape
     C = w_packed.shape[0]
-    fuses = 0
-    if x.is_cuda and (up or gamma is not None) and x.numel():
-        fuses = nv.lib("gemm_sm100").omni_conv3x3_fuses(c_int(N), c_int(H), c_int(W), c_int(C))
+    ask = x.is_cuda and (up or gamma is not None) and x.numel()
+    can = lambda: nv.lib("gemm_sm100").omni_conv3x3_fuses(c_int(N), c_int(H), c_int(W), c_int(C), c_int(1 if up else 0)) if ask else 0
+    fuses = can()
     if up and not (fuses & 2 and residual is None):
         x, up = upsample2x_nhwc(x), False
         N, H, W, _ = x.shape
-        fuses = nv.lib("gemm_sm100").omni_conv3x3_fuses(c_int(N), c_int(H), c_int(W), c_int(C)) if fuses else 0
+        fuses = can()
     make = gamma is not None and fuses & 1 and gamma.dtype == torch.bfloat16 and gamma.numel() == C and gamma.is_contiguous() and gamma.data_ptr() % 16 == 0
     if not (up or make):
         y = conv2d_nhwc(x, w_packed, bias, 3, cin, residual=residual)
