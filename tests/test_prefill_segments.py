@@ -1,0 +1,75 @@
+"""Attention of all prompt segments of a step in one launch, and decoded tokens on any rows of it, against softmax in 64 bits."""
+import pytest
+import torch
+
+from vllm_omni_b200.ops import _native as nv, kv_cache as KC
+
+pytestmark = pytest.mark.gpu
+PAGE = 16
+
+
+def _exact(q, k, v, context):
+    H, G = q.shape[1], q.shape[1] // k.shape[1]
+    k, v = (t.double().repeat_interleave(G, 1) for t in (k, v))
+    s = torch.einsum("qhd,khd->hqk", q.double(), k) * q.shape[2] ** -0.5
+    n = q.shape[0]
+    s = s.masked_fill(torch.arange(k.shape[0], device=q.device)[None] > context + torch.arange(n, device=q.device)[:, None], float("-inf"))
+    return torch.einsum("hqk,khd->qhd", s.softmax(-1), v)
+
+
+# one row, edges of a query tile (128) and block (256), contexts that end inside a page and a key tile; more than eight segments; two launches' worth of blocks
+@pytest.mark.parametrize("segs,H,Hkv,D", [
+    ([(1, 0)], 4, 1, 128), ([(257, 0), (128, 0), (129, 5)], 8, 2, 128), ([(1, 300), (256, 128), (40, 0), (700, 129)], 4, 4, 128),
+    ([(3 * i + 2, 17 * (i % 3)) for i in range(19)], 4, 2, 128), ([(130, 0), (64, 0)], 8, 8, 64), ([(66000, 0)], 1, 1, 128)])
+def test_segments(segs, H, Hkv, D):
+    g = torch.Generator(device="cuda").manual_seed(len(segs))
+    T = sum(n for n, _ in segs) + 3                                  # three rows of no segment
+    qkv = torch.randn(T, (H + 2 * Hkv) * D, device="cuda", generator=g).bfloat16()
+    q, k, v = qkv[:, :H * D].view(T, H, D), qkv[:, H * D:(H + Hkv) * D].view(T, Hkv, D), qkv[:, (H + Hkv) * D:].view(T, Hkv, D)
+    need = [-(-(n + c) // PAGE) for n, c in segs]
+    perm = torch.randperm(sum(need), generator=torch.Generator().manual_seed(3))
+    kc, vc = (torch.randn(sum(need), PAGE, Hkv, D, device="cuda", generator=g).bfloat16() for _ in range(2))
+    out = torch.full((T, H, D), 7.0, device="cuda", dtype=torch.bfloat16)
+    work, keys, at, pg = [], [], 2, 0
+    for (n, c), m in zip(segs, need):
+        table = perm[pg:pg + m].int().cuda()
+        rows = table.long()[torch.arange(n + c, device="cuda") // PAGE] * PAGE + torch.arange(n + c, device="cuda") % PAGE
+        for cache, x in ((kc, k), (vc, v)):
+            cache.view(-1, Hkv, D)[rows[c:]] = x[at:at + n]
+        work.append((at, n, c, table))
+        keys.append(rows)
+        at, pg = at + n, pg + m
+    assert KC.prefill_segments_ok(q, kc, [c for _, c in segs])
+    KC.prefill_segments(q, k, v, kc, vc, work, out=out)
+    torch.cuda.synchronize()
+    nv.check_status(q.device)
+    for (a, n, c, _), rows in zip(work, keys):
+        pick = torch.arange(n, device="cuda") if n < 2000 else torch.tensor([0, 255, 256, n // 2, n - 1], device="cuda")
+        kk, vv = kc.view(-1, Hkv, D)[rows], vc.view(-1, Hkv, D)[rows]
+        for r in ([pick] if n < 2000 else pick[:, None]):
+            last = int(r[-1]) + c + 1
+            ref = _exact(q[a + r], kk[:last], vv[:last], last - len(r)) if n >= 2000 else _exact(q[a:a + n], kk, vv, c)
+            got = out[a + r] if n >= 2000 else out[a:a + n]
+            # probabilities and results are bf16, a quarter of the exponentials a polynomial to 7.5e-5
+            assert (got.double() - ref).norm() <= 2.0 ** -8 * ref.norm()
+    assert (out[:2] == 7).all() and (out[at:] == 7).all()
+
+
+@pytest.mark.parametrize("n,H,Hkv", [(1, 8, 2), (5, 32, 4), (3, 16, 1)])
+def test_decode_on_rows_of_a_step(n, H, Hkv):
+    g = torch.Generator(device="cuda").manual_seed(n)
+    T, L = 40, 333
+    q = torch.randn(T, H, 128, device="cuda", generator=g).bfloat16()
+    kc, vc = (torch.randn(n * 21, PAGE, Hkv, 128, device="cuda", generator=g).bfloat16() for _ in range(2))
+    bt = torch.randperm(n * 21, generator=torch.Generator().manual_seed(1)).view(n, 21).int().cuda()
+    lens = torch.tensor([L - 50 * i for i in range(n)], dtype=torch.int32, device="cuda")
+    rows = torch.tensor([-1, 3, 17, 8, 0][:n], device="cuda")
+    want = KC.paged_decode(q[rows].contiguous(), kc, vc, bt, lens)
+    out = torch.full_like(q, 7.0)
+    assert KC.paged_decode(q, kc, vc, bt, lens, out=out, rows=rows) is out
+    torch.cuda.synchronize()
+    nv.check_status(q.device)
+    assert torch.equal(out[rows], want)
+    rest = torch.ones(T, dtype=torch.bool, device="cuda")
+    rest[rows] = False
+    assert (out[rest] == 7).all()

@@ -29,6 +29,7 @@
 // The MMA stream is software-pipelined (PV_t(j) is followed at once by S_t(j+1)) so that
 // the tensor pipe works on one tile while the other tile's softmax runs.  Every wait is bounded.
 #include <stdlib.h>
+#include <type_traits>
 
 #include "host_util.h"
 #include "ptx_sm100.cuh"
@@ -107,6 +108,20 @@ struct AttnPaging {
   int block_size;           // a multiple of 8 that divides 128
 };
 
+// Prompt segments of one step: causal attention of every segment's own rows against its own keys, which are rows of the projections where nothing came
+// before them and pages otherwise.  A block of the grid is one head (x) of one query block (y), the query blocks with the most keys first: in the order of the
+// rows the longest ones run last, and the chip waits for them (one prompt of 8192 tokens, 32 heads: MEASURE).
+struct NoSegs {};
+struct AttnSegs {
+  static constexpr int MAX = 8, MAX_BLOCKS = 256;
+  struct Seg {
+    CUtensorMap tmK, tmV;
+    const int* block_table;           // null: contiguous
+    int row0, len, kv_len;
+  } s[MAX];
+  unsigned short order[MAX_BLOCKS];   // segment << 12 | query block
+};
+
 __device__ __forceinline__ float ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -145,12 +160,13 @@ __device__ __forceinline__ void named_bar_sync(int id, int threads) {
 // B2 S4352 H24 (one box, medians): 4 hand-offs 0.396 ms, 1 hand-off 0.409 ms; packed-bf16 MUFU
 // exponentials and polynomial shares of 0, 1/8, 3/8 and 1/2 were within 1 % of, or slower than,
 // fp32 MUFU with a quarter of the pairs on the FMA-pipe polynomial.
-template <int NH, int HD>
+template <int NH, int HD, typename Work>
 __global__ void __launch_bounds__(ATT_THREADS, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, AttnOut out, int Sq, int Skv, int H, int Hkv,
                 const int* kv_lens, float scale_log2, int causal, int q_offset, AttnPaging pg,
-                PeerSignal sig, int* status) {
+                PeerSignal sig, int* status, const __grid_constant__ Work work) {
+  constexpr bool SEGS = std::is_same<Work, AttnSegs>::value;
   constexpr int ATT_TILE_BYTES = AttCfg<HD>::TILE_BYTES;
   constexpr int KV_STAGES = AttCfg<HD>::STAGES;
   pdl_wait();                        // key lengths and page ids are read from here on
@@ -162,15 +178,28 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int splits = out.kv_splits > 1 ? out.kv_splits : 1;
-  const int qblk = blockIdx.x / splits, split = blockIdx.x - qblk * splits;
-  const int h = blockIdx.y, b = blockIdx.z;
+  const int splits = !SEGS && out.kv_splits > 1 ? out.kv_splits : 1;
+  int qblk = blockIdx.x / splits, h = blockIdx.y, row0 = 0, kv_len = 0;
+  const int split = SEGS ? 0 : blockIdx.x - qblk * splits, b = SEGS ? 0 : blockIdx.z;
+  const CUtensorMap *pK = &tmK, *pV = &tmV;
+  const int* bt = nullptr;
+  if constexpr (SEGS) {
+    const int entry = work.order[blockIdx.y];
+    const AttnSegs::Seg& seg = work.s[entry >> 12];
+    qblk = entry & 4095; h = blockIdx.x;
+    row0 = seg.row0; kv_len = seg.kv_len; Sq = seg.len;
+    causal = 1; q_offset = kv_len - Sq;
+    pK = &seg.tmK; pV = &seg.tmV;
+    bt = seg.block_table;
+  } else {
+    kv_len = kv_lens ? min(kv_lens[b], Skv) : Skv;
+    if (pg.block_table) bt = pg.block_table + (long)b * pg.bt_stride;
+  }
   const int hkv = h / (H / Hkv);
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t sQ = smem_base;                         // 2 tiles
   const uint32_t sK = smem_base + 2 * ATT_TILE_BYTES;                    // KV_STAGES tiles
   const uint32_t sV = smem_base + (2 + KV_STAGES) * ATT_TILE_BYTES;      // KV_STAGES tiles
-  const int kv_len = kv_lens ? min(kv_lens[b], Skv) : Skv;
   // causal: query row s sees keys [0, s + q_offset]; the CTA only visits tiles its last row sees
   const int kv_cta = causal ? min(kv_len, qblk * 2 * ATT_BM + 2 * ATT_BM + q_offset) : kv_len;
   const int n_kv_all = (kv_cta + ATT_BN - 1) / ATT_BN;
@@ -196,8 +225,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     }
     fence_mbar_init();
     tma_prefetch_desc(&tmQ);
-    tma_prefetch_desc(&tmK);
-    tma_prefetch_desc(&tmV);
+    tma_prefetch_desc(pK);
+    tma_prefetch_desc(pV);
   }
   if (warp == 1) {
     tmem_alloc(smem_u32(&tmem_base_s), 512);
@@ -218,9 +247,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         const int s0 = qblk * 2 * ATT_BM + t * ATT_BM;
 #pragma unroll
         for (int x = 0; x < HD / 64; ++x)
-          tma_load_4d(sQ + t * ATT_TILE_BYTES + x * ATT_HALF_BYTES, &tmQ, qb, 64 * x, s0, h, b);
+          tma_load_4d(sQ + t * ATT_TILE_BYTES + x * ATT_HALF_BYTES, &tmQ, qb, 64 * x, row0 + s0, h, b);
       }
-      const int* bt = pg.block_table ? pg.block_table + (long)b * pg.bt_stride : nullptr;
       const int last_page = bt ? max(0, (kv_len + pg.block_size - 1) / pg.block_size - 1) : 0;
       const int pages_per_tile = bt ? ATT_BN / pg.block_size : 0;
       const uint32_t page_bytes = bt ? (uint32_t)pg.block_size * 128u : 0u;   // per 64-wide half
@@ -238,13 +266,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             const int page = bt[min(j * pages_per_tile + i, last_page)];
 #pragma unroll
             for (int x = 0; x < HD / 64; ++x)
-              tma_load_4d(sK + st * ATT_TILE_BYTES + x * ATT_HALF_BYTES + i * page_bytes, &tmK, kb, 64 * x,
+              tma_load_4d(sK + st * ATT_TILE_BYTES + x * ATT_HALF_BYTES + i * page_bytes, pK, kb, 64 * x,
                           page * pg.block_size, hkv, 0);
           }
         } else {
 #pragma unroll
           for (int x = 0; x < HD / 64; ++x)
-            tma_load_4d(sK + st * ATT_TILE_BYTES + x * ATT_HALF_BYTES, &tmK, kb, 64 * x, j * ATT_BN, hkv, b);
+            tma_load_4d(sK + st * ATT_TILE_BYTES + x * ATT_HALF_BYTES, pK, kb, 64 * x, j * ATT_BN, hkv, b);
         }
         mbar_wait(smem_u32(&v_empty[st]), ph ^ 1, &s_abort, status, ERR_WAIT_EMPTY);
         const uint32_t vb = smem_u32(&v_full[st]);
@@ -254,13 +282,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             const int page = bt[min(j * pages_per_tile + i, last_page)];
 #pragma unroll
             for (int x = 0; x < HD / 64; ++x)
-              tma_load_4d(sV + st * ATT_TILE_BYTES + x * ATT_HALF_BYTES + i * page_bytes, &tmV, vb, 64 * x,
+              tma_load_4d(sV + st * ATT_TILE_BYTES + x * ATT_HALF_BYTES + i * page_bytes, pV, vb, 64 * x,
                           page * pg.block_size, hkv, 0);
           }
         } else {
 #pragma unroll
           for (int x = 0; x < HD / 64; ++x)
-            tma_load_4d(sV + st * ATT_TILE_BYTES + x * ATT_HALF_BYTES, &tmV, vb, 64 * x, j * ATT_BN, hkv, b);
+            tma_load_4d(sV + st * ATT_TILE_BYTES + x * ATT_HALF_BYTES, pV, vb, 64 * x, j * ATT_BN, hkv, b);
         }
       }
     }
@@ -477,7 +505,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         mbar_wait(smem_u32(&o_done[t]), 0, &s_abort, status, ERR_WAIT_PV);
         tc_fence_after_sync();
       }
-      if (out.kv_splits > 1) {
+      if (!SEGS && out.kv_splits > 1) {
         // split-KV share: unnormalised O, reference exponent and row sum for the merge kernel
         const long pidx = (((long)b * H + h) * Sq + srow) * out.kv_splits + split;
         if (srow < Sq) {
@@ -507,7 +535,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         float lse_row = l > 0.f ? (m + log2f(l)) * 0.6931471805599453f : -INFINITY;
         float wp = 0.f;                          // weight of the earlier result (continuation launches)
         const __nv_bfloat16* prow = nullptr;
-        if (out.prev_o != nullptr && srow < Sq) {
+        if (!SEGS && out.prev_o != nullptr && srow < Sq) {
           const float lp = out.prev_lse[((long)b * H + h) * Sq + srow];
           prow = out.prev_o + (long)b * out.p_bs + (long)srow * out.p_rs + (long)h * out.p_hs;
           if (!(l > 0.f)) {                      // no key seen here: the earlier result stands
@@ -521,8 +549,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             lse_row = fmaxf(lse_row, lp) + log1pf(__expf(-fabsf(d)));
           }
         }
-        if (srow < Sq && out.lse) out.lse[((long)b * H + h) * Sq + srow] = lse_row;
-        if (out.n_peers > 1) {
+        if (!SEGS && srow < Sq && out.lse) out.lse[((long)b * H + h) * Sq + srow] = lse_row;
+        if (!SEGS && out.n_peers > 1) {
           // Fused exchange: rows go to their owner ranks over NVLink.  A store from the thread that
           // owns the row would put 32 separate 16-byte writes on the link per instruction, so the
           // warp's 32 rows pass through shared memory (the Q tile of this query tile is no longer
@@ -582,10 +610,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         } else {
           __nv_bfloat16* orow = nullptr;
           if (srow < Sq) {
-            if (out.o2 && srow >= out.split)
+            if (!SEGS && out.o2 && srow >= out.split)
               orow = out.o2 + (long)b * out.o2_bs + (long)(srow - out.split) * out.o2_rs + (long)h * out.o2_hs;
             else
-              orow = out.o + (long)b * out.o_bs + (long)srow * out.o_rs + (long)h * out.o_hs;
+              orow = out.o + (long)b * out.o_bs + (long)(row0 + srow) * out.o_rs + (long)h * out.o_hs;
           }
 #pragma unroll 1
           for (int c = 0; c < HD / 32; ++c) {
@@ -621,7 +649,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   tc_fence_before_sync();
   __syncthreads();
   // every peer store of this CTA was issued before the barrier above
-  if (threadIdx.x == 0) peer_signal_cta_done(sig, gridDim.x * gridDim.y * gridDim.z);
+  if (!SEGS && threadIdx.x == 0) peer_signal_cta_done(sig, gridDim.x * gridDim.y * gridDim.z);
   if (s_abort) {
     const unsigned long long t0 = globaltimer_ns();
     while (globaltimer_ns() - t0 < 200000ull) {
@@ -674,15 +702,15 @@ static int launch_attn(const CUtensorMap& tq, const CUtensorMap& tk, const CUten
                        int D = ATT_D) {
   // OMNI_ATTN_HANDOFFS (4 | 2 | 1): tuning switch, see attn_fwd_kernel
   typedef void (*KernelFn)(const CUtensorMap, const CUtensorMap, const CUtensorMap, AttnOut, int, int, int, int, const int*,
-                           float, int, int, AttnPaging, PeerSignal, int*);
+                           float, int, int, AttnPaging, PeerSignal, int*, const NoSegs);
   static KernelFn fns[2] = {nullptr, nullptr};     // [0]: head size 64, [1]: head size 128
   const int di = D == 64 ? 0 : 1;
   if (fns[di] == nullptr) {
     const char* ev = getenv("OMNI_ATTN_HANDOFFS");
     const int want = ev ? atoi(ev) : 4;
     KernelFn f;
-    if (di == 0) f = want == 1 ? attn_fwd_kernel<1, 64> : (want == 2 ? attn_fwd_kernel<2, 64> : attn_fwd_kernel<4, 64>);
-    else f = want == 1 ? attn_fwd_kernel<1, 128> : (want == 2 ? attn_fwd_kernel<2, 128> : attn_fwd_kernel<4, 128>);
+    if (di == 0) f = want == 1 ? attn_fwd_kernel<1, 64, NoSegs> : (want == 2 ? attn_fwd_kernel<2, 64, NoSegs> : attn_fwd_kernel<4, 64, NoSegs>);
+    else f = want == 1 ? attn_fwd_kernel<1, 128, NoSegs> : (want == 2 ? attn_fwd_kernel<2, 128, NoSegs> : attn_fwd_kernel<4, 128, NoSegs>);
     fns[di] = f;
   }
   static unsigned long long prepared[2] = {0, 0};
@@ -694,11 +722,90 @@ static int launch_attn(const CUtensorMap& tq, const CUtensorMap& tk, const CUten
   PeerWait unused;
   unpack_sync(sync, sig, unused);
   launch_with(!sync, 1, fns[di], grid, ATT_THREADS, di == 0 ? AttCfg<64>::SMEM : AttCfg<128>::SMEM, stream,
-      tq, tk, tv, out, Sq, Skv, H, Hkv, kv_lens, scale_log2, causal, q_offset, pg, sig, status);
+      tq, tk, tv, out, Sq, Skv, H, Hkv, kv_lens, scale_log2, causal, q_offset, pg, sig, status, NoSegs{});
+  return (int)cudaGetLastError();
+}
+
+template <int HD>
+static int launch_segs(const CUtensorMap& tq, AttnOut& out, int H, int Hkv, const AttnSegs& segs, int blocks, float scale, const AttnPaging& pg, int* status,
+                       cudaStream_t stream) {
+  static unsigned long long prepared = 0;
+  if (int e = ensure_dynamic_smem((const void*)attn_fwd_kernel<4, HD, AttnSegs>, AttCfg<HD>::SMEM, prepared)) return e;
+  launch_overlapped(attn_fwd_kernel<4, HD, AttnSegs>, dim3(H, blocks), ATT_THREADS, AttCfg<HD>::SMEM, stream, tq, tq, tq, out, 0, 0, H, Hkv, nullptr,
+                    scale * 1.4426950408889634f, 1, 0, pg, PeerSignal{}, status, segs);
   return (int)cudaGetLastError();
 }
 
 }  // namespace omni
+
+// Causal attention of the prompt segments of one step.  q, k, v: bf16 [rows, heads, D], rows of the step's projections; segment i has rows
+// [start[i], start[i] + len[i]) and, before them, context[i] tokens that are in the cache.  A segment without context reads its keys from k and v; another reads
+// all of them, its own included, from the pages (head size 128 only) that table[i] (int32 page ids) names.
+extern "C" int omni_attn_prefill_segs(const void* q, long q_rs, long q_hs, const void* k, long k_rs, long k_hs, const void* v, long v_rs, long v_hs,
+                                      const void* k_pool, const void* v_pool, int num_blocks, int block_size, void* o, long o_rs, long o_hs, int rows,
+                                      int H, int Hkv, int D, int n, const int* start, const int* len, const int* context, const void* const* table,
+                                      float scale, int* status, void* stream) {
+  using namespace omni;
+  if ((D != 64 && D != 128) || H <= 0 || Hkv <= 0 || (H % Hkv) || (o_rs & 7) || (o_hs & 7) || (reinterpret_cast<uintptr_t>(o) & 15)) return RC_BAD_ARG;
+  CUtensorMap tq, pk, pv;
+  if (rows <= 0 || n <= 0) return RC_OK;
+  if (int rc = make_qkv_tmap(&tq, q, rows, H, 1, q_rs, q_hs, rows * q_rs, ATT_BM, D)) return rc;
+  bool paged = false;
+  for (int i = 0; i < n; ++i) {
+    if (len[i] < 0 || start[i] < 0 || context[i] < 0 || (long)start[i] + len[i] > rows) return RC_BAD_ARG;
+    if (len[i] > 4096 * 2 * ATT_BM) return RC_TOO_LARGE;
+    if (context[i] > 0) {
+      if (D != 128 || table[i] == nullptr || block_size < 8 || (block_size & 7) || (ATT_BN % block_size) || num_blocks <= 0) return RC_BAD_ARG;
+      paged = true;
+    }
+  }
+  if (paged) {
+    const long pool = (long)num_blocks * block_size;
+    if (int rc = make_qkv_tmap(&pk, k_pool, (int)pool, Hkv, 1, (long)Hkv * D, D, pool * Hkv * D, block_size)) return rc;
+    if (int rc = make_qkv_tmap(&pv, v_pool, (int)pool, Hkv, 1, (long)Hkv * D, D, pool * Hkv * D, block_size)) return rc;
+  }
+  AttnOut out = {};
+  out.o = (__nv_bfloat16*)o;
+  out.o_rs = o_rs; out.o_hs = o_hs;
+  const AttnPaging pg = {nullptr, 0, block_size};
+  AttnSegs segs;
+  for (int i0 = 0; i0 < n; i0 += AttnSegs::MAX) {
+    const int m = n - i0 < AttnSegs::MAX ? n - i0 : AttnSegs::MAX;
+    int left[AttnSegs::MAX];                                 // query blocks not handed out yet: the last of a segment has the most keys
+    for (int i = 0; i < m; ++i) {
+      AttnSegs::Seg& g = segs.s[i];
+      const int a = start[i0 + i], c = context[i0 + i];
+      g.row0 = a; g.len = len[i0 + i]; g.kv_len = g.len + c;
+      g.block_table = c > 0 ? static_cast<const int*>(table[i0 + i]) : nullptr;
+      left[i] = (g.len + 2 * ATT_BM - 1) / (2 * ATT_BM);
+      if (c > 0) {
+        g.tmK = pk; g.tmV = pv;
+      } else if (g.len > 0) {
+        if (int rc = make_qkv_tmap(&g.tmK, (const __nv_bfloat16*)k + a * k_rs, g.len, Hkv, 1, k_rs, k_hs, g.len * k_rs, ATT_BM, D)) return rc;
+        if (int rc = make_qkv_tmap(&g.tmV, (const __nv_bfloat16*)v + a * v_rs, g.len, Hkv, 1, v_rs, v_hs, g.len * v_rs, ATT_BM, D)) return rc;
+      }
+    }
+    for (int i = m; i < AttnSegs::MAX; ++i) segs.s[i] = segs.s[0];
+    for (;;) {
+      int blocks = 0;
+      for (; blocks < AttnSegs::MAX_BLOCKS; ++blocks) {
+        int best = -1, most = -1;
+        for (int i = 0; i < m; ++i) {
+          const AttnSegs::Seg& g = segs.s[i];
+          const int keys = left[i] * 2 * ATT_BM + g.kv_len - g.len, seen = keys < g.kv_len ? keys : g.kv_len;
+          if (left[i] > 0 && seen > most) { most = seen; best = i; }
+        }
+        if (best < 0) break;
+        segs.order[blocks] = (unsigned short)(best << 12 | --left[best]);
+      }
+      if (blocks == 0) break;
+      const int rc = D == 64 ? launch_segs<64>(tq, out, H, Hkv, segs, blocks, scale, pg, status, (cudaStream_t)stream)
+                             : launch_segs<128>(tq, out, H, Hkv, segs, blocks, scale, pg, status, (cudaStream_t)stream);
+      if (rc) return rc;
+    }
+  }
+  return RC_OK;
+}
 
 // Strides are in elements: *_rs between consecutive sequence positions, *_hs between heads,
 // *_bs between batches; head_dim (128) is contiguous.  o2/split route query rows >= split

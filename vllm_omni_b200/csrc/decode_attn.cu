@@ -39,7 +39,20 @@ struct DecodeAttn {
   float *part_o, *part_ml;
   __nv_bfloat16* out;
   long o_rs;
+  const long long* rows;             // sequence -> row of q and out (below zero: from the end); null: the sequence's number
+  int n_rows;
+  int* status;
 };
+
+// Row of q and out; -1 where there is none, which the status word tells the host.
+__device__ __forceinline__ long da_row(const DecodeAttn& p, int seq) {
+  if (!p.rows) return seq;
+  long long r = p.rows[seq];
+  if (r < 0) r += p.n_rows;
+  if (r >= 0 && r < p.n_rows) return (long)r;
+  if (threadIdx.x == 0) atomicCAS(p.status, 0, ERR_BOUNDS);
+  return -1;
+}
 
 // UP: 9 .. 16 heads per group, the second half of the MMA's 16 rows is live.
 template <bool UP>
@@ -53,6 +66,8 @@ paged_decode_kernel(const __grid_constant__ DecodeAttn p) {
   const int hk = blockIdx.z * DA_WARPS + warp % per_block;
   if (sub >= p.subs || hk >= p.Hkv) return;
   const int G = p.H / p.Hkv, h0 = hk * G, parts = p.splits * p.subs;
+  const long q_row = da_row(p, seq);
+  if (q_row < 0) return;
   const int len = min(p.lens[seq], p.max_keys);
   const int tiles = (len + DA_KEYS - 1) / DA_KEYS, per = (tiles + p.splits - 1) / p.splits;
   const int t1 = min(tiles, (split + 1) * per);
@@ -72,7 +87,7 @@ paged_decode_kernel(const __grid_constant__ DecodeAttn p) {
   for (int u = 0; u < NH; ++u)
 #pragma unroll
     for (int c = 0; c < 4; ++c)
-      q[u][c] = u * 8 + g < G ? *reinterpret_cast<const uint4*>(p.q + (long)seq * p.q_rs + (long)(h0 + u * 8 + g) * DA_D + c * 32 + j * 8)
+      q[u][c] = u * 8 + g < G ? *reinterpret_cast<const uint4*>(p.q + q_row * p.q_rs + (long)(h0 + u * 8 + g) * DA_D + c * 32 + j * 8)
                               : make_uint4(0u, 0u, 0u, 0u);
   float m[NH], l[NH], acc[NH][8][4];
 #pragma unroll
@@ -209,7 +224,7 @@ paged_decode_kernel(const __grid_constant__ DecodeAttn p) {
           w.y = pack_bf16(acc[u][2][2 * b + hh] * f, acc[u][3][2 * b + hh] * f);
           w.z = pack_bf16(acc[u][4][2 * b + hh] * f, acc[u][5][2 * b + hh] * f);
           w.w = pack_bf16(acc[u][6][2 * b + hh] * f, acc[u][7][2 * b + hh] * f);
-          *reinterpret_cast<uint4*>(p.out + (long)seq * p.o_rs + (long)(h0 + u * 8 + h) * DA_D + b * 64 + g * 8) = w;
+          *reinterpret_cast<uint4*>(p.out + q_row * p.o_rs + (long)(h0 + u * 8 + h) * DA_D + b * 64 + g * 8) = w;
         }
       }
     }
@@ -219,11 +234,14 @@ paged_decode_kernel(const __grid_constant__ DecodeAttn p) {
 // out[seq, h] = sum_s 2^(m_s - m*) O_s / sum_s 2^(m_s - m*) l_s over a row's shares (at most 64): one block per row, its warps take
 // every fourth share, four channels per lane.
 __global__ void __launch_bounds__(128)
-paged_decode_merge_kernel(const float* part_o, const float* part_ml, int parts, int H,
-                          __nv_bfloat16* __restrict__ out, long o_rs) {
+paged_decode_merge_kernel(const __grid_constant__ DecodeAttn p, int parts) {
   pdl_begin();
   __shared__ float4 part[4][32];
+  const float *part_o = p.part_o, *part_ml = p.part_ml;
+  const int H = p.H;
   const long r = blockIdx.x;
+  const long row = da_row(p, (int)(r / H));
+  if (row < 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float2* ml = reinterpret_cast<const float2*>(part_ml) + r * parts;
   const float4* po = reinterpret_cast<const float4*>(part_o) + r * parts * (DA_D / 4) + lane;
@@ -267,7 +285,7 @@ paged_decode_merge_kernel(const float* part_o, const float* part_ml, int parts, 
   uint2 w;
   w.x = pack_bf16(acc.x * f, acc.y * f);
   w.y = pack_bf16(acc.z * f, acc.w * f);
-  *reinterpret_cast<uint2*>(out + seq * o_rs + (r - seq * H) * DA_D + lane * 4) = w;
+  *reinterpret_cast<uint2*>(p.out + row * p.o_rs + (r - seq * H) * DA_D + lane * 4) = w;
 }
 
 constexpr int DA_MAX_PARTS = 64;
@@ -302,10 +320,11 @@ extern "C" int omni_paged_decode_shares(int n, int Hkv, int max_keys) {
 }
 
 // q [n, H, 128] (row pitch q_rs elements, heads side by side), pages [blocks, block_size, Hkv, 128] with block_size a multiple of 8,
-// block_tables int32 [n, bt_stride], lens int32 [n] (counted up to max_keys), out [n, H, 128] (pitch o_rs).
+// block_tables int32 [n, bt_stride], lens int32 [n] (counted up to max_keys), out [n, H, 128] (pitch o_rs).  rows (may be null): int64 [n], sequence i
+// is row rows[i] of q and out, which then have n_rows rows.
 extern "C" int omni_paged_decode_attn(const void* q, long q_rs, const void* k, const void* v, const int* block_tables, int bt_stride,
                                       int block_size, const int* lens, int n, int H, int Hkv, int max_keys, float scale, float* part_o,
-                                      float* part_ml, void* out, long o_rs, void* stream) {
+                                      float* part_ml, void* out, long o_rs, const long long* rows, int n_rows, int* status, void* stream) {
   if (n <= 0) return RC_OK;
   if (Hkv <= 0 || H % Hkv || H / Hkv > 16 || block_size < 8 || (block_size & 7) || max_keys < 1 || n > 65535 || (q_rs & 7) || (o_rs & 7))
     return RC_BAD_ARG;
@@ -319,12 +338,13 @@ extern "C" int omni_paged_decode_attn(const void* q, long q_rs, const void* k, c
   p.q_rs = q_rs; p.block_tables = block_tables; p.bt_stride = bt_stride; p.block_size = block_size; p.lens = lens; p.max_keys = max_keys;
   p.H = H; p.Hkv = Hkv; p.scale_log2 = scale * 1.4426950408889634f;
   p.part_o = part_o; p.part_ml = part_ml; p.out = (__nv_bfloat16*)out; p.o_rs = o_rs;
+  p.rows = rows; p.n_rows = n_rows; p.status = status;
   const dim3 grid((unsigned)p.splits, (unsigned)n, (unsigned)((Hkv + DA_WARPS - 1) / DA_WARPS));
   cudaStream_t st = (cudaStream_t)stream;
   if (H / Hkv > 8) launch_overlapped(paged_decode_kernel<true>, grid, 32 * DA_WARPS, 0, st, p);
   else launch_overlapped(paged_decode_kernel<false>, grid, 32 * DA_WARPS, 0, st, p);
   if (parts == 1) return (int)cudaGetLastError();
   if (cudaError_t e = cudaGetLastError()) return (int)e;
-  launch_overlapped(paged_decode_merge_kernel, (unsigned)n * H, 128, 0, st, part_o, part_ml, parts, H, (__nv_bfloat16*)out, o_rs);
+  launch_overlapped(paged_decode_merge_kernel, (unsigned)n * H, 128, 0, st, p, parts);
   return (int)cudaGetLastError();
 }

@@ -326,7 +326,12 @@ class QwenDecoderModel(nn.Module):
         v = qkv[:, (H + Hkv) * Dh:].view(T, Hkv, Dh)
         scale = 1.0 / math.sqrt(Dh)
         o = out.view(T, H, Dh)
-        for seg in batch.prefills:
+        context = lambda seg: seg.context if k_cache is not None else 0
+        joint = bool(batch.prefills) and KC.prefill_segments_ok(q, k_cache, [context(seg) for seg in batch.prefills])
+        if joint:
+            KC.prefill_segments(q, k, v, k_cache, v_cache, [(seg.start, seg.length, context(seg), seg.block_table) for seg in batch.prefills],
+                                scale=scale, out=o)
+        for seg in () if joint else batch.prefills:
             s, n = seg.start, seg.length
             if seg.context == 0 or k_cache is None:
                 attention(q[None, s:s + n], k[None, s:s + n], v[None, s:s + n], scale=scale, causal=True,
@@ -345,9 +350,7 @@ class QwenDecoderModel(nn.Module):
                 # a decode-only step: the rows ARE the batch in order; read q and write o in place
                 KC.paged_decode(q, k_cache, v_cache, batch.decode_block_tables, batch.decode_seq_lens, scale=scale, out=o)
             else:
-                qd = q[rows].contiguous()
-                od = KC.paged_decode(qd, k_cache, v_cache, batch.decode_block_tables, batch.decode_seq_lens, scale=scale)
-                o[rows] = od
+                KC.paged_decode(q, k_cache, v_cache, batch.decode_block_tables, batch.decode_seq_lens, scale=scale, out=o, rows=rows)
         return out
 
     def forward(self, batch: ModelBatch, kv_caches=None, capture_layers=(), deepstack=None):

@@ -112,13 +112,21 @@ def decode_impl(n: int, H: int, Hkv: int, D: int, block_size: int, num_splits, q
     return "stream" if whole and (groups <= 16 or (groups > sms and not 1.8 * sms <= groups <= 2 * sms)) else "tc"
 
 
-def paged_decode(q, k_cache, v_cache, block_tables, seq_lens, scale=None, num_splits=None, out=None, impl=None):
+def paged_decode(q, k_cache, v_cache, block_tables, seq_lens, scale=None, num_splits=None, out=None, impl=None, rows=None):
     """q: [num_seqs, H, D] (one new token per sequence) -> [num_seqs, H, D].
 
+    ``rows`` (int64 [num_seqs]): sequence i is row rows[i] of q and of ``out``, which is then needed; other rows of it stay.
+
     ``impl``: "stream" (csrc/decode_attn.cu), "tc" (tcgen05 kernel) or "simt"; by default as ``decode_impl`` says."""
-    n, H, D = q.shape
+    n, H, D = q.shape if rows is None else (rows.numel(), *q.shape[1:])
     nb, bs, Hkv, _ = k_cache.shape
     scale = scale if scale is not None else 1.0 / math.sqrt(D)
+    if rows is not None:
+        if impl is None and q.is_cuda:
+            impl = decode_impl(n, H, Hkv, D, bs, num_splits, q.stride(0), out.stride(0))
+        if impl != "stream" or rows.dtype != torch.int64 or not rows.is_contiguous() or rows.device != q.device:
+            out[rows] = paged_decode(q[rows].contiguous(), k_cache, v_cache, block_tables, seq_lens, scale, num_splits)
+            return out
     if out is None:
         out = torch.empty_like(q)
     if not q.is_cuda:
@@ -140,7 +148,8 @@ def paged_decode(q, k_cache, v_cache, block_tables, seq_lens, scale=None, num_sp
         rc = lib.omni_paged_decode_attn(
             nv.ptr(q), c_long(q.stride(0)), nv.ptr(k_cache), nv.ptr(v_cache), nv.ptr(block_tables), c_int(block_tables.stride(0)), c_int(bs),
             nv.ptr(seq_lens), c_int(n), c_int(H), c_int(Hkv), c_int(max_kv), c_float(scale), nv.ptr(part),
-            nv.ptr(None if part is None else part[n * H * shares * D:]), nv.ptr(out), c_long(out.stride(0)), nv.stream_ptr())
+            nv.ptr(None if part is None else part[n * H * shares * D:]), nv.ptr(out), c_long(out.stride(0)), nv.ptr(rows), c_int(q.shape[0]),
+            nv.ptr(nv.status_word(q.device)), nv.stream_ptr())
         nv.check_rc(rc, "omni_paged_decode_attn")
         return out
     if impl == "tc":
@@ -167,6 +176,34 @@ def paged_decode(q, k_cache, v_cache, block_tables, seq_lens, scale=None, num_sp
         c_float(scale), c_int(num_splits), nv.ptr(sc[0]), nv.ptr(sc[1]), nv.ptr(out), c_long(out.stride(0)),
         nv.stream_ptr())
     nv.check_rc(rc, "omni_paged_decode")
+    return out
+
+
+def prefill_segments_ok(q, k_cache, contexts) -> bool:
+    """Whether ``prefill_segments`` takes these operands: bf16, head size 64 or 128, and pages of its kind where a segment has a context."""
+    D = q.shape[2]
+    return q.is_cuda and q.dtype == torch.bfloat16 and D in (64, 128) and (not any(contexts) or tma_pages_ok(k_cache.shape[1], D))
+
+
+def prefill_segments(q, k, v, k_cache, v_cache, segs, scale=None, out=None):
+    """Causal attention of all prompt segments of one step in one launch (csrc/attention_sm100.cu, eight segments at a time).
+
+    q [T, H, D], k, v [T, Hkv, D]: rows of the step; ``segs``: (first row, rows, context, block table) each.  A segment without context reads its keys from
+    k and v, another all of its keys from the pages, where this step's were written before.  Rows of no segment stay as they are in ``out``."""
+    T, H, D = q.shape
+    Hkv = k.shape[1]
+    assert q.stride(2) == 1 and k.stride(2) == 1 and v.stride(2) == 1 and out.stride(2) == 1
+    n = len(segs)
+    ints = lambda i: (c_int * n)(*(s[i] for s in segs))
+    tables = [s[3] if s[2] else None for s in segs]
+    assert all(t is None or (t.dtype == torch.int32 and t.stride(-1) == 1) for t in tables)
+    nb, bs = (k_cache.shape[0], k_cache.shape[1]) if k_cache is not None else (0, 0)
+    rc = nv.lib("attention_sm100").omni_attn_prefill_segs(
+        nv.ptr(q), c_long(q.stride(0)), c_long(q.stride(1)), nv.ptr(k), c_long(k.stride(0)), c_long(k.stride(1)), nv.ptr(v), c_long(v.stride(0)),
+        c_long(v.stride(1)), nv.ptr(k_cache), nv.ptr(v_cache), c_int(nb), c_int(bs), nv.ptr(out), c_long(out.stride(0)), c_long(out.stride(1)), c_int(T),
+        c_int(H), c_int(Hkv), c_int(D), c_int(n), ints(0), ints(1), ints(2), (ctypes.c_void_p * n)(*(0 if t is None else t.data_ptr() for t in tables)),
+        c_float(scale if scale is not None else 1.0 / math.sqrt(D)), nv.ptr(nv.status_word(q.device)), nv.stream_ptr())
+    nv.check_rc(rc, "omni_attn_prefill_segs")
     return out
 
 
