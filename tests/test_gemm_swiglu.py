@@ -1,0 +1,67 @@
+"""Gated layers in one launch (``gemm.linear_swiglu``) and the epilogue kernels of the general linear layers, against 64-bit sums."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+from vllm_omni_b200.ops import _native as nv, gemm
+
+pytestmark = pytest.mark.gpu
+
+
+def _rnd(seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+
+
+# rows of the few-row kernels (1 to 16), of the two-launch form (17 to 128) and of both general kernels; widths that end inside a group of 8, a chunk and a tile
+@pytest.mark.parametrize("M", [1, 7, 8, 9, 16, 17, 64, 128, 129, 300, 700, 2500])
+@pytest.mark.parametrize("F_,K", [(8, 64), (24, 200), (136, 72), (768, 512), (1000, 2048), (6144, 256)])
+def test_swiglu(M, F_, K):
+    rnd = _rnd(M + F_)
+    x, w = rnd(M, K), (rnd(2 * F_, K).float() * K ** -0.5 * 1.5).bfloat16()
+    y = gemm.linear_swiglu(x, w)
+    nv.check_status(x.device)
+    g, u = (x.double() @ w.double().T).split(F_, 1)
+    ref = F.silu(g) * u
+    # fp32 sums of K / 16 MMA steps, each off by at most an ulp of the terms' magnitudes so far; silu's slope is at most 1.1
+    mass = (x.double().abs() @ w.double().abs().T).split(F_, 1)
+    sums = 1.1 * (mass[0] * u.abs() + mass[1] * g.abs()) * (K / 16 + 1) * 2.0 ** -24
+    # result to bf16; tanh.approx in silu; where it takes two launches both halves pass through bf16 first
+    halves = (2.0 ** -8 * (g.abs() * u.abs()) * 2.2 if 16 < M <= 128 else 0.0)
+    assert torch.isfinite(y).all() and ((y.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + g.abs() * u.abs() * 2.0 ** -10 + sums + halves + 1e-5).all()
+
+
+def test_swiglu_takes_views():
+    rnd = _rnd(3)
+    x, w = rnd(2, 150, 96)[:, :, 8:72], rnd(80, 64)
+    a, b = gemm.linear_swiglu(x, w), gemm.linear_swiglu(x.contiguous(), w)
+    assert a.shape == (2, 150, 40) and torch.equal(a, b)
+
+
+# every kernel (pair of 256 / 192 / 128 columns, automatic choice) with every epilogue; ragged rows and columns; rows of a tile in two batches
+@pytest.mark.parametrize("bn", [0, 384, 448, 576])
+@pytest.mark.parametrize("act", [None, "gelu_tanh", "xielu", "silu", "relu2"])
+@pytest.mark.parametrize("B,S,N,K", [(2, 100, 200, 136), (2, 333, 520, 64), (1, 257, 8, 72)])
+@pytest.mark.parametrize("operands", ["", "bias", "bias residual", "bias gate residual"])
+def test_epilogues(bn, act, B, S, N, K, operands):
+    rnd = _rnd(S + N)
+    x, w = rnd(B, S, K), (rnd(N, K).float() * K ** -0.5).bfloat16()
+    kw = dict(bias=rnd(N) if "bias" in operands else None, residual=rnd(B, S, N) if "residual" in operands else None,
+              gate=rnd(B, N) if "gate" in operands else None, coef=(0.8, 0.6))
+    y = gemm.linear(x, w, act=act, force_bn=bn, **kw)
+    nv.check_status(x.device)
+    up = lambda t: None if t is None else t.double()
+    z = x.double() @ w.double().T
+    ref = z if kw["bias"] is None else z + up(kw["bias"])
+    size = ref.abs()
+    ref = {None: lambda t: t, "gelu_tanh": lambda t: F.gelu(t, approximate="tanh"), "silu": F.silu, "relu2": lambda t: F.relu(t).square(),
+           "xielu": lambda t: gemm.xielu(t, (0.8, 0.6))}[act](ref)
+    slack = size * 2.0 ** -10 + (ref.abs() * 2.0 ** -13 if act in ("relu2", "xielu") else 0.0)      # tanh.approx, ex2.approx; fp32 sums
+    if kw["gate"] is not None:
+        ref, slack = ref * up(kw["gate"])[:, None], slack * up(kw["gate"]).abs()[:, None]
+    if kw["residual"] is not None:
+        ref = ref + up(kw["residual"])
+    assert ((y.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + slack + 2e-5).all()
+    buf = None if kw["residual"] is None else kw["residual"].clone()
+    if buf is not None:                                              # in place: the residual is the output
+        assert torch.equal(gemm.linear(x, w, act=act, force_bn=bn, **{**kw, "residual": buf}, out=buf), y)

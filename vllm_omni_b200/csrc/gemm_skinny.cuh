@@ -80,15 +80,17 @@ __device__ __forceinline__ void skinny_finish(float (&x)[B], int m, int step, in
 
 // ---------------------------------------------------------------------------------------------------- at most 16 rows
 // NT * 8 rows of A; 16 resident warps x U chunks x 1 KB = up to 128 KB of W in flight per SM.
-template <int NT, int NW, int U, int BLOCKS>
+// GATED: W holds N / 2 gate rows and then their lift rows; a block makes 8 columns of C, silu(gate) * lift, from 8 rows of each.
+template <int NT, int NW, int U, int BLOCKS, bool GATED>
 __global__ void __launch_bounds__(32 * NW, BLOCKS)
 gemm_rows_kernel(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W, int ldw, __nv_bfloat16* C, int ldc,
                  int M, int N, int K, const __grid_constant__ GemmEpilogue epi, int resident) {
   __shared__ float part[NW][NT * 8][16];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, j = lane & 3;
   const int n0 = blockIdx.x * 16;
+  auto w_row = [&](int i) { return GATED ? min(n0 / 2 + (i & 7), N / 2 - 1) + (i >> 3) * (N / 2) : min(n0 + i, N - 1); };
   if ((int)blockIdx.x < resident) {             // W does not come from the kernel before: the first blocks' share is on its way to L2 meanwhile
-    const __nv_bfloat16* w = W + (size_t)min(n0 + (int)(threadIdx.x & 15), N - 1) * ldw;
+    const __nv_bfloat16* w = W + (size_t)w_row(threadIdx.x & 15) * ldw;
     for (int c = (threadIdx.x >> 4) * 64; c < K; c += 2 * NW * 64) prefetch_l2(w + c);
   }
   pdl_begin();
@@ -101,12 +103,27 @@ gemm_rows_kernel(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W, int ld
     for (int i = 0; i < 4; ++i) acc[t][i] = 0.f;
   }
   // columns past N repeat the last one and are not stored
-  few_rows_products<NT, NW, U>(acc, W + (size_t)min(n0 + g, N - 1) * ldw, W + (size_t)min(n0 + 8 + g, N - 1) * ldw, x, K, warp, j);
+  few_rows_products<NT, NW, U>(acc, W + (size_t)w_row(g) * ldw, W + (size_t)w_row(8 + g) * ldw, x, K, warp, j);
 #pragma unroll
   for (int t = 0; t < NT; ++t)
 #pragma unroll
     for (int i = 0; i < 4; ++i) part[warp][t * 8 + j * 2 + (i & 1)][g + 8 * (i >> 1)] = acc[t][i];
   __syncthreads();
+  if constexpr (GATED) {
+    for (int e = threadIdx.x; e < NT * 64; e += 32 * NW) {
+      const int n = n0 / 2 + (e & 7), m = e >> 3;
+      if (n < N / 2 && m < M) {
+        float gate = 0.f, lift = 0.f;
+#pragma unroll
+        for (int w = 0; w < NW; ++w) {
+          gate += part[w][m][e & 7];
+          lift += part[w][m][8 + (e & 7)];
+        }
+        C[(size_t)m * ldc + n] = __float2bfloat16(silu(gate) * lift);
+      }
+    }
+    return;
+  }
 #pragma unroll
   for (int e = threadIdx.x; e < NT * 128; e += 32 * NW) {
     const int n = n0 + (e & 15), m = e >> 4;
@@ -129,7 +146,7 @@ gemm_rows_kernel(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W, int ld
 //   more, 9 rows and up: four blocks of 4 warps where their last round is at least half full (24576 x 4096 46.1 with two blocks
 //                of 8, 42.1 with four of 4; 9216 x 2048 10.2 and 9.2), not where it is emptier (12288 x 4096 25.3 and 27.8)
 //   else         two blocks of 8 (8 rows, 32768 x 4096: 46.2; four of 4 48.0, three of 8 47.9; the copy rate would be 40.4)
-template <int NT>
+template <int NT, bool GATED>
 static void launch_rows(int tiles, const __nv_bfloat16* A, int lda, const __nv_bfloat16* W, int ldw, __nv_bfloat16* C, int ldc, int M,
                         int N, int K, const GemmEpilogue& epi, cudaStream_t stream) {
   constexpr int U = NT == 1 ? 8 : 4;
@@ -137,10 +154,10 @@ static void launch_rows(int tiles, const __nv_bfloat16* A, int lda, const __nv_b
   const auto go = [&](auto kernel, int warps, int blocks) {
     launch_overlapped(kernel, tiles, 32 * warps, 0, stream, A, lda, W, ldw, C, ldc, M, N, K, epi, blocks * sms);
   };
-  if (tiles <= sms && K > 1024) go(gemm_rows_kernel<NT, 16, U, 1>, 16, 1);
-  else if (tiles > 2 * sms && tiles <= 3 * sms) go(gemm_rows_kernel<NT, 8, U / 2, 3>, 8, 3);
-  else if (NT == 2 && tiles > 3 * sms && (last == 0 || last >= 2 * sms)) go(gemm_rows_kernel<NT, 4, U, 4>, 4, 4);
-  else go(gemm_rows_kernel<NT, 8, U, 2>, 8, 2);
+  if (tiles <= sms && K > 1024) go(gemm_rows_kernel<NT, 16, U, 1, GATED>, 16, 1);
+  else if (tiles > 2 * sms && tiles <= 3 * sms) go(gemm_rows_kernel<NT, 8, U / 2, 3, GATED>, 8, 3);
+  else if (NT == 2 && tiles > 3 * sms && (last == 0 || last >= 2 * sms)) go(gemm_rows_kernel<NT, 4, U, 4, GATED>, 4, 4);
+  else go(gemm_rows_kernel<NT, 8, U, 2, GATED>, 8, 2);
 }
 
 static int launch_rows(const void* A, int lda, const void* W, int ldw, __nv_bfloat16* C, int ldc, int M, int N, int K,
@@ -148,8 +165,9 @@ static int launch_rows(const void* A, int lda, const void* W, int ldw, __nv_bflo
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15) return RC_BAD_ARG;
   const auto a = static_cast<const __nv_bfloat16*>(A), w = static_cast<const __nv_bfloat16*>(W);
   const int tiles = (N + 15) / 16;
-  if (M <= 8) launch_rows<1>(tiles, a, lda, w, ldw, C, ldc, M, N, K, epi, stream);
-  else launch_rows<2>(tiles, a, lda, w, ldw, C, ldc, M, N, K, epi, stream);
+  const bool gated = epi.act == EPI_SWIGLU;
+  const auto go = M <= 8 ? (gated ? launch_rows<1, true> : launch_rows<1, false>) : (gated ? launch_rows<2, true> : launch_rows<2, false>);
+  go(tiles, a, lda, w, ldw, C, ldc, M, N, K, epi, stream);
   return (int)cudaGetLastError();
 }
 

@@ -224,13 +224,113 @@ __device__ __forceinline__ void epilogue_store32(const uint32_t (&v)[32], int ro
     if (col0 + j * 8 < N) *reinterpret_cast<uint4*>(out + j * 8) = o[j];
 }
 
+// Epilogues of tiles that stay on this GPU, one kernel each: the code of all activations and of the peer stores in one kernel crowds the instruction cache
+// of eight warps that run through theirs once per tile.  EPI_ANY is that kernel, for the rest (SiLU, squared ReLU, peers, two problems of different
+// activations).  us with bias, gate and residual, what there was before (one kernel
+// for all, operands read when the accumulator was there) in brackets: 8192 x 3072 x 3072 117 (121), 2048 x 3072 x 3072 35 (39), 4096 x 2048 x 2048 34 (41);
+// two problems of 4096 and 48 rows, 3072 x 3072, behind layers of the same block 68 (86).
+// EPI_SWIGLU: the accumulator's columns are 8 gate columns, their 8 lift columns, and so on (see swiglu_map); C has half as many.
+constexpr int EPI_ANY = -1, EPI_SWIGLU = 5;
+
+__device__ __forceinline__ void add_bf16x8(float (&x)[8], const uint4& u) {
+  const float2 a = unpack_bf16(u.x), b = unpack_bf16(u.y), c = unpack_bf16(u.z), d = unpack_bf16(u.w);
+  x[0] += a.x; x[1] += a.y; x[2] += b.x; x[3] += b.y;
+  x[4] += c.x; x[5] += c.y; x[6] += d.x; x[7] += d.y;
+}
+
+// CH chunks of 32 accumulator columns of one row, from column col0 (TMEM address `tmem`).  `ready` waits for the accumulator; what it does not depend on is
+// read before: the whole residual where there is no activation (a gated residual layer), else a chunk's with its bias.
+template <int MODE, int CH, typename Ready>
+__device__ __forceinline__ void drain_row(uint32_t tmem, int row, bool row_ok, int col0, int N, __nv_bfloat16* C, int ldc, const GemmEpilogue& epi,
+                                          Ready ready) {
+  __nv_bfloat16* out = C;
+  const __nv_bfloat16 *res = nullptr, *gate = nullptr;
+  if (row_ok) {
+    if (epi.c_rows_per_batch > 0) {
+      const int cb = row / epi.c_rows_per_batch;
+      out = C + (size_t)cb * epi.c_batch_stride + (size_t)(row - cb * epi.c_rows_per_batch) * ldc;
+    } else {
+      out = C + (size_t)row * ldc;
+    }
+    if (epi.residual) res = epi.residual + (size_t)row * epi.ldr;
+    if (epi.gate) gate = epi.gate + (size_t)(row / epi.rows_per_batch) * epi.gate_stride;
+  }
+  auto chunk = [&](int c, const uint4* early) {
+    const int at = col0 + c * 32;
+    uint32_t v[32];
+    tmem_ld_32x32(tmem + c * 32, v);
+    uint4 b[4], r[4];
+    if (MODE != EPI_SWIGLU) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const bool in = row_ok && at + j * 8 < N;
+        b[j] = epi.bias && in ? *reinterpret_cast<const uint4*>(epi.bias + at + j * 8) : make_uint4(0u, 0u, 0u, 0u);
+        if (!early) r[j] = res && in ? *reinterpret_cast<const uint4*>(res + at + j * 8) : make_uint4(0u, 0u, 0u, 0u);
+      }
+    }
+    tmem_wait_ld(v);
+    if (!row_ok) return;
+    if (MODE == EPI_SWIGLU) {
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+        if (at + j * 16 < N) {
+          float x[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) x[e] = silu(__uint_as_float(v[j * 16 + e])) * __uint_as_float(v[j * 16 + 8 + e]);
+          *reinterpret_cast<uint4*>(out + (at >> 1) + j * 8) =
+              make_uint4(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]), pack_bf16(x[4], x[5]), pack_bf16(x[6], x[7]));
+        }
+      return;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (at + j * 8 >= N) break;
+      float x[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) x[e] = __uint_as_float(v[j * 8 + e]);
+      if (epi.bias) add_bf16x8(x, b[j]);
+      if (MODE == ACT_GELU_TANH) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[e] = gelu_tanh(x[e]);
+      } else if (MODE == ACT_XIELU) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[e] = xielu(x[e], epi.act_c0, epi.act_c1);
+      }
+      if (gate) {
+        const uint4 g = *reinterpret_cast<const uint4*>(gate + at + j * 8);
+        const float2 g0 = unpack_bf16(g.x), g1 = unpack_bf16(g.y), g2 = unpack_bf16(g.z), g3 = unpack_bf16(g.w);
+        x[0] *= g0.x; x[1] *= g0.y; x[2] *= g1.x; x[3] *= g1.y;
+        x[4] *= g2.x; x[5] *= g2.y; x[6] *= g3.x; x[7] *= g3.y;
+      }
+      if (res) add_bf16x8(x, early ? early[j] : r[j]);
+      *reinterpret_cast<uint4*>(out + at + j * 8) = make_uint4(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]), pack_bf16(x[4], x[5]), pack_bf16(x[6], x[7]));
+    }
+  };
+  if (MODE == ACT_NONE && epi.residual) {
+    uint4 early[CH][4];
+#pragma unroll
+    for (int c = 0; c < CH; ++c)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        early[c][j] = row_ok && col0 + c * 32 + j * 8 < N ? *reinterpret_cast<const uint4*>(res + col0 + c * 32 + j * 8) : make_uint4(0u, 0u, 0u, 0u);
+    ready();
+#pragma unroll
+    for (int c = 0; c < CH; ++c)
+      if (col0 + c * 32 < N) chunk(c, early[c]);
+    return;
+  }
+  ready();
+#pragma unroll 1
+  for (int c = 0; c < CH; ++c)
+    if (col0 + c * 32 < N) chunk(c, nullptr);
+}
+
 // Peer stores (fused collectives) go through a per-warp staging block in shared memory so that
 // the warp writes whole 128-byte row segments: a store from the row-owning thread would put 32
 // separate 16-byte writes on NVLink per instruction, which is request-bound far below link speed.
 //   write phase: lane = row, `ngroups` (4 or 8) 16-byte groups, group index XOR-swizzled by the row
 //   read  phase: 8 lanes per row, 4 rows per instruction -> 4 x 128 contiguous bytes per store
 constexpr int EPI_STAGE_BYTES = 32 * 128;          // per epilogue warp: 32 rows x 64 bf16 columns
-constexpr int EPI_STAGE_TOTAL = 8 * EPI_STAGE_BYTES;
 
 __device__ __forceinline__ void epilogue_store_staged(uint32_t stg, const uint4* __restrict__ o, int ngroups, int lane,
                                                       int row0, int M, int col0, int N, __nv_bfloat16* __restrict__ C,
@@ -498,7 +598,7 @@ struct PairArgs {
   PeerWait wt;      // arrivals this launch needs before it reads its A operands
 };
 
-template <int TN>
+template <int TN, int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_pair_kernel(const __grid_constant__ PairArgs args, int* status) {
   constexpr int P_TILE_N = TN;
@@ -577,7 +677,9 @@ gemm_bf16_pair_kernel(const __grid_constant__ PairArgs args, int* status) {
           const uint32_t fb = mapa_shared(smem_u32(&full_bar[stage]), 0);
           const uint32_t sa = smem_base + stage * P_STAGE_BYTES;
           tma_load_2d_pair(sa, tmA, fb, kb * BK, mb * 2 * BM + (int)rank * BM);
-          tma_load_2d_pair(sa + P_A_BYTES, tmB, fb, kb * BK, nb * P_TILE_N + (int)rank * (P_TILE_N / 2));
+          const int w_row = nb * P_TILE_N + (int)rank * (P_TILE_N / 2);
+          if (MODE == EPI_SWIGLU) tma_load_4d_pair(sa + P_A_BYTES, tmB, fb, kb * BK, 0, 0, w_row / 16);
+          else tma_load_2d_pair(sa + P_A_BYTES, tmB, fb, kb * BK, w_row);
           if (++stage == P_STAGES) { stage = 0; phase ^= 1; }
         }
       }
@@ -624,39 +726,48 @@ gemm_bf16_pair_kernel(const __grid_constant__ PairArgs args, int* status) {
       const GemmEpilogue& epi = args.p[prob].epi;
       __nv_bfloat16* C = args.p[prob].C;
       const int ldc = args.p[prob].ldc;
-      mbar_wait(smem_u32(&tfull_bar[acc]), acc_phase, &s_abort, status, ERR_WAIT_TMEM_FULL);
-      tc_fence_after_sync();
       const int row = mb * 2 * BM + (int)rank * BM + q * 32 + lane;
       const bool row_ok = row < args.p[prob].M;
-      const __nv_bfloat16* gate_row = nullptr;
-      if (epi.gate && row_ok) gate_row = epi.gate + (size_t)(row / epi.rows_per_batch) * epi.gate_stride;
-      if (epi.scatter_P > 1 || epi.scatter_rows > 0) {
-        // fused collectives: 64 columns at a time through the staging block
-        const uint32_t stg = smem_base + P_STAGES * P_STAGE_BYTES + (warp - 2) * EPI_STAGE_BYTES;
-        const int M = args.p[prob].M;
-#pragma unroll 1
-        for (int c = half * (P_TILE_N / 64); c < (half + 1) * (P_TILE_N / 64); c += 2) {
-          const int col0 = nb * P_TILE_N + c * 32;
-          if (col0 >= N) break;
-          const int nsub = min(2, (half + 1) * (P_TILE_N / 64) - c);
-          uint4 o[8];
-          for (int sidx = 0; sidx < nsub; ++sidx) {
-            uint32_t v[32];
-            tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + acc * 256 + (c + sidx) * 32, v);
-            tmem_wait_ld();
-            if (row_ok) epilogue_math32(v, row, col0 + sidx * 32, N, epi, gate_row, o + sidx * 4);
-          }
-          epilogue_store_staged(stg, o, nsub * 4, lane, mb * 2 * BM + (int)rank * BM + q * 32, M, col0, N, C, ldc, epi);
-        }
+      auto ready = [&]() {
+        mbar_wait(smem_u32(&tfull_bar[acc]), acc_phase, &s_abort, status, ERR_WAIT_TMEM_FULL);
+        tc_fence_after_sync();
+      };
+      if constexpr (MODE != EPI_ANY) {
+        constexpr int CH = P_TILE_N / 64;
+        drain_row<MODE, CH>(tmem_base + ((uint32_t)(q * 32) << 16) + acc * 256 + half * CH * 32, row, row_ok, nb * P_TILE_N + half * CH * 32, N, C, ldc, epi,
+                            ready);
       } else {
+        ready();
+        const __nv_bfloat16* gate_row = nullptr;
+        if (epi.gate && row_ok) gate_row = epi.gate + (size_t)(row / epi.rows_per_batch) * epi.gate_stride;
+        if (epi.scatter_P > 1 || epi.scatter_rows > 0) {
+          // fused collectives: 64 columns at a time through the staging block
+          const uint32_t stg = smem_base + P_STAGES * P_STAGE_BYTES + (warp - 2) * EPI_STAGE_BYTES;
+          const int M = args.p[prob].M;
 #pragma unroll 1
-        for (int c = half * (P_TILE_N / 64); c < (half + 1) * (P_TILE_N / 64); ++c) {
-          const int col0 = nb * P_TILE_N + c * 32;
-          if (col0 >= N) break;
-          uint32_t v[32];
-          tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + acc * 256 + c * 32, v);
-          tmem_wait_ld();
-          if (row_ok) epilogue_store32(v, row, col0, N, C, ldc, epi, gate_row);
+          for (int c = half * (P_TILE_N / 64); c < (half + 1) * (P_TILE_N / 64); c += 2) {
+            const int col0 = nb * P_TILE_N + c * 32;
+            if (col0 >= N) break;
+            const int nsub = min(2, (half + 1) * (P_TILE_N / 64) - c);
+            uint4 o[8];
+            for (int sidx = 0; sidx < nsub; ++sidx) {
+              uint32_t v[32];
+              tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + acc * 256 + (c + sidx) * 32, v);
+              tmem_wait_ld();
+              if (row_ok) epilogue_math32(v, row, col0 + sidx * 32, N, epi, gate_row, o + sidx * 4);
+            }
+            epilogue_store_staged(stg, o, nsub * 4, lane, mb * 2 * BM + (int)rank * BM + q * 32, M, col0, N, C, ldc, epi);
+          }
+        } else {
+#pragma unroll 1
+          for (int c = half * (P_TILE_N / 64); c < (half + 1) * (P_TILE_N / 64); ++c) {
+            const int col0 = nb * P_TILE_N + c * 32;
+            if (col0 >= N) break;
+            uint32_t v[32];
+            tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + acc * 256 + c * 32, v);
+            tmem_wait_ld();
+            if (row_ok) epilogue_store32(v, row, col0, N, C, ldc, epi, gate_row);
+          }
         }
       }
       tc_fence_before_sync();
@@ -690,7 +801,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ PairArgs args, int* status) {
 // 148 schedulable units instead of 74 the launcher can usually find a tile width whose tile count
 // fits whole waves, and the short problem's tiles run beside the long one's instead of in a launch
 // of their own that would last a full K loop for a handful of tiles.
-template <int BN>
+template <int BN, int MODE>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_multi_kernel(const __grid_constant__ PairArgs args, int* status) {
   using Cfg = GemmCfg<BN>;
@@ -763,7 +874,8 @@ gemm_bf16_multi_kernel(const __grid_constant__ PairArgs args, int* status) {
           const uint32_t sa = smem_base + stage * Cfg::STAGE_BYTES;
           mbar_expect_tx(fb, Cfg::STAGE_BYTES);
           tma_load_2d(sa, tmA, fb, kb * BK, mb * BM);
-          tma_load_2d(sa + Cfg::A_BYTES, tmB, fb, kb * BK, nb * BN);
+          if (MODE == EPI_SWIGLU) tma_load_4d(sa + Cfg::A_BYTES, tmB, fb, kb * BK, 0, 0, nb * BN / 16);
+          else tma_load_2d(sa + Cfg::A_BYTES, tmB, fb, kb * BK, nb * BN);
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
       }
@@ -810,37 +922,45 @@ gemm_bf16_multi_kernel(const __grid_constant__ PairArgs args, int* status) {
       __nv_bfloat16* C = args.p[prob].C;
       const int ldc = args.p[prob].ldc;
       const int M = args.p[prob].M;
-      mbar_wait(smem_u32(&tfull_bar[acc]), acc_phase, &s_abort, status, ERR_WAIT_TMEM_FULL);
-      tc_fence_after_sync();
       const int row = mb * BM + q * 32 + lane;
       const bool row_ok = row < M;
-      const __nv_bfloat16* gate_row = nullptr;
-      if (epi.gate && row_ok) gate_row = epi.gate + (size_t)(row / epi.rows_per_batch) * epi.gate_stride;
-      if (epi.scatter_P > 1 || epi.scatter_rows > 0) {
-        const uint32_t stg = smem_base + STAGES * Cfg::STAGE_BYTES + (warp - 2) * EPI_STAGE_BYTES;
-#pragma unroll 1
-        for (int c = half * CH_PER_WARP; c < (half + 1) * CH_PER_WARP; c += 2) {
-          const int col0 = nb * BN + c * 32;
-          if (col0 >= N) break;
-          const int nsub = min(2, (half + 1) * CH_PER_WARP - c);
-          uint4 o[8];
-          for (int sidx = 0; sidx < nsub; ++sidx) {
-            uint32_t v[32];
-            tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + acc * Cfg::ACC_STRIDE + (c + sidx) * 32, v);
-            tmem_wait_ld();
-            if (row_ok) epilogue_math32(v, row, col0 + sidx * 32, N, epi, gate_row, o + sidx * 4);
-          }
-          epilogue_store_staged(stg, o, nsub * 4, lane, mb * BM + q * 32, M, col0, N, C, ldc, epi);
-        }
+      auto ready = [&]() {
+        mbar_wait(smem_u32(&tfull_bar[acc]), acc_phase, &s_abort, status, ERR_WAIT_TMEM_FULL);
+        tc_fence_after_sync();
+      };
+      if constexpr (MODE != EPI_ANY) {
+        drain_row<MODE, CH_PER_WARP>(tmem_base + ((uint32_t)(q * 32) << 16) + acc * Cfg::ACC_STRIDE + half * CH_PER_WARP * 32, row, row_ok,
+                                     nb * BN + half * CH_PER_WARP * 32, N, C, ldc, epi, ready);
       } else {
+        ready();
+        const __nv_bfloat16* gate_row = nullptr;
+        if (epi.gate && row_ok) gate_row = epi.gate + (size_t)(row / epi.rows_per_batch) * epi.gate_stride;
+        if (epi.scatter_P > 1 || epi.scatter_rows > 0) {
+          const uint32_t stg = smem_base + STAGES * Cfg::STAGE_BYTES + (warp - 2) * EPI_STAGE_BYTES;
 #pragma unroll 1
-        for (int c = half * CH_PER_WARP; c < (half + 1) * CH_PER_WARP; ++c) {
-          const int col0 = nb * BN + c * 32;
-          if (col0 >= N) break;
-          uint32_t v[32];
-          tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + acc * Cfg::ACC_STRIDE + c * 32, v);
-          tmem_wait_ld();
-          if (row_ok) epilogue_store32(v, row, col0, N, C, ldc, epi, gate_row);
+          for (int c = half * CH_PER_WARP; c < (half + 1) * CH_PER_WARP; c += 2) {
+            const int col0 = nb * BN + c * 32;
+            if (col0 >= N) break;
+            const int nsub = min(2, (half + 1) * CH_PER_WARP - c);
+            uint4 o[8];
+            for (int sidx = 0; sidx < nsub; ++sidx) {
+              uint32_t v[32];
+              tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + acc * Cfg::ACC_STRIDE + (c + sidx) * 32, v);
+              tmem_wait_ld();
+              if (row_ok) epilogue_math32(v, row, col0 + sidx * 32, N, epi, gate_row, o + sidx * 4);
+            }
+            epilogue_store_staged(stg, o, nsub * 4, lane, mb * BM + q * 32, M, col0, N, C, ldc, epi);
+          }
+        } else {
+#pragma unroll 1
+          for (int c = half * CH_PER_WARP; c < (half + 1) * CH_PER_WARP; ++c) {
+            const int col0 = nb * BN + c * 32;
+            if (col0 >= N) break;
+            uint32_t v[32];
+            tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + acc * Cfg::ACC_STRIDE + c * 32, v);
+            tmem_wait_ld();
+            if (row_ok) epilogue_store32(v, row, col0, N, C, ldc, epi, gate_row);
+          }
         }
       }
       tc_fence_before_sync();
@@ -867,37 +987,67 @@ gemm_bf16_multi_kernel(const __grid_constant__ PairArgs args, int* status) {
 
 static int g_pair_mode = 1;   // 0: never unless forced, 1: automatic for large problems
 
+// W [N, K] of a gated layer, gate rows first: a box of `rows` rows brings 8 gate rows, their 8 lift rows, the next 8 gate rows and so on.
+static int swiglu_map(CUtensorMap* m, const void* W, int N, int K, int ldw, int rows) {
+  EncodeTiledFn enc = get_encode_tiled();
+  if (!enc) return RC_NO_DRIVER;
+  if (reinterpret_cast<uintptr_t>(W) & 15) return RC_BAD_ARG;
+  const cuuint64_t row = (cuuint64_t)ldw * 2;
+  cuuint64_t gdim[4] = {(cuuint64_t)K, 8, 2, (cuuint64_t)N / 16}, gstr[3] = {row, row * (N / 2), row * 8};
+  cuuint32_t box[4] = {BK, 8, 2, (cuuint32_t)rows / 16}, estr[4] = {1, 1, 1, 1};
+  return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(W), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? RC_OK : RC_TMAP;
+}
+
 // w_box_rows: rows of W one TMA box brings (half a tile for the CTA-pair kernel, a whole tile for the
 // one-CTA kernel)
 static int fill_pair_problem(PairProblem& pp, const void* A, int lda, const void* W, int ldw, __nv_bfloat16* C,
                              int ldc, int M, int N, int K, const GemmEpilogue& epi, int w_box_rows) {
   int rc = make_tmap_2d(&pp.tmA, A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)M, (uint64_t)K, (uint64_t)lda * 2, BM, BK);
   if (rc) return rc;
-  rc = make_tmap_2d(&pp.tmB, W, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)N, (uint64_t)K, (uint64_t)ldw * 2, w_box_rows, BK);
+  rc = epi.act == EPI_SWIGLU ? swiglu_map(&pp.tmB, W, N, K, ldw, w_box_rows)
+                             : make_tmap_2d(&pp.tmB, W, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)N, (uint64_t)K, (uint64_t)ldw * 2, w_box_rows, BK);
   if (rc) return rc;
   pp.C = C; pp.ldc = ldc; pp.M = M; pp.epi = epi;
   return RC_OK;
 }
 
-template <int TN>
+// the kernel of a launch's epilogues
+static int epilogue_mode(const PairArgs& args) {
+  const GemmEpilogue& e = args.p[0].epi;
+  for (int i = 0; i < args.n_problems; ++i) {
+    const GemmEpilogue& f = args.p[i].epi;
+    if (f.scatter_P > 1 || f.scatter_rows > 0 || f.act != e.act) return EPI_ANY;
+  }
+  return e.act == ACT_NONE || e.act == ACT_GELU_TANH || e.act == ACT_XIELU || e.act == EPI_SWIGLU ? e.act : EPI_ANY;
+}
+
+template <int TN, int MODE>
 static int launch_gemm_pair(const PairArgs& args, int* status, int max_pairs, cudaStream_t stream) {
   using Cfg = PairCfg<TN>;
   static unsigned long long prepared = 0;
-  if (int e = ensure_dynamic_smem((const void*)gemm_bf16_pair_kernel<TN>, Cfg::SMEM_BYTES, prepared)) return e;
+  if (int e = ensure_dynamic_smem((const void*)gemm_bf16_pair_kernel<TN, MODE>, Cfg::SMEM_BYTES, prepared)) return e;
   const int num_n = (args.N + TN - 1) / TN;
   int num_tiles = 0;
   for (int i = 0; i < args.n_problems; ++i) num_tiles += ((args.p[i].M + 2 * BM - 1) / (2 * BM)) * num_n;
   const int pairs = num_tiles < max_pairs ? num_tiles : max_pairs;
-  launch_with(!args.wt.counter && !args.sig.n, 1, gemm_bf16_pair_kernel<TN>, 2 * pairs, GEMM_THREADS, Cfg::SMEM_BYTES, stream, args, status);
+  launch_with(!args.wt.counter && !args.sig.n, 1, gemm_bf16_pair_kernel<TN, MODE>, 2 * pairs, GEMM_THREADS, Cfg::SMEM_BYTES, stream, args, status);
   return (int)cudaGetLastError();
 }
 
-static int launch_pair_tn(int tn, const PairArgs& args, int* status, int pairs, cudaStream_t s) {
-  switch (tn) {
-    case 256: return launch_gemm_pair<256>(args, status, pairs, s);
-    case 192: return launch_gemm_pair<192>(args, status, pairs, s);
-    default: return launch_gemm_pair<128>(args, status, pairs, s);
+#define OMNI_BY_MODE(launch, W)                                                     \
+  switch (epilogue_mode(args)) {                                                    \
+    case ACT_NONE: return launch<W, ACT_NONE>(args, status, units, s);              \
+    case ACT_GELU_TANH: return launch<W, ACT_GELU_TANH>(args, status, units, s);    \
+    case ACT_XIELU: return launch<W, ACT_XIELU>(args, status, units, s);            \
+    case EPI_SWIGLU: return launch<W, EPI_SWIGLU>(args, status, units, s);          \
+    default: return launch<W, EPI_ANY>(args, status, units, s);                     \
   }
+
+static int launch_pair_tn(int tn, const PairArgs& args, int* status, int units, cudaStream_t s) {
+  if (tn == 256) OMNI_BY_MODE(launch_gemm_pair, 256)
+  if (tn == 192) OMNI_BY_MODE(launch_gemm_pair, 192)
+  OMNI_BY_MODE(launch_gemm_pair, 128)
 }
 
 // how many CTA pairs can be resident at once (one CTA per SM, two SMs of one TPC per pair)
@@ -905,7 +1055,7 @@ static int max_resident_pairs() {
   static int cached = 0;
   if (cached) return cached;
   int n = 0;
-  if (cudaFuncSetAttribute(gemm_bf16_pair_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  if (cudaFuncSetAttribute(gemm_bf16_pair_kernel<256, EPI_ANY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            PairCfg<256>::SMEM_BYTES) == cudaSuccess) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(sm_count() & ~1);
@@ -916,7 +1066,7 @@ static int max_resident_pairs() {
     at.val.clusterDim.x = 2; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&n, gemm_bf16_pair_kernel<256>, &cfg) != cudaSuccess) n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, gemm_bf16_pair_kernel<256, EPI_ANY>, &cfg) != cudaSuccess) n = 0;
   }
   (void)cudaGetLastError();
   if (n <= 0 || n > sm_count() / 2) n = sm_count() / 2;
@@ -965,26 +1115,25 @@ static int launch_gemm(const CUtensorMap& tmA, const void* W, __nv_bfloat16* C, 
 }
 
 
-template <int BN>
+template <int BN, int MODE>
 static int launch_gemm_multi(const PairArgs& args, int* status, int max_ctas, cudaStream_t stream) {
   using Cfg = GemmCfg<BN>;
   static unsigned long long prepared = 0;
-  if (int e = ensure_dynamic_smem((const void*)gemm_bf16_multi_kernel<BN>, Cfg::SMEM_BYTES, prepared)) return e;
+  if (int e = ensure_dynamic_smem((const void*)gemm_bf16_multi_kernel<BN, MODE>, Cfg::SMEM_BYTES, prepared)) return e;
   const int num_n = (args.N + BN - 1) / BN;
   int num_tiles = 0;
   for (int i = 0; i < args.n_problems; ++i) num_tiles += ((args.p[i].M + BM - 1) / BM) * num_n;
   const int grid = num_tiles < max_ctas ? num_tiles : max_ctas;
-  launch_with(!args.wt.counter && !args.sig.n, 1, gemm_bf16_multi_kernel<BN>, grid, GEMM_THREADS, Cfg::SMEM_BYTES, stream, args, status);
+  launch_with(!args.wt.counter && !args.sig.n, 1, gemm_bf16_multi_kernel<BN, MODE>, grid, GEMM_THREADS, Cfg::SMEM_BYTES, stream, args, status);
   return (int)cudaGetLastError();
 }
 
-static int launch_multi_bn(int bn, const PairArgs& args, int* status, int ctas, cudaStream_t s) {
-  switch (bn) {
-    case 256: return launch_gemm_multi<256>(args, status, ctas, s);
-    case 192: return launch_gemm_multi<192>(args, status, ctas, s);
-    default: return launch_gemm_multi<128>(args, status, ctas, s);
-  }
+static int launch_multi_bn(int bn, const PairArgs& args, int* status, int units, cudaStream_t s) {
+  if (bn == 256) OMNI_BY_MODE(launch_gemm_multi, 256)
+  if (bn == 192) OMNI_BY_MODE(launch_gemm_multi, 192)
+  OMNI_BY_MODE(launch_gemm_multi, 128)
 }
+#undef OMNI_BY_MODE
 
 // Which kernel and tile width finish a list of (one or two) problems soonest.  A wave of tiles costs
 // time in proportion to the tile width (K and the 128 rows per SM are the same for every choice);
@@ -1054,7 +1203,7 @@ extern "C" int omni_gemm_bf16_coef(const void* A, int lda, const void* W, int ld
   if (M <= 0 || N <= 0 || K <= 0) return sync ? RC_BAD_ARG : RC_OK;
   if ((K & 7) || (N & 7) || (lda & 7) || (ldw & 7) || (ldc & 7) || (ldr & 7) || (gate_stride & 7))
     return RC_BAD_ARG;
-  if (gate && rows_per_batch <= 0) return RC_BAD_ARG;
+  if ((gate && rows_per_batch <= 0) || act == EPI_SWIGLU) return RC_BAD_ARG;
   GemmEpilogue epi;
   epi.bias = static_cast<const __nv_bfloat16*>(bias);
   epi.residual = static_cast<const __nv_bfloat16*>(residual);
@@ -1103,19 +1252,19 @@ extern "C" int omni_gemm_bf16_coef(const void* A, int lda, const void* W, int ld
   // problem with at least one full wave of 256 x 256 tiles
   TilePlan plan = {false, 0};
   if (force_bn == 0) plan = plan_tiles(&M, 1, N, ctas, g_pair_mode == 1 ? max_resident_pairs() : 0, g_pair_mode == 1);
-  if (force_bn >= 384 || (force_bn == 0 && plan.pair)) {
+  if (force_bn >= 384 || force_bn == 0) {
     const int pairs = max_resident_pairs();
+    const bool pair = force_bn || plan.pair;
     const int tn = force_bn == 576 ? 256 : (force_bn == 448 ? 192 : (force_bn == 384 ? 128 :
                    (force_bn == 512 ? pick_pair_tn(M, N, pairs) : plan.bn)));
     PairArgs args = {};
     args.n_problems = 1; args.N = N; args.K = K;
     unpack_sync(sync, args.sig, args.wt);
-    rc = fill_pair_problem(args.p[0], A, lda, W, ldw, c, ldc, M, N, K, epi, tn / 2);
+    rc = fill_pair_problem(args.p[0], A, lda, W, ldw, c, ldc, M, N, K, epi, pair ? tn / 2 : tn);
     if (rc) return rc;
-    return launch_pair_tn(tn, args, status, pairs, s);
+    return pair ? launch_pair_tn(tn, args, status, pairs, s) : launch_multi_bn(tn, args, status, ctas, s);
   }
-  const int bn = force_bn ? force_bn : plan.bn;
-  switch (bn) {
+  switch (force_bn) {
     case 256: return launch_gemm<256>(tmA, W, c, ldc, M, N, K, ldw, epi, status, ctas, s, 1, nullptr, nullptr, sync);
     case 192: return launch_gemm<192>(tmA, W, c, ldc, M, N, K, ldw, epi, status, ctas, s, 1, nullptr, nullptr, sync);
     case 128: return launch_gemm<128>(tmA, W, c, ldc, M, N, K, ldw, epi, status, ctas, s, 1, nullptr, nullptr, sync);
@@ -1211,7 +1360,7 @@ struct OmniGemmDesc {
 
 static int desc_epilogue(const OmniGemmDesc& d, omni::GemmEpilogue& epi) {
   if ((d.lda & 7) || (d.ldw & 7) || (d.ldc & 7) || (d.ldr & 7) || (d.gate_stride & 7)) return omni::RC_BAD_ARG;
-  if (d.act == omni::ACT_XIELU) return omni::RC_BAD_ARG;      // has numbers of its own
+  if (d.act == omni::ACT_XIELU || d.act == omni::EPI_SWIGLU) return omni::RC_BAD_ARG;      // has numbers of its own; has an entry of its own
   if (d.gate && d.rows_per_batch <= 0) return omni::RC_BAD_ARG;
   if (d.c_rows_per_batch > 0 && (d.c_batch_stride & 7)) return omni::RC_BAD_ARG;
   epi = omni::GemmEpilogue{};
@@ -1274,6 +1423,28 @@ extern "C" int omni_gemm_bf16_dual_sync(const OmniGemmDesc* d0, const OmniGemmDe
 extern "C" int omni_gemm_bf16_dual(const OmniGemmDesc* d0, const OmniGemmDesc* d1, int N, int K, int force_pair,
                                    int* status, void* stream) {
   return omni_gemm_bf16_dual_sync(d0, d1, N, K, force_pair, nullptr, status, stream);
+}
+
+// C[M, F] = silu(A gate^T) * (A lift^T), W [2 F, K] with the F gate rows first; F and K multiples of 8.  -5: these rows are faster as two launches (17 to 128
+// rows that gemm_skinny_kernel takes).
+extern "C" int omni_gemm_bf16_swiglu(const void* A, int lda, const void* W, int ldw, void* C, int ldc, int M, int F, int K, int* status, void* stream) {
+  using namespace omni;
+  if (M <= 0 || F <= 0 || K <= 0) return RC_OK;
+  if ((K & 7) || (F & 7) || (lda & 7) || (ldw & 7) || (ldc & 7)) return RC_BAD_ARG;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  GemmEpilogue epi = {};
+  epi.rows_per_batch = 1;
+  epi.act = EPI_SWIGLU;
+  const FewRows few = few_rows(M, 2 * F, K);
+  if (few == FewRows::skinny) return -5;
+  if (few == FewRows::rows) return launch_rows(A, lda, W, ldw, static_cast<__nv_bfloat16*>(C), ldc, M, 2 * F, K, epi, s);
+  const int N = 2 * F, ctas = sm_count(), pairs = max_resident_pairs();
+  const TilePlan plan = plan_tiles(&M, 1, N, ctas, g_pair_mode == 1 ? pairs : 0, g_pair_mode == 1);
+  PairArgs args = {};
+  args.n_problems = 1; args.N = N; args.K = K;
+  unpack_sync(nullptr, args.sig, args.wt);
+  if (int rc = fill_pair_problem(args.p[0], A, lda, W, ldw, static_cast<__nv_bfloat16*>(C), ldc, M, N, K, epi, plan.pair ? plan.bn / 2 : plan.bn)) return rc;
+  return plan.pair ? launch_pair_tn(plan.bn, args, status, pairs, s) : launch_multi_bn(plan.bn, args, status, ctas, s);
 }
 
 // 0: the CTA-pair kernel runs only when forced (force_bn = 512); 1: automatic for large problems.

@@ -49,6 +49,13 @@ class FusedLinear(nn.Module):
             y = gemm.linear(x, self.weight, self.bias, act=act, residual=residual, gate=gate, out=out, **kw)
         return y
 
+    def swiglu(self, x):
+        """silu(first half) * second half of the layer's outputs."""
+        if self.fp8 is None and not self.lora and self.bias is None:
+            return gemm.linear_swiglu(x, self.weight)
+        from ...ops import fused
+        return fused.silu_mul(self(x))
+
     def extra_repr(self):
         return f"in={self.in_features}, out={self.out_features}, bias={self.bias is not None}"
 

@@ -415,7 +415,7 @@ class QwenDecoderModel(nn.Module):
                 if shared is not None:
                     x.add_(shared.to(x.dtype))
             else:
-                h = fused.silu_mul(layer.gate_up(xn))
+                h = layer.gate_up.swiglu(xn)
                 if self.tp_reduce is not None:
                     self.tp_reduce.linear(layer.down, h, residual=x, out=x, capacity=tp_cap)
                 else:

@@ -144,6 +144,26 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None, a
     return None if to_peers else out
 
 
+def linear_swiglu(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+    """silu(x @ gate.T) * (x @ lift.T) with w = [gate | lift] rows: on a GPU in one launch (the product of both never reaches memory, and neither half is
+    rounded before they meet), for rows that the few-row kernels split over clusters in two."""
+    from .fused import silu_mul
+    F_, K = w.shape[0] // 2, w.shape[1]
+    if x.is_cuda and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and w.shape[0] % 16 == 0 and K % 8 == 0 and x.numel() and w.stride(1) == 1 \
+            and w.stride(0) % 8 == 0:
+        x2 = x.reshape(-1, K)
+        if x2.stride(1) != 1 or x2.stride(0) % 8:
+            x2 = x2.contiguous()
+        out = torch.empty(*x.shape[:-1], F_, dtype=x.dtype, device=x.device)
+        rc = nv.lib("gemm_sm100").omni_gemm_bf16_swiglu(nv.ptr(x2), ctypes.c_int(x2.stride(0)), nv.ptr(w), ctypes.c_int(w.stride(0)), nv.ptr(out),
+                                                        ctypes.c_int(F_), ctypes.c_int(x2.shape[0]), ctypes.c_int(F_), ctypes.c_int(K),
+                                                        nv.ptr(nv.status_word(x.device)), nv.stream_ptr())
+        if rc != -5:
+            nv.check_rc(rc, "omni_gemm_bf16_swiglu")
+            return out
+    return silu_mul(linear(x, w))
+
+
 def _linear_f32(x, w, bias, out, act=None, coef=(0.0, 0.0)):
     """Exact mode: true fp32 products on the CUDA cores (csrc/gemm_f32.cu); ``act(x @ w.T (+ bias))`` only."""
     K, N = x.shape[-1], w.shape[0]
