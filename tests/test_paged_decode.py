@@ -77,3 +77,29 @@ def test_pages_of_other_sizes_keep_fp32_weights(bs, H, Hkv):
     # the result's rounding to bf16 alone; fp32 scores, weights and sums are 2^-14 and below
     bound = ref.abs() * 2.0 ** -8 + torch.einsum("nhk,nkhd->nhd", w, vv.abs()) * 2.0 ** -14
     assert ((out.double() - ref).abs() <= bound).all()
+
+
+# shares of very different and of like lengths (as many as make one round of warps), sequences without keys, more sequences than add up their lengths, a block each
+@pytest.mark.parametrize("H,Hkv,lens", [(32, 4, [4000, 3, 0, 70] + [17] * 40 + [900]), (8, 1, [2500] + [1] * 200), (16, 8, [0, 0, 5]), (32, 8, [33] * 700),
+                                        (12, 3, [16 * i for i in range(50)]), (16, 1, [5000, 0, 40]), (8, 8, [1] * 450), (4, 1, [7000])])
+def test_shares_by_the_lengths(H, Hkv, lens):
+    D, bs, n = 128, 16, len(lens)
+    g = torch.Generator(device="cuda").manual_seed(n)
+    per = [-(-l // bs) for l in lens]
+    k, v = (torch.randn(max(1, sum(per)), bs, Hkv, D, generator=g, device="cuda").bfloat16() for _ in range(2))
+    order = torch.randperm(sum(per), generator=torch.Generator().manual_seed(n)).tolist()
+    tables, at = torch.zeros(n, max(per) + 3, dtype=torch.int32), 0
+    for s in range(n):
+        tables[s, :per[s]] = torch.tensor(order[at:at + per[s]], dtype=torch.int32)
+        at += per[s]
+    q = torch.randn(n, H, D, generator=g, device="cuda").bfloat16()
+    out = KC.paged_decode(q, k, v, tables.cuda(), torch.tensor(lens, dtype=torch.int32, device="cuda"), out=torch.full_like(q, 9.0), impl="stream")
+    for s, l in enumerate(lens):
+        if l == 0:
+            assert (out[s] == 0).all()
+            continue
+        kk, vv = (t[order[sum(per[:s]):sum(per[:s + 1])]].reshape(-1, Hkv, D)[:l].double().repeat_interleave(H // Hkv, 1) for t in (k, v))
+        w = torch.softmax(torch.einsum("hd,khd->hk", q[s].double(), kk) * D ** -0.5, -1)
+        ref = torch.einsum("hk,khd->hd", w, vv)
+        bound = torch.einsum("hk,khd->hd", w, vv.abs()) * 2.0 ** -8 + ref.abs() * 2.0 ** -8 + 1e-5          # as above
+        assert ((out[s].double() - ref).abs() <= bound).all(), (s, l)

@@ -34,7 +34,8 @@ struct DecodeAttn {
   int bt_stride, block_size;
   const int* lens;
   int max_keys;                      // no sequence has more
-  int H, Hkv, splits, subs;          // shares of the keys: blocks, and warps of a block
+  int n, H, Hkv, splits, subs;       // shares of the keys: blocks, and warps of a block
+  int room;                          // warps that a round leaves for whole shares, see plan_shares; 0: a sequence's shares are its keys / splits
   float scale_log2;
   float *part_o, *part_ml;
   __nv_bfloat16* out;
@@ -45,31 +46,41 @@ struct DecodeAttn {
 };
 
 // Row of q and out; -1 where there is none, which the status word tells the host.
+template <bool ROWS>
 __device__ __forceinline__ long da_row(const DecodeAttn& p, int seq) {
-  if (!p.rows) return seq;
+  if (!ROWS) return seq;
   long long r = p.rows[seq];
   if (r < 0) r += p.n_rows;
   if (r >= 0 && r < p.n_rows) return (long)r;
-  if (threadIdx.x == 0) atomicCAS(p.status, 0, ERR_BOUNDS);
+  atomicCAS(p.status, 0, ERR_BOUNDS);
   return -1;
 }
 
 // UP: 9 .. 16 heads per group, the second half of the MMA's 16 rows is live.
-template <bool UP>
+template <bool UP, bool ROWS>
 __global__ void __launch_bounds__(32 * DA_WARPS, UP ? 2 : 3)
 paged_decode_kernel(const __grid_constant__ DecodeAttn p) {
   pdl_begin();
   constexpr int NH = UP ? 2 : 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, j = lane & 3;
-  const int seq = blockIdx.y, split = blockIdx.x;
+  const int seq = blockIdx.x, split = blockIdx.y;
   const int per_block = min(DA_WARPS, p.Hkv), sub = warp / per_block;
   const int hk = blockIdx.z * DA_WARPS + warp % per_block;
   if (sub >= p.subs || hk >= p.Hkv) return;
   const int G = p.H / p.Hkv, h0 = hk * G, parts = p.splits * p.subs;
-  const long q_row = da_row(p, seq);
+  const long q_row = da_row<ROWS>(p, seq);
   if (q_row < 0) return;
   const int len = min(p.lens[seq], p.max_keys);
-  const int tiles = (len + DA_KEYS - 1) / DA_KEYS, per = (tiles + p.splits - 1) / p.splits;
+  const int tiles = (len + DA_KEYS - 1) / DA_KEYS;
+  int per = (tiles + p.splits - 1) / p.splits;
+  if (p.room) {
+    // Shares of at least a warp's part of all keys: those in use are one round of warps then.  Blocks past a sequence's shares leave; they are the
+    // grid's last ones.
+    int all = 0;
+    for (int i = lane; i < p.n; i += 32) all += (min(p.lens[i], p.max_keys) + DA_KEYS - 1) / DA_KEYS;
+    all = __reduce_add_sync(0xffffffffu, all) * p.Hkv;
+    if (4 * all > 5 * p.room) per = max(per, (all + p.room - 1) / p.room * p.subs);
+  }
   const int t1 = min(tiles, (split + 1) * per);
   if (split * per + sub >= t1) {      // no keys (a table wider than the sequence): weight zero, and no sum for the merge to read
     if (parts > 1 && lane < G) {
@@ -233,15 +244,13 @@ paged_decode_kernel(const __grid_constant__ DecodeAttn p) {
 
 // out[seq, h] = sum_s 2^(m_s - m*) O_s / sum_s 2^(m_s - m*) l_s over a row's shares (at most 64): one block per row, its warps take
 // every fourth share, four channels per lane.
+template <bool ROWS>
 __global__ void __launch_bounds__(128)
 paged_decode_merge_kernel(const __grid_constant__ DecodeAttn p, int parts) {
   pdl_begin();
   __shared__ float4 part[4][32];
   const float *part_o = p.part_o, *part_ml = p.part_ml;
-  const int H = p.H;
   const long r = blockIdx.x;
-  const long row = da_row(p, (int)(r / H));
-  if (row < 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float2* ml = reinterpret_cast<const float2*>(part_ml) + r * parts;
   const float4* po = reinterpret_cast<const float4*>(part_o) + r * parts * (DA_D / 4) + lane;
@@ -281,18 +290,24 @@ paged_decode_merge_kernel(const __grid_constant__ DecodeAttn p, int parts) {
     acc.x += x.x; acc.y += x.y; acc.z += x.z; acc.w += x.w;
   }
   const float f = den > 0.f ? 1.0f / den : 0.f;
-  const long seq = r / H;
+  const int seq = (int)blockIdx.x / p.H;
+  const long row = da_row<ROWS>(p, seq);
+  if (row < 0) return;                                         // no share was written, and nothing of it is
   uint2 w;
   w.x = pack_bf16(acc.x * f, acc.y * f);
   w.y = pack_bf16(acc.z * f, acc.w * f);
-  *reinterpret_cast<uint2*>(p.out + row * p.o_rs + (r - seq * H) * DA_D + lane * 4) = w;
+  *reinterpret_cast<uint2*>(p.out + row * p.o_rs + ((int)blockIdx.x - seq * p.H) * DA_D + lane * 4) = w;
 }
 
-constexpr int DA_MAX_PARTS = 64;
+constexpr int DA_MAX_PARTS = 64, DA_EVEN = 128;          // every warp adds up that many lengths at most
 
-// Shares of a sequence's keys: about `target` warps in all, at least two tiles of 16 keys each.  Twelve warps fit an SM; two rounds of them
-// even out lengths (8 sequences of 4096 keys, 8 KV heads: 20 warps per SM 1.05 and 18 1.12 times as long as 24).  Blocks of fewer KV
-// heads hold shares of one sequence, whose sums are many and small: 20, since 24 took 1.11 times the tensor-core kernel's time for 72
+// Shares of a sequence's keys: room for about `target` warps in all, at least two tiles of 16 keys each.  Twelve warps fit an SM.  Two rounds of them let
+// long sequences among short ones have many shares (8 sequences of 4096 keys, 8 KV heads: 20 warps per SM 1.05 and 18 1.12 times as long as 24), but of
+// sequences that are alike one round is faster: fewer starts, fewer sums.  The kernel, which knows the lengths, uses as many shares as make one round
+// (room).  us, as many as two rounds in brackets: 32 heads, 8 KV heads, 12 sequences of
+// about 2600 keys 30.5 (34.6), 48 of them 93 (103), 16 of 60 to 4000 keys 29.4 (32.7); 4 KV heads, 24 of about 440 12.5 (14.8).  Up to a quarter more keys than
+// a round's warps have tiles they keep a tile each: 32 of 90 keys, 8 KV heads, 9.4, in shares of two 11.1.
+// Blocks of fewer KV heads hold shares of one sequence, whose sums are many and small: 20, since 24 took 1.11 times the tensor-core kernel's time for 72
 // sequences of 1024 keys in tables of 4096 and 1 KV head, and 20 never more than 1.01 of it.  A single sequence has at most
 // 64 shares: 131072 keys of 4 KV heads take 148 us, the tensor-core kernel 246 (the copy rate would be 41; more shares would reach more SMs).
 static void plan_shares(int n, int Hkv, int max_keys, int& splits, int& subs) {
@@ -326,7 +341,7 @@ extern "C" int omni_paged_decode_attn(const void* q, long q_rs, const void* k, c
                                       int block_size, const int* lens, int n, int H, int Hkv, int max_keys, float scale, float* part_o,
                                       float* part_ml, void* out, long o_rs, const long long* rows, int n_rows, int* status, void* stream) {
   if (n <= 0) return RC_OK;
-  if (Hkv <= 0 || H % Hkv || H / Hkv > 16 || block_size < 8 || (block_size & 7) || max_keys < 1 || n > 65535 || (q_rs & 7) || (o_rs & 7))
+  if (Hkv <= 0 || H % Hkv || H / Hkv > 16 || block_size < 8 || (block_size & 7) || max_keys < 1 || (q_rs & 7) || (o_rs & 7))
     return RC_BAD_ARG;
   if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(out)) & 15)
     return RC_BAD_ARG;
@@ -336,15 +351,22 @@ extern "C" int omni_paged_decode_attn(const void* q, long q_rs, const void* k, c
   if (parts > 1 && (!part_o || !part_ml)) return RC_BAD_ARG;
   p.q = (const __nv_bfloat16*)q; p.k = (const __nv_bfloat16*)k; p.v = (const __nv_bfloat16*)v;
   p.q_rs = q_rs; p.block_tables = block_tables; p.bt_stride = bt_stride; p.block_size = block_size; p.lens = lens; p.max_keys = max_keys;
+  p.n = n;
+  // rounding up gives every sequence at most one share more; sequences and heads that fill half of a round by themselves get two, and so on
+  const int round = (H / Hkv > 8 ? 8 : 12) * sm_count(), rest = n * p.subs * Hkv;
+  p.room = parts > 1 && n <= DA_EVEN && n * Hkv >= 32 ? (2 * rest + round - 1) / round * round - rest : 0;
   p.H = H; p.Hkv = Hkv; p.scale_log2 = scale * 1.4426950408889634f;
   p.part_o = part_o; p.part_ml = part_ml; p.out = (__nv_bfloat16*)out; p.o_rs = o_rs;
   p.rows = rows; p.n_rows = n_rows; p.status = status;
-  const dim3 grid((unsigned)p.splits, (unsigned)n, (unsigned)((Hkv + DA_WARPS - 1) / DA_WARPS));
+  const dim3 grid((unsigned)n, (unsigned)p.splits, (unsigned)((Hkv + DA_WARPS - 1) / DA_WARPS));
   cudaStream_t st = (cudaStream_t)stream;
-  if (H / Hkv > 8) launch_overlapped(paged_decode_kernel<true>, grid, 32 * DA_WARPS, 0, st, p);
-  else launch_overlapped(paged_decode_kernel<false>, grid, 32 * DA_WARPS, 0, st, p);
+  const bool up = H / Hkv > 8;
+  // One round of blocks has to lie evenly on the SMs, which it does not where it is dealt out around the last blocks of the kernel before: overlapped, a step of
+  // 48 sequences of about 2600 keys (4096-wide dense decoder, four layers) took 1347 us instead of 903, with two rounds 1069.
+  launch_with(p.room == 0, 1, rows ? (up ? paged_decode_kernel<true, true> : paged_decode_kernel<false, true>)
+                         : (up ? paged_decode_kernel<true, false> : paged_decode_kernel<false, false>), grid, 32 * DA_WARPS, 0, st, p);
   if (parts == 1) return (int)cudaGetLastError();
   if (cudaError_t e = cudaGetLastError()) return (int)e;
-  launch_overlapped(paged_decode_merge_kernel, (unsigned)n * H, 128, 0, st, p, parts);
+  launch_overlapped(rows ? paged_decode_merge_kernel<true> : paged_decode_merge_kernel<false>, (unsigned)n * H, 128, 0, st, p, parts);
   return (int)cudaGetLastError();
 }
