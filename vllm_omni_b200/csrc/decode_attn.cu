@@ -246,10 +246,9 @@ paged_decode_kernel(const __grid_constant__ DecodeAttn p) {
 // every fourth share, four channels per lane.
 template <bool ROWS>
 __global__ void __launch_bounds__(128)
-paged_decode_merge_kernel(const __grid_constant__ DecodeAttn p, int parts) {
+paged_decode_merge_kernel(const float* part_o, const float* part_ml, int parts, int H, __nv_bfloat16* __restrict__ out, long o_rs, const long long* rows, int n_rows) {
   pdl_begin();
   __shared__ float4 part[4][32];
-  const float *part_o = p.part_o, *part_ml = p.part_ml;
   const long r = blockIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float2* ml = reinterpret_cast<const float2*>(part_ml) + r * parts;
@@ -290,13 +289,17 @@ paged_decode_merge_kernel(const __grid_constant__ DecodeAttn p, int parts) {
     acc.x += x.x; acc.y += x.y; acc.z += x.z; acc.w += x.w;
   }
   const float f = den > 0.f ? 1.0f / den : 0.f;
-  const int seq = (int)blockIdx.x / p.H;
-  const long row = da_row<ROWS>(p, seq);
-  if (row < 0) return;                                         // no share was written, and nothing of it is
+  const int seq = (int)blockIdx.x / H;
+  long row = seq;
+  if (ROWS) {
+    row = rows[seq];
+    if (row < 0) row += n_rows;
+    if (row < 0 || row >= n_rows) return;
+  }
   uint2 w;
   w.x = pack_bf16(acc.x * f, acc.y * f);
   w.y = pack_bf16(acc.z * f, acc.w * f);
-  *reinterpret_cast<uint2*>(p.out + row * p.o_rs + ((int)blockIdx.x - seq * p.H) * DA_D + lane * 4) = w;
+  *reinterpret_cast<uint2*>(out + row * o_rs + ((int)blockIdx.x - seq * H) * DA_D + lane * 4) = w;
 }
 
 constexpr int DA_MAX_PARTS = 64, DA_EVEN = 128;          // every warp adds up that many lengths at most
@@ -367,6 +370,6 @@ extern "C" int omni_paged_decode_attn(const void* q, long q_rs, const void* k, c
                          : (up ? paged_decode_kernel<true, false> : paged_decode_kernel<false, false>), grid, 32 * DA_WARPS, 0, st, p);
   if (parts == 1) return (int)cudaGetLastError();
   if (cudaError_t e = cudaGetLastError()) return (int)e;
-  launch_overlapped(rows ? paged_decode_merge_kernel<true> : paged_decode_merge_kernel<false>, (unsigned)n * H, 128, 0, st, p, parts);
+  launch_overlapped(rows ? paged_decode_merge_kernel<true> : paged_decode_merge_kernel<false>, (unsigned)n * H, 128, 0, st, part_o, part_ml, parts, H, (__nv_bfloat16*)out, o_rs, rows, n_rows);
   return (int)cudaGetLastError();
 }
