@@ -85,3 +85,15 @@ def test_edges_of_the_rules(rows, n, k):
     y = gemm.linear(x, w, b, residual=res)
     _check(y, x.double() @ w.double().T + b.double() + res.double(), x.double().abs() @ w.double().abs().T)
     nv.check_status()
+
+
+@pytest.mark.parametrize("rows", [17, 23, 24, 25])
+@pytest.mark.parametrize("per_sm,k", [(0.5, 9216), (1, 136), (1.5, 4096), (2, 72), (2.5, 512), (3.5, 264), (4.5, 1024), (5.5, 64)])
+def test_splits_of_17_to_24_rows(rows, per_sm, k):
+    """Every split of the three-tile form, and the rows and widths past it."""
+    n = int(per_sm * torch.cuda.get_device_properties(0).multi_processor_count) * 16 - 8
+    g = torch.Generator(device="cuda").manual_seed(rows + k)
+    x, w, r = (torch.randn(*s, generator=g, device="cuda").bfloat16() for s in ((rows, k), (n, k), (rows, n)))
+    y = gemm.linear(x, w, residual=r)
+    _check(y, x.double() @ w.double().T + r.double(), x.double().abs() @ w.double().abs().T)
+    nv.check_status()

@@ -2,10 +2,10 @@
 // is that of streaming W from HBM plus a launch's fixed chain of latencies, and a tile per 128..256 columns leaves most SMs
 // idle (16 tiles of 128 columns for a 2048-wide layer).
 //
-// gemm_rows_kernel     M <= 16: 16 columns of C per block, the contraction dealt out to its warps.  W goes from HBM straight into
+// gemm_rows_kernel     M <= 24: 16 columns of C per block, the contraction dealt out to its warps.  W goes from HBM straight into
 //                      MMA fragments: no shared-memory ring, no barriers and no tensor memory to set up, which is what a
 //                      launch of a few microseconds is made of.
-// gemm_skinny_kernel   17 <= M <= 128: the operands change places, 128 rows of W are the M side of a tcgen05 MMA and MT = 32 / 64 /
+// gemm_skinny_kernel   M <= 128: the operands change places, 128 rows of W are the M side of a tcgen05 MMA and MT = 32 / 64 /
 //                      128 rows of A its N side; the contraction is split over the S = 1, 2, 4 or 8 CTAs of a cluster, each
 //                      streaming its own K range through a TMA ring.  Partial sums (fp32) meet over distributed shared
 //                      memory in rank order: the result does not depend on timing.
@@ -78,7 +78,7 @@ __device__ __forceinline__ void skinny_finish(float (&x)[B], int m, int step, in
   }
 }
 
-// ---------------------------------------------------------------------------------------------------- at most 16 rows
+// ---------------------------------------------------------------------------------------------------- at most 24 rows
 // NT * 8 rows of A; 16 resident warps x U chunks x 1 KB = up to 128 KB of W in flight per SM.
 // GATED: W holds N / 2 gate rows and then their lift rows; a block makes 8 columns of C, silu(gate) * lift, from 8 rows of each.
 template <int NT, int NW, int U, int BLOCKS, bool GATED>
@@ -146,6 +146,9 @@ gemm_rows_kernel(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W, int ld
 //   more, 9 rows and up: four blocks of 4 warps where their last round is at least half full (24576 x 4096 46.1 with two blocks
 //                of 8, 42.1 with four of 4; 9216 x 2048 10.2 and 9.2), not where it is emptier (12288 x 4096 25.3 and 27.8)
 //   else         two blocks of 8 (8 rows, 32768 x 4096: 46.2; four of 4 48.0, three of 8 47.9; the copy rate would be 40.4)
+// 17 to 24 rows, whose products leave registers for fewer loads (17 and 24 rows; gemm_skinny_kernel in brackets): up to one tile per SM 16 warps
+// (2048 x 6144 8.1 / 8.7 (10.0)), up to two two blocks of 8 with twice the loads (4096 x 4096 9.1 / 9.8 (10.6)), up to three those with half
+// (6144 x 4096 12.2 / 13.3 (14.3)), more four of 4 (9216 x 2048 9.4 / 10.2 (11.6)), with half the loads past a round of them (12288 x 2048 12.0 / 12.8 (14.9)).
 template <int NT, bool GATED>
 static void launch_rows(int tiles, const __nv_bfloat16* A, int lda, const __nv_bfloat16* W, int ldw, __nv_bfloat16* C, int ldc, int M,
                         int N, int K, const GemmEpilogue& epi, cudaStream_t stream) {
@@ -154,7 +157,13 @@ static void launch_rows(int tiles, const __nv_bfloat16* A, int lda, const __nv_b
   const auto go = [&](auto kernel, int warps, int blocks) {
     launch_overlapped(kernel, tiles, 32 * warps, 0, stream, A, lda, W, ldw, C, ldc, M, N, K, epi, blocks * sms);
   };
-  if (tiles <= sms && K > 1024) go(gemm_rows_kernel<NT, 16, U, 1, GATED>, 16, 1);
+  if constexpr (NT == 3) {
+    if (tiles <= sms) go(gemm_rows_kernel<3, 16, 2, 1, GATED>, 16, 1);
+    else if (tiles <= 2 * sms) go(gemm_rows_kernel<3, 8, 4, 2, GATED>, 8, 2);
+    else if (tiles <= 3 * sms) go(gemm_rows_kernel<3, 8, 2, 2, GATED>, 8, 2);
+    else if (tiles <= 4 * sms) go(gemm_rows_kernel<3, 4, 4, 4, GATED>, 4, 4);
+    else go(gemm_rows_kernel<3, 4, 2, 4, GATED>, 4, 4);
+  } else if (tiles <= sms && K > 1024) go(gemm_rows_kernel<NT, 16, U, 1, GATED>, 16, 1);
   else if (tiles > 2 * sms && tiles <= 3 * sms) go(gemm_rows_kernel<NT, 8, U / 2, 3, GATED>, 8, 3);
   else if (NT == 2 && tiles > 3 * sms && (last == 0 || last >= 2 * sms)) go(gemm_rows_kernel<NT, 4, U, 4, GATED>, 4, 4);
   else go(gemm_rows_kernel<NT, 8, U, 2, GATED>, 8, 2);
@@ -166,7 +175,8 @@ static int launch_rows(const void* A, int lda, const void* W, int ldw, __nv_bflo
   const auto a = static_cast<const __nv_bfloat16*>(A), w = static_cast<const __nv_bfloat16*>(W);
   const int tiles = (N + 15) / 16;
   const bool gated = epi.act == EPI_SWIGLU;
-  const auto go = M <= 8 ? (gated ? launch_rows<1, true> : launch_rows<1, false>) : (gated ? launch_rows<2, true> : launch_rows<2, false>);
+  const auto go = M <= 8 ? (gated ? launch_rows<1, true> : launch_rows<1, false>)
+                : M <= 16 ? (gated ? launch_rows<2, true> : launch_rows<2, false>) : (gated ? launch_rows<3, true> : launch_rows<3, false>);
   go(tiles, a, lda, w, ldw, C, ldc, M, N, K, epi, stream);
   return (int)cudaGetLastError();
 }
@@ -380,7 +390,9 @@ static int launch_skinny_mt(const CUtensorMap& tmW, const void* A, int lda, __nv
 //                    blocks per SM, or four of very long rows, that costs more than it saves.  us, general kernel in brackets: 13 rows 16384 x 4096 30.0
 //                    (37.3), 16 rows 16384 x 3584 28.3 (33.9), 16384 x 4096 31.5 (28.7), 13824 x 4096 24.4 (25.7), 12288 x 12288 1.05 times
 //                    as long, 8192 x 4096 18.1 (20.5).  Up to 8 rows the products are half as many and it pays at any length.
-//   17 to 32         up to as many tiles as SMs: 17 rows 10240 x 2048 12.5 (17.1), 12288 x 1024 8.0 (11.6), 32 rows 18432 x 2048 15.4 (16.7)
+//   17 to 24         gemm_rows_kernel up to 5 blocks per SM and contractions of 4096, or a block per SM and 9216: 17 rows 4096 x 12288 22.4 (20.6), 32768 x 2048
+//                    30.8 (29.6)
+//   17 to 32         else up to as many tiles as SMs: 17 rows 10240 x 2048 12.5 (17.1), 12288 x 1024 8.0 (11.6), 32 rows 18432 x 2048 15.4 (16.7)
 //   33 to 64         up to half as many; above, the general kernels stream W as fast and read A less often: 64 rows 9216 x 2048 12.7 (13.8),
 //                    10240 x 2048 14.4 (13.2)
 //   65 to 128        up to a third, and contractions long enough for the split: exchange and epilogue of 128 rows take 4 us, which a split
@@ -393,6 +405,8 @@ static FewRows few_rows(int M, int N, int K) {
     const long a_kb = (long)M * K * 2 / 1024, blocks = (N + 15) / 16;
     return M > 8 && ((a_kb > 120 && blocks > 6L * sm_count()) || (a_kb >= 384 && blocks > 4L * sm_count())) ? FewRows::no : FewRows::rows;
   }
+  const long blocks = (N + 15) / 16;
+  if (M <= 24 && ((blocks <= sm_count() && K <= 9216) || (blocks <= 5.25 * sm_count() && K <= 4096))) return FewRows::rows;
   if (M <= 64) return tiles * (M <= 32 ? 1 : 2) <= sm_count() ? FewRows::skinny : FewRows::no;
   return M <= 128 && tiles * 3 <= sm_count() && num_kb >= 16 && num_kb * 4 >= tiles * 3 ? FewRows::skinny : FewRows::no;
 }
