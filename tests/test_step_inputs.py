@@ -120,3 +120,25 @@ def test_positions_of_two_axes_keep_the_general_form():
     x, cos, sin = m.rows_and_rotation(ModelBatch(ids, pos, None))
     c, s = m.rope.cos_sin_for(pos, m.cfg.mrope_section, False)
     assert torch.equal(x, m.embed_tokens[ids]) and torch.equal(cos, c) and torch.equal(sin, s)
+
+
+@pytest.mark.parametrize("experts,per_token", [(0, 8), (8, 5), (8, 6)])         # 3 sequences: 15 and 18 choices of 8 experts
+@pytest.mark.parametrize("once", [True, False])
+def test_padding_rows_of_a_step(experts, per_token, once, monkeypatch):
+    """Without experts, or with two choices per expert, they see one key, else row 0's; either way its pages, and they write nothing."""
+    long = experts and per_token == 5
+    m = _decoder(False)
+    m.cfg.num_experts, m.cfg.num_experts_per_tok, m.uses_seq_table = experts, per_token, True
+    kv = [tuple(torch.zeros(8, 16, 1, 128, device="cuda", dtype=torch.bfloat16) for _ in range(2))]
+    r = DecodeGraphRunner(m, kv, max_blocks=5, buckets=(8,))
+    i32 = lambda *v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    b = ModelBatch(torch.arange(3, device="cuda"), torch.arange(3, device="cuda"), i32(4, 5, 6), [], decode_rows=torch.arange(3, device="cuda"),
+                   decode_block_tables=i32(7, 8, 9)[:, None], decode_seq_lens=i32(20, 30, 40))
+    b.seqs = SeqTable(None, i32(19, 29, 39), None, None, None, 3, 3, 0, None, None)
+    if not once:
+        monkeypatch.setattr(DecodeGraphRunner, "_fill_once", lambda *a: False)
+    st = r._bucket(3)
+    r._fill(st, b)
+    assert st.lens.tolist() == [20, 30, 40] + [20 if long else 1] * 5
+    assert st.ctx.tolist() == [19, 29, 39] + [19 if long else 0] * 5
+    assert st.slots.tolist() == [4, 5, 6] + [-1] * 5 and st.tables[:, 0].tolist() == [7, 8, 9] + [7] * 5

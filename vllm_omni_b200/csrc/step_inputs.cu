@@ -13,14 +13,14 @@ namespace omni {
 
 constexpr int FILL_JOBS = 16;
 
-// Row i < n of `dst` takes row order[i] (ordered) or i of `src`; rows past n repeat row 0's source or become -1 (pad_ones).  Bytes past
+// Row i < n of `dst` takes row order[i] (ordered) or i of `src`; rows past n repeat row 0's source or become int32 -1, 1 or 0 (pad 1, 2, 3).  Bytes past
 // src_bytes of a row are zero.  src == nullptr: zeros everywhere.
 struct FillJob {
   const unsigned char* src;
   unsigned char* dst;
   long src_pitch, dst_pitch;
   int src_bytes, dst_bytes;
-  int ordered, pad_ones;
+  int ordered, pad;
 };
 struct FillStep {
   FillJob jobs[FILL_JOBS];
@@ -37,13 +37,13 @@ fill_step_kernel(const __grid_constant__ FillStep p) {
   const long from = j.ordered ? p.order[live ? i : 0] : (live ? i : 0);
   const unsigned char* s = j.src ? j.src + from * j.src_pitch : nullptr;
   unsigned char* d = j.dst + (long)i * j.dst_pitch;
-  const bool ones = !live && j.pad_ones;
+  const int pad = live ? 0 : j.pad;
   const bool words = ((reinterpret_cast<uintptr_t>(s) | reinterpret_cast<uintptr_t>(d) | (unsigned)j.src_bytes | (unsigned)j.dst_bytes) & 3) == 0;
   if (words) {
     for (int c = threadIdx.x; c < j.dst_bytes / 4; c += 128)
-      reinterpret_cast<uint32_t*>(d)[c] = ones ? 0xffffffffu : (s && c < j.src_bytes / 4 ? reinterpret_cast<const uint32_t*>(s)[c] : 0u);
+      reinterpret_cast<uint32_t*>(d)[c] = pad ? (pad == 1 ? 0xffffffffu : (uint32_t)(pad == 2)) : (s && c < j.src_bytes / 4 ? reinterpret_cast<const uint32_t*>(s)[c] : 0u);
   } else {
-    for (int c = threadIdx.x; c < j.dst_bytes; c += 128) d[c] = ones ? 0xff : (s && c < j.src_bytes ? s[c] : 0);
+    for (int c = threadIdx.x; c < j.dst_bytes; c += 128) d[c] = pad ? (pad == 1 ? 0xff : (unsigned char)(pad == 2 && (c & 3) == 0)) : (s && c < j.src_bytes ? s[c] : 0);
   }
 }
 

@@ -5,7 +5,9 @@ decoder issues several hundred small kernels per step.  ``DecodeGraphRunner`` ke
 bucket, a set of STATIC input tensors (token ids / embedding overlay, positions, slot mapping,
 block tables, sequence lengths), copies each step's values into them, and replays one captured
 graph of ``decoder.forward`` on them.  Rows beyond the live batch repeat row 0 with slot -1 (the
-KV write skips them), so a bucket never computes on undefined data.
+KV write skips them), so a bucket never computes on undefined data.  Where a decoder says so (``short_padding``) they see row 0's first key only,
+so that a batch of 17 does not pay for 15 contexts of that length more; a decoder with experts says so for larger batches only, because rows that differ
+from row 0 choose other experts, whose weights cost more than the keys.
 
 The reference gets the same effect from vLLM's CUDA-graph runner plus dedicated buffers for the
 talker's multi-token step (vllm_omni/worker/gpu_model_runner.py:71-89, 1085-1112).
@@ -67,6 +69,7 @@ class DecodeGraphRunner:
         dev = decoder.embed_tokens.device
         self.device, self.dtype = dev, decoder.embed_tokens.dtype
         self.use_graph = (dev.type == "cuda") if use_graph is None else bool(use_graph and dev.type == "cuda")
+        self.short_padding = getattr(decoder, "short_padding", lambda n: False)
         self._state: dict[int, _Bucket] = {}
         self.replays = 0
 
@@ -94,7 +97,7 @@ class DecodeGraphRunner:
         order = b.decode_rows
         if not (order.device == st.ids.device and order.dtype == torch.int64 and order.is_contiguous()):
             return False
-        f, pos = StepFill(order.numel(), st.n), b.positions
+        f, pos, short = StepFill(order.numel(), st.n), b.positions, self.short_padding(order.numel())
         ok = f.put(st.ids, b.input_ids, True)
         if st.pos.dim() == 2:
             for ax in range(st.pos.shape[0]):
@@ -102,9 +105,9 @@ class DecodeGraphRunner:
         else:
             ok = ok and f.put(st.pos, pos, True)
         ok = ok and f.put(st.slots, b.slot_mapping, True, pad_ones=True) and f.put(st.tables, b.decode_block_tables, False, narrow=True) \
-            and f.put(st.lens, b.decode_seq_lens, False)
+            and f.put(st.lens, b.decode_seq_lens, False, pad_to=1 if short else None)
         if st.seqs is not None:
-            ok = ok and f.put(st.ctx, b.seqs.context, True)
+            ok = ok and f.put(st.ctx, b.seqs.context, True, pad_to=0 if short else None)
             if st.seqs.state_in is not None:
                 ok = ok and f.put(st.seqs.state_in, b.seqs.state_in, True) and f.put(st.seqs.state_out, b.seqs.state_out, False, pad_ones=True)
         if b.input_embeds is not None:
@@ -121,7 +124,7 @@ class DecodeGraphRunner:
         if st.ids.is_cuda and self._fill_once(st, b):
             return n
         order = b.decode_rows                      # rows of the step's batch in decode order (identity here)
-        pad = st.n - n
+        pad, short = st.n - n, self.short_padding(n)
 
         def put(dst, src, dim=0):
             src = src.index_select(dim, order) if order is not None else src
@@ -147,9 +150,11 @@ class DecodeGraphRunner:
         st.lens[:n].copy_(b.decode_seq_lens)
         if pad:
             st.tables[n:].copy_(st.tables[:1].expand(pad, -1))
-            st.lens[n:].copy_(st.lens[:1].expand(pad))
+            st.lens[n:].copy_(torch.ones_like(st.lens[n:]) if short else st.lens[:1].expand(pad))
         if st.seqs is not None:
             put(st.ctx, b.seqs.context)
+            if pad and short:
+                st.ctx[n:].zero_()
             if st.seqs.state_in is not None:
                 put(st.seqs.state_in, b.seqs.state_in)
                 st.seqs.state_out[:n].copy_(b.seqs.state_out)

@@ -242,6 +242,9 @@ class FikizenLayer(nn.Module):
 
 
 class FikizenDecoder(PackedDecoder):
+    def short_padding(self, n: int) -> bool:
+        return True                      # padding rows of a captured decode step may see one key only
+
     def __init__(self, cfg: FikizenConfig, dtype=torch.bfloat16, device=None):
         super().__init__()
         self.cfg, self.dtype_ = cfg, dtype

@@ -194,6 +194,12 @@ class QwenDecoderModel(nn.Module):
         self.tp_reduce = None
         self.local_heads = (cfg.num_attention_heads, cfg.num_key_value_heads)   # (q, kv) heads on this rank
 
+    def short_padding(self, n: int) -> bool:
+        """Padding rows of a captured step of ``n`` sequences may see one key only (engine/graph_runner.py).  With experts they choose others than row 0 then:
+        from two tokens per expert on few that no token has chosen (36 sequences, 128 experts, top 8: one more per layer, 1 us, against the
+        keys of 28 contexts; 20 sequences: two more)."""
+        return not self.cfg.num_experts or n * self.cfg.num_experts_per_tok >= 2 * self.cfg.num_experts
+
     @property
     def kv_heads_local(self) -> int:
         """KV heads whose pages this rank keeps (all of them without tensor parallelism)."""

@@ -14,7 +14,7 @@ _JOBS = 16
 
 class _Job(ctypes.Structure):
     _fields_ = [("src", c_void_p), ("dst", c_void_p), ("src_pitch", c_long), ("dst_pitch", c_long), ("src_bytes", c_int),
-                ("dst_bytes", c_int), ("ordered", c_int), ("pad_ones", c_int)]
+                ("dst_bytes", c_int), ("ordered", c_int), ("pad", c_int)]
 
 
 class _Fill(ctypes.Structure):
@@ -34,8 +34,10 @@ class StepFill:
     def __init__(self, n: int, rows: int):
         self.a, self.n, self.rows, self.count, self.keep = _Fill(), n, rows, 0, []
 
-    def put(self, dst: torch.Tensor, src: torch.Tensor | None, ordered: bool, pad_ones: bool = False, narrow: bool = False) -> bool:
-        """dst [rows] or [rows, c]; src the same with n rows and c columns, or with ``narrow`` fewer (the rest of a row is zeroed)."""
+    def put(self, dst: torch.Tensor, src: torch.Tensor | None, ordered: bool, pad_ones: bool = False, narrow: bool = False,
+            pad_to: int | None = None) -> bool:
+        """dst [rows] or [rows, c]; src the same with n rows and c columns, or with ``narrow`` fewer (the rest of a row is zeroed).  Rows past n repeat
+        row 0 of src, or are -1 (``pad_ones``), or the int32 ``pad_to``, 0 or 1."""
         if self.count == _JOBS:
             return False
         j = self.a.jobs[self.count]
@@ -49,7 +51,8 @@ class StepFill:
                 return False
             j.src, j.src_pitch, j.src_bytes = src.data_ptr(), src.stride(0) * size, (src.shape[1] if src.dim() == 2 else 1) * size
             self.keep.append(src)
-        j.ordered, j.pad_ones = int(ordered), int(pad_ones)
+        assert pad_to is None or (pad_to in (0, 1) and dst.dtype == torch.int32)
+        j.ordered, j.pad = int(ordered), 1 if pad_ones else {None: 0, 1: 2, 0: 3}[pad_to]
         self.count += 1
         return True
 
