@@ -1489,9 +1489,9 @@ extern "C" int omni_gemm_bf16_experts(const void* A, int lda, const void* W, int
   using namespace omni;
   if (act != ACT_NONE && act != ACT_RELU2 && act != 5) return RC_BAD_ARG;
   if (M <= 0 || N <= 0 || K <= 0 || num_tiles <= 0) return RC_OK;
-  if ((K & 7) || (N & 7) || (lda & 7) || num_experts <= 0 || !tile_expert || !tile_row0 || !tile_rows) return RC_BAD_ARG;
+  if ((K & 7) || (N & 7) || (lda & 7) || (ldc & 7) || (reinterpret_cast<uintptr_t>(C) & 15) || num_experts <= 0 || !tile_expert || !tile_row0 || !tile_rows) return RC_BAD_ARG;
   ExpertArgs a = {};
-  if (int rc = make_tmap_2d(&a.tmX, A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)M, (uint64_t)K, (uint64_t)lda * 2, 64, 64)) return rc;
+  if (int rc = make_tmap_2d(&a.tmX, A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)M, (uint64_t)K, (uint64_t)lda * 2, tile == 256 ? ExpertPairCfg::BOX : 64, 64)) return rc;
   if (act == 5) {
     EncodeTiledFn enc = get_encode_tiled();
     if (!enc) return RC_NO_DRIVER;
