@@ -94,7 +94,8 @@ def test_expert_rows(act, T):
 
 
 @pytest.mark.parametrize("n_pairs,E,lo,hi,tile", [(1, 1, 0, 1, 64), (5000, 128, 0, 128, 64), (5000, 128, 0, 128, 128), (3000, 7, 2, 5, 128), (2048, 1024, 0, 1024, 128),
-                                                     (70001, 64, 0, 64, 256), (70001, 64, 0, 64, 128), (1300, 4, 1, 4, 256)])
+                                                     (70001, 64, 0, 64, 256), (70001, 64, 0, 64, 128), (1300, 4, 1, 4, 256),
+                                                     (8192, 128, 0, 128, 128), (8193, 128, 0, 128, 128), (16385, 1024, 100, 900, 256)])
 def test_even_plan(n_pairs, E, lo, hi, tile):
     g = torch.Generator(device="cuda").manual_seed(n_pairs)
     ids = (torch.rand(n_pairs, generator=g, device="cuda") ** 2 * E).int().clamp(max=E - 1)
