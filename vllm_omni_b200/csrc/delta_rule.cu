@@ -4,7 +4,10 @@
 //                       every n-th key row; per token convolution, unit lengths, decays, both reads of the state, the write,
 //                       norm and gate.  Decoded tokens take exactly one turn (one launch does the whole mixer, and the state
 //                       is read and written once); the exact mode walks whole portions.  States too large for one block are
-//                       cut into column slices, whose results go to `raw`
+//                       cut into column slices, whose results go to `raw`.  One token per sequence is a chain of latencies around 128 KB of
+//                       state per block: what it starts from is fetched before or together.  A step of a mixer of 16 heads of 128 x 128 and
+//                       three attention layers: 16 sequences 309.5 -> 307.8 us, 20 380 -> 375, 64 503 -> 499 (taps and channels one after the
+//                       other, gate and gain at the end, new history in a pass of its own)
 //   omni_delta_finish   norm and gate of the results in `raw`
 #include "delta_rule.cuh"
 
@@ -15,9 +18,8 @@ typedef __nv_bfloat16 bf16;
 constexpr int DS_THREADS = 256;
 
 template <typename T, bool CHANNEL, int NR>
-__global__ void __launch_bounds__(DS_THREADS)
+__global__ void __launch_bounds__(DS_THREADS, NR <= 4 ? 3 : NR <= 16 ? 2 : 1)
 delta_steps_kernel(const DeltaRule p, const int cw) {
-  pdl_begin();
   extern __shared__ __align__(16) float sm[];
   __shared__ float sh[64];
   const int tid = threadIdx.x;
@@ -32,8 +34,19 @@ delta_steps_kernel(const DeltaRule p, const int cw) {
   float* s_d = s_k + p.dp;                                   // [dp] channel: decay
   float* s_a = s_d + p.dp;                                   // [dp] channel: removal rate
   float* s_v = s_a + p.dp;                                   // [w]
-  float* red = s_v + cw;                                     // [RG, w]
+  float* s_g = s_v + cw;                                     // [2, w] gate's logits, of every other token: read when the next one's are fetched
+  float* s_w = s_g + 2 * cw;                                 // [w] gain
+  float* red = s_w + cw;                                     // [RG, w]
   float* red2 = red + 4 * DS_THREADS;
+  {
+    // The state is on its way to L2 before the kernel before has ended.  It only hints: the row is read past L1 and once more below, and one that is out
+    // of range or about to change costs a wasted fetch.
+    const int row = __ldcg(p.state_in + seq), per_row = (w * 4 + 127) / 128;
+    if (row >= 0 && row < p.num_state)
+      for (int l = tid; l < p.dp * per_row; l += DS_THREADS)
+        prefetch_l2(p.state + (((long)row * p.H + h) * p.dp + l / per_row) * p.vp + c0 + l % per_row * 32);
+  }
+  pdl_begin();
   const int q0 = p.q_start[seq], n = p.q_start[seq + 1] - q0, ctx = p.context[seq];
   if (n <= 0) return;
   int sin, sout;
@@ -64,6 +77,17 @@ delta_steps_kernel(const DeltaRule p, const int cw) {
     const long row = q0 + t;
     const T* pr = proj + row * p.ldp;
     float ss[2] = {0.f, 0.f};                                // sums of squares of q and k
+    float rate = 0.f, za = 0.f, zb = 0.f;
+    if (!CHANNEL) {
+      rate = p.rate[h];
+      za = (float)pr[p.a_col + h] + p.dt_bias[h];
+      zb = (float)pr[p.b_col + h];
+    }
+    if (gridDim.z == 1)                                      // fetched with everything else, used last
+      for (int c = tid; c < w; c += DS_THREADS) {
+        s_g[(t & 1) * cw + c] = (float)pr[p.g_col + h * p.vp + c];
+        s_w[c] = p.gain[(long)h * p.gain_hs + c];
+      }
     if (CHANNEL) {
       const T* z = static_cast<const T*>(p.z) + row * p.ldz;
       for (int c = tid; c < p.dp; c += DS_THREADS) {
@@ -77,19 +101,49 @@ delta_steps_kernel(const DeltaRule p, const int cw) {
       }
       for (int c = tid; c < w; c += DS_THREADS) s_v[c] = (float)pr[p.v_col + h * p.vp + c0 + c];
     } else {
-      for (int i = tid; i < 2 * p.dp + w; i += DS_THREADS) {
-        const int c = channel_of(i);
-        float x = 0.f;
-        for (int j = 0; j < p.taps; ++j) x = fmaf(p.conv[(long)j * C + c], conv_x(t - hl + j, c), x);
-        x = x / (1.0f + expf(-x));
-        if (i < p.dp) {
-          s_q[i] = x;
-          ss[0] = fmaf(x, x, ss[0]);
-        } else if (i < 2 * p.dp) {
-          s_k[i - p.dp] = x;
-          ss[1] = fmaf(x, x, ss[1]);
-        } else {
-          s_v[i - 2 * p.dp] = x;
+      // two elements of a thread and four taps at a time: their loads are under way together
+      const int count = 2 * p.dp + w;
+      const bool keep = t == n - 1 && sout >= 0, keeps_qk = h == g * R && blockIdx.z == 0;
+      for (int i0 = tid; i0 < count; i0 += 2 * DS_THREADS) {
+        float x[2] = {0.f, 0.f};
+        for (int j0 = 0; j0 < p.taps; j0 += 4) {
+          float cv[2][4], in[2][4];
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const int i = i0 + u * DS_THREADS, c = channel_of(i);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const bool live = i < count && j0 + j < p.taps;
+              cv[u][j] = live ? p.conv[(long)(j0 + j) * C + c] : 0.f;
+              in[u][j] = live ? conv_x(t - hl + j0 + j, c) : 0.f;
+            }
+          }
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const int i = i0 + u * DS_THREADS, c = channel_of(i);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              if (j0 + j < p.taps) x[u] = fmaf(cv[u][j], in[u][j], x[u]);
+              // new history (a row of its own): the last token's inputs but the oldest; the group's first head writes q and k, every block its values
+              if (keep && i < count && (keeps_qk || i >= 2 * p.dp) && j0 + j > 0 && j0 + j < p.taps)
+                hist[((long)sout * hl + j0 + j - 1) * C + c] = (T)in[u][j];
+            }
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int i = i0 + u * DS_THREADS;
+          if (i >= count) continue;
+          x[u] = x[u] / (1.0f + expf(-x[u]));
+          if (i < p.dp) {
+            s_q[i] = x[u];
+            ss[0] = fmaf(x[u], x[u], ss[0]);
+          } else if (i < 2 * p.dp) {
+            s_k[i - p.dp] = x[u];
+            ss[1] = fmaf(x[u], x[u], ss[1]);
+          } else {
+            s_v[i - 2 * p.dp] = x[u];
+          }
         }
       }
     }
@@ -97,8 +151,8 @@ delta_steps_kernel(const DeltaRule p, const int cw) {
     const float ik = 1.0f / sqrtf(ss[1] + p.unit_eps);
     float decay = 1.f, beta = 1.f, o_mul = 1.f;
     if (!CHANNEL) {
-      decay = expf(p.rate[h] * dr_softplus((float)pr[p.a_col + h] + p.dt_bias[h]));
-      beta = dr_sigmoid((float)pr[p.b_col + h]);
+      decay = expf(rate * dr_softplus(za));
+      beta = dr_sigmoid(zb);
       o_mul = p.q_mul / sqrtf(ss[0] + p.unit_eps);
     }
     // what the old state answers to the unit key
@@ -180,11 +234,10 @@ delta_steps_kernel(const DeltaRule p, const int cw) {
       block_sum<1>(so, sh);
       if (tid < nc) {
         const float s = rms_scale(so[0], p.dv, p.eps);
-        const float* gain = p.gain + (long)h * p.gain_hs + tid * 4;
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const float gz = (float)pr[p.g_col + col + e], open = dr_sigmoid(gz);
-          static_cast<T*>(p.out)[row * p.ldo + col + e] = (T)(res[e] * s * gain[e] * (CHANNEL ? open : gz * open));
+          const float gz = s_g[(t & 1) * cw + tid * 4 + e], open = dr_sigmoid(gz);
+          static_cast<T*>(p.out)[row * p.ldo + col + e] = (T)(res[e] * s * s_w[tid * 4 + e] * (CHANNEL ? open : gz * open));
         }
       }
     }
@@ -195,14 +248,6 @@ delta_steps_kernel(const DeltaRule p, const int cw) {
   for (int i = 0; i < NR; ++i) {
     const int r = rg + i * RG;
     if (act && r < p.dp) *reinterpret_cast<float4*>(S1 + (long)r * p.vp) = S[i];
-  }
-  if (!CHANNEL && hl > 0) {
-    // new history: the group's first head writes q and k, every block its values
-    const bool first = h == g * R && blockIdx.z == 0;
-    for (int i = first ? tid : 2 * p.dp + tid; i < 2 * p.dp + w; i += DS_THREADS) {
-      const int c = channel_of(i);
-      for (int m = 0; m < hl; ++m) hist[((long)sout * hl + m) * C + c] = (T)conv_x(n - hl + m, c);
-    }
   }
 }
 
@@ -273,7 +318,7 @@ template <typename T, bool CHANNEL>
 static int launch_steps(const DeltaRule& p, int cw, cudaStream_t st) {
   const int nc = cw / 4, RG = DS_THREADS / nc, rows = (p.dp + RG - 1) / RG;
   const dim3 grid(p.seq_list ? p.n_list : p.num_seqs, p.H, (p.vp + cw - 1) / cw);
-  const int smem = (4 * p.dp + cw + 8 * DS_THREADS) * 4;
+  const int smem = (4 * p.dp + 4 * cw + 8 * DS_THREADS) * 4;
   if (smem > 47 * 1024) return RC_TOO_LARGE;
   if (rows <= 4) launch_overlapped(delta_steps_kernel<T, CHANNEL, 4>, grid, DS_THREADS, smem, st, p, cw);
   else if (rows <= 8) launch_overlapped(delta_steps_kernel<T, CHANNEL, 8>, grid, DS_THREADS, smem, st, p, cw);
