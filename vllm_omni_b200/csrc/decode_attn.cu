@@ -27,6 +27,8 @@ __device__ __forceinline__ float da_ex2(float x) {
   return y;
 }
 
+constexpr int DA_EVEN = 128;          // every warp adds up that many lengths at most
+
 struct DecodeAttn {
   const __nv_bfloat16 *q, *k, *v;
   long q_rs;
@@ -35,6 +37,7 @@ struct DecodeAttn {
   const int* lens;
   int max_keys;                      // no sequence has more
   int n, H, Hkv, splits, subs;       // shares of the keys: blocks, and warps of a block
+  int by_seq;                        // neighbours in the grid are sequences, else shares of one
   int room;                          // warps that a round leaves for whole shares, see plan_shares; 0: a sequence's shares are its keys / splits
   float scale_log2;
   float *part_o, *part_ml;
@@ -63,7 +66,7 @@ paged_decode_kernel(const __grid_constant__ DecodeAttn p) {
   pdl_begin();
   constexpr int NH = UP ? 2 : 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, j = lane & 3;
-  const int seq = blockIdx.x, split = blockIdx.y;
+  const int seq = p.by_seq ? blockIdx.x : blockIdx.y, split = p.by_seq ? blockIdx.y : blockIdx.x;
   const int per_block = min(DA_WARPS, p.Hkv), sub = warp / per_block;
   const int hk = blockIdx.z * DA_WARPS + warp % per_block;
   if (sub >= p.subs || hk >= p.Hkv) return;
@@ -76,10 +79,24 @@ paged_decode_kernel(const __grid_constant__ DecodeAttn p) {
   if (p.room) {
     // Shares of at least a warp's part of all keys: those in use are one round of warps then.  Blocks past a sequence's shares leave; they are the
     // grid's last ones.
-    int all = 0;
-    for (int i = lane; i < p.n; i += 32) all += (min(p.lens[i], p.max_keys) + DA_KEYS - 1) / DA_KEYS;
+    int t[DA_EVEN / 32], all = 0;
+#pragma unroll
+    for (int i = 0; i < DA_EVEN / 32; ++i) {
+      t[i] = lane + i * 32 < p.n ? (min(p.lens[lane + i * 32], p.max_keys) + DA_KEYS - 1) / DA_KEYS : 0;
+      all += t[i];
+    }
     all = __reduce_add_sync(0xffffffffu, all) * p.Hkv;
-    if (4 * all > 5 * p.room) per = max(per, (all + p.room - 1) / p.room * p.subs);
+    if (4 * all > 5 * p.room) {
+      // a sequence's last share is a smaller one: `room` has a warp for each of them, a round has more where that many are not needed
+      const int round = p.room + p.n * p.subs * p.Hkv, safe = (all + p.room - 1) / p.room * p.subs, even = (all + round - 1) / round * p.subs;
+      int shares = 0;
+      if (even < safe) {
+#pragma unroll
+        for (int i = 0; i < DA_EVEN / 32; ++i) shares += (t[i] + even - 1) / even;
+        shares = __reduce_add_sync(0xffffffffu, shares) * p.subs * p.Hkv;
+      }
+      per = max(per, even < safe && shares <= round ? even : safe);
+    }
   }
   const int t1 = min(tiles, (split + 1) * per);
   if (split * per + sub >= t1) {      // no keys (a table wider than the sequence): weight zero, and no sum for the merge to read
@@ -302,13 +319,14 @@ paged_decode_merge_kernel(const float* part_o, const float* part_ml, int parts, 
   *reinterpret_cast<uint2*>(out + row * o_rs + ((int)blockIdx.x - seq * H) * DA_D + lane * 4) = w;
 }
 
-constexpr int DA_MAX_PARTS = 64, DA_EVEN = 128;          // every warp adds up that many lengths at most
+constexpr int DA_MAX_PARTS = 64;
 
 // Shares of a sequence's keys: room for about `target` warps in all, at least two tiles of 16 keys each.  Twelve warps fit an SM.  Two rounds of them let
 // long sequences among short ones have many shares (8 sequences of 4096 keys, 8 KV heads: 20 warps per SM 1.05 and 18 1.12 times as long as 24), but of
 // sequences that are alike one round is faster: fewer starts, fewer sums.  The kernel, which knows the lengths, uses as many shares as make one round
 // (room).  us, as many as two rounds in brackets: 32 heads, 8 KV heads, 12 sequences of
-// about 2600 keys 30.5 (34.6), 48 of them 93 (103), 16 of 60 to 4000 keys 29.4 (32.7); 4 KV heads, 24 of about 440 12.5 (14.8).  Up to a quarter more keys than
+// about 2600 keys 30.5 (34.6), 48 of them 93 (103), 16 of 60 to 4000 keys 29.4 (32.7); 4 KV heads, 24 of about 440 12.5 (14.8).
+// Where rounding up leaves the round room, shares are a tile shorter: 8 sequences of 3500 keys, 4 KV heads, between their projections 24.6 (24.7; 25.9 without), 20 of 700 22.1 (21.5; 23.5).  Up to a quarter more keys than
 // a round's warps have tiles they keep a tile each: 32 of 90 keys, 8 KV heads, 9.4, in shares of two 11.1.
 // Blocks of fewer KV heads hold shares of one sequence, whose sums are many and small: 20, since 24 took 1.11 times the tensor-core kernel's time for 72
 // sequences of 1024 keys in tables of 4096 and 1 KV head, and 20 never more than 1.01 of it.  A single sequence has at most
@@ -361,7 +379,10 @@ extern "C" int omni_paged_decode_attn(const void* q, long q_rs, const void* k, c
   p.H = H; p.Hkv = Hkv; p.scale_log2 = scale * 1.4426950408889634f;
   p.part_o = part_o; p.part_ml = part_ml; p.out = (__nv_bfloat16*)out; p.o_rs = o_rs;
   p.rows = rows; p.n_rows = n_rows; p.status = status;
-  const dim3 grid((unsigned)n, (unsigned)p.splits, (unsigned)((Hkv + DA_WARPS - 1) / DA_WARPS));
+  // blocks without keys come last where there may be many of them; else a sequence's blocks side by side: 3 sequences of 60 to 3500 keys, 4 KV heads, between
+  // their projections 15.1 us (15.9)
+  p.by_seq = p.room > 0 || n > 65535;
+  const dim3 grid((unsigned)(p.by_seq ? n : p.splits), (unsigned)(p.by_seq ? p.splits : n), (unsigned)((Hkv + DA_WARPS - 1) / DA_WARPS));
   cudaStream_t st = (cudaStream_t)stream;
   const bool up = H / Hkv > 8;
   // One round of blocks has to lie evenly on the SMs, which it does not where it is dealt out around the last blocks of the kernel before: overlapped, a step of
