@@ -23,7 +23,6 @@ delta_steps_kernel(const DeltaRule p, const int cw) {
   extern __shared__ __align__(16) float sm[];
   __shared__ float sh[64];
   const int tid = threadIdx.x;
-  const int seq = p.seq_list ? min(max(p.seq_list[blockIdx.x], 0), p.num_seqs - 1) : blockIdx.x;
   const int h = blockIdx.y, R = p.H / p.G, g = h / R;
   const int c0 = blockIdx.z * cw, w = min(cw, p.vp - c0);
   const int nc = w / 4, RG = DS_THREADS / nc;                // four-column groups, key rows side by side
@@ -39,14 +38,16 @@ delta_steps_kernel(const DeltaRule p, const int cw) {
   float* red = s_w + cw;                                     // [RG, w]
   float* red2 = red + 4 * DS_THREADS;
   {
-    // The state is on its way to L2 before the kernel before has ended.  It only hints: the row is read past L1 and once more below, and one that is out
-    // of range or about to change costs a wasted fetch.
-    const int row = __ldcg(p.state_in + seq), per_row = (w * 4 + 127) / 128;
+    // The state is on its way to L2 before the kernel before has ended.  It only hints: sequence and row are read past L1 and once more below, and a row that is
+    // out of range or about to change costs a wasted fetch.
+    const int s = p.seq_list ? min(max(__ldcg(p.seq_list + blockIdx.x), 0), p.num_seqs - 1) : blockIdx.x;
+    const int row = __ldcg(p.state_in + s), per_row = (w * 4 + 127) / 128;
     if (row >= 0 && row < p.num_state)
       for (int l = tid; l < p.dp * per_row; l += DS_THREADS)
         prefetch_l2(p.state + (((long)row * p.H + h) * p.dp + l / per_row) * p.vp + c0 + l % per_row * 32);
   }
   pdl_begin();
+  const int seq = p.seq_list ? min(max(p.seq_list[blockIdx.x], 0), p.num_seqs - 1) : blockIdx.x;
   const int q0 = p.q_start[seq], n = p.q_start[seq + 1] - q0, ctx = p.context[seq];
   if (n <= 0) return;
   int sin, sout;
