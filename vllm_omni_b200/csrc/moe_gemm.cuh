@@ -6,7 +6,7 @@
 // GATED: W [E, 2 N, K] holds gate and lift rows; one 5-D box brings 8 gate rows, their 8 lift rows, the next 8 gate rows and so on, so that both
 // values of an output lie 8 lanes apart in a warp and silu(gate) * lift leaves the accumulators without passing through memory.
 // 128 experts, 2048 -> 2 x 768 -> 2048, top 8, whole layer on cold caches: 64 tokens 200 us (two grouped launches of 128-row tiles around a SwiGLU
-// kernel: 239), 256 tokens 211 us (241), 2463 tokens 304 us (about 440); the weights alone take 182 us.
+// kernel: 239), 256 tokens 211 us (241), 2463 tokens 290 us (about 440); the weights alone take 182 us.
 #pragma once
 
 namespace omni {
