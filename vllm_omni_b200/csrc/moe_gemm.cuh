@@ -213,7 +213,8 @@ expert_gemm_kernel(const __grid_constant__ ExpertArgs a, int* status) {
 }
 
 // Tiles of up to 256 rows, on CTA pairs: each CTA brings 128 rows of W and half of the tile's rows, and one MMA of 256 outputs reads both.  On single CTAs these
-// tiles are bound by what L2 delivers (154 rows: 1.1 MB per 128 x 2048 weights, 10.5 TB/s in all); a pair fetches 0.8.  128 experts, 2048 -> 2 x 768 and
+// tiles are bound by what L2 delivers (154 rows: 1.1 MB per 128 x 2048 weights, 10.5 TB/s in all); a pair fetches 0.8, and what bounds it is HBM
+// (2463 tokens: weights and rows at 0.94 and 0.96 of the copy rate).  128 experts, 2048 -> 2 x 768 and
 // 768 -> 2048, top 8, both with the drain of this file: 1400 tokens 152 -> 144 and 79 -> 77 us, 2463 162 -> 155 and 89 -> 86, 4000 204 -> 192 and 124 -> 111,
 // 8000 340 -> 322 and 210 -> 191.  Tiles of up to 128 rows gain nothing (600 tokens 132.6 -> 132 and 70.7 -> 72.7, 1000 135 -> 135 and 72.7 -> 75.3).
 struct ExpertPairCfg {
