@@ -79,11 +79,11 @@ def test_pages_of_other_sizes_keep_fp32_weights(bs, H, Hkv):
     assert ((out.double() - ref).abs() <= bound).all()
 
 
-# shares of very different and of like lengths (as many as make one round of warps), sequences without keys, more sequences than add up their lengths, a block each
+# shares of very different and of like lengths, sequences without keys, sequences by the hundred, a block each
 @pytest.mark.parametrize("H,Hkv,lens", [(32, 4, [4000, 3, 0, 70] + [17] * 40 + [900]), (8, 1, [2500] + [1] * 200), (16, 8, [0, 0, 5]), (32, 8, [33] * 700),
                                         (12, 3, [16 * i for i in range(50)]), (16, 1, [5000, 0, 40]), (8, 8, [1] * 450), (4, 1, [7000]),
-                                        (32, 4, [3500] * 8), (32, 4, [700] * 20), (32, 4, [3500] * 7 + [1])])          # a round's room used up, and not
-def test_shares_by_the_lengths(H, Hkv, lens):
+                                        (32, 4, [3500] * 8), (32, 4, [700] * 20), (32, 4, [3500] * 7 + [1])])
+def test_shares_of_lengths(H, Hkv, lens):
     D, bs, n = 128, 16, len(lens)
     g = torch.Generator(device="cuda").manual_seed(n)
     per = [-(-l // bs) for l in lens]
@@ -104,3 +104,21 @@ def test_shares_by_the_lengths(H, Hkv, lens):
         ref = torch.einsum("hk,khd->hd", w, vv)
         bound = torch.einsum("hk,khd->hd", w, vv.abs()) * 2.0 ** -8 + ref.abs() * 2.0 ** -8 + 1e-5          # as above
         assert ((out[s].double() - ref).abs() <= bound).all(), (s, l)
+
+
+# batches of less and of more than a round of warps, both group sizes; one block of tables throughout
+@pytest.mark.parametrize("H,Hkv,n,length", [(32, 4, 64, 1800), (32, 8, 8, 3500), (32, 8, 48, 2600), (16, 1, 40, 700), (32, 4, 3, 2000)])
+def test_neighbours_leave_a_sequence_alone(H, Hkv, n, length):
+    """A sequence's result has the same bits whatever the lengths of the others in its batch."""
+    D, bs, width = 128, 16, 256
+    g = torch.Generator(device="cuda").manual_seed(n)
+    k, v = (torch.randn(2 * width, bs, Hkv, D, generator=g, device="cuda").bfloat16() for _ in range(2))
+    q = torch.randn(n, H, D, generator=g, device="cuda").bfloat16()
+    tables = torch.arange(width, 2 * width, dtype=torch.int32, device="cuda").repeat(n, 1)         # the others share their pages
+    tables[0] -= width
+    def first(others):
+        lens = torch.tensor([length] + [others(i) for i in range(1, n)], dtype=torch.int32, device="cuda")
+        return KC.paged_decode(q, k, v, tables, lens, impl="stream")[0]
+    want = first(lambda i: length)
+    for others in (lambda i: 1, lambda i: 4096, lambda i: 1 + 997 * i % 4096, lambda i: 0):
+        assert torch.equal(first(others), want)

@@ -27,8 +27,6 @@ __device__ __forceinline__ float da_ex2(float x) {
   return y;
 }
 
-constexpr int DA_EVEN = 128;          // every warp adds up that many lengths at most
-
 struct DecodeAttn {
   const __nv_bfloat16 *q, *k, *v;
   long q_rs;
@@ -36,9 +34,7 @@ struct DecodeAttn {
   int bt_stride, block_size;
   const int* lens;
   int max_keys;                      // no sequence has more
-  int n, H, Hkv, splits, subs;       // shares of the keys: blocks, and warps of a block
-  int by_seq;                        // neighbours in the grid are sequences, else shares of one
-  int room;                          // warps that a round leaves for whole shares, see plan_shares; 0: a sequence's shares are its keys / splits
+  int H, Hkv, splits, subs;          // shares of the keys: blocks, and warps of a block
   float scale_log2;
   float *part_o, *part_ml;
   __nv_bfloat16* out;
@@ -66,7 +62,7 @@ paged_decode_kernel(const __grid_constant__ DecodeAttn p) {
   pdl_begin();
   constexpr int NH = UP ? 2 : 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, j = lane & 3;
-  const int seq = p.by_seq ? blockIdx.x : blockIdx.y, split = p.by_seq ? blockIdx.y : blockIdx.x;
+  const int seq = blockIdx.y, split = blockIdx.x;
   const int per_block = min(DA_WARPS, p.Hkv), sub = warp / per_block;
   const int hk = blockIdx.z * DA_WARPS + warp % per_block;
   if (sub >= p.subs || hk >= p.Hkv) return;
@@ -74,30 +70,7 @@ paged_decode_kernel(const __grid_constant__ DecodeAttn p) {
   const long q_row = da_row<ROWS>(p, seq);
   if (q_row < 0) return;
   const int len = min(p.lens[seq], p.max_keys);
-  const int tiles = (len + DA_KEYS - 1) / DA_KEYS;
-  int per = (tiles + p.splits - 1) / p.splits;
-  if (p.room) {
-    // Shares of at least a warp's part of all keys: those in use are one round of warps then.  Blocks past a sequence's shares leave; they are the
-    // grid's last ones.
-    int t[DA_EVEN / 32], all = 0;
-#pragma unroll
-    for (int i = 0; i < DA_EVEN / 32; ++i) {
-      t[i] = lane + i * 32 < p.n ? (min(p.lens[lane + i * 32], p.max_keys) + DA_KEYS - 1) / DA_KEYS : 0;
-      all += t[i];
-    }
-    all = __reduce_add_sync(0xffffffffu, all) * p.Hkv;
-    if (4 * all > 5 * p.room) {
-      // a sequence's last share is a smaller one: `room` has a warp for each of them, a round has more where that many are not needed
-      const int round = p.room + p.n * p.subs * p.Hkv, safe = (all + p.room - 1) / p.room * p.subs, even = (all + round - 1) / round * p.subs;
-      int shares = 0;
-      if (even < safe) {
-#pragma unroll
-        for (int i = 0; i < DA_EVEN / 32; ++i) shares += (t[i] + even - 1) / even;
-        shares = __reduce_add_sync(0xffffffffu, shares) * p.subs * p.Hkv;
-      }
-      per = max(per, even < safe && shares <= round ? even : safe);
-    }
-  }
+  const int tiles = (len + DA_KEYS - 1) / DA_KEYS, per = (tiles + p.splits - 1) / p.splits;
   const int t1 = min(tiles, (split + 1) * per);
   if (split * per + sub >= t1) {      // no keys (a table wider than the sequence): weight zero, and no sum for the merge to read
     if (parts > 1 && lane < G) {
@@ -321,14 +294,12 @@ paged_decode_merge_kernel(const float* part_o, const float* part_ml, int parts, 
 
 constexpr int DA_MAX_PARTS = 64;
 
-// Shares of a sequence's keys: room for about `target` warps in all, at least two tiles of 16 keys each.  Twelve warps fit an SM.  Two rounds of them let
-// long sequences among short ones have many shares (8 sequences of 4096 keys, 8 KV heads: 20 warps per SM 1.05 and 18 1.12 times as long as 24), but of
-// sequences that are alike one round is faster: fewer starts, fewer sums.  The kernel, which knows the lengths, uses as many shares as make one round
-// (room).  us, as many as two rounds in brackets: 32 heads, 8 KV heads, 12 sequences of
-// about 2600 keys 30.5 (34.6), 48 of them 93 (103), 16 of 60 to 4000 keys 29.4 (32.7); 4 KV heads, 24 of about 440 12.5 (14.8).
-// Where rounding up leaves the round room, shares are a tile shorter: 8 sequences of 3500 keys, 4 KV heads, between their projections 24.6 (24.7; 25.9 without), 20 of 700 22.1 (21.5; 23.5).  Up to a quarter more keys than
-// a round's warps have tiles they keep a tile each: 32 of 90 keys, 8 KV heads, 9.4, in shares of two 11.1.
-// Blocks of fewer KV heads hold shares of one sequence, whose sums are many and small: 20, since 24 took 1.11 times the tensor-core kernel's time for 72
+// Shares of a sequence's keys: about `target` warps in all, at least two tiles of 16 keys each.  Twelve warps fit an SM; two rounds of them
+// even out lengths (8 sequences of 4096 keys, 8 KV heads: 20 warps per SM 1.05 and 18 1.12 times as long as 24).  The number depends on how many sequences
+// there are and on the table's width, never on the lengths: a sequence's result is the same whatever its neighbours hold, and probabilities are rounded
+// against the maximum of short shares.  (As many shares as make one round of warps, from the sum of the lengths: 48 sequences of about 2600 keys, 32 heads,
+// 8 KV heads 93 us instead of 103, but 2 to 5 % further from 64-bit results: 64 sequences of 900 to 2700 keys, 4 KV heads 0.00214 instead of 0.00208.)  Blocks of fewer KV
+// heads hold shares of one sequence, whose sums are many and small: 20, since 24 took 1.11 times the tensor-core kernel's time for 72
 // sequences of 1024 keys in tables of 4096 and 1 KV head, and 20 never more than 1.01 of it.  A single sequence has at most
 // 64 shares: 131072 keys of 4 KV heads take 148 us, the tensor-core kernel 246 (the copy rate would be 41; more shares would reach more SMs).
 static void plan_shares(int n, int Hkv, int max_keys, int& splits, int& subs) {
@@ -362,7 +333,7 @@ extern "C" int omni_paged_decode_attn(const void* q, long q_rs, const void* k, c
                                       int block_size, const int* lens, int n, int H, int Hkv, int max_keys, float scale, float* part_o,
                                       float* part_ml, void* out, long o_rs, const long long* rows, int n_rows, int* status, void* stream) {
   if (n <= 0) return RC_OK;
-  if (Hkv <= 0 || H % Hkv || H / Hkv > 16 || block_size < 8 || (block_size & 7) || max_keys < 1 || (q_rs & 7) || (o_rs & 7))
+  if (Hkv <= 0 || H % Hkv || H / Hkv > 16 || block_size < 8 || (block_size & 7) || max_keys < 1 || n > 65535 || (q_rs & 7) || (o_rs & 7))
     return RC_BAD_ARG;
   if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(out)) & 15)
     return RC_BAD_ARG;
@@ -372,22 +343,16 @@ extern "C" int omni_paged_decode_attn(const void* q, long q_rs, const void* k, c
   if (parts > 1 && (!part_o || !part_ml)) return RC_BAD_ARG;
   p.q = (const __nv_bfloat16*)q; p.k = (const __nv_bfloat16*)k; p.v = (const __nv_bfloat16*)v;
   p.q_rs = q_rs; p.block_tables = block_tables; p.bt_stride = bt_stride; p.block_size = block_size; p.lens = lens; p.max_keys = max_keys;
-  p.n = n;
-  // rounding up gives every sequence at most one share more; sequences and heads that fill half of a round by themselves get two, and so on
-  const int round = (H / Hkv > 8 ? 8 : 12) * sm_count(), rest = n * p.subs * Hkv;
-  p.room = parts > 1 && n <= DA_EVEN && n * Hkv >= 32 ? (2 * rest + round - 1) / round * round - rest : 0;
   p.H = H; p.Hkv = Hkv; p.scale_log2 = scale * 1.4426950408889634f;
   p.part_o = part_o; p.part_ml = part_ml; p.out = (__nv_bfloat16*)out; p.o_rs = o_rs;
   p.rows = rows; p.n_rows = n_rows; p.status = status;
-  // blocks without keys come last where there may be many of them; else a sequence's blocks side by side: 3 sequences of 60 to 3500 keys, 4 KV heads, between
-  // their projections 15.1 us (15.9)
-  p.by_seq = p.room > 0 || n > 65535;
-  const dim3 grid((unsigned)(p.by_seq ? n : p.splits), (unsigned)(p.by_seq ? p.splits : n), (unsigned)((Hkv + DA_WARPS - 1) / DA_WARPS));
+  const dim3 grid((unsigned)p.splits, (unsigned)n, (unsigned)((Hkv + DA_WARPS - 1) / DA_WARPS));
   cudaStream_t st = (cudaStream_t)stream;
   const bool up = H / Hkv > 8;
-  // One round of blocks has to lie evenly on the SMs, which it does not where it is dealt out around the last blocks of the kernel before: overlapped, a step of
-  // 48 sequences of about 2600 keys (4096-wide dense decoder, four layers) took 1347 us instead of 903, with two rounds 1069.
-  launch_with(p.room == 0, 1, rows ? (up ? paged_decode_kernel<true, true> : paged_decode_kernel<false, true>)
+  // The blocks of many sequences are dealt out unevenly around the last blocks of the kernel before, few ones gain from the early start.  Decode steps of four
+  // layers in us, ordinary launch (overlapped): 4096 wide, 8 KV heads, 50 sequences of 4000 keys 957 (1123), 24 of 1000 521 (527), 14 of 300 494.8 (493.5), 8 of 800
+  // 431 (430); 2048 wide, 4 KV heads, 20 of 500 263 (270), 14 of 300 217.8 (217.3); experts, 4 KV heads, 64 of 2048 1128 (1205), 32 of 90 856 (858).
+  launch_with(n <= 16, 1, rows ? (up ? paged_decode_kernel<true, true> : paged_decode_kernel<false, true>)
                          : (up ? paged_decode_kernel<true, false> : paged_decode_kernel<false, false>), grid, 32 * DA_WARPS, 0, st, p);
   if (parts == 1) return (int)cudaGetLastError();
   if (cudaError_t e = cudaGetLastError()) return (int)e;
