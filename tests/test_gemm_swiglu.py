@@ -38,6 +38,19 @@ def test_swiglu_takes_views():
     assert a.shape == (2, 150, 40) and torch.equal(a, b)
 
 
+@pytest.mark.parametrize("M", [4, 64, 300])
+def test_swiglu_of_rows_narrower_than_the_weights(M):
+    """As in ``linear``, rows of fewer channels meet the first columns of the weights; each row stays a row."""
+    rnd = _rnd(M)
+    x, w = rnd(M, 512), (rnd(2 * 96, 1024).float() * 512 ** -0.5).bfloat16()
+    g, u = (x.double() @ w[:, :512].double().T).split(96, 1)
+    ref = F.silu(g) * u
+    y = gemm.linear_swiglu(x, w)
+    nv.check_status(x.device)
+    # both halves and the result rounded to bf16; tanh.approx in silu, whose slope is at most 1.1
+    assert y.shape == ref.shape and ((y.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + g.abs() * u.abs() * (2.2 * 2.0 ** -8 + 2.0 ** -10) + 1e-4).all()
+
+
 # every kernel (pair of 256 / 192 / 128 columns, automatic choice) with every epilogue; ragged rows and columns; rows of a tile in two batches
 @pytest.mark.parametrize("bn", [0, 384, 448, 576])
 @pytest.mark.parametrize("act", [None, "gelu_tanh", "xielu", "silu", "relu2"])

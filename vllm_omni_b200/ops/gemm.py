@@ -149,8 +149,9 @@ def linear_swiglu(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     rounded before they meet), for rows that the few-row kernels split over clusters in two."""
     from .fused import silu_mul
     F_, K = w.shape[0] // 2, w.shape[1]
-    if x.is_cuda and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and w.shape[0] % 16 == 0 and K % 8 == 0 and x.numel() and w.stride(1) == 1 \
-            and w.stride(0) % 8 == 0:
+    # rows narrower than w meet its first columns, as in linear(): not for the launch below, which would take them for fewer, longer rows
+    if x.is_cuda and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.shape[-1] == K and w.shape[0] % 16 == 0 and K % 8 == 0 and x.numel() \
+            and w.stride(1) == 1 and w.stride(0) % 8 == 0:
         x2 = x.reshape(-1, K)
         if x2.stride(1) != 1 or x2.stride(0) % 8:
             x2 = x2.contiguous()
