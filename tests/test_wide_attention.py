@@ -46,6 +46,25 @@ def test_wide_attention_growing_maxima():
         assert (out.double() - ref).norm() <= 2 ** -8 * ref.norm()
 
 
+@pytest.mark.parametrize("workers", [0, 1, 5])
+def test_scores_of_minus_infinity(workers):
+    """Rows whose first keys score -inf (products past the range of fp32) beside rows of the same warp whose maxima grow: those keys weigh nothing."""
+    N, dead = 640, 300
+    g = torch.Generator(device="cuda").manual_seed(4)
+    q, k, v = (torch.randn(1, N, 384, device="cuda", generator=g).bfloat16() for _ in range(3))
+    k *= torch.linspace(1, 12, N, device="cuda")[None, :, None].bfloat16()
+    q[..., 0], k[..., 0] = 0.0, 0.0
+    q[:, ::3, 0], k[:, :dead, 0] = -1e30, 1e30
+    out = C._wide_head_flash(q, k, v, 384 ** -0.5, workers)
+    torch.cuda.synchronize()
+    nv.check_status(q.device)
+    s = q.double() @ k.double().transpose(1, 2) * 384 ** -0.5
+    s[:, ::3, :dead] = float("-inf")
+    ref = torch.softmax(s, -1) @ v.double()
+    # probabilities and results are bf16, the exponentials 2^-22
+    assert torch.isfinite(out).all() and (out.double() - ref).norm() <= 2 ** -8 * ref.norm()
+
+
 def test_wide_attention_width_outside_the_kernel():
     """512 channels stay with the two GEMMs around the row softmax, whose scores pass through bf16 as well."""
     g = torch.Generator(device="cuda").manual_seed(2)

@@ -261,7 +261,7 @@ wide_attn_kernel(const __grid_constant__ WideAttn a, int* status) {
       const bool grow = __any_sync(0xffffffffu, m_new > m + 8.0f) && !first;
       float alpha = 1.f;
       if (grow) {
-        alpha = wide_ex2(m - m_new);
+        alpha = m_new == -INFINITY ? 1.f : wide_ex2(m - m_new);      // a row of -inf scores so far beside one that grows
         la = mul2(la, pack2(alpha, alpha));
         lb = mul2(lb, pack2(alpha, alpha));
       }
