@@ -93,6 +93,30 @@ def test_expert_rows(act, T):
     assert same.sum() >= T - 4 and ((y - ref).abs() <= bound + 0.01 * ref.abs())[same].all()
 
 
+@pytest.mark.parametrize("act", [0, 3, 5])                             # none, squared ReLU, SwiGLU
+@pytest.mark.parametrize("tile", [64, 128, 256])
+@pytest.mark.parametrize("pitch,base", [(3, 0), (0, 1), (8, 4), (5, 7)])
+def test_expert_gemm_into_any_rows(act, tile, pitch, base):
+    """C of any pitch and base gets the bits of one whose rows lie on 16 bytes, and nothing beside them is written."""
+    from ctypes import c_int
+    E, N, K, rows = 3, 136, 72, [tile, 0, tile - 15, 1]
+    g = torch.Generator(device="cuda").manual_seed(tile)
+    a, w = (torch.randn(*s, generator=g, device="cuda").bfloat16() for s in ((sum(rows), K), (E, (2 if act == 5 else 1) * N, K)))
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    used = [i for i, r in enumerate(rows) if r]
+    te, t0, tn = i32([i % E for i in used] + [-1]), i32([sum(rows[:i]) for i in used] + [0]), i32([rows[i] for i in used] + [0])
+    def run(ld, at):
+        c = torch.full((sum(rows) * ld + 16,), 7.0, device="cuda", dtype=torch.bfloat16)
+        nv.check_rc(nv.lib("gemm_sm100").omni_gemm_bf16_experts(nv.ptr(a), c_int(K), nv.ptr(w), c_int(E), nv.ptr(c[at:]), c_int(ld), c_int(sum(rows)), c_int(N), c_int(K),
+                                                                nv.ptr(te), nv.ptr(t0), nv.ptr(tn), c_int(len(te)), c_int(tile), c_int(act),
+                                                                nv.ptr(nv.status_word(a.device)), nv.stream_ptr()), "experts")
+        nv.check_status(a.device)
+        body = c[at:at + sum(rows) * ld].view(-1, ld)
+        assert (c[:at] == 7).all() and (c[at + sum(rows) * ld:] == 7).all() and (body[:, N:] == 7).all()
+        return body[:, :N]
+    assert torch.equal(run(N + pitch, base), run(N, 0))
+
+
 @pytest.mark.parametrize("n_pairs,E,lo,hi,tile", [(1, 1, 0, 1, 64), (5000, 128, 0, 128, 64), (5000, 128, 0, 128, 128), (3000, 7, 2, 5, 128), (2048, 1024, 0, 1024, 128),
                                                      (70001, 64, 0, 64, 256), (70001, 64, 0, 64, 128), (1300, 4, 1, 4, 256),
                                                      (8192, 128, 0, 128, 128), (8193, 128, 0, 128, 128), (16385, 1024, 100, 900, 256)])

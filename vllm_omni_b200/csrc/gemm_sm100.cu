@@ -1482,14 +1482,15 @@ extern "C" int omni_gemm_bf16_grouped(const void* A, int lda, const void* W, int
 
 // Grouped GEMM over experts whose rows sit back to back (no padding): M rows in A and C in total, tile t covers rows [tile_row0[t],
 // tile_row0[t] + tile_rows[t]) of expert tile_expert[t] (-1 = unused, after all used ones); no tile has more than `tile` (64, 128 or 256) rows.
-// C[M, N] = act(A W[e]^T), W [E, N, K]; act 5: W [E, 2 N, K], C = silu(A W[e, :N]^T) * (A W[e, N:]^T), N a multiple of 8.
+// C[M, N] = act(A W[e]^T), W [E, N, K]; act 5: W [E, 2 N, K], C = silu(A W[e, :N]^T) * (A W[e, N:]^T), N a multiple of 8.  C: any
+// pitch and base.
 extern "C" int omni_gemm_bf16_experts(const void* A, int lda, const void* W, int num_experts, void* C, int ldc, int M, int N, int K,
                                       const int* tile_expert, const int* tile_row0, const int* tile_rows, int num_tiles, int tile,
                                       int act, int* status, void* stream) {
   using namespace omni;
   if (act != ACT_NONE && act != ACT_RELU2 && act != 5) return RC_BAD_ARG;
   if (M <= 0 || N <= 0 || K <= 0 || num_tiles <= 0) return RC_OK;
-  if ((K & 7) || (N & 7) || (lda & 7) || (ldc & 7) || (reinterpret_cast<uintptr_t>(C) & 15) || num_experts <= 0 || !tile_expert || !tile_row0 || !tile_rows) return RC_BAD_ARG;
+  if ((K & 7) || (N & 7) || (lda & 7) || num_experts <= 0 || !tile_expert || !tile_row0 || !tile_rows) return RC_BAD_ARG;
   ExpertArgs a = {};
   if (int rc = make_tmap_2d(&a.tmX, A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)M, (uint64_t)K, (uint64_t)lda * 2, tile == 256 ? ExpertPairCfg::BOX : 64, 64)) return rc;
   if (act == 5) {
@@ -1508,6 +1509,7 @@ extern "C" int omni_gemm_bf16_experts(const void* A, int lda, const void* W, int
     return rc;
   }
   a.c = static_cast<__nv_bfloat16*>(C); a.ldc = ldc; a.N = N; a.K = K;
+  a.by16 = (ldc & 7) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0;
   a.tile_expert = tile_expert; a.tile_row0 = tile_row0; a.tile_rows = tile_rows; a.max_tiles = num_tiles; a.act = act;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   return act == 5 ? launch_expert<true>(a, tile, status, s) : launch_expert<false>(a, tile, status, s);

@@ -26,6 +26,7 @@ struct ExpertArgs {
   int N, K;                                   // outputs per row, contraction
   const int *tile_expert, *tile_row0, *tile_rows;
   int max_tiles, act;
+  int by16;                                   // rows of C begin on 16 bytes
 };
 
 __device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap* tmap, uint32_t cluster_bar, int c0, int c1, int c2) {
@@ -52,7 +53,7 @@ __device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* tma
 
 // A warp's share of a finished tile: its 32 lanes of the accumulator, every other chunk of 16 rows; `out` and `cols` from the warp's first column on.  A lane
 // holds a column of the result.  GATED: lanes of a gate row take the even rows of C, lanes of its lift row the odd ones, and store where they stand.  Else the
-// chunk is turned in `turned` (1 KB of this warp) and leaves in pieces of 16 bytes: 16000 tokens of 128 x (768 -> 2048) on pairs 480 -> 349 us (427 -> 396 on
+// chunk is turned in `turned` (1 KB of this warp) and leaves in pieces of 16 bytes where C lies on such: 16000 tokens of 128 x (768 -> 2048) on pairs 480 -> 349 us (427 -> 396 on
 // single CTAs); the gated half as many stores are no faster that way (560 us, 611 turned).
 template <bool GATED>
 __device__ __forceinline__ void expert_drain(uint32_t acc, __nv_bfloat16* turned, __nv_bfloat16* out, int rows, int half, int lane, int cols, const ExpertArgs& a) {
@@ -77,6 +78,11 @@ __device__ __forceinline__ void expert_drain(uint32_t acc, __nv_bfloat16* turned
         float x = __uint_as_float(v[i]);
         if (a.act == ACT_RELU2) x = fmaxf(x, 0.f) * fmaxf(x, 0.f);
         turned[i * 32 + lane] = __float2bfloat16(x);
+      }
+      if (!a.by16) {                          // a lane's own column
+        for (int i = 0; i < 16; ++i)
+          if (c + i < rows && lane < cols) out[(long)(c + i) * a.ldc + lane] = turned[i * 32 + lane];
+        continue;
       }
       __syncwarp();
 #pragma unroll
