@@ -46,6 +46,15 @@ def test_wide_attention_growing_maxima():
         assert (out.double() - ref).norm() <= 2 ** -8 * ref.norm()
 
 
+def test_wide_attention_of_shared_keys():
+    """Two batch entries with the same keys and values (a batch stride of zero)."""
+    g = torch.Generator(device="cuda").manual_seed(6)
+    q, k, v = (torch.randn(n, 264, 384, device="cuda", generator=g).bfloat16() for n in (2, 1, 1))
+    out = C.wide_head_attention(q, k.expand(2, -1, -1), v.expand(2, -1, -1))
+    nv.check_status(q.device)
+    assert torch.equal(out, C.wide_head_attention(q, k.repeat(2, 1, 1), v.repeat(2, 1, 1)))
+
+
 @pytest.mark.parametrize("workers", [0, 1, 5])
 def test_scores_of_minus_infinity(workers):
     """Rows whose first keys score -inf (products past the range of fp32) beside rows of the same warp whose maxima grow: those keys weigh nothing."""
