@@ -55,6 +55,17 @@ def test_segments(segs, H, Hkv, D):
     assert (out[:2] == 7).all() and (out[at:] == 7).all()
 
 
+@pytest.mark.parametrize("lengths,launches", [([5] * 8, 1), ([5] * 9, 2), ([300] * 19, 3), ([64000], 1), ([65536], 1), ([65537], 2), ([0] * 9, 0)])
+def test_launches_are_counted(lengths, launches):
+    T = max(1, sum(lengths))
+    q = torch.zeros(T, 1, 64, device="cuda", dtype=torch.bfloat16)
+    segs = [(sum(lengths[:i]), n, 0, None) for i, n in enumerate(lengths)]
+    before = nv.launch_count
+    KC.prefill_segments(q, q, q, None, None, segs, out=torch.empty_like(q))
+    assert nv.launch_count - before == launches
+    nv.check_status(q.device)
+
+
 @pytest.mark.parametrize("n,H,Hkv", [(1, 8, 2), (5, 32, 4), (3, 16, 1)])
 def test_decode_on_rows_of_a_step(n, H, Hkv):
     g = torch.Generator(device="cuda").manual_seed(n)

@@ -46,6 +46,14 @@ def test_wide_attention_growing_maxima():
         assert (out.double() - ref).norm() <= 2 ** -8 * ref.norm()
 
 
+@pytest.mark.parametrize("N,workers,launches", [(256, 1, 1), (512, 2, 1), (512, 3, 2), (300, 2, 1), (300, 6, 2)])
+def test_launches_are_counted(N, workers, launches):
+    q = torch.zeros(1, N, 384, device="cuda", dtype=torch.bfloat16)
+    before = nv.launch_count
+    C._wide_head_flash(q, q, q, 1.0, workers)
+    assert nv.launch_count - before == launches
+
+
 def test_wide_attention_of_shared_keys():
     """Two batch entries with the same keys and values (a batch stride of zero)."""
     g = torch.Generator(device="cuda").manual_seed(6)

@@ -27,6 +27,12 @@ launch_count = 0
 _timing: list | None = None      # (entry point, start event, stop event) while kernel timing is on
 
 
+def count_launches(n: int) -> None:
+    """Launches of a call beyond those its entry point stands for."""
+    global launch_count
+    launch_count += n
+
+
 def enable_kernel_timing(on: bool = True) -> None:
     """Bracket every native launch with CUDA events; read the result with ``kernel_timing_summary``."""
     global _timing

@@ -358,6 +358,8 @@ def _wide_head_flash(q, k, v, scale, workers: int = 0):
     ops = [a for t in (q, k, v, out) for a in (nv.ptr(t), c_long(t.stride(1)), c_long(t.stride(0) if B > 1 else N * t.stride(1)))]
     nv.check_rc(lib.omni_attn_wide(*ops, c_int(B), c_int(N), c_int(C), ctypes.c_float(scale), c_int(workers), nv.ptr(scratch),
                                    nv.ptr(nv.status_word(q.device)), nv.stream_ptr()), "omni_attn_wide")
+    if workers != B * (-(-N // 256)):                    # tiles that pairs share are merged
+        nv.count_launches(1)
     return out
 
 

@@ -204,6 +204,9 @@ def prefill_segments(q, k, v, k_cache, v_cache, segs, scale=None, out=None):
         c_int(H), c_int(Hkv), c_int(D), c_int(n), ints(0), ints(1), ints(2), (ctypes.c_void_p * n)(*(0 if t is None else t.data_ptr() for t in tables)),
         c_float(scale if scale is not None else 1.0 / math.sqrt(D)), nv.ptr(nv.status_word(q.device)), nv.stream_ptr())
     nv.check_rc(rc, "omni_attn_prefill_segs")
+    if n > 8 or T > 248 * 256:                               # more than eight segments or 256 blocks of 256 rows
+        blocks = [sum(-(-s[1] // 256) for s in segs[i:i + 8]) for i in range(0, n, 8)]
+        nv.count_launches(sum(-(-b // 256) for b in blocks) - 1)
     return out
 
 
