@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import torch
 from torch import nn
+from torch.nn.modules.module import _has_any_global_hook
 
 from ...ops import gemm
 
@@ -50,8 +51,10 @@ class FusedLinear(nn.Module):
         return y
 
     def swiglu(self, x):
-        """silu(first half) * second half of the layer's outputs."""
-        if self.fp8 is None and not self.lora and self.bias is None:
+        """silu(first half) * second half of the layer's outputs, which exist as such only where something else needs them: adapters, fp8 weights, a bias,
+        hooks, a forward of one's own."""
+        hooked = self._forward_hooks or self._forward_pre_hooks or self._backward_hooks or self._backward_pre_hooks or _has_any_global_hook()
+        if self.fp8 is None and not self.lora and self.bias is None and not hooked and getattr(self.forward, "__func__", None) is FusedLinear.forward:
             return gemm.linear_swiglu(x, self.weight)
         from ...ops import fused
         return fused.silu_mul(self(x))
