@@ -2,11 +2,12 @@
 //
 //   C[M,N] (bf16) = epilogue( A[M,K] (bf16, row-major) * W[N,K]^T (bf16, row-major) )
 //
-// i.e. the nn.Linear contraction with both operands K-major.  Two kernels share one epilogue:
+// i.e. the nn.Linear contraction with both operands K-major.  Three kernels:
 //
-// gemm_bf16_kernel<BN>       one CTA per SM walks a strided list of 128 x BN output tiles
-//                            (BN = 128 / 192 / 256).  Also runs the expert GEMM over padded segments, where
-//                            every 128-row tile names its expert, and the implicit-GEMM convolution,
+// gemm_bf16_multi_kernel<BN> one CTA per SM walks a strided list of 128 x BN output tiles
+//                            (BN = 128 / 192 / 256) of one linear layer or of two of the same (N, K).
+// gemm_bf16_kernel<BN>       the same tiles of the expert GEMM over padded segments, where
+//                            every 128-row tile names its expert, and of the implicit-GEMM convolution,
 //                            where the A tile of a (tap, channel block) is a shifted 4-D TMA box.
 // gemm_bf16_pair_kernel<TN>  two CTAs of a cluster (cta_group::2) compute one 256 x TN tile; each
 //                            stages its own 128 rows of A and half of the W tile, the even CTA issues
@@ -17,7 +18,7 @@
 // convolutions on CTA pairs (conv_pair.cuh) and the GEMM of all experts over rows that sit back to
 // back (moe_gemm.cuh).
 //
-// Roles inside a CTA (both kernels):
+// Roles inside a CTA (all three):
 //   warp 0    TMA producer: cp.async.bulk.tensor loads of the A / W k-blocks (128-byte
 //             swizzle) into a multi-stage shared-memory ring, completion on mbarriers
 //   warp 1    MMA issuer: one elected thread issues tcgen05.mma (K=16 per instruction) with
@@ -357,7 +358,7 @@ template <int BN>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  __nv_bfloat16* __restrict__ C, int ldc, int M, int N, int K, GemmEpilogue epi,
-                 const int* tile_expert, ConvGeom conv, PeerSignal sig, PeerWait wt, int* status) {
+                 const int* tile_expert, ConvGeom conv, int* status) {
   using Cfg = GemmCfg<BN>;
   constexpr int STAGES = Cfg::STAGES;
 
@@ -407,7 +408,6 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
-      peer_wait_arrivals(wt, &s_abort, status);   // A may hold rows that peers write (fused exchange)
       for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
         int mb, nb;
         tile_coords(t, num_m, num_n, mb, nb);
@@ -479,7 +479,6 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     const int q = warp & 3;         // TMEM lane quadrant this warp may read
     const int half = (warp - 2) >> 2;  // which half of the tile's columns this warp drains
     constexpr int CH_PER_WARP = BN / 64;
-    const bool peer_stores = (epi.scatter_P > 1 || epi.scatter_rows > 0) && conv.taps == 0;
     int acc = 0;
     uint32_t acc_phase = 0;
     for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
@@ -500,35 +499,14 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         row_ok = y < conv.H && x < conv.W;
         row = (img * conv.H + y) * conv.W + x;
       }
-      const __nv_bfloat16* gate_row = nullptr;
-      if (epi.gate && row_ok) gate_row = epi.gate + (size_t)(row / epi.rows_per_batch) * epi.gate_stride;
-      if (peer_stores) {
-        // fused collectives: 64 columns at a time through the staging block
-        const uint32_t stg = smem_base + STAGES * Cfg::STAGE_BYTES + (warp - 2) * EPI_STAGE_BYTES;
 #pragma unroll 1
-        for (int c = half * CH_PER_WARP; c < (half + 1) * CH_PER_WARP; c += 2) {
-          const int col0 = nb * BN + c * 32;
-          if (col0 >= N) break;
-          const int nsub = min(2, (half + 1) * CH_PER_WARP - c);
-          uint4 o[8];
-          for (int sidx = 0; sidx < nsub; ++sidx) {
-            uint32_t v[32];
-            tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + acc * Cfg::ACC_STRIDE + (c + sidx) * 32, v);
-            tmem_wait_ld();
-            if (row_ok) epilogue_math32(v, row, col0 + sidx * 32, N, epi, gate_row, o + sidx * 4);
-          }
-          epilogue_store_staged(stg, o, nsub * 4, lane, mb * BM + q * 32, M, col0, N, C, ldc, epi);
-        }
-      } else {
-#pragma unroll 1
-        for (int c = half * CH_PER_WARP; c < (half + 1) * CH_PER_WARP; ++c) {
-          const int col0 = nb * BN + c * 32;
-          if (col0 >= N) break;
-          uint32_t v[32];
-          tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + acc * Cfg::ACC_STRIDE + c * 32, v);
-          tmem_wait_ld();
-          if (row_ok) epilogue_store32(v, row, col0, N, C, ldc, epi, gate_row);
-        }
+      for (int c = half * CH_PER_WARP; c < (half + 1) * CH_PER_WARP; ++c) {
+        const int col0 = nb * BN + c * 32;
+        if (col0 >= N) break;
+        uint32_t v[32];
+        tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + acc * Cfg::ACC_STRIDE + c * 32, v);
+        tmem_wait_ld();
+        if (row_ok) epilogue_store32(v, row, col0, N, C, ldc, epi, nullptr);
       }
       tc_fence_before_sync();
       __syncwarp();
@@ -540,11 +518,6 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
   tc_fence_before_sync();
   __syncthreads();
-  if (threadIdx.x == 0) {
-    // every peer store of this CTA was issued before the barrier above
-    peer_signal_cta_done(sig, gridDim.x);
-    peer_wait_cta_exit(wt, gridDim.x);
-  }
   if (s_abort) {
     // give copies and MMAs that may still be in flight time to land before TMEM and
     // shared memory are handed back
@@ -1093,10 +1066,10 @@ template <int BN>
 static int launch_gemm(const CUtensorMap& tmA, const void* W, __nv_bfloat16* C, int ldc, int M,
                        int N, int K, int ldw, const GemmEpilogue& epi, int* status, int max_ctas,
                        cudaStream_t stream, int num_experts = 1, const int* tile_expert = nullptr,
-                       const ConvGeom* conv = nullptr, const OmniSync* sync = nullptr) {
+                       const ConvGeom* conv = nullptr) {
   using Cfg = GemmCfg<BN>;
   CUtensorMap tmB;
-  // weights as [E, N, K]; a plain linear layer is E = 1
+  // weights as [E, N, K]; a convolution is E = 1
   int rc = make_tmap_3d(&tmB, W, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (uint64_t)K, (uint64_t)N,
                         (uint64_t)num_experts, (uint64_t)ldw * 2, (uint64_t)N * ldw * 2, BK, BN);
   if (rc) return rc;
@@ -1106,11 +1079,7 @@ static int launch_gemm(const CUtensorMap& tmA, const void* W, __nv_bfloat16* C, 
   int grid = num_tiles < max_ctas ? num_tiles : max_ctas;
   ConvGeom geom = {};
   if (conv) geom = *conv;
-  PeerSignal sig;
-  PeerWait wt;
-  unpack_sync(sync, sig, wt);
-  launch_with(!sync, 1, gemm_bf16_kernel<BN>, grid, GEMM_THREADS, Cfg::SMEM_BYTES, stream, tmA, tmB, C, ldc, M, N, K, epi, tile_expert, geom, sig,
-              wt, status);
+  launch_overlapped(gemm_bf16_kernel<BN>, grid, GEMM_THREADS, Cfg::SMEM_BYTES, stream, tmA, tmB, C, ldc, M, N, K, epi, tile_expert, geom, status);
   return (int)cudaGetLastError();
 }
 
@@ -1159,6 +1128,21 @@ static TilePlan plan_tiles(const int* Ms, int n_problems, int N, int ctas, int p
     }
   }
   return best;
+}
+
+// force_bn 0: as plan_tiles says; 128, 192, 256: tiles of that width on single CTAs; 384, 448, 576: tiles of 128, 192, 256 columns on CTA pairs; 512: on pairs,
+// as pick_pair_tn says.  False: another number.
+static bool choose_plan(TilePlan& plan, int M, int N, int force_bn, int ctas) {
+  const int pairs = max_resident_pairs();
+  switch (force_bn) {
+    case 0: plan = plan_tiles(&M, 1, N, ctas, g_pair_mode == 1 ? pairs : 0, g_pair_mode == 1); return true;
+    case 128: case 192: case 256: plan = {false, force_bn}; return true;
+    case 384: plan = {true, 128}; return true;
+    case 448: plan = {true, 192}; return true;
+    case 576: plan = {true, 256}; return true;
+    case 512: plan = {true, pick_pair_tn(M, N, pairs)}; return true;
+    default: return false;
+  }
 }
 
 static int pick_bn(int M, int N, int ctas) {
@@ -1243,33 +1227,13 @@ extern "C" int omni_gemm_bf16_coef(const void* A, int lda, const void* W, int ld
       default: break;
     }
   }
-  CUtensorMap tmA;
-  int rc = make_tmap_2d(&tmA, A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)M, (uint64_t)K,
-                        (uint64_t)lda * 2, BM, BK);
-  if (rc) return rc;
-  // force_bn = 576 / 448 / 384 selects the CTA-pair kernel with a 256 / 192 / 128 wide tile on two
-  // SMs, 512 the pair kernel with the launcher's choice of width; in automatic mode the pair kernel takes every
-  // problem with at least one full wave of 256 x 256 tiles
-  TilePlan plan = {false, 0};
-  if (force_bn == 0) plan = plan_tiles(&M, 1, N, ctas, g_pair_mode == 1 ? max_resident_pairs() : 0, g_pair_mode == 1);
-  if (force_bn >= 384 || force_bn == 0) {
-    const int pairs = max_resident_pairs();
-    const bool pair = force_bn || plan.pair;
-    const int tn = force_bn == 576 ? 256 : (force_bn == 448 ? 192 : (force_bn == 384 ? 128 :
-                   (force_bn == 512 ? pick_pair_tn(M, N, pairs) : plan.bn)));
-    PairArgs args = {};
-    args.n_problems = 1; args.N = N; args.K = K;
-    unpack_sync(sync, args.sig, args.wt);
-    rc = fill_pair_problem(args.p[0], A, lda, W, ldw, c, ldc, M, N, K, epi, pair ? tn / 2 : tn);
-    if (rc) return rc;
-    return pair ? launch_pair_tn(tn, args, status, pairs, s) : launch_multi_bn(tn, args, status, ctas, s);
-  }
-  switch (force_bn) {
-    case 256: return launch_gemm<256>(tmA, W, c, ldc, M, N, K, ldw, epi, status, ctas, s, 1, nullptr, nullptr, sync);
-    case 192: return launch_gemm<192>(tmA, W, c, ldc, M, N, K, ldw, epi, status, ctas, s, 1, nullptr, nullptr, sync);
-    case 128: return launch_gemm<128>(tmA, W, c, ldc, M, N, K, ldw, epi, status, ctas, s, 1, nullptr, nullptr, sync);
-    default: return RC_BAD_ARG;
-  }
+  TilePlan plan;
+  if (!choose_plan(plan, M, N, force_bn, ctas)) return RC_BAD_ARG;
+  PairArgs args = {};
+  args.n_problems = 1; args.N = N; args.K = K;
+  unpack_sync(sync, args.sig, args.wt);
+  if (int rc = fill_pair_problem(args.p[0], A, lda, W, ldw, c, ldc, M, N, K, epi, plan.pair ? plan.bn / 2 : plan.bn)) return rc;
+  return plan.pair ? launch_pair_tn(plan.bn, args, status, max_resident_pairs(), s) : launch_multi_bn(plan.bn, args, status, ctas, s);
 }
 
 extern "C" int omni_gemm_bf16_sync(const void* A, int lda, const void* W, int ldw, void* C, int ldc,
@@ -1426,8 +1390,9 @@ extern "C" int omni_gemm_bf16_dual(const OmniGemmDesc* d0, const OmniGemmDesc* d
 }
 
 // C[M, F] = silu(A gate^T) * (A lift^T), W [2 F, K] with the F gate rows first; F and K multiples of 8.  -5: these rows are faster as two launches (17 to 128
-// rows that gemm_skinny_kernel takes).
-extern "C" int omni_gemm_bf16_swiglu(const void* A, int lda, const void* W, int ldw, void* C, int ldc, int M, int F, int K, int* status, void* stream) {
+// rows that gemm_skinny_kernel takes).  force_bn as for the other linear layers.
+extern "C" int omni_gemm_bf16_swiglu(const void* A, int lda, const void* W, int ldw, void* C, int ldc, int M, int F, int K, int force_bn, int* status,
+                                     void* stream) {
   using namespace omni;
   if (M <= 0 || F <= 0 || K <= 0) return RC_OK;
   if ((K & 7) || (F & 7) || (lda & 7) || (ldw & 7) || (ldc & 7)) return RC_BAD_ARG;
@@ -1435,16 +1400,17 @@ extern "C" int omni_gemm_bf16_swiglu(const void* A, int lda, const void* W, int 
   GemmEpilogue epi = {};
   epi.rows_per_batch = 1;
   epi.act = EPI_SWIGLU;
-  const FewRows few = few_rows(M, 2 * F, K);
+  const FewRows few = force_bn ? FewRows::no : few_rows(M, 2 * F, K);
   if (few == FewRows::skinny) return -5;
   if (few == FewRows::rows) return launch_rows(A, lda, W, ldw, static_cast<__nv_bfloat16*>(C), ldc, M, 2 * F, K, epi, s);
-  const int N = 2 * F, ctas = sm_count(), pairs = max_resident_pairs();
-  const TilePlan plan = plan_tiles(&M, 1, N, ctas, g_pair_mode == 1 ? pairs : 0, g_pair_mode == 1);
+  const int N = 2 * F, ctas = sm_count();
+  TilePlan plan;
+  if (!choose_plan(plan, M, N, force_bn, ctas)) return RC_BAD_ARG;
   PairArgs args = {};
   args.n_problems = 1; args.N = N; args.K = K;
   unpack_sync(nullptr, args.sig, args.wt);
   if (int rc = fill_pair_problem(args.p[0], A, lda, W, ldw, static_cast<__nv_bfloat16*>(C), ldc, M, N, K, epi, plan.pair ? plan.bn / 2 : plan.bn)) return rc;
-  return plan.pair ? launch_pair_tn(plan.bn, args, status, pairs, s) : launch_multi_bn(plan.bn, args, status, ctas, s);
+  return plan.pair ? launch_pair_tn(plan.bn, args, status, max_resident_pairs(), s) : launch_multi_bn(plan.bn, args, status, ctas, s);
 }
 
 // 0: the CTA-pair kernel runs only when forced (force_bn = 512); 1: automatic for large problems.

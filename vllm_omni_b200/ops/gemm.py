@@ -144,7 +144,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None, a
     return None if to_peers else out
 
 
-def linear_swiglu(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+def linear_swiglu(x: torch.Tensor, w: torch.Tensor, force_bn: int = 0) -> torch.Tensor:
     """silu(x @ gate.T) * (x @ lift.T) with w = [gate | lift] rows: on a GPU in one launch (the product of both never reaches memory, and neither half is
     rounded before they meet), for rows that the few-row kernels split over clusters in two."""
     from .fused import silu_mul
@@ -157,7 +157,7 @@ def linear_swiglu(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
             x2 = x2.contiguous()
         out = torch.empty(*x.shape[:-1], F_, dtype=x.dtype, device=x.device)
         rc = nv.lib("gemm_sm100").omni_gemm_bf16_swiglu(nv.ptr(x2), ctypes.c_int(x2.stride(0)), nv.ptr(w), ctypes.c_int(w.stride(0)), nv.ptr(out),
-                                                        ctypes.c_int(F_), ctypes.c_int(x2.shape[0]), ctypes.c_int(F_), ctypes.c_int(K),
+                                                        ctypes.c_int(F_), ctypes.c_int(x2.shape[0]), ctypes.c_int(F_), ctypes.c_int(K), ctypes.c_int(force_bn),
                                                         nv.ptr(nv.status_word(x.device)), nv.stream_ptr())
         if rc != -5:
             nv.check_rc(rc, "omni_gemm_bf16_swiglu")
