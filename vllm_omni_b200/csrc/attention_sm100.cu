@@ -122,12 +122,6 @@ struct AttnSegs {
   unsigned short order[MAX_BLOCKS];   // segment << 12 | query block
 };
 
-__device__ __forceinline__ float ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
 // 2^x for a pair, on the FMA and integer pipes: n = round(x), r = x - n in [-0.5, 0.5],
 // 2^r by a degree-3 polynomial (relative error 7.5e-5, far inside bf16's 2^-9), and n added
 // into the exponent field.  x is clamped at -126 so the exponent cannot wrap.
@@ -435,7 +429,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       if (j == 0) {
         m = m_new;
       } else if (__any_sync(0xffffffffu, grow)) {
-        const float alpha = ex2(m - m_new);
+        const float alpha = ex2_approx(m - m_new);
         const uint64_t alpha2 = pack2(alpha, alpha);
         l2a = mul2(l2a, alpha2);
         l2b = mul2(l2b, alpha2);
@@ -469,8 +463,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             unpack2(p2, p0, p1);
           } else {
             unpack2(x2, p0, p1);
-            p0 = ex2(p0);
-            p1 = ex2(p1);
+            p0 = ex2_approx(p0);
+            p1 = ex2_approx(p1);
             p2 = pack2(p0, p1);
           }
           if (e & 2) l2b = add2(l2b, p2); else l2a = add2(l2a, p2);

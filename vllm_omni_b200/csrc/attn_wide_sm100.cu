@@ -37,18 +37,6 @@ struct WideAttn {
 // worker w has the units [wide_start(w), wide_start(w + 1)) of tiles * steps
 __device__ __forceinline__ int wide_start(const WideAttn& a, int w) { return (int)((long)w * a.tiles * a.steps / a.workers); }
 
-__device__ __forceinline__ float wide_ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
-__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap* tmap, uint32_t cluster_bar, int c0, int c1, int c2) {
-  asm volatile("cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-               :
-               : "r"(dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(cluster_bar), "r"(c0), "r"(c1), "r"(c2)
-               : "memory");
-}
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(AW_THREADS, 1)
 wide_attn_kernel(const __grid_constant__ WideAttn a, int* status) {
   extern __shared__ uint8_t smem_raw[];
@@ -261,7 +249,7 @@ wide_attn_kernel(const __grid_constant__ WideAttn a, int* status) {
       const bool grow = __any_sync(0xffffffffu, m_new > m + 8.0f) && !first;
       float alpha = 1.f;
       if (grow) {
-        alpha = m_new == -INFINITY ? 1.f : wide_ex2(m - m_new);      // a row of -inf scores so far beside one that grows
+        alpha = m_new == -INFINITY ? 1.f : ex2_approx(m - m_new);      // a row of -inf scores so far beside one that grows
         la = mul2(la, pack2(alpha, alpha));
         lb = mul2(lb, pack2(alpha, alpha));
       }
@@ -273,8 +261,8 @@ wide_attn_kernel(const __grid_constant__ WideAttn a, int* status) {
         for (int e = 0; e < 32; e += 2) {
           float p0, p1;
           unpack2(fma2(pack2(__uint_as_float(v[e]), __uint_as_float(v[e + 1])), scale2, negm2), p0, p1);
-          p0 = wide_ex2(p0);
-          p1 = wide_ex2(p1);
+          p0 = ex2_approx(p0);
+          p1 = ex2_approx(p1);
           if (e & 2) lb = add2(lb, pack2(p0, p1)); else la = add2(la, pack2(p0, p1));
           v[e >> 1] = pack_bf16(p0, p1);
         }
@@ -392,7 +380,7 @@ wide_attn_merge_kernel(const __grid_constant__ WideAttn a) {
   for (int p = w; wide_start(a, p) < end && p < a.workers; ++p) {
     const long slot = slot_of(p);
     const float2 ml = a.part_ml[slot * 128 + row];
-    const float s = ml.x == -INFINITY ? 0.f : wide_ex2(ml.x - M);
+    const float s = ml.x == -INFINITY ? 0.f : ex2_approx(ml.x - M);
     l = fmaf(ml.y, s, l);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -447,7 +435,8 @@ extern "C" int omni_attn_wide_workers(int B, int N, long* scratch_floats) {
 }
 
 // out[b, r, :] = softmax(scale q[b, r] k[b]^T) v[b] for one head of 384 channels; q, k, v, out bf16 [B, N, 384] with row and batch strides in elements
-// (multiples of 8) and contiguous channels, bases on 16 bytes.  workers 0: as omni_attn_wide_workers says; scratch as it says.
+// (multiples of 8) and contiguous channels, bases on 16 bytes.  workers: what omni_attn_wide_workers says, or any other number of pairs; scratch (may be null where
+// no tile is shared): 4 * 128 * (384 + 2) floats for each.
 extern "C" int omni_attn_wide(const void* q, long q_rs, long q_bs, const void* k, long k_rs, long k_bs, const void* v, long v_rs, long v_bs, void* out,
                               long o_rs, long o_bs, int B, int N, int C, float scale, int workers, float* scratch, int* status, void* stream) {
   using namespace omni;
@@ -465,8 +454,8 @@ extern "C" int omni_attn_wide(const void* q, long q_rs, long q_bs, const void* k
   const long tiles = (long)B * a.tiles_per;
   if (tiles * a.steps > 0x3fffffffL) return RC_TOO_LARGE;
   a.tiles = (int)tiles;
-  a.workers = workers > 0 ? workers : wide_workers(tiles, a.steps, sm_count() / 2);
-  if (a.workers > tiles * a.steps) return RC_BAD_ARG;
+  if (workers < 1 || workers > tiles * a.steps) return RC_BAD_ARG;
+  a.workers = workers;
   a.scale_log2 = scale * 1.4426950408889634f;
   const bool shared = a.workers != a.tiles;
   if (shared && (scratch == nullptr || (reinterpret_cast<uintptr_t>(scratch) & 15))) return RC_BAD_ARG;

@@ -50,11 +50,6 @@ struct WinPrefill {
   int tab_stride;       // floats between the bias rows of two heads
 };
 
-__device__ __forceinline__ float wp_ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
 __device__ __forceinline__ float wp_rcp(float x) {
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -75,7 +70,7 @@ __device__ __forceinline__ uint32_t bit_range(int a, int b) {
 }
 
 // sigmoid of a gate logit
-__device__ __forceinline__ float wp_open(float z) { return wp_rcp(1.0f + wp_ex2(-WP_LOG2E * z)); }
+__device__ __forceinline__ float wp_open(float z) { return wp_rcp(1.0f + ex2_approx(-WP_LOG2E * z)); }
 
 // 16 channels of a row, times f, channel by channel times the opening of their logits z where `gated`
 __device__ __forceinline__ void wp_store16(__nv_bfloat16* dst, const float (&v)[16], float f, bool gated, const uint4 (&z)[2]) {
@@ -333,7 +328,7 @@ attn_window_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid
     float b_const = CAP ? C : 0.f;               // what a score without bias is relative to
     if (BOUNDED) {
       const float ref = fmaxf(C, m);
-      l2a = p.sink ? pack2(wp_ex2(m - ref), 0.f) : 0ull;
+      l2a = p.sink ? pack2(ex2_approx(m - ref), 0.f) : 0ull;
       m = ref;
       b_const = C - ref;
     }
@@ -379,7 +374,7 @@ attn_window_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid
           if (CAP) {
             // cap tanh(s / cap) = C - 2C / (1 + 2^y); the pair shares one reciprocal, and |y| <= 60 keeps the
             // product of the two denominators finite (there the bound is reached to the last bit)
-            const uint64_t e2 = pack2(wp_ex2(fminf(y0, 60.f)), wp_ex2(fminf(y1, 60.f)));
+            const uint64_t e2 = pack2(ex2_approx(fminf(y0, 60.f)), ex2_approx(fminf(y1, 60.f)));
             float a0, a1;
             unpack2(add2(e2, pack2(1.f, 1.f)), a0, a1);
             const float k = neg2C * wp_rcp(a0 * a1);
@@ -420,8 +415,8 @@ attn_window_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid
           if (!BOUNDED) x2 = add2(x2, negm2);
           float e0, e1;
           unpack2(x2, e0, e1);
-          e0 = wp_ex2(e0);
-          e1 = wp_ex2(e1);
+          e0 = ex2_approx(e0);
+          e1 = ex2_approx(e1);
           const uint64_t p2 = pack2(e0, e1);
           if (e & 2) l2b = add2(l2b, p2); else l2a = add2(l2a, p2);
           pk[e >> 1] = pack_bf16(e0, e1);
@@ -457,11 +452,11 @@ attn_window_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid
       table_done();
       const float m_new = fmaxf(m, fmaxf(fmaxf(ma, mb), fmaxf(mc, md)));
       if (j == 0) {
-        if (m != -INFINITY) l2a = pack2(wp_ex2(m - m_new), 0.f);          // the sink's share so far
+        if (m != -INFINITY) l2a = pack2(ex2_approx(m - m_new), 0.f);          // the sink's share so far
         m = m_new;
       } else if (__any_sync(0xffffffffu, m_new > m + 8.0f)) {
         // rare: O follows the new reference; the scores wait in their own TMEM columns meanwhile
-        const float alpha = m_new == -INFINITY ? 1.f : wp_ex2(m - m_new);
+        const float alpha = m_new == -INFINITY ? 1.f : ex2_approx(m - m_new);
         l2a = mul2(l2a, pack2(alpha, alpha));
         l2b = mul2(l2b, pack2(alpha, alpha));
         tmem_st_32x32(tS, v0);

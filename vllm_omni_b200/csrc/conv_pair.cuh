@@ -56,12 +56,6 @@ struct Conv3Args {
   GemmEpilogue epi;
 };
 
-__device__ __forceinline__ void add8(float (&f)[8], const uint4& u) {
-  const float2 a = unpack_bf16(u.x), b = unpack_bf16(u.y), c = unpack_bf16(u.z), d = unpack_bf16(u.w);
-  f[0] += a.x; f[1] += a.y; f[2] += b.x; f[3] += b.y;
-  f[4] += c.x; f[5] += c.y; f[6] += d.x; f[7] += d.y;
-}
-
 // not inlined: few convolutions have one, and its code would crowd the instruction cache
 __device__ __noinline__ float conv3_act(float x, int act) {
   if (act == ACT_GELU_TANH) return gelu_tanh(x);
@@ -69,7 +63,7 @@ __device__ __noinline__ float conv3_act(float x, int act) {
   return act == ACT_RELU2 ? fmaxf(x, 0.f) * fmaxf(x, 0.f) : x;
 }
 __device__ __forceinline__ void conv3_finish(float (&f)[8], const GemmEpilogue& epi, int col) {
-  if (epi.bias) add8(f, *reinterpret_cast<const uint4*>(epi.bias + col));
+  if (epi.bias) add_bf16x8(f, *reinterpret_cast<const uint4*>(epi.bias + col));
   if (epi.act != ACT_NONE) {
     f[0] = conv3_act(f[0], epi.act); f[1] = conv3_act(f[1], epi.act); f[2] = conv3_act(f[2], epi.act); f[3] = conv3_act(f[3], epi.act);
     f[4] = conv3_act(f[4], epi.act); f[5] = conv3_act(f[5], epi.act); f[6] = conv3_act(f[6], epi.act); f[7] = conv3_act(f[7], epi.act);
@@ -307,7 +301,7 @@ conv3x3_pair_kernel(const __grid_constant__ Conv3Args a, int* status) {
 #pragma unroll
           for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(v[c * 8 + e]);
           conv3_finish(f, a.epi, col);
-          if (a.epi.residual) add8(f, lds128(at(buf, in_tile)));
+          if (a.epi.residual) add_bf16x8(f, lds128(at(buf, in_tile)));
           const uint4 w = make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
           sts128(at(buf, in_tile), w);
           if (norm) {                                       // of the rounded values

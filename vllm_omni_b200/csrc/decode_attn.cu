@@ -21,12 +21,6 @@ namespace omni {
 
 constexpr int DA_D = 128, DA_WARPS = 4, DA_KEYS = 16;
 
-__device__ __forceinline__ float da_ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
 struct DecodeAttn {
   const __nv_bfloat16 *q, *k, *v;
   long q_rs;
@@ -167,11 +161,11 @@ paged_decode_kernel(const __grid_constant__ DecodeAttn p) {
       mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
       m[u] = fmaxf(m[u], mx);
       const float top = m[u] == -INFINITY ? 0.f : m[u];        // only scores of -inf so far: all weights are zero
-      const float alpha = da_ex2(before - top);
+      const float alpha = ex2_approx(before - top);
       l[u] *= alpha;
 #pragma unroll
       for (int n = 0; n < 2; ++n) {
-        const float e0 = da_ex2(s[n][2 * u] - top), e1 = da_ex2(s[n][2 * u + 1] - top);
+        const float e0 = ex2_approx(s[n][2 * u] - top), e1 = ex2_approx(s[n][2 * u + 1] - top);
         l[u] += e0 + e1;
         pw[u][n] = pack_bf16(e0, e1);
       }
@@ -248,7 +242,7 @@ paged_decode_merge_kernel(const float* part_o, const float* part_ml, int parts, 
   float top = fmaxf(a.x, b.x);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-  const float wa = a.x == -INFINITY ? 0.f : da_ex2(a.x - top), wb = b.x == -INFINITY ? 0.f : da_ex2(b.x - top);
+  const float wa = a.x == -INFINITY ? 0.f : ex2_approx(a.x - top), wb = b.x == -INFINITY ? 0.f : ex2_approx(b.x - top);
   float den = a.y * wa + b.y * wb;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) den += __shfl_xor_sync(0xffffffffu, den, o);

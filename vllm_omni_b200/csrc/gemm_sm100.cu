@@ -142,11 +142,6 @@ __device__ __forceinline__ __nv_bfloat16* epilogue_dest(int row, int col0, __nv_
   return cbase + (size_t)row * ldc + dcol;
 }
 
-__device__ __forceinline__ float ex2_approx(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
 // c0 z^2 + z / 2 above zero, c1 (e^z - 1 - z) + z / 2 below; near zero, where e^z - 1 - z would cancel, the first terms of its
 // series (the next one is below 1e-5 of the result)
 __device__ __forceinline__ float xielu(float z, float c0, float c1) {

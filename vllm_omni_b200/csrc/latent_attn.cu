@@ -250,11 +250,6 @@ struct LatentDecode {
 constexpr int LD_KEYS = 32, LD_ROWS = 16, LD_MAX_STAGES = 8;
 constexpr float LD_LOG2E = 1.4426950408889634f;
 
-__device__ __forceinline__ float ld_ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
 // contiguous bytes to shared memory, counted on an mbarrier (both addresses and the size: multiples of 16)
 __device__ __forceinline__ void ld_bulk(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes),
@@ -409,9 +404,9 @@ latent_decode_kernel(const LatentDecode p, const int stages) {
 #pragma unroll
         for (int o = 8; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         const float m_new = fmaxf(m_run, mx);                // finite: a tile holds at least one visible key
-        const float alpha = ld_ex2(m_run - m_new);
-        y.x = ld_ex2(y.x - m_new);
-        y.y = ld_ex2(y.y - m_new);
+        const float alpha = ex2_approx(m_run - m_new);
+        y.x = ex2_approx(y.x - m_new);
+        y.y = ex2_approx(y.y - m_new);
         l_run = fmaf(l_run, alpha, y.x + y.y);               // this thread's keys only; summed at the end
         m_run = m_new;
         if ((gt & 15) == 0) s_alpha[grp][srow] = alpha;
@@ -490,8 +485,8 @@ latent_decode_kernel(const LatentDecode p, const int stages) {
     if (!WIDE) {                                             // group 0 has a tile wherever group 1 has one
       const float m1 = s_m[1][r];
       const float top = fmaxf(m, m1);
-      f0 = m == -INFINITY ? 0.f : ld_ex2(m - top);
-      f1 = m1 == -INFINITY ? 0.f : ld_ex2(m1 - top);
+      f0 = m == -INFINITY ? 0.f : ex2_approx(m - top);
+      f1 = m1 == -INFINITY ? 0.f : ex2_approx(m1 - top);
       l = l * f0 + s_l[1][r] * f1;
       m = top;
     }
@@ -531,7 +526,7 @@ latent_merge_kernel(const LatentDecode p) {
   float den = 0.f;
   for (int s = 0; s < p.splits; ++s) {
     const float ms = p.part_ml[2 * (base + s)];
-    den += ms == -INFINITY ? 0.f : p.part_ml[2 * (base + s) + 1] * ld_ex2(ms - top);
+    den += ms == -INFINITY ? 0.f : p.part_ml[2 * (base + s) + 1] * ex2_approx(ms - top);
   }
   const float f = 1.0f / den;
   for (int c = threadIdx.x * 4; c < p.rank_p; c += 512) {
@@ -539,7 +534,7 @@ latent_merge_kernel(const LatentDecode p) {
     for (int s = 0; s < p.splits; ++s) {
       const float ms = p.part_ml[2 * (base + s)];
       if (ms == -INFINITY) continue;
-      const float a = ld_ex2(ms - top) * f;
+      const float a = ex2_approx(ms - top) * f;
       const float4 v = *reinterpret_cast<const float4*>(p.part_o + (base + s) * p.rank_p + c);
       o.x = fmaf(v.x, a, o.x); o.y = fmaf(v.y, a, o.y); o.z = fmaf(v.z, a, o.z); o.w = fmaf(v.w, a, o.w);
     }
