@@ -110,7 +110,8 @@ struct AttnPaging {
 
 // Prompt segments of one step: causal attention of every segment's own rows against its own keys, which are rows of the projections where nothing came
 // before them and pages otherwise.  A block of the grid is one head (x) of one query block (y), the query blocks with the most keys first: in the order of the
-// rows the longest ones run last, and the chip waits for them (one prompt of 8192 tokens, 32 heads: MEASURE).
+// rows the longest ones run last, and the chip waits for them (32 heads, us, in the order of the rows in brackets: one prompt of 8192 tokens 453 (496), of 2048
+// 50 (60), two of 4096 259 (283), three of 1414, 705 and 333 48 (48)).
 struct NoSegs {};
 struct AttnSegs {
   static constexpr int MAX = 8, MAX_BLOCKS = 256;

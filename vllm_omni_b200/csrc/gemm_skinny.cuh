@@ -391,7 +391,8 @@ static int launch_skinny_mt(const CUtensorMap& tmW, const void* A, int lda, __nv
 //                    (37.3), 16 rows 16384 x 3584 28.3 (33.9), 16384 x 4096 31.5 (28.7), 13824 x 4096 24.4 (25.7), 12288 x 12288 1.05 times
 //                    as long, 8192 x 4096 18.1 (20.5).  Up to 8 rows the products are half as many and it pays at any length.
 //   17 to 24         gemm_rows_kernel up to 5 blocks per SM and contractions of 4096, or a block per SM and 9216: 17 rows 4096 x 12288 22.4 (20.6), 32768 x 2048
-//                    30.8 (29.6)
+//                    30.8 (29.6).  Which rows these are: steps that are not replayed from a captured batch (mixed ones, contexts past the captured tables),
+//                    since captured batches have 16 or 32 rows and a vocabulary is wider than that
 //   17 to 32         else up to as many tiles as SMs: 17 rows 10240 x 2048 12.5 (17.1), 12288 x 1024 8.0 (11.6), 32 rows 18432 x 2048 15.4 (16.7)
 //   33 to 64         up to half as many; above, the general kernels stream W as fast and read A less often: 64 rows 9216 x 2048 12.7 (13.8),
 //                    10240 x 2048 14.4 (13.2)

@@ -1,8 +1,9 @@
 // Expert GEMMs over rows that sit back to back (mixture of experts, more than a few tokens):  C[r, n] = act(sum_k A[r, k] W[e(r), n, k]).
 //
 // The weights are the M side of the MMA (128 rows of W) and a tile's rows of A its N side, because experts get any number of rows: the N of an
-// MMA goes in steps of 16 (154 rows cost 160, not the 256 of two 128-row tiles), every weight is fetched once per tile of up to 256 rows, and a
-// tile of few rows leaves the shared memory to the weights' ring.  XR (64, 128 or 256) is the most rows a tile may have.
+// MMA goes in steps of 16, or of 32 on CTA pairs (154 rows cost 160, not the 256 of two 128-row tiles), every weight is fetched once per tile of up to
+// 256 rows, and a tile of few rows leaves the shared memory to the weights' ring.  XR is the most rows a tile may have: 64 or 128 on single CTAs
+// (expert_gemm_kernel), 256 on pairs (expert_pair_kernel).
 // GATED: W [E, 2 N, K] holds gate and lift rows; one 5-D box brings 8 gate rows, their 8 lift rows, the next 8 gate rows and so on, so that both
 // values of an output lie 8 lanes apart in a warp and silu(gate) * lift leaves the accumulators without passing through memory.
 // 128 experts, 2048 -> 2 x 768 -> 2048, top 8, whole layer on cold caches: 64 tokens 200 us (two grouped launches of 128-row tiles around a SwiGLU

@@ -211,7 +211,8 @@ def prefill_segments(q, k, v, k_cache, v_cache, segs, scale=None, out=None):
 
 
 def paged_prefill(q, k_cache, v_cache, block_table, kv_len: int, scale=None, out=None):
-    """Causal attention of the LAST ``T`` tokens of one sequence against its whole paged context.
+    """Causal attention of the LAST ``T`` tokens of one sequence against its whole paged context (a decoder's step takes all of its portions through
+    ``prefill_segments``).
 
     q: [T, H, D]; block_table: int32 [max_blocks]; kv_len: tokens in the cache including these T
     (their K/V already written).  Query row i sees keys [0, kv_len - T + i]."""
