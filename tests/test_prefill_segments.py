@@ -66,6 +66,30 @@ def test_launches_are_counted(lengths, launches):
     nv.check_status(q.device)
 
 
+# Rows 192 to 199 of the first prompt share a warp with the second one's, whose scores against the first one's keys then grow in the second key tile only
+@pytest.mark.parametrize("context", [0, 130])
+@pytest.mark.parametrize("D", [64, 128])
+def test_results_do_not_depend_on_the_next_segment(context, D):
+    if context and D == 64:
+        pytest.skip("pages have 128 channels")
+    g = torch.Generator(device="cuda").manual_seed(D)
+    n, H = 200, 8
+    q, k, v = (torch.randn(n + 60, H, D, device="cuda", generator=g).bfloat16() for _ in range(3))
+    m = -(-(n + context) // PAGE)
+    table = torch.arange(m, dtype=torch.int32, device="cuda")
+    kc, vc = (torch.randn(m, PAGE, H, D, device="cuda", generator=g).bfloat16() for _ in range(2))
+    for cache, x in ((kc, k), (vc, v)):
+        cache.view(-1, H, D)[context:context + n] = x[:n]
+    segs = [(0, n, context, table if context else None), (n, 60, 0, None)]
+    got = []
+    for scale in (0.0, 8.0):
+        q[n:] = scale * k[150]
+        got.append(KC.prefill_segments(q, k, v, kc, vc, segs, out=torch.empty_like(q))[:n])
+    torch.cuda.synchronize()
+    nv.check_status(q.device)
+    assert torch.equal(*got)
+
+
 @pytest.mark.parametrize("n,H,Hkv", [(1, 8, 2), (5, 32, 4), (3, 16, 1)])
 def test_decode_on_rows_of_a_step(n, H, Hkv):
     g = torch.Generator(device="cuda").manual_seed(n)

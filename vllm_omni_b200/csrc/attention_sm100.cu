@@ -373,8 +373,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     uint64_t l2a = 0ull, l2b = 0ull;     // four partial row sums (two packed pairs)
     // A tile that is not in use has no work at all; a warp whose 32 rows all lie past the last
     // query row (decode: a handful of real rows per tile) only keeps the barrier protocol going.
-    // Its rows of S come from zero-filled Q rows, so the stale bits the P*V MMA reads as their P
-    // are zeros, and nothing of those rows is stored.
+    // Its rows of S come from zero-filled Q rows (or the next segment's), so the stale bits the P*V MMA
+    // reads as their P are zeros (or anything), and nothing of those rows is stored.
     const bool tile_used = t < n_qt;
     const bool rows_used = tile_used && (srow - lane) < Sq;
     for (int j = 0; tile_used && j < n_kv; ++j) {
@@ -426,7 +426,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
       const float m_new = fmaxf(m, mx);
       // lazy rescale, decided per warp because tcgen05.ld/st are warp-wide
-      const bool grow = m_new > m + 8.0f;
+      // (rows past a segment are the next one's, not zeros: they may not decide for its last rows)
+      const bool grow = m_new > m + 8.0f && (!SEGS || srow < Sq);
       if (j == 0) {
         m = m_new;
       } else if (__any_sync(0xffffffffu, grow)) {
