@@ -90,6 +90,12 @@ def test_results_do_not_depend_on_the_next_segment(context, D):
     assert torch.equal(*got)
 
 
+def test_steps_past_the_launch_limit_go_segment_by_segment():
+    q = torch.empty(1 << 20, 1, 64, device="cuda", dtype=torch.bfloat16)
+    assert KC.prefill_segments_ok(q, None, [0])
+    assert not KC.prefill_segments_ok(torch.empty((1 << 20) + 1, 1, 64, device="cuda", dtype=torch.bfloat16), None, [0])
+
+
 @pytest.mark.parametrize("n,H,Hkv", [(1, 8, 2), (5, 32, 4), (3, 16, 1)])
 def test_decode_on_rows_of_a_step(n, H, Hkv):
     g = torch.Generator(device="cuda").manual_seed(n)

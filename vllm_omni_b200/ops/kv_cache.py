@@ -180,9 +180,10 @@ def paged_decode(q, k_cache, v_cache, block_tables, seq_lens, scale=None, num_sp
 
 
 def prefill_segments_ok(q, k_cache, contexts) -> bool:
-    """Whether ``prefill_segments`` takes these operands: bf16, head size 64 or 128, and pages of its kind where a segment has a context."""
-    D = q.shape[2]
-    return q.is_cuda and q.dtype == torch.bfloat16 and D in (64, 128) and (not any(contexts) or tma_pages_ok(k_cache.shape[1], D))
+    """Whether ``prefill_segments`` takes these operands: bf16, head size 64 or 128, at most 4096 query blocks of 256 rows, and pages of its kind where a
+    segment has a context."""
+    T, _, D = q.shape
+    return q.is_cuda and q.dtype == torch.bfloat16 and D in (64, 128) and T <= 4096 * 256 and (not any(contexts) or tma_pages_ok(k_cache.shape[1], D))
 
 
 def prefill_segments(q, k, v, k_cache, v_cache, segs, scale=None, out=None):
