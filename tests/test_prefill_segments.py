@@ -114,3 +114,29 @@ def test_decode_on_rows_of_a_step(n, H, Hkv):
     rest = torch.ones(T, dtype=torch.bool, device="cuda")
     rest[rows] = False
     assert (out[rest] == 7).all()
+
+
+# more sequences than one early launch takes, groups of 12 heads, rows from both ends, every length down to one key
+@pytest.mark.parametrize("n,H,Hkv", [(40, 32, 4), (20, 48, 4), (17, 12, 1)])
+def test_many_decoded_rows_of_a_step(n, H, Hkv):
+    g = torch.Generator(device="cuda").manual_seed(n)
+    T, L = 2 * n + 5, 900
+    q = torch.randn(T, H, 128, device="cuda", generator=g).bfloat16()
+    m = -(-L // PAGE)
+    kc, vc = (torch.randn(n * m, PAGE, Hkv, 128, device="cuda", generator=g).bfloat16() for _ in range(2))
+    bt = torch.randperm(n * m, generator=torch.Generator().manual_seed(1)).view(n, m).int().cuda()
+    lens = [max(1, L - i * i * 7) if i % 2 else max(1, 40 - i) for i in range(n)]
+    rows = torch.randperm(T, generator=torch.Generator().manual_seed(2))[:n].cuda()
+    rows[::3] -= T
+    out = torch.full_like(q, 7.0)
+    KC.paged_decode(q, kc, vc, bt, torch.tensor(lens, dtype=torch.int32, device="cuda"), out=out, rows=rows, impl="stream")
+    torch.cuda.synchronize()
+    nv.check_status(q.device)
+    for i in range(n):
+        keys = bt[i].long().repeat_interleave(PAGE)[:lens[i]] * PAGE + torch.arange(lens[i], device="cuda") % PAGE
+        ref = _exact(q[rows[i]][None], kc.view(-1, Hkv, 128)[keys], vc.view(-1, Hkv, 128)[keys], lens[i] - 1)
+        # probabilities and results are bf16
+        assert (out[rows[i]][None].double() - ref).norm() <= 2.0 ** -8 * ref.norm()
+    rest = torch.ones(T, dtype=torch.bool, device="cuda")
+    rest[rows] = False
+    assert (out[rest] == 7).all()
