@@ -273,3 +273,20 @@ def test_single_rows_leave_history_alone():
     layer = Gated(GATED["base"], torch.float32, "cpu")
     d = layer.rows(30, 1)
     compare(run(layer, [d, d], [{0: 20, 1: 1}, {0: 1, 1: 20}, {0: 9, 1: 9}], ("cpu", torch.float32, 0))[1], layer.expected(d), 5e-5)
+
+
+# blocks of the token-by-token kernel against the SMs: at most one for each, two, three and more; states of every number of rows a thread
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 5e-5), (torch.bfloat16, 0.02)])
+@pytest.mark.parametrize("kind,size", [pytest.param(Gated, (8, 4, 32, 48, 3), id="gated4"), pytest.param(Gated, (8, 2, 64, 128, 4), id="gated8"),
+                                       pytest.param(Gated, (8, 8, 128, 128, 2), id="gated16"), pytest.param(Channel, (8, 64), id="channel4"),
+                                       pytest.param(Channel, (8, 96), id="channel12"), pytest.param(Channel, (8, 128), id="channel16")])
+def test_grids_of_steps(kind, size, dtype, tol):
+    mode = ("cuda", dtype, tol)
+    layer = kind(size, dtype, "cuda")
+    data = [layer.rows(4, i % 5) for i in range(70)]
+    want = [layer.expected(d) for d in data[:5]]
+    for n in (18, 19, 37, 38, 70):
+        got = run(layer, data[:n], [{i: 2 + i % 2 for i in range(n)}, {i: 2 - i % 2 for i in range(n)}], mode, impl="steps")
+        for i, g in enumerate(got):
+            compare(g, want[i % 5], tol)

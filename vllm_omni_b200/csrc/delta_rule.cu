@@ -4,12 +4,11 @@
 //                       every n-th key row; per token convolution, unit lengths, decays, both reads of the state, the write,
 //                       norm and gate.  Decoded tokens take exactly one turn (one launch does the whole mixer, and the state
 //                       is read and written once); the exact mode walks whole portions.  States too large for one block are
-//                       cut into column slices, whose results go to `raw`.  One token per sequence is a chain of latencies around 128 KB of
-//                       state per block: what it starts from is fetched before or together.  A decode step of the
-//                       2048-wide decoder with one such mixer of 16 heads of 128 x 128 in four layers: 16 sequences of 3000 tokens 272.3 us, 20
-//                       340.9, 32 347.9, 64 464.4 (taps and channels one after the other, gate and gain at the end, new history in a pass of its
-//                       own: 274.1, 345.3, 351.7, 469.0)
+//                       cut into column slices, whose results go to `raw`.  A token is a chain of latencies around up to 128 KB of state in
+//                       registers, which is fetched into L2 before the kernel before has ended
 //   omni_delta_finish   norm and gate of the results in `raw`
+#include <type_traits>
+
 #include "delta_rule.cuh"
 
 namespace omni {
@@ -18,8 +17,9 @@ typedef __nv_bfloat16 bf16;
 
 constexpr int DS_THREADS = 256;
 
-template <typename T, bool CHANNEL, int NR>
-__global__ void __launch_bounds__(DS_THREADS, NR <= 4 ? 3 : NR <= 16 ? 2 : 1)
+// BLOCKS: of an SM, as many as there are registers for (0: what the compiler makes of it)
+template <typename T, bool CHANNEL, int NR, int BLOCKS>
+__global__ void __launch_bounds__(DS_THREADS, BLOCKS)
 delta_steps_kernel(const DeltaRule p, const int cw) {
   extern __shared__ __align__(16) float sm[];
   __shared__ float sh[64];
@@ -34,13 +34,12 @@ delta_steps_kernel(const DeltaRule p, const int cw) {
   float* s_d = s_k + p.dp;                                   // [dp] channel: decay
   float* s_a = s_d + p.dp;                                   // [dp] channel: removal rate
   float* s_v = s_a + p.dp;                                   // [w]
-  float* s_g = s_v + cw;                                     // [2, w] gate's logits, of every other token: read when the next one's are fetched
-  float* s_w = s_g + 2 * cw;                                 // [w] gain
-  float* red = s_w + cw;                                     // [RG, w]
+  float* red = s_v + cw;                                     // [RG, w]
   float* red2 = red + 4 * DS_THREADS;
-  {
-    // The state is on its way to L2 before the kernel before has ended.  It only hints: sequence and row are read past L1 and once more below, and a row that is
-    // out of range or about to change costs a wasted fetch.
+  if (gridDim.z == 1) {
+    // The state is on its way to L2 before the kernel before has ended: decode steps of the 2048-wide decoder with one mixer of 16 heads of 128 x 128 and one of
+    // 16 x 64 per channel in four layers, 16 sequences of 3000 tokens 273.7 us (275.4 without), 20 344.8 (346.1), 64 470.2 (471.6).  Slices of a wide state gain
+    // nothing.  It only hints: sequence and row are read past L1 and once more below, and a row that is out of range or about to change costs a wasted fetch.
     const int s = p.seq_list ? min(max(__ldcg(p.seq_list + blockIdx.x), 0), p.num_seqs - 1) : blockIdx.x;
     const int row = __ldcg(p.state_in + s), per_row = (w * 4 + 127) / 128;
     if (row >= 0 && row < p.num_state)
@@ -79,17 +78,6 @@ delta_steps_kernel(const DeltaRule p, const int cw) {
     const long row = q0 + t;
     const T* pr = proj + row * p.ldp;
     float ss[2] = {0.f, 0.f};                                // sums of squares of q and k
-    float rate = 0.f, za = 0.f, zb = 0.f;
-    if (!CHANNEL) {
-      rate = p.rate[h];
-      za = (float)pr[p.a_col + h] + p.dt_bias[h];
-      zb = (float)pr[p.b_col + h];
-    }
-    if (gridDim.z == 1)                                      // fetched with everything else, used last
-      for (int c = tid; c < w; c += DS_THREADS) {
-        s_g[(t & 1) * cw + c] = (float)pr[p.g_col + h * p.vp + c];
-        s_w[c] = p.gain[(long)h * p.gain_hs + c];
-      }
     if (CHANNEL) {
       const T* z = static_cast<const T*>(p.z) + row * p.ldz;
       for (int c = tid; c < p.dp; c += DS_THREADS) {
@@ -103,49 +91,19 @@ delta_steps_kernel(const DeltaRule p, const int cw) {
       }
       for (int c = tid; c < w; c += DS_THREADS) s_v[c] = (float)pr[p.v_col + h * p.vp + c0 + c];
     } else {
-      // two elements of a thread and four taps at a time: their loads are under way together
-      const int count = 2 * p.dp + w;
-      const bool keep = t == n - 1 && sout >= 0, keeps_qk = h == g * R && blockIdx.z == 0;
-      for (int i0 = tid; i0 < count; i0 += 2 * DS_THREADS) {
-        float x[2] = {0.f, 0.f};
-        for (int j0 = 0; j0 < p.taps; j0 += 4) {
-          float cv[2][4], in[2][4];
-#pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const int i = i0 + u * DS_THREADS, c = channel_of(i);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const bool live = i < count && j0 + j < p.taps;
-              cv[u][j] = live ? p.conv[(long)(j0 + j) * C + c] : 0.f;
-              in[u][j] = live ? conv_x(t - hl + j0 + j, c) : 0.f;
-            }
-          }
-#pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const int i = i0 + u * DS_THREADS, c = channel_of(i);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              if (j0 + j < p.taps) x[u] = fmaf(cv[u][j], in[u][j], x[u]);
-              // new history (a row of its own): the last token's inputs but the oldest; the group's first head writes q and k, every block its values
-              if (keep && i < count && (keeps_qk || i >= 2 * p.dp) && j0 + j > 0 && j0 + j < p.taps)
-                hist[((long)sout * hl + j0 + j - 1) * C + c] = (T)in[u][j];
-            }
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const int i = i0 + u * DS_THREADS;
-          if (i >= count) continue;
-          x[u] = x[u] / (1.0f + expf(-x[u]));
-          if (i < p.dp) {
-            s_q[i] = x[u];
-            ss[0] = fmaf(x[u], x[u], ss[0]);
-          } else if (i < 2 * p.dp) {
-            s_k[i - p.dp] = x[u];
-            ss[1] = fmaf(x[u], x[u], ss[1]);
-          } else {
-            s_v[i - 2 * p.dp] = x[u];
-          }
+      for (int i = tid; i < 2 * p.dp + w; i += DS_THREADS) {
+        const int c = channel_of(i);
+        float x = 0.f;
+        for (int j = 0; j < p.taps; ++j) x = fmaf(p.conv[(long)j * C + c], conv_x(t - hl + j, c), x);
+        x = x / (1.0f + expf(-x));
+        if (i < p.dp) {
+          s_q[i] = x;
+          ss[0] = fmaf(x, x, ss[0]);
+        } else if (i < 2 * p.dp) {
+          s_k[i - p.dp] = x;
+          ss[1] = fmaf(x, x, ss[1]);
+        } else {
+          s_v[i - 2 * p.dp] = x;
         }
       }
     }
@@ -153,8 +111,8 @@ delta_steps_kernel(const DeltaRule p, const int cw) {
     const float ik = 1.0f / sqrtf(ss[1] + p.unit_eps);
     float decay = 1.f, beta = 1.f, o_mul = 1.f;
     if (!CHANNEL) {
-      decay = expf(rate * dr_softplus(za));
-      beta = dr_sigmoid(zb);
+      decay = expf(p.rate[h] * dr_softplus((float)pr[p.a_col + h] + p.dt_bias[h]));
+      beta = dr_sigmoid((float)pr[p.b_col + h]);
       o_mul = p.q_mul / sqrtf(ss[0] + p.unit_eps);
     }
     // what the old state answers to the unit key
@@ -236,10 +194,11 @@ delta_steps_kernel(const DeltaRule p, const int cw) {
       block_sum<1>(so, sh);
       if (tid < nc) {
         const float s = rms_scale(so[0], p.dv, p.eps);
+        const float* gain = p.gain + (long)h * p.gain_hs + tid * 4;
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const float gz = s_g[(t & 1) * cw + tid * 4 + e], open = dr_sigmoid(gz);
-          static_cast<T*>(p.out)[row * p.ldo + col + e] = (T)(res[e] * s * s_w[tid * 4 + e] * (CHANNEL ? open : gz * open));
+          const float gz = (float)pr[p.g_col + col + e], open = dr_sigmoid(gz);
+          static_cast<T*>(p.out)[row * p.ldo + col + e] = (T)(res[e] * s * gain[e] * (CHANNEL ? open : gz * open));
         }
       }
     }
@@ -250,6 +209,14 @@ delta_steps_kernel(const DeltaRule p, const int cw) {
   for (int i = 0; i < NR; ++i) {
     const int r = rg + i * RG;
     if (act && r < p.dp) *reinterpret_cast<float4*>(S1 + (long)r * p.vp) = S[i];
+  }
+  if (!CHANNEL && hl > 0) {
+    // new history: the group's first head writes q and k, every block its values
+    const bool first = h == g * R && blockIdx.z == 0;
+    for (int i = first ? tid : 2 * p.dp + tid; i < 2 * p.dp + w; i += DS_THREADS) {
+      const int c = channel_of(i);
+      for (int m = 0; m < hl; ++m) hist[((long)sout * hl + m) * C + c] = (T)conv_x(n - hl + m, c);
+    }
   }
 }
 
@@ -320,12 +287,24 @@ template <typename T, bool CHANNEL>
 static int launch_steps(const DeltaRule& p, int cw, cudaStream_t st) {
   const int nc = cw / 4, RG = DS_THREADS / nc, rows = (p.dp + RG - 1) / RG;
   const dim3 grid(p.seq_list ? p.n_list : p.num_seqs, p.H, (p.vp + cw - 1) / cw);
-  const int smem = (4 * p.dp + 4 * cw + 8 * DS_THREADS) * 4;
+  const int smem = (4 * p.dp + cw + 8 * DS_THREADS) * 4;
   if (smem > 47 * 1024) return RC_TOO_LARGE;
-  if (rows <= 4) launch_overlapped(delta_steps_kernel<T, CHANNEL, 4>, grid, DS_THREADS, smem, st, p, cw);
-  else if (rows <= 8) launch_overlapped(delta_steps_kernel<T, CHANNEL, 8>, grid, DS_THREADS, smem, st, p, cw);
-  else if (rows <= 16) launch_overlapped(delta_steps_kernel<T, CHANNEL, 16>, grid, DS_THREADS, smem, st, p, cw);
-  else if (rows <= 24) launch_overlapped(delta_steps_kernel<T, CHANNEL, 24>, grid, DS_THREADS, smem, st, p, cw);
+  // Registers as the grid leaves them: a lone block of an SM has twice the loads in flight, and where there are more blocks than SMs they run beside each other
+  // rather than in turn.  us, one kernel for all grids in brackets: 16 heads of 128 x 128, a portion of 200 tokens 792 (1102), 16 of 64 418 (419); of 64 x 64
+  // 611 (660) and 230 (265); per channel, 16 x 128, 16 of 64 tokens 379 (539), 64 single tokens 44 (58); 16 x 64, 64 of 20 229 (278).  Gated states of at most
+  // four rows per thread get three blocks from the compiler by itself (64 x 64, 64 of 20: 232; bound to three 248).
+  const long blocks = (long)grid.x * grid.y * grid.z, per_sm = (blocks + sm_count() - 1) / sm_count();
+  auto go = [&](auto n) {
+    constexpr int NR = decltype(n)::value, MOST = NR <= 4 ? 3 : NR <= 16 ? 2 : 1;
+    launch_overlapped(per_sm == 1   ? delta_steps_kernel<T, CHANNEL, NR, 1>
+                      : per_sm == 2 ? delta_steps_kernel<T, CHANNEL, NR, MOST < 2 ? MOST : 2>
+                                    : delta_steps_kernel<T, CHANNEL, NR, NR <= 4 && !CHANNEL ? 0 : MOST>,
+                      grid, DS_THREADS, smem, st, p, cw);
+  };
+  if (rows <= 4) go(std::integral_constant<int, 4>());
+  else if (rows <= 8) go(std::integral_constant<int, 8>());
+  else if (rows <= 16) go(std::integral_constant<int, 16>());
+  else if (rows <= 24) go(std::integral_constant<int, 24>());
   else return RC_TOO_LARGE;
   return (int)cudaGetLastError();
 }
