@@ -97,3 +97,11 @@ def test_splits_of_17_to_24_rows(rows, per_sm, k):
     y = gemm.linear(x, w, residual=r)
     _check(y, x.double() @ w.double().T + r.double(), x.double().abs() @ w.double().abs().T)
     nv.check_status()
+
+
+# both sides of every limit of the rule for 17 to 24 rows: rounds of blocks that are four fifths full and not, the longest contraction of each
+@pytest.mark.parametrize("rows", [17, 24])
+@pytest.mark.parametrize("n,k", [(1888, 2048), (1888, 2056), (1904, 9216), (1904, 9224), (3776, 2048), (3776, 2056), (3800, 4096), (3800, 4104), (5680, 3072),
+                                 (5680, 3080), (5696, 4096), (5696, 4104), (9472, 2560), (9472, 2568), (12432, 2048), (12432, 2056), (12440, 2048)])
+def test_edges_of_17_to_24_rows(rows, n, k):
+    test_edges_of_the_rules(rows, n, k)

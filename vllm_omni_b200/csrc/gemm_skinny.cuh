@@ -390,8 +390,13 @@ static int launch_skinny_mt(const CUtensorMap& tmW, const void* A, int lda, __nv
 //                    blocks per SM, or four of very long rows, that costs more than it saves.  us, general kernel in brackets: 13 rows 16384 x 4096 30.0
 //                    (37.3), 16 rows 16384 x 3584 28.3 (33.9), 16384 x 4096 31.5 (28.7), 13824 x 4096 24.4 (25.7), 12288 x 12288 1.05 times
 //                    as long, 8192 x 4096 18.1 (20.5).  Up to 8 rows the products are half as many and it pays at any length.
-//   17 to 24         gemm_rows_kernel up to 5 blocks per SM and contractions of 4096, or a block per SM and 9216: 17 rows 4096 x 12288 22.4 (20.6), 32768 x 2048
-//                    30.8 (29.6).  Which rows these are: steps that are not replayed from a captured batch (mixed ones, contexts past the captured tables),
+//   17 to 24         gemm_rows_kernel up to 5 blocks per SM and contractions of 2048; of 9216, 4096, 4096 and 2560 with one to four where those fill four fifths of
+//                    a round, and of 3072 and 2560 with three and four that do not.  17 and 24 rows on weights from memory, gemm_skinny_kernel in brackets: 10240 x 2048 12.8
+//                    and 13.4 (13.2, 13.5), 2048 x 9216 11.6, 12.3 (12.3, 12.4), 4096 x 4096 9.5, 10.2 (10.7), 8192 x 2560 10.9, 11.7 (11.8); beyond: 1024 x 8192
+//                    9.6, 10.0 (8.6), 2560 x 4096 9.2, 9.4 (8.5), 7168 x 4096 16.2, 17.3 (15.0), 10240 x 4096 23.8, 25.6 (21.0), 12288 x 4096 24.3, 25.4 (23.4).  A
+//                    gated layer, for which the alternative is two launches: up to 9216, 4096 with two to four blocks per SM, 2560 with five (17 and 24 rows, two
+//                    launches in brackets: 2560 x 4096 8.5, 9.0 (10.0), 8192 x 4096 16.0, 17.4 (17.4), 10240 x 3072 18.0, 19.0 (17.6), 12288 x 2048 12.3, 13.1 (16.5)).
+//                    Which rows these are: steps that are not replayed from a captured batch (mixed ones, contexts past the captured tables),
 //                    since captured batches have 16 or 32 rows and a vocabulary is wider than that
 //   17 to 32         else up to as many tiles as SMs: 17 rows 10240 x 2048 12.5 (17.1), 12288 x 1024 8.0 (11.6), 32 rows 18432 x 2048 15.4 (16.7)
 //   33 to 64         up to half as many; above, the general kernels stream W as fast and read A less often: 64 rows 9216 x 2048 12.7 (13.8),
@@ -400,14 +405,19 @@ static int launch_skinny_mt(const CUtensorMap& tmW, const void* A, int lda, __nv
 //                    wins back from 16 K blocks on and, with less to split by, from three quarters of the number of tiles: 128 rows 1536 x 768
 //                    9.8 (9.2), 1536 x 1024 8.1 (10.0), 4096 x 1024 11.2 (10.0), 4096 x 2048 12.9 (13.0); 65 rows 4096 x 1536 10.3 (10.7)
 enum class FewRows { no, rows, skinny };
-static FewRows few_rows(int M, int N, int K) {
+static FewRows few_rows(int M, int N, int K, bool gated = false) {
   const int tiles = (N + 127) / 128, num_kb = (K + 63) / 64;
   if (M <= 16) {
     const long a_kb = (long)M * K * 2 / 1024, blocks = (N + 15) / 16;
     return M > 8 && ((a_kb > 120 && blocks > 6L * sm_count()) || (a_kb >= 384 && blocks > 4L * sm_count())) ? FewRows::no : FewRows::rows;
   }
   const long blocks = (N + 15) / 16;
-  if (M <= 24 && ((blocks <= sm_count() && K <= 9216) || (blocks <= 5.25 * sm_count() && K <= 4096))) return FewRows::rows;
+  if (M <= 24 && blocks <= 5.25 * sm_count()) {
+    const long rounds = (blocks + sm_count() - 1) / sm_count();
+    const bool full = 5 * blocks >= 4 * rounds * sm_count();
+    const int most = gated ? (rounds == 1 ? 9216 : rounds > 4 ? 2560 : 4096) : rounds > 4 ? 2048 : rounds == 4 ? 2560 : full ? (rounds == 1 ? 9216 : 4096) : rounds == 3 ? 3072 : 2048;
+    if (K <= most) return FewRows::rows;
+  }
   if (M <= 64) return tiles * (M <= 32 ? 1 : 2) <= sm_count() ? FewRows::skinny : FewRows::no;
   return M <= 128 && tiles * 3 <= sm_count() && num_kb >= 16 && num_kb * 4 >= tiles * 3 ? FewRows::skinny : FewRows::no;
 }

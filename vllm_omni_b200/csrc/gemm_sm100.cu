@@ -1395,7 +1395,7 @@ extern "C" int omni_gemm_bf16_swiglu(const void* A, int lda, const void* W, int 
   GemmEpilogue epi = {};
   epi.rows_per_batch = 1;
   epi.act = EPI_SWIGLU;
-  const FewRows few = force_bn ? FewRows::no : few_rows(M, 2 * F, K);
+  const FewRows few = force_bn ? FewRows::no : few_rows(M, 2 * F, K, true);
   if (few == FewRows::skinny) return -5;
   if (few == FewRows::rows) return launch_rows(A, lda, W, ldw, static_cast<__nv_bfloat16*>(C), ldc, M, 2 * F, K, epi, s);
   const int N = 2 * F, ctas = sm_count();
