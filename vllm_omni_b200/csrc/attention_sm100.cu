@@ -426,10 +426,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
       const float m_new = fmaxf(m, mx);
       // lazy rescale, decided per warp because tcgen05.ld/st are warp-wide
-      // (rows past a segment are the next one's, not zeros: they may not decide for its last rows)
-      const bool grow = m_new > m + 8.0f && (!SEGS || srow < Sq);
+      const bool grow = m_new > m + 8.0f;
       if (j == 0) {
-        m = m_new;
+        // rows past a segment are the next one's, not zeros: they may not decide for its last rows, and from infinity nothing grows
+        m = !SEGS || srow < Sq ? m_new : INFINITY;
       } else if (__any_sync(0xffffffffu, grow)) {
         const float alpha = ex2_approx(m - m_new);
         const uint64_t alpha2 = pack2(alpha, alpha);
