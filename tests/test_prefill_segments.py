@@ -55,6 +55,13 @@ def test_segments(segs, H, Hkv, D):
     assert (out[:2] == 7).all() and (out[at:] == 7).all()
 
 
+# a lone segment of one round of blocks, which goes to the kernel of a single sequence, and just past its limits
+@pytest.mark.parametrize("segs,H,Hkv,D", [([(1000, 0)], 4, 2, 128), ([(999, 0)], 4, 2, 128), ([(300, 700)], 8, 2, 128), ([(17, 1300)], 16, 4, 128), ([(1027, 0)], 2, 2, 64),
+                                          ([(1300, 33)], 24, 4, 128), ([(1300, 33)], 25, 5, 128)])
+def test_lone_segment(segs, H, Hkv, D):
+    test_segments(segs, H, Hkv, D)
+
+
 @pytest.mark.parametrize("lengths,launches", [([5] * 8, 1), ([5] * 9, 2), ([300] * 19, 3), ([64000], 1), ([65536], 1), ([65537], 2), ([0] * 9, 0)])
 def test_launches_are_counted(lengths, launches):
     T = max(1, sum(lengths))
