@@ -79,11 +79,11 @@ def test_pages_of_other_sizes_keep_fp32_weights(bs, H, Hkv):
     assert ((out.double() - ref).abs() <= bound).all()
 
 
-# shares of very different and of like lengths, sequences without keys, sequences by the hundred, a block each
+# shares of very different and of like lengths (as many as make one round of warps), sequences without keys, more sequences than add up their lengths, a block each
 @pytest.mark.parametrize("H,Hkv,lens", [(32, 4, [4000, 3, 0, 70] + [17] * 40 + [900]), (8, 1, [2500] + [1] * 200), (16, 8, [0, 0, 5]), (32, 8, [33] * 700),
                                         (12, 3, [16 * i for i in range(50)]), (16, 1, [5000, 0, 40]), (8, 8, [1] * 450), (4, 1, [7000]),
-                                        (32, 4, [3500] * 8), (32, 4, [700] * 20), (32, 4, [3500] * 7 + [1])])
-def test_shares_of_lengths(H, Hkv, lens):
+                                        (32, 4, [3500] * 8), (32, 4, [700] * 20), (32, 4, [3500] * 7 + [1])])          # a round's room used up, and not
+def test_shares_by_the_lengths(H, Hkv, lens):
     D, bs, n = 128, 16, len(lens)
     g = torch.Generator(device="cuda").manual_seed(n)
     per = [-(-l // bs) for l in lens]
