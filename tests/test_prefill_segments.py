@@ -147,3 +147,16 @@ def test_many_decoded_rows_of_a_step(n, H, Hkv):
     rest = torch.ones(T, dtype=torch.bool, device="cuda")
     rest[rows] = False
     assert (out[rest] == 7).all()
+
+
+@pytest.mark.parametrize("impl", ["stream", "tc", "simt"])
+def test_rows_of_a_step_take_the_kernel_asked_for(impl):
+    g = torch.Generator(device="cuda").manual_seed(5)
+    q = torch.randn(9, 8, 128, device="cuda", generator=g).bfloat16()
+    kc, vc = (torch.randn(30, PAGE, 2, 128, device="cuda", generator=g).bfloat16() for _ in range(2))
+    bt = torch.arange(30, dtype=torch.int32, device="cuda").view(3, 10)
+    lens = torch.tensor([150, 90, 33], dtype=torch.int32, device="cuda")
+    rows = torch.tensor([7, 0, -3], device="cuda")
+    out = KC.paged_decode(q, kc, vc, bt, lens, out=torch.zeros_like(q), rows=rows, impl=impl)
+    assert torch.equal(out[rows], KC.paged_decode(q[rows].contiguous(), kc, vc, bt, lens, impl=impl))
+    nv.check_status(q.device)

@@ -122,10 +122,11 @@ def paged_decode(q, k_cache, v_cache, block_tables, seq_lens, scale=None, num_sp
     nb, bs, Hkv, _ = k_cache.shape
     scale = scale if scale is not None else 1.0 / math.sqrt(D)
     if rows is not None:
+        asked = impl
         if impl is None and q.is_cuda:
             impl = decode_impl(n, H, Hkv, D, bs, num_splits, q.stride(0), out.stride(0))
         if impl != "stream" or rows.dtype != torch.int64 or not rows.is_contiguous() or rows.device != q.device:
-            out[rows] = paged_decode(q[rows].contiguous(), k_cache, v_cache, block_tables, seq_lens, scale, num_splits)
+            out[rows] = paged_decode(q[rows].contiguous(), k_cache, v_cache, block_tables, seq_lens, scale, num_splits, impl=asked)
             return out
     if out is None:
         out = torch.empty_like(q)
